@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "pair.cuh"
+#include "taylor.cuh"
 
 namespace vext {
 
@@ -50,10 +51,14 @@ struct BatchSys {
     const float4 *tf;
     const double *td;
     int n_types;
+    int flush;                  // list_flush
     int near_mode;              // 1: cutoff test on near pairs, 2: none needed
     int bi, bj, bk, nrj, nrk;   // region grid (pose -> region)
     float *out;                 // [O][S^3]
     float *grad;                // [O][S^3][6] (forward + adjoint batches), else null
+    float *init, *init_grad;    // where the local expansions' values stand (out and grad, or
+                                // device scratch when those are host memory)
+    const double *poly;         // [regions][kTaylorPolyPad], or null: inner pairs are summed here
     double *out64;              // FP64 copy of the energies [O][S^3], or null
 };
 
@@ -79,6 +84,36 @@ struct BatchArgs {
     int *status;
 };
 
+__device__ __forceinline__ long long pose_index(const BatchSys &y, int o, int gi, int gj,
+                                                int gk) {
+    return ((((long long)o * y.S + gi) * y.S + gj) * y.S) + gk;
+}
+
+// Add the local expansion of region `reg` at pose idx (director o, center c
+// relative to the origin): the degree 0-3 polynomial here, the rest from
+// taylor_eval_kernel's output.
+__device__ __forceinline__ void add_expansion(const BatchSys &y, int reg, long long idx, int o,
+                                              double cx, double cy, double cz, double &e,
+                                              double (&g)[6]) {
+    const double *p = y.poly + (size_t)reg * kTaylorPolyPad;
+    const double u[3] = {y.axes[3 * o], y.axes[3 * o + 1], y.axes[3 * o + 2]};
+    double a[3], b[3];
+    e += taylor_poly_grad(p, cx + y.off0 * u[0], cy + y.off0 * u[1], cz + y.off0 * u[2], a) +
+         taylor_poly_grad(p, cx + y.off1 * u[0], cy + y.off1 * u[1], cz + y.off1 * u[2], b);
+    e += (double)y.init[idx];
+    const float2 *gi = reinterpret_cast<const float2 *>(y.init_grad + 6 * idx);
+    const float2 g0 = gi[0], g1 = gi[1], g2 = gi[2];
+    const double w[3] = {y.off0 * a[0] + y.off1 * b[0], y.off0 * a[1] + y.off1 * b[1],
+                         y.off0 * a[2] + y.off1 * b[2]};
+    const double wu = w[0] * u[0] + w[1] * u[1] + w[2] * u[2];
+    g[0] += a[0] + b[0] + (double)g0.x;
+    g[1] += a[1] + b[1] + (double)g0.y;
+    g[2] += a[2] + b[2] + (double)g1.x;
+    g[3] += w[0] - wu * u[0] + (double)g1.y;
+    g[4] += w[1] - wu * u[1] + (double)g2.x;
+    g[5] += w[2] - wu * u[2] + (double)g2.y;
+}
+
 // Forward + adjoint item: the same staged pipeline with the AdjAcc pair loops
 // (pair.cuh); writes the energy and [dE/dc, tangent dE/du] of every pose.
 // Far entries come in two passes, inner (no cutoff mask, shift summed once
@@ -91,7 +126,7 @@ struct BatchArgs {
 // pair too close to the cutoff for the FP32 test; 2: the smallest
 // | |d0 . u| - |T*| | (symmetric sites), 2 |o| times which is the former.
 template <int CB, int G, int P, bool NEWTON, bool RCP1, int UNROLL, int FLUSH, bool GSUM,
-          int BORDER, bool OUTER>
+          int BORDER, bool OUTER, bool EXPAND>
 __device__ __forceinline__ bool batch_item_adj(const BatchArgs &a, const BatchSys &y,
                                                const RegionInfo &r, Stager &st, double *ed,
                                                const float4 *stf, const double *std4,
@@ -171,19 +206,25 @@ __device__ __forceinline__ bool batch_item_adj(const BatchArgs &a, const BatchSy
             uz[j] = make_float2((float)y.axes[3 * o0 + 2], (float)y.axes[3 * o1 + 2]);
         }
         const FarGeom g = far_geom(cx, cy, cz, y.off0, y.off1, y.rc2f);
-        // inner entries, the shell, then (symmetric sites) the outer shell,
-        // where only the near site of each director can be inside
+        // inner entries (with a local expansion only those too near for it),
+        // the shell, then (symmetric sites) the outer shell, where only the
+        // near site of each director can be inside, and with an expansion the
+        // near shell, where only the other site can be outside
         const int n_outer = SYM && OUTER ? r.n_outer : 0;
+        const bool expand = EXPAND && y.poly;
+        const int n_trim = SYM && OUTER && expand ? r.n_shella : 0;
 #pragma unroll 1
-        for (int pass = 0; pass < 3; ++pass) {
+        for (int pass = 0; pass < (EXPAND ? 4 : 3); ++pass) {
             ChunkPlan plan;
             if (pass == 0)
-                plan.init_range(r.off + r.n_near, 0, r.n_inner);
+                plan.init_range(r.off + r.n_near, 0, expand ? r.n_mid : r.n_inner);
             else if (pass == 1)
-                plan.init_range(r.off + r.n_near + r.n_inner, 0,
-                                r.n_total - r.n_near - r.n_inner - n_outer);
-            else
+                plan.init_range(r.off + r.n_near + r.n_inner + n_trim, 0,
+                                r.n_total - r.n_near - r.n_inner - n_trim - n_outer);
+            else if (pass == 2)
                 plan.init_range(r.off + r.n_total - n_outer, 0, n_outer);
+            else
+                plan.init_range(r.off + r.n_near + r.n_inner, 0, n_trim);
             stage_prologue(st, plan, y.hi, y.lo, seq);
             for (int c = 0; c < plan.n_chunks; ++c) {
                 if (!stage_wait(st, plan, c, seq, a.status)) return false;
@@ -192,16 +233,21 @@ __device__ __forceinline__ bool batch_item_adj(const BatchArgs &a, const BatchSy
                 plan.chunk(c, start, len, near);
                 const float4 *hb = st.hib + ((seq + c) % kStages) * kCH;
                 constexpr int GNT = GSUM ? NT : 0;
-                if (pass == 2) {
-                    if constexpr (SYM && OUTER)
-                        far_chunk_outer<P, FLUSH, UNROLL, GNT, BORDER>(hb, stf, len, g, ux, uy,
-                                                                       uz, acc, gsum, border);
+                if (pass >= 2) {
+                    if constexpr (SYM && OUTER) {
+                        if (!EXPAND || pass == 2)
+                            far_chunk_outer<P, FLUSH, UNROLL, GNT, BORDER>(
+                                hb, stf, len, g, ux, uy, uz, acc, gsum, border);
+                        else
+                            far_chunk_outer<P, FLUSH, UNROLL, GNT, BORDER, true>(
+                                hb, stf, len, g, ux, uy, uz, acc, gsum, border);
+                    }
                 } else if (pass == 1) {
                     far_chunk_adj<P, NEWTON, FLUSH, true, RCP1, UNROLL, GNT, BORDER, SYM>(
                         hb, stf, len, g, ux, uy, uz, acc, shift_sum, gsum, border);
                 } else {
                     far_chunk_adj<P, NEWTON, FLUSH, false, RCP1, UNROLL, GNT, 0, SYM>(
-                        hb, stf, len, g, ux, uy, uz, acc, shift_sum, gsum);
+                        hb, stf, len, g, ux, uy, uz, acc, shift_sum, gsum, nullptr, y.flush);
                 }
                 stage_next(st, plan, y.hi, y.lo, c, seq);
             }
@@ -230,7 +276,9 @@ __device__ __forceinline__ bool batch_item_adj(const BatchArgs &a, const BatchSy
 // single-site pass (far_chunk_outer).  BORDER: 0 none, 1 the
 // cutoff-border test per site (|q - rc^2|), 2 per director (| |d0 . u| -
 // |T*| |, symmetric sites only).
-template <int CB, int G, int P, int MINB, int ADJ, int BORDER = 0, bool OUTER = false>
+// EXPAND: systems may have local expansions (taylor.cuh).
+template <int CB, int G, int P, int MINB, int ADJ, int BORDER = 0, bool OUTER = false,
+          bool EXPAND = false>
 __global__ void __launch_bounds__(CB *G, MINB) batch_field_kernel(BatchArgs a) {
     constexpr int NT = CB * G, PP = P / 2;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -276,7 +324,7 @@ __global__ void __launch_bounds__(CB *G, MINB) batch_field_kernel(BatchArgs a) {
         if constexpr (ADJ) {
             double *gsum = reinterpret_cast<double *>(std4 + 4 * y.n_types);
             if (!batch_item_adj<CB, G, P, ADJ == 2, ADJ == 1 || ADJ >= 5, kUnroll,
-                                ADJ == 6 ? 16 : ADJ == 7 ? 64 : 128, kGsum, BORDER, OUTER>(
+                                ADJ == 6 ? 16 : ADJ == 7 ? 64 : 128, kGsum, BORDER, OUTER, EXPAND>(
                     a, y, r, st, ed, stf, std4, gsum, seq, cx, cy, cz, obase, e, gr, border))
                 return;
         } else {
@@ -312,7 +360,14 @@ __global__ void __launch_bounds__(CB *G, MINB) batch_field_kernel(BatchArgs a) {
             }
             seq += plan.n_chunks;
 #pragma unroll
-            for (int p = 0; p < P; ++p) e[p] = acc[p][0] + acc[p][1] + 2.0 * shift_near;
+            for (int p = 0; p < P; ++p) {
+                e[p] = acc[p][0] + acc[p][1] + 2.0 * shift_near;
+                if (EXPAND && y.poly && cvalid && obase + G * p < y.O) {
+                    const double *tp = y.poly + (size_t)w.y * kTaylorPolyPad;
+                    e[p] += taylor_pair(tp, cx, cy, cz, y.off0, y.off1, ux[p], uy[p], uz[p]);
+                    e[p] += (double)y.init[pose_index(y, obase + G * p, gi, gj, gk)];
+                }
+            }
         }
         // ---- far pairs (packed FP32x2)
         {
@@ -329,16 +384,24 @@ __global__ void __launch_bounds__(CB *G, MINB) batch_field_kernel(BatchArgs a) {
             }
             const FarGeom g = far_geom(cx, cy, cz, y.off0, y.off1, y.rc2f);
             double shift_sum = 0.0;
-            // inner entries, then the shell, whose outer entries (symmetric
-            // sites) take the near site of each director alone
-            const int shell_n = r.n_total - r.n_near - r.n_inner;
+            // inner entries (with a local expansion only those too near for
+            // it), with an expansion of symmetric sites the near shell, then
+            // the shell, whose outer entries (symmetric sites) take the near
+            // site of each director alone
             const bool sym = y.off0 != 0.0 && y.off1 == -y.off0;
+            const bool expand = EXPAND && y.poly;
+            const int n_trim = sym && expand ? r.n_shella : 0;
+            const int shell_n = r.n_total - r.n_near - r.n_inner - n_trim;
             const int outer_at = shell_n - (sym ? r.n_outer : 0);
 #pragma unroll 1
-            for (int pass = 0; pass < 2; ++pass) {
+            for (int pass = 0; pass < (EXPAND ? 3 : 2); ++pass) {
+                const bool trim = EXPAND && pass == 2;
                 ChunkPlan plan;
-                plan.init_range(r.off + r.n_near + (pass ? r.n_inner : 0), 0,
-                                pass ? shell_n : r.n_inner);
+                if (pass == 0)
+                    plan.init_range(r.off + r.n_near, 0, expand ? r.n_mid : r.n_inner);
+                else
+                    plan.init_range(r.off + r.n_near + r.n_inner + (trim ? 0 : n_trim), 0,
+                                    trim ? n_trim : shell_n);
                 stage_prologue(st, plan, y.hi, y.lo, seq);
                 for (int c = 0; c < plan.n_chunks; ++c) {
                     if (!stage_wait(st, plan, c, seq, a.status)) return;
@@ -346,13 +409,16 @@ __global__ void __launch_bounds__(CB *G, MINB) batch_field_kernel(BatchArgs a) {
                     bool near;
                     plan.chunk(c, start, len, near);
                     const float4 *hb = st.hib + ((seq + c) % kStages) * kCH;
-                    if (pass && sym)
-                        far_chunk_fwd<P, 16, true, true>(hb, stf, len, g, ux, uy, uz, acc,
-                                                         shift_sum, outer_at - start);
+                    if (trim)
+                        far_chunk_trim<P, 16>(hb, stf, len, g, ux, uy, uz, acc);
+                    else if (pass && sym)
+                        far_chunk_fwd<P, true, true>(hb, stf, len, g, ux, uy, uz, acc, shift_sum,
+                                                     16, outer_at - start);
                     else if (pass)
-                        far_chunk_fwd<P, 16, true>(hb, stf, len, g, ux, uy, uz, acc, shift_sum);
+                        far_chunk_fwd<P, true>(hb, stf, len, g, ux, uy, uz, acc, shift_sum, 16);
                     else
-                        far_chunk_fwd<P, 16, false>(hb, stf, len, g, ux, uy, uz, acc, shift_sum);
+                        far_chunk_fwd<P, false>(hb, stf, len, g, ux, uy, uz, acc, shift_sum,
+                                                y.flush);
                     stage_next(st, plan, y.hi, y.lo, c, seq);
                 }
                 seq += plan.n_chunks;
@@ -369,9 +435,13 @@ __global__ void __launch_bounds__(CB *G, MINB) batch_field_kernel(BatchArgs a) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int o = obase + G * (2 * j + h);
-                    const double v = e[2 * j + h];
+                    double v = e[2 * j + h];
                     if (o < y.O) {
                         const long long idx = (long long)o * S3 + cg;
+                        if constexpr (ADJ) {
+                            if (EXPAND && y.poly)
+                                add_expansion(y, w.y, idx, o, cx, cy, cz, v, gr[2 * j + h]);
+                        }
                         y.out[idx] = (float)v;
                         if (y.out64) y.out64[idx] = v;
                         if constexpr (ADJ) {
@@ -538,11 +608,14 @@ struct BatchKernel {
     void (*fn)(BatchArgs);
     int threads;
     const char *name;
+    void (*fn_expand)(BatchArgs) = nullptr;   // the same for batches with local expansions
 };
 
 static const BatchKernel kForwardKernels[] = {
-    {batch_field_kernel<16, 8, 4, 4, 0>, 128, "128x4"},
-    {batch_field_kernel<16, 16, 2, 3, 0>, 256, "256x2"}};
+    {batch_field_kernel<16, 8, 4, 4, 0>, 128, "128x4",
+     batch_field_kernel<16, 8, 4, 4, 0, 0, false, true>},
+    {batch_field_kernel<16, 16, 2, 3, 0>, 256, "256x2",
+     batch_field_kernel<16, 16, 2, 3, 0, 0, false, true>}};
 static const BatchKernel kAdjointKernels[] = {
     {batch_field_kernel<16, 16, 2, 2, 1, true>, 256, "256x2"},
     {batch_field_kernel<16, 8, 4, 2, 1, true>, 128, "128x4"},
@@ -564,27 +637,43 @@ static const BatchKernel kAdjointFlush64Kernels[] = {   // accuracy/speed study
 // 8-center regions x 64-director items (the same 512 poses per staged
 // entry): a smaller region radius, hence shorter near and shell lists
 static const BatchKernel kForwardCb8Kernels[] = {
-    {batch_field_kernel<8, 16, 4, 4, 0>, 128, "8c 128x4"},
-    {batch_field_kernel<8, 32, 2, 3, 0>, 256, "8c 256x2"}};
+    {batch_field_kernel<8, 16, 4, 4, 0>, 128, "8c 128x4",
+     batch_field_kernel<8, 16, 4, 4, 0, 0, false, true>},
+    {batch_field_kernel<8, 32, 2, 3, 0>, 256, "8c 256x2",
+     batch_field_kernel<8, 32, 2, 3, 0, 0, false, true>}};
 // symmetric sites: border per director, outer shell in the single-site pass
 static const BatchKernel kAdjointCb8Kernels[] = {
-    {batch_field_kernel<8, 16, 4, 3, 8, 2, true>, 128, "8c 128x4/3 gsum"},
-    {batch_field_kernel<8, 16, 4, 2, 1, 2, true>, 128, "8c 128x4"},
-    {batch_field_kernel<8, 32, 2, 2, 1, 2, true>, 256, "8c 256x2"},
-    {batch_field_kernel<8, 16, 4, 3, 11, 2, true>, 128, "8c 128x4/3 gsum unroll2"},
-    {batch_field_kernel<8, 16, 4, 2, 12, 2, true>, 128, "8c 128x4 unroll2"},
-    {batch_field_kernel<8, 16, 4, 3, 17, 2, true>, 128, "8c 128x4/3 gsum unroll4"}};
+    {batch_field_kernel<8, 16, 4, 3, 8, 2, true>, 128, "8c 128x4/3 gsum",
+     batch_field_kernel<8, 16, 4, 3, 8, 2, true, true>},
+    {batch_field_kernel<8, 16, 4, 2, 1, 2, true>, 128, "8c 128x4",
+     batch_field_kernel<8, 16, 4, 2, 1, 2, true, true>},
+    {batch_field_kernel<8, 32, 2, 2, 1, 2, true>, 256, "8c 256x2",
+     batch_field_kernel<8, 32, 2, 2, 1, 2, true, true>},
+    {batch_field_kernel<8, 16, 4, 3, 11, 2, true>, 128, "8c 128x4/3 gsum unroll2",
+     batch_field_kernel<8, 16, 4, 3, 11, 2, true, true>},
+    {batch_field_kernel<8, 16, 4, 2, 12, 2, true>, 128, "8c 128x4 unroll2",
+     batch_field_kernel<8, 16, 4, 2, 12, 2, true, true>},
+    {batch_field_kernel<8, 16, 4, 3, 17, 2, true>, 128, "8c 128x4/3 gsum unroll4",
+     batch_field_kernel<8, 16, 4, 3, 17, 2, true, true>}};
 // the same with the outer shell in the two-site shell pass (timing study)
 static const BatchKernel kAdjointCb8TwoSiteKernels[] = {
-    {batch_field_kernel<8, 16, 4, 3, 11, 2>, 128, "8c 128x4/3 gsum unroll2, two-site outer"},
-    {batch_field_kernel<8, 16, 4, 3, 17, 2>, 128, "8c 128x4/3 gsum unroll4, two-site outer"}};
+    {batch_field_kernel<8, 16, 4, 3, 11, 2>, 128, "8c 128x4/3 gsum unroll2, two-site outer",
+     batch_field_kernel<8, 16, 4, 3, 11, 2, false, true>},
+    {batch_field_kernel<8, 16, 4, 3, 17, 2>, 128, "8c 128x4/3 gsum unroll4, two-site outer",
+     batch_field_kernel<8, 16, 4, 3, 17, 2, false, true>}};
 static const BatchKernel kAdjointCb8SiteBorderKernels[] = {   // any sites: border per site
-    {batch_field_kernel<8, 16, 4, 3, 8, 1>, 128, "8c 128x4/3 gsum, border/site"},
-    {batch_field_kernel<8, 16, 4, 2, 1, 1>, 128, "8c 128x4, border/site"},
-    {batch_field_kernel<8, 32, 2, 2, 1, 1>, 256, "8c 256x2, border/site"},
-    {batch_field_kernel<8, 16, 4, 3, 11, 1>, 128, "8c 128x4/3 gsum unroll2, border/site"},
-    {batch_field_kernel<8, 16, 4, 2, 12, 1>, 128, "8c 128x4 unroll2, border/site"},
-    {batch_field_kernel<8, 16, 4, 3, 17, 1>, 128, "8c 128x4/3 gsum unroll4, border/site"}};
+    {batch_field_kernel<8, 16, 4, 3, 8, 1>, 128, "8c 128x4/3 gsum, border/site",
+     batch_field_kernel<8, 16, 4, 3, 8, 1, false, true>},
+    {batch_field_kernel<8, 16, 4, 2, 1, 1>, 128, "8c 128x4, border/site",
+     batch_field_kernel<8, 16, 4, 2, 1, 1, false, true>},
+    {batch_field_kernel<8, 32, 2, 2, 1, 1>, 256, "8c 256x2, border/site",
+     batch_field_kernel<8, 32, 2, 2, 1, 1, false, true>},
+    {batch_field_kernel<8, 16, 4, 3, 11, 1>, 128, "8c 128x4/3 gsum unroll2, border/site",
+     batch_field_kernel<8, 16, 4, 3, 11, 1, false, true>},
+    {batch_field_kernel<8, 16, 4, 2, 12, 1>, 128, "8c 128x4 unroll2, border/site",
+     batch_field_kernel<8, 16, 4, 2, 12, 1, false, true>},
+    {batch_field_kernel<8, 16, 4, 3, 17, 1>, 128, "8c 128x4/3 gsum unroll4, border/site",
+     batch_field_kernel<8, 16, 4, 3, 17, 1, false, true>}};
 // the same without the cutoff-border test (timing study: its cost)
 static const BatchKernel kAdjointCb8NoBorderKernels[] = {
     {batch_field_kernel<8, 16, 4, 3, 8>, 128, "8c 128x4/3 gsum, no border test"},
@@ -664,7 +753,17 @@ struct vext_batch_s {
     int size = 0, n_axes = 0;
     Options opt;
     BatchSys *d_sys = nullptr;
-    std::vector<std::pair<float *, float *>> targets;   // current (out, grad) of each system
+    struct Target {   // (the layout of these words in BatchSys)
+        float *out, *grad, *init, *init_grad;
+        bool operator==(const Target &o) const {
+            return out == o.out && grad == o.grad && init == o.init && init_grad == o.init_grad;
+        }
+    };
+    std::vector<Target> targets;          // current outputs of each system
+    std::vector<TaylorPlan> plans;        // local expansions (poly null: none)
+    std::vector<const RegionSet *> lists; // each system's region lists
+    float *d_sums = nullptr;              // expansion sums of one system at a time
+    size_t sums_cap = 0;
     int4 *d_items = nullptr, *d_sample = nullptr;
     int n_items = 0, n_sample = 0;
     int *d_counter = nullptr, *d_refine = nullptr;
@@ -693,9 +792,19 @@ struct vext_batch_s {
         cudaFree(d_refine);
         cudaFree(d_axes);
         cudaFree(d_status);
+        cudaFree(d_sums);
+        for (TaylorPlan &p : plans) p.release();
         if (stream) cudaStreamDestroy(stream);
     }
 };
+
+// Whether the batch's kernels trim the near shell of symmetric sites (the
+// expansion then holds those entries): the default forward + adjoint kernels
+// and, per system, the forward ones.
+static bool batch_trims(vext_batch b, const System &sys) {
+    const bool sym = sys.offsets[0] != 0.0 && sys.offsets[1] == -sys.offsets[0];
+    return b->adj ? b->kind == 6 : sym;
+}
 
 // Staging + converted near chunk + type tables (+ the FP64 gradient sums of
 // 16 centers x 32 directors for the adjoint kernels that park them there).
@@ -704,8 +813,17 @@ static size_t batch_smem(int max_types, bool adj) {
            (adj ? (size_t)kGradWords * 16 * 32 * sizeof(double) : 0);
 }
 
+// expand: evaluate the local expansions into the outputs first (a whole
+// pass; the tuner's samples run without).
 static int batch_launch(vext_batch b, const BatchConfig &cfg, const int4 *items, int n_items,
-                        cudaStream_t st) {
+                        bool expand, cudaStream_t st) {
+    for (size_t k = 0; expand && k < b->plans.size(); ++k) {
+        if (!b->plans[k].poly) continue;
+        const System &sys = b->systems[k]->sys;
+        VEXT_TRY(taylor_enqueue(sys, *b->lists[k], b->n_axes, b->plans[k], batch_trims(b, sys),
+                                b->d_sums, &b->d_sys[k].init, nullptr, &b->d_sys[k].init_grad,
+                                st));
+    }
     BatchArgs a;
     a.sys = b->d_sys;
     a.items = items;
@@ -721,7 +839,7 @@ static int batch_launch(vext_batch b, const BatchConfig &cfg, const int4 *items,
     VEXT_CUDA(cudaMemsetAsync(b->d_counter, 0, sizeof(int), st));
     VEXT_CUDA(cudaMemsetAsync(b->d_refine, 0, sizeof(int), st));
     const BatchKernel &k = batch_kernel(b->kind, cfg.shape);
-    k.fn<<<cfg.grid, k.threads, smem, st>>>(a);
+    (b->d_sums ? k.fn_expand : k.fn)<<<cfg.grid, k.threads, smem, st>>>(a);
     VEXT_CUDA(cudaGetLastError());
     if (b->adj) {
         batch_refine_adj_kernel<<<1184, 256, 0, st>>>(a);
@@ -752,13 +870,24 @@ static std::map<TuneKey, TunePick> g_tune_cache;
 // pick for this class (the pick is then replaced)
 constexpr int kVariantTuneAfresh = 2048;
 
+static bool device_memory(const void *p) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
+}
+
 // Shared by vext_batch_create, vext_batch_create_adjoint and the cached
 // one-system batch of vext_field_adjoint_device (which already holds its
-// system's lock: lock_systems = false).
+// system's lock: lock_systems = false, and says with `rule_axes` how many
+// directors the whole call has and with `init` where expansion values may
+// stand when the outputs are host memory).
 int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
                 const double *axes, const vext_options *opt, float *const *outputs,
                 float *const *gradients, double *const *outputs_f64, bool lock_systems,
-                vext_batch *out) {
+                vext_batch *out, int rule_axes, float *const *init) {
     if (!out || n_systems < 1 || !systems || !outputs || size < 1 || n_axes < 1 || !axes)
         return fail(VEXT_ERR_ARGUMENT, "bad batch arguments");
     for (int k = 0; k < n_systems; ++k)
@@ -854,6 +983,7 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
         for (const RegionInfo &r : rs->h_info) rho = std::max(rho, r.rho);
         y.near_mode =
             rs->r_split + 2.0 * (rho + list_sys->max_offset) + 1e-6 < sys->cutoff ? 2 : 1;
+        y.flush = list_flush(*rs, sys->cutoff);
         y.bi = rs->bi;
         y.bj = rs->bj;
         y.bk = rs->bk;
@@ -861,6 +991,9 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
         y.nrk = rs->n_rk;
         y.out = outputs[k];
         y.grad = gradients ? gradients[k] : nullptr;
+        y.init = init ? init[0] : y.out;
+        y.init_grad = init ? init[1] : y.grad;
+        y.poly = nullptr;
         y.out64 = outputs_f64 ? outputs_f64[k] : nullptr;
         b->max_types = std::max(b->max_types, sys->n_types);
         b->poses += S3 * n_axes;
@@ -907,7 +1040,23 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
     if (b->kind == 6 || b->kind == 10)
         for (const BatchSys &y : hs)
             if (y.off0 == 0.0 || y.off1 != -y.off0) b->kind = 9;
-    for (const BatchSys &y : hs) b->targets.push_back({y.out, y.grad});
+    // local expansions: the kinds whose kernels use them, where the rule of
+    // taylor_worthwhile says so and their values can stand in device memory
+    b->plans.resize(n_systems);
+    const bool expands = b->kind == 0 || b->kind == 6 || b->kind == 7 || b->kind == 9 ||
+                         b->kind == 10;
+    for (int k = 0; k < n_systems; ++k) {
+        b->lists.push_back(lists[owner[k]]);
+        const System &sys = systems[k]->sys;
+        const RegionSet &rs = *b->lists[k];
+        if (!expands || !taylor_worthwhile(sys, rs, rule_axes ? rule_axes : n_axes, b->adj) ||
+            !device_memory(hs[k].init) || (b->adj && !device_memory(hs[k].init_grad)))
+            continue;
+        VEXT_TRY(taylor_prepare(sys, rs, n_axes, b->d_axes, b->adj, b->plans[k], b->stream));
+        VEXT_TRY(ensure_capacity(b->d_sums, b->sums_cap, taylor_workspace(rs)));
+        hs[k].poly = b->plans[k].poly;
+    }
+    for (const BatchSys &y : hs) b->targets.push_back({y.out, y.grad, y.init, y.init_grad});
     VEXT_CUDA(cudaMalloc(&b->d_sys, sizeof(BatchSys) * n_systems));
     VEXT_CUDA(cudaMemcpy(b->d_sys, hs.data(), sizeof(BatchSys) * n_systems, cudaMemcpyHostToDevice));
     VEXT_CUDA(cudaMalloc(&b->d_items, sizeof(int4) * hitems.size()));
@@ -936,10 +1085,11 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
     for (int k = 0; k < n_kernels; ++k) {
         if (b->opt.batch_shape && k != b->opt.batch_shape - 1) continue;   // pinned shape
         const BatchKernel &bk = batch_kernel(b->kind, k);
-        VEXT_CUDA(cudaFuncSetAttribute(bk.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        const auto fn = b->d_sums ? bk.fn_expand : bk.fn;
+        VEXT_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)smem));
         int occ = 0;
-        VEXT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, bk.fn, bk.threads, smem));
+        VEXT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, bk.threads, smem));
         if (occ < 1) continue;
         if (n_cands < kMaxCandidates) cands[n_cands++] = {k, sms * occ};
         if (occ >= 4 && n_cands < kMaxCandidates && !b->opt.batch_shape)
@@ -950,7 +1100,7 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
     for (int c = 0; c < n_cands; ++c) b->cands[c] = cands[c];
     // a process-wide cache of the winners per (device, kernel table, size
     // class): later batches of the same class skip the timing runs
-    const TuneKey key{dev, b->kind, size_class};
+    const TuneKey key{dev, b->kind + (b->d_sums ? 64 : 0), size_class};
     bool cached = false;
     if (!b->opt.batch_shape && !(b->opt.variant & kVariantTuneAfresh)) {
         std::lock_guard<std::mutex> guard(g_tune_lock);
@@ -972,11 +1122,12 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
         const int n_warm = std::min(b->n_sample, sms);
         for (int c = 0; c < n_cands; ++c) {
             // warm-up on a few items (module load, first-launch costs)
-            VEXT_TRY(batch_launch(b, cands[c], b->d_sample, n_warm, b->stream));
+            VEXT_TRY(batch_launch(b, cands[c], b->d_sample, n_warm, false, b->stream));
             float ms = 1e30f;
             for (int rep = 0; rep < 2; ++rep) {   // best of two: launch noise
                 VEXT_CUDA(cudaEventRecord(e0, b->stream));
-                VEXT_TRY(batch_launch(b, cands[c], b->d_sample, b->n_sample, b->stream));
+                VEXT_TRY(batch_launch(b, cands[c], b->d_sample, b->n_sample, false,
+                                      b->stream));
                 VEXT_CUDA(cudaEventRecord(e1, b->stream));
                 VEXT_CUDA(cudaEventSynchronize(e1));
                 float t = 0;
@@ -1004,7 +1155,7 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
     if (status) return fail(VEXT_ERR_TIMEOUT, "a device wait gave up during batch tuning");
     // ---- capture the whole batch into a graph
     VEXT_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    const int rc = batch_launch(b, b->config, b->d_items, b->n_items, b->stream);
+    const int rc = batch_launch(b, b->config, b->d_items, b->n_items, true, b->stream);
     cudaGraph_t g = nullptr;
     const cudaError_t end = cudaStreamEndCapture(b->stream, &g);
     if (rc) {
@@ -1024,7 +1175,7 @@ extern "C" int vext_batch_create(int n_systems, const vext_system *systems, int 
                                  int n_axes, const double *axes, const vext_options *opt,
                                  float *const *outputs, vext_batch *out) {
     return batch_build(n_systems, systems, size, n_axes, axes, opt, outputs, nullptr, nullptr,
-                       true, out);
+                       true, out, 0, nullptr);
 }
 
 extern "C" int vext_batch_create_adjoint(int n_systems, const vext_system *systems, int size,
@@ -1033,7 +1184,7 @@ extern "C" int vext_batch_create_adjoint(int n_systems, const vext_system *syste
                                          float *const *gradients, vext_batch *out) {
     if (!gradients) return fail(VEXT_ERR_ARGUMENT, "gradient outputs required");
     return batch_build(n_systems, systems, size, n_axes, axes, opt, energies, gradients, nullptr,
-                       true, out);
+                       true, out, 0, nullptr);
 }
 
 namespace vext {
@@ -1044,19 +1195,26 @@ int batch_replay(vext_batch b, cudaStream_t stream) {
     return 0;
 }
 
-// Point system k's float32 energy / gradient outputs at `out` / `grad` for the
-// replays that follow on `stream`: a stream-ordered update of the device copy
-// of its BatchSys, which the captured kernels read at run time (no rebuild).
-int batch_retarget(vext_batch b, int k, float *out, float *grad, cudaStream_t stream) {
+// Point system k's float32 energy / gradient outputs at `out` / `grad` (and
+// its expansion values at `init` / `init_grad`) for the replays that follow on
+// `stream`: a stream-ordered update of the device copy of its BatchSys, which
+// the captured kernels read at run time (no rebuild).
+int batch_retarget(vext_batch b, int k, float *out, float *grad, float *init, float *init_grad,
+                   cudaStream_t stream) {
     if (k < 0 || k >= (int)b->systems.size()) return fail(VEXT_ERR_ARGUMENT, "bad system index");
     if (!out || (b->adj && !grad)) return fail(VEXT_ERR_ARGUMENT, "null output");
-    static_assert(offsetof(BatchSys, grad) == offsetof(BatchSys, out) + sizeof(float *),
-                  "out and grad must be adjacent");
-    float *ptrs[2] = {out, b->adj ? grad : nullptr};
-    if (b->targets[k].first == ptrs[0] && b->targets[k].second == ptrs[1]) return 0;
+    using Target = vext_batch_s::Target;
+    static_assert(offsetof(BatchSys, grad) - offsetof(BatchSys, out) == offsetof(Target, grad) &&
+                      offsetof(BatchSys, init) - offsetof(BatchSys, out) ==
+                          offsetof(Target, init) &&
+                      offsetof(BatchSys, init_grad) - offsetof(BatchSys, out) ==
+                          offsetof(Target, init_grad),
+                  "the output words must be adjacent");
+    const Target to{out, b->adj ? grad : nullptr, init, b->adj ? init_grad : nullptr};
+    if (b->targets[k] == to) return 0;
     VEXT_CUDA(cudaMemcpyAsync(reinterpret_cast<char *>(b->d_sys + k) + offsetof(BatchSys, out),
-                              ptrs, sizeof ptrs, cudaMemcpyHostToDevice, stream));
-    b->targets[k] = {ptrs[0], ptrs[1]};
+                              &to, sizeof to, cudaMemcpyHostToDevice, stream));
+    b->targets[k] = to;
     return 0;
 }
 

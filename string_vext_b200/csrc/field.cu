@@ -20,6 +20,7 @@
 #include <cuda.h>
 
 #include "pair.cuh"
+#include "taylor.cuh"
 
 namespace vext {
 
@@ -41,6 +42,9 @@ struct FieldArgs {
     const float4 *tf;
     const double *td;
     int n_types;
+    int flush;                // list_flush
+    const double *poly;       // [regions][kTaylorPolyPad] local expansions, whose further
+                              // degrees stand in e64; null: inner pairs are summed directly
     double *e64;              // [O][S^3]
     int *status;
 };
@@ -55,7 +59,7 @@ __device__ __forceinline__ void center_of(const FieldArgs &a, const RegionInfo &
 
 // Near pairs in FP64 over every region's near entries (all entries for the
 // FP64 oracle region set); MODE as in near_chunk (pair.cuh).  Writes e64.
-template <int CB, int G, int P, int MODE>
+template <int CB, int G, int P, int MODE, bool EXPAND = false>
 __global__ void __launch_bounds__(CB *G, 1) field_near_kernel(FieldArgs a) {
     constexpr int NT = CB * G;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -113,7 +117,14 @@ __global__ void __launch_bounds__(CB *G, 1) field_near_kernel(FieldArgs a) {
 #pragma unroll
         for (int p = 0; p < P; ++p) {
             const int o = obase + G * p;
-            if (o < a.O) a.e64[(size_t)o * S3 + cg] = acc[p][0] + acc[p][1] + 2.0 * shift_near;
+            if (o >= a.O) continue;
+            double e = acc[p][0] + acc[p][1] + 2.0 * shift_near;
+            if (EXPAND) {
+                e += taylor_pair(a.poly + (size_t)blockIdx.x * kTaylorPolyPad, cx, cy, cz, a.off0,
+                                 a.off1, ux[p], uy[p], uz[p]);
+                e += a.e64[(size_t)o * S3 + cg];
+            }
+            a.e64[(size_t)o * S3 + cg] = e;
         }
     }
 }
@@ -183,9 +194,11 @@ __global__ void __launch_bounds__(CB *G, MINB) field_far_kernel(FieldArgs a) {
     }
 }
 
-// The default far kernel: far_chunk_fwd over the inner entries (no mask) and
-// then the shell entries; same thread layout and output as field_far_kernel.
-template <int CB, int G, int P, int MINB>
+// The default far kernel: far_chunk_fwd over the inner entries (no mask; with
+// a local expansion only those too near for it), with an expansion of
+// symmetric sites far_chunk_trim over the near shell, and far_chunk_fwd over
+// the (rest of the) shell; same thread layout and output as field_far_kernel.
+template <int CB, int G, int P, int MINB, bool EXPAND = false>
 __global__ void __launch_bounds__(CB *G, MINB) field_far2_kernel(FieldArgs a) {
     constexpr int NT = CB * G, PP = P / 2;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -220,13 +233,18 @@ __global__ void __launch_bounds__(CB *G, MINB) field_far2_kernel(FieldArgs a) {
         uz[j] = make_float2((float)a.axes[3 * o0 + 2], (float)a.axes[3 * o1 + 2]);
         acc[2 * j] = acc[2 * j + 1] = 0.0;
     }
+    const int n_trim = EXPAND && a.off0 != 0.0 && a.off1 == -a.off0 ? r.n_shella : 0;
     double shift_sum = 0.0;
     unsigned seq = 0;
 #pragma unroll 1
-    for (int pass = 0; pass < 2; ++pass) {   // inner entries, then the shell
+    for (int pass = 0; pass < (EXPAND ? 3 : 2); ++pass) {
+        const bool trim = EXPAND && pass == 2;
         ChunkPlan plan;
-        plan.init_range(r.off + r.n_near + (pass ? r.n_inner : 0), 0,
-                        pass ? r.n_total - r.n_near - r.n_inner : r.n_inner);
+        if (pass == 0)
+            plan.init_range(r.off + r.n_near, 0, EXPAND ? r.n_mid : r.n_inner);
+        else
+            plan.init_range(r.off + r.n_near + r.n_inner + (trim ? 0 : n_trim), 0,
+                            trim ? n_trim : r.n_total - r.n_near - r.n_inner - n_trim);
         stage_prologue(st, plan, a.hi, a.lo, seq);
         for (int c = 0; c < plan.n_chunks; ++c) {
             if (!stage_wait(st, plan, c, seq, a.status)) return;
@@ -234,8 +252,9 @@ __global__ void __launch_bounds__(CB *G, MINB) field_far2_kernel(FieldArgs a) {
             bool near;
             plan.chunk(c, start, len, near);
             const float4 *hb = st.hib + ((seq + c) % kStages) * kCH;
-            if (pass) far_chunk_fwd<P, 16, true>(hb, stf, len, g, ux, uy, uz, acc, shift_sum);
-            else far_chunk_fwd<P, 16, false>(hb, stf, len, g, ux, uy, uz, acc, shift_sum);
+            if (trim) far_chunk_trim<P, 16>(hb, stf, len, g, ux, uy, uz, acc);
+            else if (pass) far_chunk_fwd<P, true>(hb, stf, len, g, ux, uy, uz, acc, shift_sum, 16);
+            else far_chunk_fwd<P, false>(hb, stf, len, g, ux, uy, uz, acc, shift_sum, a.flush);
             stage_next(st, plan, a.hi, a.lo, c, seq);
         }
         seq += plan.n_chunks;
@@ -561,24 +580,32 @@ static int launch_t(K kern, dim3 grid, int threads, size_t smem, const FieldArgs
 
 // Near (FP64) kernel over every region.  mode 0 = the FP64 oracle kernel
 // (must run on an all-near region set), 1 = mixed with cutoff test, 2 =
-// mixed without (near pairs provably inside the cutoff).
+// mixed without (near pairs provably inside the cutoff).  EXPAND: add the
+// local expansions (FieldArgs::poly, and e64's contents).
+template <bool EXPAND>
 static int launch_near(const FieldArgs &a, int cb, int mode, cudaStream_t stream) {
     const size_t smem = near_smem(a.n_types);
-    if (cb == 32) {
-        dim3 grid(a.n_regions, (a.O + 31) / 32);
-        if (mode == 0) return launch_t(field_near_kernel<32, 8, 4, 0>, grid, 256, smem, a, stream);
-        if (mode == 1) return launch_t(field_near_kernel<32, 8, 4, 1>, grid, 256, smem, a, stream);
-        return launch_t(field_near_kernel<32, 8, 4, 2>, grid, 256, smem, a, stream);
+    const dim3 grid(a.n_regions, cb == 32 ? (a.O + 31) / 32 : (a.O + 63) / 64);
+    if constexpr (!EXPAND) {
+        if (cb == 32) {
+            if (mode == 0)
+                return launch_t(field_near_kernel<32, 8, 4, 0>, grid, 256, smem, a, stream);
+            if (mode == 1)
+                return launch_t(field_near_kernel<32, 8, 4, 1>, grid, 256, smem, a, stream);
+            return launch_t(field_near_kernel<32, 8, 4, 2>, grid, 256, smem, a, stream);
+        }
+        if (mode == 0)
+            return cb == 8
+                       ? launch_t(field_near_kernel<8, 16, 4, 0>, grid, 128, smem, a, stream)
+                       : launch_t(field_near_kernel<16, 16, 4, 0>, grid, 256, smem, a, stream);
     }
-    dim3 grid(a.n_regions, (a.O + 63) / 64);
-    if (cb == 8) {
-        if (mode == 0) return launch_t(field_near_kernel<8, 16, 4, 0>, grid, 128, smem, a, stream);
-        if (mode == 1) return launch_t(field_near_kernel<8, 16, 4, 1>, grid, 128, smem, a, stream);
-        return launch_t(field_near_kernel<8, 16, 4, 2>, grid, 128, smem, a, stream);
-    }
-    if (mode == 0) return launch_t(field_near_kernel<16, 16, 4, 0>, grid, 256, smem, a, stream);
-    if (mode == 1) return launch_t(field_near_kernel<16, 16, 4, 1>, grid, 256, smem, a, stream);
-    return launch_t(field_near_kernel<16, 16, 4, 2>, grid, 256, smem, a, stream);
+    if (cb == 8)
+        return mode == 1
+                   ? launch_t(field_near_kernel<8, 16, 4, 1, EXPAND>, grid, 128, smem, a, stream)
+                   : launch_t(field_near_kernel<8, 16, 4, 2, EXPAND>, grid, 128, smem, a, stream);
+    return mode == 1
+               ? launch_t(field_near_kernel<16, 16, 4, 1, EXPAND>, grid, 256, smem, a, stream)
+               : launch_t(field_near_kernel<16, 16, 4, 2, EXPAND>, grid, 256, smem, a, stream);
 }
 
 // Far kernels (threads = CB x G, directors per CTA = G x P):
@@ -588,15 +615,17 @@ static int launch_near(const FieldArgs &a, int cb, int mode, cudaStream_t stream
 //            cutoff mask, reciprocal of q per lane cubed, no Newton step
 //   9:       field_far_kernel <16, 8, 4>: reciprocal of q^3 per lane + Newton
 //            step, every entry masked (the earlier kernel, for comparison)
+template <bool EXPAND>
 static int launch_far(const FieldArgs &a, int cb, int variant, cudaStream_t stream) {
     const size_t smem = far_smem(a.n_types);
     if (cb == 8)
-        return launch_t(field_far2_kernel<8, 16, 4, 6>, dim3(a.n_regions, (a.O + 63) / 64), 128,
-                        smem, a, stream);
+        return launch_t(field_far2_kernel<8, 16, 4, EXPAND ? 5 : 6, EXPAND>,
+                        dim3(a.n_regions, (a.O + 63) / 64), 128, smem, a, stream);
     const dim3 grid(a.n_regions, (a.O + 31) / 32);
     if (cb == 32) return launch_t(field_far2_kernel<32, 8, 4, 2>, grid, 256, smem, a, stream);
     if (variant == 9) return launch_t(field_far_kernel<16, 8, 4, 4>, grid, 128, smem, a, stream);
-    return launch_t(field_far2_kernel<16, 8, 4, 6>, grid, 128, smem, a, stream);
+    return launch_t(field_far2_kernel<16, 8, 4, EXPAND ? 5 : 6, EXPAND>, grid, 128, smem, a,
+                    stream);
 }
 
 static FieldArgs make_args(System *sys, const RegionSet *rs, int n_axes, const double *d_axes,
@@ -623,14 +652,17 @@ static FieldArgs make_args(System *sys, const RegionSet *rs, int n_axes, const d
     a.tf = sys->d_tf;
     a.td = sys->d_td;
     a.n_types = sys->n_types;
+    a.flush = list_flush(*rs, sys->cutoff);
+    a.poly = nullptr;
     a.e64 = d_e64;
     a.status = sys->d_status;
     return a;
 }
 
-// The near kernel writes e64, the far kernel adds its sums to it.
-int launch_field(System *sys, const RegionSet *rs, int n_axes, const double *d_axes,
-                 double *d_e64, int cb, int variant, cudaStream_t stream) {
+// Local expansions (when they pay) into e64, the near kernel adds to them or
+// writes e64, the far kernel adds its sums to it.
+int launch_field(System *sys, const RegionSet *rs, int n_axes, const double *axes_host,
+                 const double *d_axes, double *d_e64, int cb, int variant, cudaStream_t stream) {
     FieldArgs a = make_args(sys, rs, n_axes, d_axes, d_e64);
     sys->split_timed = false;
     if (rs->r_split >= 1e29 && variant == kPlainVariant) {            // plain FP64 baseline
@@ -643,15 +675,32 @@ int launch_field(System *sys, const RegionSet *rs, int n_axes, const double *d_a
         VEXT_CUDA(cudaGetLastError());
         return 0;
     }
-    if (rs->r_split >= 1e29) return launch_near(a, cb, 0, stream);   // FP64 oracle
+    if (rs->r_split >= 1e29) return launch_near<false>(a, cb, 0, stream);   // FP64 oracle
     // near pairs are at most r_split + 2 (rho + max|offset|) apart
     double rho = 0;
     for (const RegionInfo &r : rs->h_info) rho = std::max(rho, r.rho);
     const int near_mode = rs->r_split + 2.0 * (rho + sys->max_offset) + 1e-6 < sys->cutoff ? 2 : 1;
-    VEXT_TRY(launch_near(a, cb, near_mode, stream));
+    if (variant != 9 && cb != 32 && taylor_worthwhile(*sys, *rs, n_axes, false)) {
+        TaylorPlan &plan = sys->field_plan;
+        if (sys->field_plan_set != rs || sys->field_plan_axes.size() != 3 * (size_t)n_axes ||
+            !std::equal(axes_host, axes_host + 3 * n_axes, sys->field_plan_axes.begin())) {
+            sys->field_plan_set = nullptr;
+            VEXT_TRY(taylor_prepare(*sys, *rs, n_axes, d_axes, false, plan, stream));
+            sys->field_plan_set = rs;
+            sys->field_plan_axes.assign(axes_host, axes_host + 3 * n_axes);
+        }
+        VEXT_TRY(ensure_capacity(sys->d_sums, sys->sums_cap, taylor_workspace(*rs)));
+        const bool sym = a.off0 != 0.0 && a.off1 == -a.off0;
+        VEXT_TRY(taylor_enqueue(*sys, *rs, n_axes, plan, sym, sys->d_sums, nullptr, d_e64,
+                                nullptr, stream));
+        a.poly = plan.poly;
+    }
+    VEXT_TRY(a.poly ? launch_near<true>(a, cb, near_mode, stream)
+                    : launch_near<false>(a, cb, near_mode, stream));
     VEXT_CUDA(cudaEventRecord(sys->ev[5], stream));   // near | far split of the timing
     sys->split_timed = true;
-    return launch_far(a, cb, variant, stream);
+    return a.poly ? launch_far<true>(a, cb, variant, stream)
+                  : launch_far<false>(a, cb, variant, stream);
 }
 
 // Everything on device pointers and `stream`; region lists are built (with
@@ -689,7 +738,7 @@ static int field_device(System *sys, int size, int n_axes, const double *axes_ho
     VEXT_CUDA(cudaMemsetAsync(sys->d_refine, 0, sizeof(int), stream));
     const FieldArgs a = make_args(sys, rs, n_axes, sys->d_axes, sys->d_e64);
     VEXT_CUDA(cudaEventRecord(sys->ev[0], stream));
-    VEXT_TRY(launch_field(sys, rs, n_axes, sys->d_axes, sys->d_e64, cb,
+    VEXT_TRY(launch_field(sys, rs, n_axes, axes_host, sys->d_axes, sys->d_e64, cb,
                           o.mode == VEXT_MODE_FP64_PLAIN   ? kPlainVariant
                           : o.mode == VEXT_MODE_FP32_NAIVE ? kNaiveVariant
                                                            : o.variant,
@@ -826,12 +875,23 @@ static int field_adjoint_device(vext_system h, int size, int n_axes, const doubl
                           sys->adj_key[2] == o.band_hi &&
                           sys->adj_key[3] == batch_key(o) &&
                           sys->adj_energy64 == energy_f64;
+        // outputs in host memory: expansion values stand in device scratch
+        float *init[2] = {energy, gradient};
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, energy) != cudaSuccess) cudaGetLastError();
+        else if (at.type == cudaMemoryTypeHost) {
+            const size_t n = (size_t)(S3 * n_axes);
+            VEXT_TRY(ensure_capacity(sys->d_f32, sys->f32_cap, n));
+            VEXT_TRY(ensure_capacity(sys->d_g32, sys->g32_cap, 6 * n));
+            init[0] = sys->d_f32;
+            init[1] = sys->d_g32;
+        }
         if (!same) {
             if (sys->adj_batch) vext_batch_destroy(sys->adj_batch);   // (host parts stay)
             sys->adj_batch = nullptr;
             vext_batch b = nullptr;
             VEXT_TRY(batch_build(1, &h, size, n_axes, axes, opt, &energy, &gradient,
-                                 energy_f64 ? &energy_f64 : nullptr, false, &b));
+                                 energy_f64 ? &energy_f64 : nullptr, false, &b, n_axes, init));
             sys->adj_batch = b;
             sys->adj_size = size;
             sys->adj_axes.assign(axes, axes + 3 * n_axes);
@@ -843,7 +903,7 @@ static int field_adjoint_device(vext_system h, int size, int n_axes, const doubl
         }
         // other float32 outputs than the last call's: a stream-ordered update
         // of the batch's output pointers, no rebuild
-        VEXT_TRY(batch_retarget(sys->adj_batch, 0, energy, gradient, stream));
+        VEXT_TRY(batch_retarget(sys->adj_batch, 0, energy, gradient, init[0], init[1], stream));
         return batch_replay(sys->adj_batch, stream);
     }
     if (o.mode != VEXT_MODE_FP64 && o.mode != VEXT_MODE_FP64_PLAIN)
@@ -964,7 +1024,7 @@ extern "C" int vext_field_adjoint(vext_system h, int size, int n_axes, const dou
                 float *gk = sys->d_g32 + 6 * blk * (size_t)k * S3;
                 vext_batch b = nullptr;
                 VEXT_TRY(batch_build(1, &h, size, nk, axes + 3 * blk * k, opt, &ek, &gk, nullptr,
-                                     false, &b));
+                                     false, &b, n_axes, nullptr));
                 sys->host_parts.push_back(b);
                 cudaEvent_t ev;
                 VEXT_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));

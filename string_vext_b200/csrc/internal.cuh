@@ -40,6 +40,11 @@ struct alignas(16) RegionInfo {
                         // region (they follow the near entries; the shell ones come last)
     int n_outer;        // the last shell entries: beyond rc + rho + 1e-3 A of the origin,
                         // hence beyond rc of every pose center of the region
+    int n_mid;          // the first of the inner entries: too near the origin for its local
+                        // expansion (taylor.cuh), which covers the rest
+    int n_shella;       // the first of the shell entries: so near that a symmetric director's
+                        // site on the entry's side is inside the cutoff for every pose
+    int pad[2];
 };
 static_assert(sizeof(RegionInfo) % 16 == 0, "RegionInfo must stay 16-byte aligned");
 
@@ -53,6 +58,9 @@ struct RegionSet {
     int n_regions = 0;
     int n_ri = 0, n_rj = 0, n_rk = 0;       // regions per axis
     long long n_entries = 0, n_near = 0, n_outer = 0;
+    long long n_taylor = 0;                 // inner entries of the expansions (taylor.cuh)
+    double d_taylor = 1e30;                 // their smallest distance from the origin
+    double taylor_radius = 0;               // every site of a region lies this near its origin
     RegionInfo *d_info = nullptr;
     float4 *d_hi = nullptr, *d_lo = nullptr;
     std::vector<RegionInfo> h_info;
@@ -60,6 +68,24 @@ struct RegionSet {
     bool stale = false;                     // rebuild before the next use
     float build_ms = 0;
     ~RegionSet();
+};
+
+// One system's local expansions in a field or batch (taylor.cuh): the
+// evaluation matrix and the per-region polynomials (null poly: the system's
+// inner pairs are summed directly).
+struct TaylorPlan {
+    double *poly = nullptr;     // [n_regions][kTaylorPolyPad]
+    float *matrix = nullptr;    // [kTaylorPad][rows]
+    size_t poly_cap = 0, matrix_cap = 0;
+    int rows = 0;               // outputs of a region's poses, padded to the tile
+    int outs = 0;               // outputs per pose: 1 (energy) or 7
+    void release() {
+        cudaFree(poly);
+        cudaFree(matrix);
+        poly = nullptr;
+        matrix = nullptr;
+        poly_cap = matrix_cap = 0;
+    }
 };
 
 // One system's view for the warp-per-pose kernel (posebatch.cu).
@@ -110,6 +136,12 @@ struct System {
     size_t e64T_cap = 0;
     int *d_flags = nullptr;        // [0] non-finite count
     size_t flags_cap = 0;
+    // local expansions of the field path: plan of the last (lists, directors)
+    TaylorPlan field_plan;
+    const RegionSet *field_plan_set = nullptr;
+    std::vector<double> field_plan_axes;
+    float *d_sums = nullptr;
+    size_t sums_cap = 0;
     // scratch of the pose path
     void *d_pose_scratch = nullptr;
     size_t pose_scratch_cap = 0;
@@ -154,9 +186,10 @@ struct System {
 int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
                 const double *axes, const vext_options *opt, float *const *outputs,
                 float *const *gradients, double *const *outputs_f64, bool lock_systems,
-                vext_batch *out);
+                vext_batch *out, int rule_axes, float *const *init);
 int batch_replay(vext_batch b, cudaStream_t stream);
-int batch_retarget(vext_batch b, int k, float *out, float *grad, cudaStream_t stream);
+int batch_retarget(vext_batch b, int k, float *out, float *grad, float *init, float *init_grad,
+                   cudaStream_t stream);
 
 // Region sets (system.cu)
 int get_field_regions(System *sys, int size, int cb, double r_split, RegionSet **out,
@@ -209,6 +242,13 @@ inline double floor_clear_radius2(const System &sys) {
     return rf * rf;
 }
 
+// Far entries per FP32 energy partial in the unmasked pass over inner entries:
+// 16, or 8 where the lists set the nearer ones apart (RegionInfo::n_mid).  A
+// partial's rounding grows with its sum, and with the nearest entries next to
+// one another partials over 16 gave 1.55e-4 instead of 1.26e-4 K at worst in a
+// slab framework whose pairs were summed unsorted to 1.24e-4 K.
+inline int list_flush(const RegionSet &rs, double cutoff) { return rs.d_taylor < cutoff ? 8 : 16; }
+
 // Directors per work item of a batch with these options (32 or 64; its
 // regions hold 512 / that many grid centers).
 int batch_item_directors(const Options &o, bool adjoint);
@@ -226,8 +266,8 @@ int pose_warp_enqueue(System *sys, const RegionSet *rs, int n, const double *cen
                       double *gq, double *gu, cudaStream_t st);
 
 // Field kernel launcher (field.cu): computes E64 [O][S^3] for all regions.
-int launch_field(System *sys, const RegionSet *rs, int n_axes, const double *d_axes,
-                 double *d_e64, int cb, int variant, cudaStream_t stream);
+int launch_field(System *sys, const RegionSet *rs, int n_axes, const double *axes_host,
+                 const double *d_axes, double *d_e64, int cb, int variant, cudaStream_t stream);
 
 }  // namespace vext
 

@@ -16,6 +16,12 @@ __device__ __forceinline__ float set_lt(float a, float b) {
     return r;
 }
 
+__device__ __forceinline__ float set_ge(float a, float b) {
+    float r;
+    asm("set.ge.f32.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // FP64 reciprocal: hardware seed (relative error <= 2^-23) refined by
 // Newton-Raphson steps r' = r + r (1 - s r), each squaring the relative error
 // and leaving it one-sided (r under-estimates): one step leaves <= 2^-46
@@ -508,7 +514,7 @@ __device__ __forceinline__ void far_chunk(const float4 *hb, const float4 *stf, i
 // Newton step), n3 = n1^3 = q^-3, e = n3 (c12 n3 - c6); MASK as in
 // far_chunk_adj (inner entries: no mask, shift summed once per entry into
 // shift_sum, to be added twice -- both sites -- to every energy).  FP32
-// partials over FLUSH entries are flushed into the FP64 acc.  Shell entries
+// partials over `flush` entries are flushed into the FP64 acc.  Shell entries
 // beyond every site's cutoff (the list radius carries the region radius on
 // top) are skipped: they would add exactly nothing.
 // OUTER (symmetric sites, MASK): entries [outer_from, len) are outer shell
@@ -517,22 +523,22 @@ __device__ __forceinline__ void far_chunk(const float4 *hb, const float4 *stf, i
 // |d0|^2 + o^2 > rc^2 and adds exact zeros; only the near site (q = |d0|^2 +
 // o^2 - |2 o t|, the same FP32 fma as its two-site q) is evaluated there, so
 // the partials, and the result, are bit for bit those of the two-site loop.
-template <int P, int FLUSH, bool MASK, bool OUTER = false>
+template <int P, bool MASK, bool OUTER = false>
 __device__ __forceinline__ void far_chunk_fwd(const float4 *hb, const float4 *stf, int len,
                                               const FarGeom &g, const float2 (&ux)[P / 2],
                                               const float2 (&uy)[P / 2],
                                               const float2 (&uz)[P / 2], double (&acc)[P],
-                                              double &shift_sum, int outer_from = 0) {
+                                              double &shift_sum, int flush, int outer_from = 0) {
     static_assert(!OUTER || MASK, "outer entries are shell entries");
     constexpr int PP = P / 2;
     const float2 nam = make_float2(-fabsf(g.m0.x), -fabsf(g.m0.x));   // -|m0|
 #pragma unroll 1
-    for (int e0 = 0; e0 < len; e0 += FLUSH) {
+    for (int e0 = 0; e0 < len; e0 += flush) {
         float2 fa[PP];
         float fs = 0.f;
 #pragma unroll
         for (int j = 0; j < PP; ++j) fa[j] = make_float2(0.f, 0.f);
-        const int e1 = min(e0 + FLUSH, len);
+        const int e1 = min(e0 + flush, len);
         const int em = OUTER ? max(e0, min(e1, outer_from)) : e1;
 #pragma unroll 2
         for (int e = e0; e < em; ++e) {
@@ -614,6 +620,58 @@ __device__ __forceinline__ void far_chunk_fwd(const float4 *hb, const float4 *st
         for (int j = 0; j < PP; ++j) {
             acc[2 * j] += (double)fa[j].x;
             acc[2 * j + 1] += (double)fa[j].y;
+        }
+    }
+}
+
+// Near shell entries (RegionInfo::n_shella) of a region whose local expansion
+// (taylor.cuh) holds them as if inside, symmetric sites: the site on the
+// entry's side has q <= |d0|^2 + o^2 < rc^2 for every pose; where the other
+// site, q = |d0|^2 + o^2 + |2 o t|, lies outside, its pair is taken out of
+// acc again.
+template <int P, int FLUSH>
+__device__ __forceinline__ void far_chunk_trim(const float4 *hb, const float4 *stf, int len,
+                                               const FarGeom &g, const float2 (&ux)[P / 2],
+                                               const float2 (&uy)[P / 2],
+                                               const float2 (&uz)[P / 2], double (&acc)[P]) {
+    constexpr int PP = P / 2;
+    const float2 am = make_float2(fabsf(g.m0.x), fabsf(g.m0.x));
+#pragma unroll 1
+    for (int e0 = 0; e0 < len; e0 += FLUSH) {
+        float2 fa[PP];
+#pragma unroll
+        for (int j = 0; j < PP; ++j) fa[j] = make_float2(0.f, 0.f);
+        const int e1 = min(e0 + FLUSH, len);
+#pragma unroll 2
+        for (int e = e0; e < e1; ++e) {
+            const float4 h = hb[e];
+            const float4 tp = stf[__float_as_int(h.w)];
+            const float dx = h.x - g.cx, dy = h.y - g.cy, dz = h.z - g.cz;
+            const float dd = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+            const float2 k0 = make_float2(dd + g.oo0, dd + g.oo0), dx2 = make_float2(dx, dx),
+                         dy2 = make_float2(dy, dy), dz2 = make_float2(dz, dz),
+                         c12 = make_float2(tp.x, tp.x), mc6 = make_float2(-tp.y, -tp.y),
+                         sh = make_float2(tp.z, tp.z);
+#pragma unroll
+            for (int j = 0; j < PP; ++j) {
+                const float2 t =
+                    __ffma2_rn(dx2, ux[j], __ffma2_rn(dy2, uy[j], __fmul2_rn(dz2, uz[j])));
+                const float2 d2 = __ffma2_rn(am, make_float2(fabsf(t.x), fabsf(t.y)), k0);
+                float r0, r1;
+                asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(d2.x));
+                asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(d2.y));
+                const float2 n1 = make_float2(r0, r1);
+                float2 n3 = __fmul2_rn(__fmul2_rn(n1, n1), n1);
+                const float2 m = make_float2(set_ge(d2.x, g.rc2f), set_ge(d2.y, g.rc2f));
+                n3 = __fmul2_rn(n3, m);
+                fa[j] = __ffma2_rn(m, sh, fa[j]);
+                fa[j] = __ffma2_rn(n3, __ffma2_rn(c12, n3, mc6), fa[j]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < PP; ++j) {
+            acc[2 * j] -= (double)fa[j].x;
+            acc[2 * j + 1] -= (double)fa[j].y;
         }
     }
 }
@@ -785,7 +843,8 @@ __device__ __forceinline__ void grad_load(double *gsum, AdjAcc (&acc)[P]) {
 // pose of the region): no mask, and the shift, the same for every pose, is
 // summed once per entry into shift_sum (the caller adds 2 x shift_sum, both
 // sites, to every energy).  FP32 partials are flushed into the FP64 AdjAcc:
-// the energy every 16 entries, the gradient sums every FLUSH entries.
+// the energy every `eb` entries (16, or list_flush's 8), the gradient sums
+// every FLUSH entries.
 // GSUM_NT > 0: the gradient partials go to the shared-memory sums
 // (grad_slot<GSUM_NT>(gsum, ...)) instead of acc (whose energies stay).
 // border (masked entries only, when non-null): per director the smallest
@@ -802,7 +861,7 @@ __device__ __forceinline__ void far_chunk_adj(const float4 *hb, const float4 *st
                                               const float2 (&uy)[P / 2],
                                               const float2 (&uz)[P / 2], AdjAcc (&acc)[P],
                                               double &shift_sum, double *gsum = nullptr,
-                                              float *border = nullptr) {
+                                              float *border = nullptr, int eb = 16) {
     constexpr int PP = P / 2;
     const float2 one2 = make_float2(1.f, 1.f);
     const float2 mrc2 = make_float2(-g.rc2f, -g.rc2f);
@@ -819,12 +878,12 @@ __device__ __forceinline__ void far_chunk_adj(const float4 *hb, const float4 *st
             }
         const int e1 = min(e0 + FLUSH, len);
 #pragma unroll 1
-        for (int b0 = e0; b0 < e1; b0 += 16) {   // energy partials: 16 entries
+        for (int b0 = e0; b0 < e1; b0 += eb) {   // energy partials: eb entries
         float2 fe[PP];
         float fs = 0.f;
 #pragma unroll
         for (int j = 0; j < PP; ++j) fe[j] = make_float2(0.f, 0.f);
-        const int b1 = min(b0 + 16, e1);
+        const int b1 = min(b0 + eb, e1);
 #pragma unroll UNROLL
         for (int e = b0; e < b1; ++e) {
             float2 k0, k1, dx2, dy2, dz2, c12, c6, sh, mc6, m2c12;
@@ -970,7 +1029,11 @@ __device__ __forceinline__ void far_chunk_adj(const float4 *hb, const float4 *st
 // where the near site is site 0, -1 where it is site 1), flushed as H_0 =
 // (A + B) / 2, H_1 = (A - B) / 2 and F_0 - F_1 = C (f[0] of the symmetric
 // loops).  BORDER 2: the per-director cutoff-border test of far_chunk_adj.
-template <int P, int FLUSH, int UNROLL, int GSUM_NT, int BORDER>
+// TRIM: the near shell entries instead (far_chunk_trim: the site on the
+// entry's side is inside for every pose, and the local expansion holds both
+// sites as if inside): the other site's pair, q = k0 + |m_0| |t| (again its
+// own fma bit for bit), is taken out of the sums where it lies outside.
+template <int P, int FLUSH, int UNROLL, int GSUM_NT, int BORDER, bool TRIM = false>
 __device__ __forceinline__ void far_chunk_outer(const float4 *hb, const float4 *stf, int len,
                                                 const FarGeom &g, const float2 (&ux)[P / 2],
                                                 const float2 (&uy)[P / 2],
@@ -979,8 +1042,12 @@ __device__ __forceinline__ void far_chunk_outer(const float4 *hb, const float4 *
                                                 float *border = nullptr) {
     static_assert(BORDER != 1, "the outer loop serves the symmetric-site kernels");
     constexpr int PP = P / 2;
-    const float2 nam = make_float2(-fabsf(g.m0.x), -fabsf(g.m0.x));   // -|m0|
-    const bool m0neg = g.m0.x < 0.f;   // site 0 is the near one where t > 0
+    // near site: -|m0| and site 0 where t > 0 (m0 < 0); the other site: |m0|
+    // and site 0 where t <= 0
+    const float am = TRIM ? fabsf(g.m0.x) : -fabsf(g.m0.x);
+    const float2 nam = make_float2(am, am);
+    const bool m0neg = (g.m0.x < 0.f) != TRIM;
+    constexpr double kSign = TRIM ? -1.0 : 1.0;
 #pragma unroll 1
     for (int e0 = 0; e0 < len; e0 += FLUSH) {
         float2 fa[PP][3], fb[PP][3], fc[PP];
@@ -1006,7 +1073,7 @@ __device__ __forceinline__ void far_chunk_outer(const float4 *hb, const float4 *
                     const float4 tp = stf[__float_as_int(h.w)];   // (c12, c6, shift, -)
                     const float dx = h.x - g.cx, dy = h.y - g.cy, dz = h.z - g.cz;
                     const float dd = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                    if (dd > g.out2) continue;
+                    if (!TRIM && dd > g.out2) continue;
                     k0 = make_float2(dd + g.oo0, dd + g.oo0);
                     dx2 = make_float2(dx, dx);
                     dy2 = make_float2(dy, dy);
@@ -1033,7 +1100,9 @@ __device__ __forceinline__ void far_chunk_outer(const float4 *hb, const float4 *
                     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(d2.y));
                     const float2 n1 = make_float2(r0, r1);
                     float2 n3 = __fmul2_rn(__fmul2_rn(n1, n1), n1);
-                    const float2 m = make_float2(set_lt(d2.x, g.rc2f), set_lt(d2.y, g.rc2f));
+                    const float2 m =
+                        TRIM ? make_float2(set_ge(d2.x, g.rc2f), set_ge(d2.y, g.rc2f))
+                             : make_float2(set_lt(d2.x, g.rc2f), set_lt(d2.y, g.rc2f));
                     n3 = __fmul2_rn(n3, m);
                     fe[j] = __ffma2_rn(m, sh, fe[j]);
                     fe[j] = __ffma2_rn(n3, __ffma2_rn(c12, n3, mc6), fe[j]);
@@ -1051,8 +1120,8 @@ __device__ __forceinline__ void far_chunk_outer(const float4 *hb, const float4 *
             }
 #pragma unroll
             for (int j = 0; j < PP; ++j) {
-                acc[2 * j].e += (double)fe[j].x;
-                acc[2 * j + 1].e += (double)fe[j].y;
+                acc[2 * j].e += kSign * (double)fe[j].x;
+                acc[2 * j + 1].e += kSign * (double)fe[j].y;
             }
         }
 #pragma unroll
@@ -1065,18 +1134,18 @@ __device__ __forceinline__ void far_chunk_outer(const float4 *hb, const float4 *
                     const double a = (double)(l ? fa[j][k].y : fa[j][k].x);
                     const double b = (double)(l ? fb[j][k].y : fb[j][k].x);
                     if constexpr (GSUM_NT > 0) {
-                        grad_slot<GSUM_NT>(gsum, p, k) += 0.5 * (a + b);
-                        grad_slot<GSUM_NT>(gsum, p, 3 + k) += 0.5 * (a - b);
+                        grad_slot<GSUM_NT>(gsum, p, k) += 0.5 * kSign * (a + b);
+                        grad_slot<GSUM_NT>(gsum, p, 3 + k) += 0.5 * kSign * (a - b);
                     } else {
-                        acc[p].h[0][k] += 0.5 * (a + b);
-                        acc[p].h[1][k] += 0.5 * (a - b);
+                        acc[p].h[0][k] += 0.5 * kSign * (a + b);
+                        acc[p].h[1][k] += 0.5 * kSign * (a - b);
                     }
                 }
                 const double c = (double)(l ? fc[j].y : fc[j].x);
                 if constexpr (GSUM_NT > 0)
-                    grad_slot<GSUM_NT>(gsum, p, 6) += c;
+                    grad_slot<GSUM_NT>(gsum, p, 6) += kSign * c;
                 else
-                    acc[p].f[0] += c;
+                    acc[p].f[0] += kSign * c;
             }
     }
 }

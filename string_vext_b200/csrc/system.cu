@@ -20,6 +20,7 @@
 #include <map>
 
 #include "internal.cuh"
+#include "taylor.cuh"
 
 namespace vext {
 
@@ -110,6 +111,30 @@ struct BuildArgs {
     double r_near0;   // r_split + max|offset| (+ margin)
     double r_inner0;  // cutoff - max|offset| (- margin): inner entries lie within r_inner0 - rho
     double r_outer0;  // cutoff + 1e-3 A: outer shell entries lie beyond r_outer0 + rho
+    double r_taylor;  // inner entries beyond it belong to the local expansion
+    double r_shella0; // shell entries within r_shella0 - rho: the nearer of two symmetric sites
+                      // is inside the cutoff for every pose (0: none are set apart)
+};
+
+// Class boundaries (squared distance from the origin) of one region, in
+// increasing order: near | mid | taylor | shell a | shell | outer is the order
+// of the classes and of the entries.
+constexpr int kClasses = 6;
+struct ClassRadii {
+    double rl, at[kClasses - 1];
+    __device__ ClassRadii(const BuildArgs &a, const RegionInfo &r) {
+        rl = a.r_list0 + r.rho;
+        const double rn = a.r_near0 + r.rho, ri = fmax(a.r_inner0 - r.rho, 0.0),
+                     ra = fmax(a.r_shella0 - r.rho, 0.0), ro = a.r_outer0 + r.rho;
+        at[0] = rn * rn;
+        at[2] = fmax(ri * ri, at[0]);
+        at[1] = fmin(fmax(a.r_taylor * a.r_taylor, at[0]), at[2]);
+        at[3] = fmax(ra * ra, at[2]);
+        at[4] = fmax(ro * ro, at[3]);
+    }
+};
+struct ClassCounts {
+    int n[kClasses];
 };
 
 // Visit every candidate image of atom j for a region; f(dist2, rel) per image.
@@ -182,83 +207,104 @@ __device__ __forceinline__ void block_scan2(int a, int b, int &pa, int &pb, int 
     __syncthreads();
 }
 
-constexpr int kBuildThreads = 256;
+// Threads per region of the list builds: field lists take 128 (fewer idle
+// threads in the last round of atoms, half the counts to hand over), pose bins
+// 256.
+constexpr int kBuildThreads = 256, kFieldBuildThreads = 128;
 
 // Per region: the entries of each class, and per thread (atoms j = tid, tid +
-// kBuildThreads, ...) its (near, inner, shell, outer) counts for the fill.
-__global__ void __launch_bounds__(kBuildThreads)
-    region_count_kernel(BuildArgs a, RegionInfo *regs, int n_regions, int4 *counts) {
+// NT, ...) its counts per class for the fill.
+template <int NT>
+__global__ void __launch_bounds__(NT)
+    region_count_kernel(BuildArgs a, RegionInfo *regs, int n_regions, ClassCounts *counts) {
     const int region = blockIdx.x;
     if (region >= n_regions) return;
     const RegionInfo r = regs[region];
-    const double rl = a.r_list0 + r.rho, rn = a.r_near0 + r.rho, rn2 = rn * rn;
-    const double ri = a.r_inner0 - r.rho, ri2 = ri > 0 ? ri * ri : 0.0;
-    const double ro = a.r_outer0 + r.rho, ro2 = ro * ro;
-    int near = 0, inner = 0, outer = 0, total = 0;
-    for (int j = threadIdx.x; j < a.n_atoms; j += kBuildThreads)
-        for_each_image(a, r, j, rl, [&](double q, double, double, double) {
-            ++total;
-            near += q < rn2;
-            inner += q >= rn2 && q < ri2;
-            outer += q >= rn2 && q >= ri2 && q >= ro2;
+    const ClassRadii cls(a, r);
+    int from[kClasses] = {0, 0, 0, 0, 0, 0};   // entries at or beyond each boundary
+    for (int j = threadIdx.x; j < a.n_atoms; j += NT)
+        for_each_image(a, r, j, cls.rl, [&](double q, double, double, double) {
+            ++from[0];
+#pragma unroll
+            for (int i = 1; i < kClasses; ++i) from[i] += q >= cls.at[i - 1];
         });
-    counts[(long long)region * kBuildThreads + threadIdx.x] =
-        make_int4(near, inner, total - near - inner - outer, outer);
+    ClassCounts c;
+#pragma unroll
+    for (int i = 0; i < kClasses; ++i) c.n[i] = from[i] - (i + 1 < kClasses ? from[i + 1] : 0);
+    counts[(long long)region * NT + threadIdx.x] = c;
     __shared__ int sh[128];
-    int pa, pb, ta, tb, pc, pd, tc, td;
-    block_scan2<kBuildThreads>(near, total, pa, pb, ta, tb, sh);
-    block_scan2<kBuildThreads>(inner, outer, pc, pd, tc, td, sh);
+    int p, q, t[kClasses];
+#pragma unroll
+    for (int i = 0; i < kClasses; i += 2)
+        block_scan2<NT>(c.n[i], c.n[i + 1], p, q, t[i], t[i + 1], sh);
     if (threadIdx.x == 0) {
-        regs[region].n_near = ta;
-        regs[region].n_total = tb;
-        regs[region].n_inner = tc;
-        regs[region].n_outer = td;
+        RegionInfo &w = regs[region];
+        w.n_near = t[0];
+        w.n_mid = t[1];
+        w.n_inner = t[1] + t[2];
+        w.n_shella = t[3];
+        w.n_outer = t[5];
+        w.n_total = t[0] + t[1] + t[2] + t[3] + t[4] + t[5];
     }
 }
 
-// Entry order inside each class: thread-major (thread t's atoms t, t +
-// kBuildThreads, ... in turn, each atom's images in enumeration order), so a
-// thread's slots follow from a block scan of the per-thread counts that
-// region_count_kernel stored and the candidates are enumerated once here.
-__global__ void __launch_bounds__(kBuildThreads, 2)
-    region_fill_kernel(BuildArgs a, const RegionInfo *regs, int n_regions, const int4 *counts,
-                       float4 *hi, float4 *lo, int *status) {
+// Entry order inside each class: thread-major (thread t's atoms t, t + NT,
+// ... in turn, each atom's images in enumeration order), so a thread's slots
+// follow from a block scan of the per-thread counts that region_count_kernel
+// stored and the candidates are enumerated once here.
+template <int NT>
+__global__ void __launch_bounds__(NT, 512 / NT)
+    region_fill_kernel(BuildArgs a, const RegionInfo *regs, int n_regions,
+                       const ClassCounts *counts, float4 *hi, float4 *lo, int *status) {
     const int region = blockIdx.x;
     if (region >= n_regions) return;
     const RegionInfo r = regs[region];
-    const double rl = a.r_list0 + r.rho, rn = a.r_near0 + r.rho, rn2 = rn * rn;
-    const double ri = a.r_inner0 - r.rho, ri2 = ri > 0 ? ri * ri : 0.0;
-    const double ro = a.r_outer0 + r.rho, ro2 = ro * ro;
+    const ClassRadii cls(a, r);
     __shared__ int sh[128];
-    // entry order: near | far inner | far shell | outer shell
-    const int end_shell = r.n_total - r.n_outer;
-    const int4 c = counts[(long long)region * kBuildThreads + threadIdx.x];
-    int pn, pi, tn, ti, ps, po, ts, to;
-    block_scan2<kBuildThreads>(c.x, c.y, pn, pi, tn, ti, sh);
-    block_scan2<kBuildThreads>(c.z, c.w, ps, po, ts, to, sh);
-    if (threadIdx.x == 0 && (tn != r.n_near || ti != r.n_inner ||
-                             ts != end_shell - r.n_near - r.n_inner || to != r.n_outer))
+    const ClassCounts c = counts[(long long)region * NT + threadIdx.x];
+    // this thread's next slot and end per class (indexed by unrolled loops
+    // only: a runtime index would put them in local memory)
+    int w[kClasses], end[kClasses], t[kClasses];
+#pragma unroll
+    for (int i = 0; i < kClasses; i += 2)
+        block_scan2<NT>(c.n[i], c.n[i + 1], w[i], w[i + 1], t[i], t[i + 1], sh);
+    if (threadIdx.x == 0 && (t[0] != r.n_near || t[1] != r.n_mid || t[1] + t[2] != r.n_inner ||
+                             t[3] != r.n_shella || t[5] != r.n_outer ||
+                             t[0] + t[1] + t[2] + t[3] + t[4] + t[5] != r.n_total))
         atomicExch(status, DEV_BAD_LIST);
-    // this thread's next slot and end per class (scalars: an indexed array
-    // would live in local memory)
-    int wn = pn, wi = r.n_near + pi, ws = r.n_near + r.n_inner + ps, wo = end_shell + po;
-    const int en = wn + c.x, ei = wi + c.y, es = ws + c.z, eo = wo + c.w;
-    for (int j = threadIdx.x; j < a.n_atoms; j += kBuildThreads) {
-        const int t = a.type[j];
-        for_each_image(a, r, j, rl, [&](double q, double x, double y, double z) {
-            const int cls = q < rn2 ? 0 : (q < ri2 ? 1 : (q < ro2 ? 2 : 3));
-            const int slot = cls == 0 ? wn++ : (cls == 1 ? wi++ : (cls == 2 ? ws++ : wo++));
-            const int lim = cls == 0 ? en : (cls == 1 ? ei : (cls == 2 ? es : eo));
+    int base = 0;
+#pragma unroll
+    for (int i = 0; i < kClasses; ++i) {
+        w[i] += base;
+        end[i] = w[i] + c.n[i];
+        base += t[i];
+    }
+    for (int j = threadIdx.x; j < a.n_atoms; j += NT) {
+        const int ty = a.type[j];
+        for_each_image(a, r, j, cls.rl, [&](double q, double x, double y, double z) {
+            int k = 0;
+#pragma unroll
+            for (int i = 1; i < kClasses; ++i) k += q >= cls.at[i - 1];
+            int slot = 0, lim = 0;
+#pragma unroll
+            for (int i = 0; i < kClasses; ++i)
+                if (k == i) {
+                    slot = w[i]++;
+                    lim = end[i];
+                }
             if (slot >= lim) {
                 atomicExch(status, DEV_BAD_LIST);
                 return;
             }
             const float hx = (float)x, hy = (float)y, hz = (float)z;
-            hi[r.off + slot] = make_float4(hx, hy, hz, __int_as_float(t));
+            hi[r.off + slot] = make_float4(hx, hy, hz, __int_as_float(ty));
             lo[r.off + slot] = make_float4((float)(x - hx), (float)(y - hy), (float)(z - hz), 0.f);
         });
     }
-    if (wn != en || wi != ei || ws != es || wo != eo) atomicExch(status, DEV_BAD_LIST);
+    bool full = true;
+#pragma unroll
+    for (int i = 0; i < kClasses; ++i) full = full && w[i] == end[i];
+    if (!full) atomicExch(status, DEV_BAD_LIST);
 }
 
 // ------------------------------------------------------------ region sets
@@ -277,7 +323,7 @@ RegionSet::~RegionSet() {
 namespace {
 struct BuildScratch {
     std::mutex lock;
-    int4 *ptr = nullptr;
+    ClassCounts *ptr = nullptr;
     size_t cap = 0;
     unsigned long long ctx_id = 0;
 };
@@ -335,6 +381,12 @@ static int build_lists(System *sys, RegionSet *rs, cudaStream_t stream) {
     a.r_near0 = rs->r_split + sys->max_offset + 1e-6;
     a.r_inner0 = sys->cutoff - sys->max_offset - 1e-6;
     a.r_outer0 = sys->cutoff + 1e-3;
+    // field lists set the entries of the local expansion apart, and those near
+    // shell entries whose nearer site is always inside: |d0|^2 + o^2 < rc^2
+    // for every center (|d0| the entry's distance from it)
+    a.r_taylor = rs->d_taylor;
+    const double ra2 = sys->cutoff * sys->cutoff - sys->max_offset * sys->max_offset;
+    a.r_shella0 = rs->d_taylor < sys->cutoff && ra2 > 0 ? std::sqrt(ra2) - 1e-3 : 0.0;
     const int n = rs->n_regions;
     if (!rs->d_info) VEXT_CUDA(cudaMalloc(&rs->d_info, sizeof(RegionInfo) * n));
     VEXT_CUDA(cudaMemcpyAsync(rs->d_info, rs->h_info.data(), sizeof(RegionInfo) * n,
@@ -348,23 +400,32 @@ static int build_lists(System *sys, RegionSet *rs, cudaStream_t stream) {
         scratch.ptr = nullptr;
         scratch.cap = 0;
     }
-    VEXT_TRY(ensure_capacity(scratch.ptr, scratch.cap, (size_t)n * kBuildThreads));
+    const bool field = rs->size > 0;
+    VEXT_TRY(ensure_capacity(scratch.ptr, scratch.cap,
+                             (size_t)n * (field ? kFieldBuildThreads : kBuildThreads)));
     scratch.ctx_id = ctx;
-    region_count_kernel<<<n, kBuildThreads, 0, stream>>>(a, rs->d_info, n, scratch.ptr);
+    if (field)
+        region_count_kernel<kFieldBuildThreads>
+            <<<n, kFieldBuildThreads, 0, stream>>>(a, rs->d_info, n, scratch.ptr);
+    else
+        region_count_kernel<kBuildThreads>
+            <<<n, kBuildThreads, 0, stream>>>(a, rs->d_info, n, scratch.ptr);
     VEXT_CUDA(cudaGetLastError());
     VEXT_CUDA(cudaMemcpyAsync(rs->h_info.data(), rs->d_info, sizeof(RegionInfo) * n,
                               cudaMemcpyDeviceToHost, stream));
     VEXT_CUDA(cudaStreamSynchronize(stream));
-    long long off = 0, near = 0, outer = 0;
+    long long off = 0, near = 0, outer = 0, taylor = 0;
     for (auto &r : rs->h_info) {
         r.off = off;
         off += r.n_total;
         near += r.n_near;
         outer += r.n_outer;
+        taylor += r.n_inner - r.n_mid;
     }
     rs->n_entries = off;
     rs->n_near = near;
     rs->n_outer = outer;
+    rs->n_taylor = taylor;
     VEXT_CUDA(cudaMemcpyAsync(rs->d_info, rs->h_info.data(), sizeof(RegionInfo) * n,
                               cudaMemcpyHostToDevice, stream));
     if (off > rs->capacity || !rs->d_hi) {
@@ -376,8 +437,12 @@ static int build_lists(System *sys, RegionSet *rs, cudaStream_t stream) {
         VEXT_CUDA(cudaMalloc(&rs->d_lo, sizeof(float4) * std::max<long long>(off, 1)));
         rs->capacity = std::max<long long>(off, 1);
     }
-    region_fill_kernel<<<n, kBuildThreads, 0, stream>>>(a, rs->d_info, n, scratch.ptr, rs->d_hi,
-                                                        rs->d_lo, sys->d_status);
+    if (field)
+        region_fill_kernel<kFieldBuildThreads><<<n, kFieldBuildThreads, 0, stream>>>(
+            a, rs->d_info, n, scratch.ptr, rs->d_hi, rs->d_lo, sys->d_status);
+    else
+        region_fill_kernel<kBuildThreads><<<n, kBuildThreads, 0, stream>>>(
+            a, rs->d_info, n, scratch.ptr, rs->d_hi, rs->d_lo, sys->d_status);
     VEXT_CUDA(cudaGetLastError());
     VEXT_CUDA(cudaEventRecord(e1, stream));
     VEXT_CUDA(cudaEventSynchronize(e1));
@@ -387,12 +452,19 @@ static int build_lists(System *sys, RegionSet *rs, cudaStream_t stream) {
     return check_status(sys, stream);
 }
 
+static double det3(const Mat3 &m) {
+    const double *h = m.m;
+    return h[0] * (h[4] * h[8] - h[5] * h[7]) - h[1] * (h[3] * h[8] - h[5] * h[6]) +
+           h[2] * (h[3] * h[7] - h[4] * h[6]);
+}
+
 int get_field_regions(System *sys, int size, int cb, double r_split, RegionSet **out,
                       cudaStream_t stream) {
     for (RegionSet *rs : sys->sets)
         if (rs->size == size && rs->bi * rs->bj * rs->bk == cb && rs->r_split == r_split) {
             if (rs->stale) {
-                for (auto &r : rs->h_info) r.n_near = r.n_total = r.n_inner = r.n_outer = 0;
+                for (auto &r : rs->h_info)
+                    r.n_near = r.n_total = r.n_inner = r.n_outer = r.n_mid = r.n_shella = 0;
                 VEXT_TRY(build_lists(sys, rs, stream));
             }
             *out = rs;
@@ -407,6 +479,7 @@ int get_field_regions(System *sys, int size, int cb, double r_split, RegionSet *
     rs->n_rk = (size + rs->bk - 1) / rs->bk;
     rs->n_regions = rs->n_ri * rs->n_rj * rs->n_rk;
     rs->h_info.resize(rs->n_regions);
+    const double rho = block_radius(sys->H, size, rs->bi, rs->bj, rs->bk) + 1e-9;
     int idx = 0;
     for (int I = 0; I < rs->n_ri; ++I)
         for (int J = 0; J < rs->n_rj; ++J)
@@ -419,12 +492,25 @@ int get_field_regions(System *sys, int size, int cb, double r_split, RegionSet *
                 r.ni = std::min(rs->bi, size - r.i0);
                 r.nj = std::min(rs->bj, size - r.j0);
                 r.nk = std::min(rs->bk, size - r.k0);
-                // origin = mean of the block's centers ((i + .5)/S ...)
-                r.of[0] = (r.i0 + 0.5 * r.ni) / size;
-                r.of[1] = (r.j0 + 0.5 * r.nj) / size;
-                r.of[2] = (r.k0 + 0.5 * r.nk) / size;
-                r.rho = block_radius(sys->H, size, r.ni, r.nj, r.nk) + 1e-9;
+                // origin = mean of a whole block's centers ((i + .5)/S ...), also
+                // where the grid's edge cuts the block: the centers sit at the
+                // same places relative to it in every region
+                r.of[0] = (r.i0 + 0.5 * rs->bi) / size;
+                r.of[1] = (r.j0 + 0.5 * rs->bj) / size;
+                r.of[2] = (r.k0 + 0.5 * rs->bk) / size;
+                r.rho = rho;
             }
+    if (r_split < 1e29) {
+        rs->taylor_radius = sys->max_offset + rho;
+        const double start = std::max(taylor_start(*sys, rs->taylor_radius),
+                                      r_split + rs->taylor_radius);
+        const double inner = sys->cutoff - rs->taylor_radius;
+        const double volume = 1.0 / std::fabs(det3(sys->Hinv));
+        // too few entries for an expansion to pay (taylor_worthwhile): unsorted
+        if (start < inner && 4.18879 * (inner * inner * inner - start * start * start) *
+                                     sys->n_atoms / volume >= kTaylorMinEntries)
+            rs->d_taylor = start;
+    }
     int rc = build_lists(sys, rs, stream);
     if (rc) {
         delete rs;
@@ -442,7 +528,8 @@ int get_bin_regions(System *sys, double r_split, RegionSet **out, cudaStream_t s
     for (RegionSet *rs : sys->sets)
         if (rs->size == 0 && rs->r_split == r_split && rs->bin_width == bin_width) {
             if (rs->stale) {
-                for (auto &r : rs->h_info) r.n_near = r.n_total = r.n_inner = r.n_outer = 0;
+                for (auto &r : rs->h_info)
+                    r.n_near = r.n_total = r.n_inner = r.n_outer = r.n_mid = r.n_shella = 0;
                 VEXT_TRY(build_lists(sys, rs, stream));
             }
             *out = rs;
@@ -522,6 +609,8 @@ System::~System() {
     drop_adjoint_batch();   // it points into the region sets
     for (RegionSet *rs : sets) delete rs;
     cudaFree(d_g32);
+    field_plan.release();
+    cudaFree(d_sums);
     cudaFree(d_frac);
     cudaFree(d_type);
     cudaFree(d_tf);
