@@ -762,6 +762,9 @@ struct vext_batch_s {
     std::vector<Target> targets;          // current outputs of each system
     std::vector<TaylorPlan> plans;        // local expansions (poly null: none)
     std::vector<const RegionSet *> lists; // each system's region lists
+    std::vector<int> slab_items, slab_plane;   // first item and first grid plane of each slab,
+                                               // then the ends (see batch_run_slab)
+    int *d_slab_counts = nullptr;              // refinement records of each slab
     float *d_sums = nullptr;              // expansion sums of one system at a time
     size_t sums_cap = 0;
     int4 *d_items = nullptr, *d_sample = nullptr;
@@ -793,6 +796,7 @@ struct vext_batch_s {
         cudaFree(d_axes);
         cudaFree(d_status);
         cudaFree(d_sums);
+        cudaFree(d_slab_counts);
         for (TaylorPlan &p : plans) p.release();
         if (stream) cudaStreamDestroy(stream);
     }
@@ -883,11 +887,12 @@ static bool device_memory(const void *p) {
 // one-system batch of vext_field_adjoint_device (which already holds its
 // system's lock: lock_systems = false, and says with `rule_axes` how many
 // directors the whole call has and with `init` where expansion values may
-// stand when the outputs are host memory).
+// stand when the outputs are host memory; slabs > 1 orders the queue of a
+// one-system batch for batch_run_slab).
 int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
                 const double *axes, const vext_options *opt, float *const *outputs,
                 float *const *gradients, double *const *outputs_f64, bool lock_systems,
-                vext_batch *out, int rule_axes, float *const *init) {
+                vext_batch *out, int rule_axes, float *const *init, int slabs) {
     if (!out || n_systems < 1 || !systems || !outputs || size < 1 || n_axes < 1 || !axes)
         return fail(VEXT_ERR_ARGUMENT, "bad batch arguments");
     for (int k = 0; k < n_systems; ++k)
@@ -1012,6 +1017,24 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
     std::vector<int4> hitems(items.size());
     for (const auto &it : items) hitems[(size_t)start[(size_t)(max_len - it.first)]++] = it.second;
     b->n_items = (int)hitems.size();
+    if (slabs > 1) {
+        // slab by slab (region planes along the slowest axis), longest first in each
+        const RegionSet &rs = *lists[owner[0]];
+        const int per = rs.n_rj * rs.n_rk;
+        auto slab_of = [&](const int4 &it) { return (int)((long long)(it.y / per) * slabs / rs.n_ri); };
+        std::stable_sort(hitems.begin(), hitems.end(),
+                         [&](const int4 &x, const int4 &y) { return slab_of(x) < slab_of(y); });
+        b->slab_items.assign(slabs + 1, 0);
+        b->slab_plane.assign(slabs + 1, 0);
+        for (const int4 &it : hitems) ++b->slab_items[slab_of(it) + 1];
+        for (int k = 0; k < slabs; ++k) {
+            b->slab_items[k + 1] += b->slab_items[k];
+            // first region plane I with I * slabs / n_ri > k
+            const int end = (int)(((long long)(k + 1) * rs.n_ri + slabs - 1) / slabs);
+            b->slab_plane[k + 1] = std::min(size, end * rs.bi);
+        }
+        VEXT_CUDA(cudaMalloc(&b->d_slab_counts, sizeof(int) * slabs));
+    }
     // the tuning sample: a strided subset of the queue (so it keeps the mix of
     // long and short items), every 128th item for large queues but at least
     // 16 items per SM, so that the persistent CTAs stay busy while it is
@@ -1175,7 +1198,7 @@ extern "C" int vext_batch_create(int n_systems, const vext_system *systems, int 
                                  int n_axes, const double *axes, const vext_options *opt,
                                  float *const *outputs, vext_batch *out) {
     return batch_build(n_systems, systems, size, n_axes, axes, opt, outputs, nullptr, nullptr,
-                       true, out, 0, nullptr);
+                       true, out, 0, nullptr, 1);
 }
 
 extern "C" int vext_batch_create_adjoint(int n_systems, const vext_system *systems, int size,
@@ -1184,7 +1207,7 @@ extern "C" int vext_batch_create_adjoint(int n_systems, const vext_system *syste
                                          float *const *gradients, vext_batch *out) {
     if (!gradients) return fail(VEXT_ERR_ARGUMENT, "gradient outputs required");
     return batch_build(n_systems, systems, size, n_axes, axes, opt, energies, gradients, nullptr,
-                       true, out, 0, nullptr);
+                       true, out, 0, nullptr, 1);
 }
 
 namespace vext {
@@ -1193,6 +1216,31 @@ namespace vext {
 int batch_replay(vext_batch b, cudaStream_t stream) {
     VEXT_CUDA(cudaGraphLaunch(b->exec, stream));
     return 0;
+}
+
+// Run slab k (of a batch built with slabs > 1) on `stream`, slabs in order: the
+// poses of grid planes [*plane0, *plane1) along the slowest axis are final
+// once it is done, so a caller can copy them while the next slab runs.
+int batch_run_slab(vext_batch b, int k, cudaStream_t stream, int *plane0, int *plane1) {
+    const int first = b->slab_items[k], n = b->slab_items[k + 1] - first;
+    *plane0 = b->slab_plane[k];
+    *plane1 = b->slab_plane[k + 1];
+    VEXT_TRY(batch_launch(b, b->config, b->d_items + first, n, k == 0, stream));
+    VEXT_CUDA(cudaMemcpyAsync(b->d_slab_counts + k, b->d_refine, sizeof(int),
+                              cudaMemcpyDeviceToDevice, stream));
+    return 0;
+}
+
+// vext_batch_status over all slabs.
+int batch_slab_status(vext_batch b) {
+    std::vector<int> counts(b->slab_items.size() - 1);
+    VEXT_CUDA(cudaMemcpy(counts.data(), b->d_slab_counts, sizeof(int) * counts.size(),
+                         cudaMemcpyDeviceToHost));
+    for (int c : counts)
+        if (c > b->refine_cap)
+            return fail(VEXT_ERR_CAPACITY, "%d poses in the refinement band; %d refined", c,
+                        b->refine_cap);
+    return vext_batch_status(b);
 }
 
 // Point system k's float32 energy / gradient outputs at `out` / `grad` (and

@@ -891,7 +891,7 @@ static int field_adjoint_device(vext_system h, int size, int n_axes, const doubl
             sys->adj_batch = nullptr;
             vext_batch b = nullptr;
             VEXT_TRY(batch_build(1, &h, size, n_axes, axes, opt, &energy, &gradient,
-                                 energy_f64 ? &energy_f64 : nullptr, false, &b, n_axes, init));
+                                 energy_f64 ? &energy_f64 : nullptr, false, &b, n_axes, init, 1));
             sys->adj_batch = b;
             sys->adj_size = size;
             sys->adj_axes.assign(axes, axes + 3 * n_axes);
@@ -974,6 +974,75 @@ static void *mapped_host_range(void *p, size_t bytes) {
     return first.devicePointer;
 }
 
+// Page-locked outputs of vext_field_adjoint (mixed mode; d_f32 and d_g32 hold
+// the results on the device).  Slabs of 24 MB and more: below that the copy
+// of a slab is short of the bus rate, and eight hide all but the last one.
+static int adjoint_pinned(vext_system h, int size, int n_axes, const double *axes,
+                          const Options &o, const vext_options *opt, float *energy,
+                          float *gradient, cudaStream_t st) {
+    System *sys = &h->sys;
+    const size_t S3 = (size_t)size * size * size, n = S3 * n_axes;
+    const int slabs =
+        (int)std::max<size_t>(1, std::min<size_t>({8, (size_t)size / 4, 28 * n / (24u << 20)}));
+    if (slabs == 1) {
+        VEXT_TRY(field_adjoint_device(h, size, n_axes, axes, o, opt, sys->d_f32, sys->d_g32,
+                                      nullptr, nullptr, st));
+        VEXT_CUDA(cudaMemcpyAsync(energy, sys->d_f32, sizeof(float) * n, cudaMemcpyDeviceToHost,
+                                  st));
+        VEXT_CUDA(cudaMemcpyAsync(gradient, sys->d_g32, sizeof(float) * 6 * n,
+                                  cudaMemcpyDeviceToHost, st));
+        VEXT_CUDA(cudaStreamSynchronize(st));
+        return vext_batch_status(sys->adj_batch);
+    }
+    for (int k = 0; k < 3 * n_axes; ++k)
+        if (!std::isfinite(axes[k])) return fail(VEXT_ERR_ARGUMENT, "non-finite director");
+    const double key[4] = {o.r_split, o.band_lo, o.band_hi, batch_key(o)};
+    const bool same = sys->slab_batch && sys->slab_size == size && sys->slab_count == slabs &&
+                      sys->slab_axes.size() == 3 * (size_t)n_axes &&
+                      std::equal(axes, axes + 3 * n_axes, sys->slab_axes.begin()) &&
+                      std::equal(key, key + 4, sys->slab_key);
+    if (!same) {
+        if (sys->slab_batch) vext_batch_destroy(sys->slab_batch);
+        sys->slab_batch = nullptr;
+        VEXT_TRY(batch_build(1, &h, size, n_axes, axes, opt, &sys->d_f32, &sys->d_g32, nullptr,
+                             false, &sys->slab_batch, n_axes, nullptr, slabs));
+        sys->slab_size = size;
+        sys->slab_count = slabs;
+        sys->slab_axes.assign(axes, axes + 3 * n_axes);
+        std::copy(key, key + 4, sys->slab_key);
+    }
+    VEXT_TRY(batch_retarget(sys->slab_batch, 0, sys->d_f32, sys->d_g32, sys->d_f32, sys->d_g32,
+                            st));
+    // a slab of the [directors][S][S][S] arrays: one row of consecutive planes
+    // per director
+    auto copy_rows = [&](float *to, const float *from, size_t words, int p0, int p1) {
+        const size_t plane = sizeof(float) * words * size * size, off = plane * p0;
+        return cudaMemcpy2DAsync(reinterpret_cast<char *>(to) + off, plane * size,
+                                 reinterpret_cast<const char *>(from) + off, plane * size,
+                                 plane * (p1 - p0), n_axes, cudaMemcpyDeviceToHost, sys->aux);
+    };
+    auto run = [&]() -> int {
+        for (int k = 0; k < slabs; ++k) {
+            int p0 = 0, p1 = 0;
+            VEXT_TRY(batch_run_slab(sys->slab_batch, k, st, &p0, &p1));
+            VEXT_CUDA(cudaEventRecord(sys->ev[5], st));
+            VEXT_CUDA(cudaStreamWaitEvent(sys->aux, sys->ev[5], 0));
+            if (p1 <= p0) continue;
+            VEXT_CUDA(copy_rows(energy, sys->d_f32, 1, p0, p1));
+            VEXT_CUDA(copy_rows(gradient, sys->d_g32, 6, p0, p1));
+        }
+        return 0;
+    };
+    const int rc = run();
+    // both streams end before the call does, also on an error
+    const cudaError_t e0 = cudaStreamSynchronize(sys->aux), e1 = cudaStreamSynchronize(st);
+    sys->split_timed = false;   // ev[5] was used here
+    VEXT_TRY(rc);
+    VEXT_CUDA(e0);
+    VEXT_CUDA(e1);
+    return batch_slab_status(sys->slab_batch);
+}
+
 extern "C" int vext_field_adjoint(vext_system h, int size, int n_axes, const double *axes,
                                   const vext_options *opt, float *energy, float *gradient) {
     if (!h) return fail(VEXT_ERR_ARGUMENT, "null system");
@@ -988,18 +1057,13 @@ extern "C" int vext_field_adjoint(vext_system h, int size, int n_axes, const dou
     VEXT_TRY(ensure_capacity(sys->d_g32, sys->g32_cap, 6 * n));
     cudaStream_t st = sys->stream;
     if (o.mode == VEXT_MODE_MIXED) {
-        // page-locked host outputs: one batch over all directors writes the
-        // float32 results straight into them (the transfer runs beside the
-        // pair work)
-        float *de = static_cast<float *>(mapped_host_range(energy, sizeof(float) * n));
-        float *dg = de ? static_cast<float *>(mapped_host_range(gradient, sizeof(float) * 6 * n))
-                       : nullptr;
-        if (de && dg) {
-            VEXT_TRY(field_adjoint_device(h, size, n_axes, axes, o, opt, de, dg, nullptr, nullptr,
-                                          st));
-            VEXT_CUDA(cudaStreamSynchronize(st));
-            return vext_batch_status(sys->adj_batch);
-        }
+        // page-locked host outputs: results in device memory, copied out by
+        // slabs of grid planes, a slab while the next one computes.  (Kernels
+        // storing straight into host memory kept up only behind much more pair
+        // work: their 8- and 24-byte segments crossed PCIe at about 6 GB/s.)
+        const bool mapped = mapped_host_range(energy, sizeof(float) * n) &&
+                            mapped_host_range(gradient, sizeof(float) * 6 * n);
+        if (mapped) return adjoint_pinned(h, size, n_axes, axes, o, opt, energy, gradient, st);
     }
     if (o.mode == VEXT_MODE_MIXED) {
         // pageable host outputs: one batch per block of the batch's work-item
@@ -1024,7 +1088,7 @@ extern "C" int vext_field_adjoint(vext_system h, int size, int n_axes, const dou
                 float *gk = sys->d_g32 + 6 * blk * (size_t)k * S3;
                 vext_batch b = nullptr;
                 VEXT_TRY(batch_build(1, &h, size, nk, axes + 3 * blk * k, opt, &ek, &gk, nullptr,
-                                     false, &b, n_axes, nullptr));
+                                     false, &b, n_axes, nullptr, 1));
                 sys->host_parts.push_back(b);
                 cudaEvent_t ev;
                 VEXT_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));

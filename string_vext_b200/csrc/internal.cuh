@@ -176,6 +176,12 @@ struct System {
     std::vector<double> host_axes;
     double host_key[4] = {0, 0, 0, 0};
     float *host_e = nullptr, *host_g = nullptr;
+    // the same entry into page-locked buffers: one batch over all directors,
+    // its poses slab by slab along the slowest grid axis (batch_run_slab)
+    vext_batch slab_batch = nullptr;
+    int slab_size = 0, slab_count = 0;
+    std::vector<double> slab_axes;
+    double slab_key[4] = {0, 0, 0, 0};
     std::mutex lock;
     void drop_adjoint_batch();   // both caches (they point into the region sets)
     void drop_host_parts();
@@ -186,8 +192,10 @@ struct System {
 int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
                 const double *axes, const vext_options *opt, float *const *outputs,
                 float *const *gradients, double *const *outputs_f64, bool lock_systems,
-                vext_batch *out, int rule_axes, float *const *init);
+                vext_batch *out, int rule_axes, float *const *init, int slabs);
 int batch_replay(vext_batch b, cudaStream_t stream);
+int batch_run_slab(vext_batch b, int k, cudaStream_t stream, int *plane0, int *plane1);
+int batch_slab_status(vext_batch b);
 int batch_retarget(vext_batch b, int k, float *out, float *grad, float *init, float *init_grad,
                    cudaStream_t stream);
 

@@ -593,6 +593,9 @@ void System::drop_adjoint_batch() {
     adj_batch = nullptr;
     adj_size = 0;
     adj_axes.clear();
+    if (slab_batch) vext_batch_destroy(slab_batch);
+    slab_batch = nullptr;
+    slab_axes.clear();
     drop_host_parts();
 }
 

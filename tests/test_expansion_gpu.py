@@ -116,3 +116,22 @@ def test_batch_mixes_systems_with_and_without_expansions():
         batch.close()
     for s in systems:
         s.close()
+
+
+@pytest.mark.parametrize("size,n_axes", [(30, 96), (33, 70)])
+def test_page_locked_outputs_by_slabs(size, n_axes):
+    """Outputs of 50 MB and more leave by slabs of grid planes while the next
+    slab computes (33 planes in four slabs, the last block of them partial):
+    the same bits as the device entry, twice, also into a second buffer."""
+    axes = directors(n_axes)
+    shape = (n_axes,) + (size,) * 3
+    with VextSystem(synth.small_field()) as system:
+        e = torch.empty(shape, dtype=torch.float32, device="cuda")
+        g = torch.empty(shape + (6,), dtype=torch.float32, device="cuda")
+        system.field_adjoint_device(size, axes, e, g)
+        torch.cuda.synchronize()
+        kept = []
+        for _ in range(2):
+            kept.append(system.field_adjoint(size, axes, pinned=True))
+            np.testing.assert_array_equal(kept[-1][0], e.cpu().numpy())
+            np.testing.assert_array_equal(kept[-1][1], g.cpu().numpy())
