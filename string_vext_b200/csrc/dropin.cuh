@@ -7,6 +7,7 @@
 namespace vext {
 
 constexpr int kCsrChunk = 256;   // neighbours staged per shared-memory chunk
+constexpr int kCsrAxes = 32, kCsrLanes = 4;   // directors per CTA, lanes per director
 
 // Per-image record on the device: x, y, z, c12, c6, shift, floor2, pad.
 struct CsrArgs {
@@ -21,7 +22,7 @@ struct CsrArgs {
     double *out;             // [n][n_axes]
 };
 
-// One CTA per center; defined in dropin.cu.
-__global__ void csr_kernel(CsrArgs a);
+// Launch the pair kernel (dropin.cu).
+int csr_launch(const CsrArgs &a, cudaStream_t stream);
 
 }  // namespace vext

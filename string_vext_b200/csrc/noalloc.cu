@@ -201,9 +201,7 @@ extern "C" int evaluate_reused_neighbors_noalloc(int n_centers, int n_axes, int 
     a.starts = d_start;
     a.indices = d_idx;
     a.out = d_out;
-    const int threads = n_axes >= 128 ? 128 : ((n_axes + 31) / 32) * 32;
-    csr_kernel<<<n_eval, threads, 0, st>>>(a);
-    VEXT_CUDA(cudaGetLastError());
+    VEXT_TRY(csr_launch(a, st));
     const unsigned long long none = (unsigned long long)n_out;
     VEXT_CUDA(cudaMemcpyAsync(d_first, &none, sizeof none, cudaMemcpyHostToDevice, st));
     noalloc_first_nonfinite_kernel<<<148, 256, 0, st>>>(d_out, (long long)n_out, d_first);
