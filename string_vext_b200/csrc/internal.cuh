@@ -273,6 +273,12 @@ int pose_warp_enqueue(System *sys, const RegionSet *rs, int n, const double *cen
                       const double *quats, const Options &o, double *energy, double *gc,
                       double *gq, double *gu, cudaStream_t st);
 
+// One system's view of its bin lists for the pose kernels.
+PoseBatchSys pose_describe(const System *sys, const RegionSet *rs);
+int warps_per_pose(long long n);
+// Its device copy, uploaded when it changed.
+int pose_upload_desc(System *sys, const RegionSet *rs, const PoseBatchSys **out);
+
 // Field kernel launcher (field.cu): computes E64 [O][S^3] for all regions.
 int launch_field(System *sys, const RegionSet *rs, int n_axes, const double *axes_host,
                  const double *d_axes, double *d_e64, int cb, int variant, cudaStream_t stream);

@@ -32,14 +32,18 @@
 //      (legacy_policy.h:9-12, RC_main.cu:1853-1854); on convergence the loop
 //      stops before the copy;
 //   8. s0 = (s2 positions, smoothed angles wrapped into [0, 2 pi]) (copy2s0).
-// Steps 2-8 run in two single-CTA kernels (one thread per image); the two
-// pose evaluations are the only heavy work.  One iteration is captured in a
-// CUDA graph and replayed; the host reads the stop flag only at check
-// iterations.
+// Paths of up to kLoopImages images run many iterations in one cooperative
+// launch (string_loop_kernel): a CTA evaluates one image, and between two grid
+// barriers every CTA does steps 2-8 for the whole path itself.  Longer paths
+// and the reference differences run steps 2-8 in two single-CTA kernels (one
+// thread per image) around the pose kernels, one iteration captured in a CUDA
+// graph and replayed.  The host reads the stop flag only at check iterations
+// (the graphs) or between launches.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
-#include "internal.cuh"
+#include "poseeval.cuh"
 
 namespace vext {
 
@@ -100,6 +104,97 @@ __global__ void string_fd_pose_kernel(StringArgs a) {
     }
 }
 
+// The steps of one image, shared by the kernels below.
+
+// g_k = h_k dE/dx_k from dE/dcenter and dE/ddirector.
+__device__ __forceinline__ void string_gradient(const StringArgs &a, const double *s,
+                                                const double *gc, const double *gu, double *g) {
+    // dE/dfrac_k = sum_j H[k][j] dE/dcart_j
+    for (int k = 0; k < 3; ++k)
+        g[k] = a.hf * (a.H.m[3 * k] * gc[0] + a.H.m[3 * k + 1] * gc[1] +
+                       a.H.m[3 * k + 2] * gc[2]);
+    // director u = (cg cb, sg cb, -sb); dE/dalpha = 0 for a linear guest
+    const double cb = cos(s[4]), sb = sin(s[4]), cg = cos(s[5]), sg = sin(s[5]);
+    g[3] = 0.0;
+    g[4] = a.ha * (gu[0] * (-cg * sb) + gu[1] * (-sg * sb) + gu[2] * (-cb));
+    g[5] = a.ha * (gu[0] * (-sg * cb) + gu[1] * (cg * cb));
+}
+
+// The normalised step from s along -g.
+__device__ __forceinline__ void string_move(const StringArgs &a, const double *s, double *g,
+                                            double *o) {
+    for (int k = 0; k < 6; ++k) g[k] = trunc_r(g[k], a.rounding);
+    const double lt = trunc_r(sqrt(g[0] * g[0] + g[1] * g[1] + g[2] * g[2]), a.rounding);
+    const double lr = trunc_r(sqrt(g[3] * g[3] + g[4] * g[4] + g[5] * g[5]), a.rounding);
+    for (int k = 0; k < 3; ++k)
+        o[k] = lt < a.hf ? s[k] - a.hf * g[k] : s[k] - a.hf * trunc_r(g[k] / lt, a.rounding);
+    for (int k = 3; k < 6; ++k)
+        o[k] = lr < a.ha ? s[k] - a.ha * g[k] : s[k] - a.ha * trunc_r(g[k] / lr, a.rounding);
+}
+
+// End fixing of image i: image 0 keeps its axis coordinate; the last image
+// keeps its axis coordinate and takes the other five from image 0; an interior
+// image outside [0, 1] along the axis copies the nearest image inside.  moved
+// [n][6] and its axis coordinates ax[stride k]: the values before fixing.
+__device__ __forceinline__ void string_fix(const StringArgs &a, int i, const double *s0,
+                                           const double *moved, int stride, const double *ax,
+                                           double *o) {
+    const int n = a.n, d = a.axis;
+    for (int k = 0; k < 6; ++k) o[k] = moved[6 * i + k];
+    if (i == 0) {
+        o[d] = s0[d];
+    } else if (i == n - 1) {
+        for (int k = 0; k < 6; ++k) o[k] = k == d ? s0[6 * (n - 1) + d] : moved[k];
+    } else {
+        const double v = ax[stride * i];
+        int src = -1;
+        if (v < 0) {
+            for (int ii = i + 1; ii < n; ++ii)
+                if (ax[stride * ii] > 0) {
+                    src = ii;
+                    break;
+                }
+        } else if (v > 1) {
+            for (int ii = i - 1; ii >= 0; --ii)
+                if (ax[stride * ii] < 1) {
+                    src = ii;
+                    break;
+                }
+        }
+        if (src >= 0)
+            for (int k = 0; k < 6; ++k) o[k] = moved[6 * src + k];
+    }
+}
+
+// Segment lengths cum[1..n-1] -> running sums in image order (cum[0] = 0).
+__device__ __forceinline__ void running_sum(double *cum, int n) {
+    double c = 0;
+    cum[0] = 0;
+    for (int k = 1; k < n; ++k) {
+        c += cum[k];
+        cum[k] = c;
+    }
+}
+
+// Position of image i at equal arc lengths along the images `from` [n][6].
+__device__ __forceinline__ void string_reparametrise(int i, int n, const double *cum,
+                                                     const double *from, double *out) {
+    const double L = cum[n - 1];
+    const double t = (double)i / (n - 1);
+    // segment ii with cum[ii]/L <= t <= cum[ii+1]/L (binary search)
+    int lo = 0, hi = n - 2;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (cum[mid] / L <= t) lo = mid;
+        else hi = mid - 1;
+    }
+    const int ii = lo;
+    const double l0 = cum[ii] / L, l1 = cum[ii + 1] / L;
+    const double *p0 = from + 6 * ii, *p1 = from + 6 * (ii + 1);
+    for (int k = 0; k < 3; ++k)
+        out[k] = l1 > l0 ? p0[k] + (t - l0) * ((p1[k] - p0[k]) / (l1 - l0)) : p0[k];
+}
+
 // Steps 2-4 (and the pose of s2).  One CTA, thread i = image i (n <= 1024 =
 // blockDim): the step in registers, end fixing and segment lengths through
 // shared memory, the running sum of the lengths by one thread in image order.
@@ -107,7 +202,6 @@ __global__ void __launch_bounds__(1024) string_step_kernel(StringArgs a) {
     __shared__ double ax[1024];       // axis coordinate of every stepped image (before fixing)
     __shared__ double cum[1024];      // segment lengths, then their running sums
     __shared__ double cart[3][1024];  // Cartesian positions of the fixed images
-    __shared__ double pre0[6];        // image 0 before fixing
     if (a.flags[0]) return;   // converged earlier (uniform over the CTA)
     const int n = a.n, d = a.axis, i = threadIdx.x;
     double o[6];
@@ -120,59 +214,16 @@ __global__ void __launch_bounds__(1024) string_step_kernel(StringArgs a) {
             for (int k = 0; k < 6; ++k) g[k] = e7[k + 1] - e7[0];
             a.e0[i] = e7[0];
         } else {
-            // dE/dfrac_k = sum_j H[k][j] dE/dcart_j
-            for (int k = 0; k < 3; ++k)
-                g[k] = a.hf * (a.H.m[3 * k] * a.gc[3 * i] + a.H.m[3 * k + 1] * a.gc[3 * i + 1] +
-                               a.H.m[3 * k + 2] * a.gc[3 * i + 2]);
-            // director u = (cg cb, sg cb, -sb); dE/dalpha = 0 for a linear guest
-            const double cb = cos(s[4]), sb = sin(s[4]), cg = cos(s[5]), sg = sin(s[5]);
-            const double *gu = a.gu + 3 * i;
-            g[3] = 0.0;
-            g[4] = a.ha * (gu[0] * (-cg * sb) + gu[1] * (-sg * sb) + gu[2] * (-cb));
-            g[5] = a.ha * (gu[0] * (-sg * cb) + gu[1] * (cg * cb));
+            string_gradient(a, s, a.gc + 3 * i, a.gu + 3 * i, g);
         }
-        for (int k = 0; k < 6; ++k) g[k] = trunc_r(g[k], a.rounding);
-        const double lt = trunc_r(sqrt(g[0] * g[0] + g[1] * g[1] + g[2] * g[2]), a.rounding);
-        const double lr = trunc_r(sqrt(g[3] * g[3] + g[4] * g[4] + g[5] * g[5]), a.rounding);
-        for (int k = 0; k < 3; ++k)
-            o[k] = lt < a.hf ? s[k] - a.hf * g[k] : s[k] - a.hf * trunc_r(g[k] / lt, a.rounding);
-        for (int k = 3; k < 6; ++k)
-            o[k] = lr < a.ha ? s[k] - a.ha * g[k] : s[k] - a.ha * trunc_r(g[k] / lr, a.rounding);
+        string_move(a, s, g, o);
         // the values before fixing (s2), read by the images that copy them
         for (int k = 0; k < 6; ++k) a.s2[6 * i + k] = o[k];
         ax[i] = o[d];
-        if (i == 0)
-            for (int k = 0; k < 6; ++k) pre0[k] = o[k];
     }
     __syncthreads();
     if (i < n) {
-        // end fixing: image 0 keeps its axis coordinate; the last image keeps
-        // its axis coordinate and takes the other five from image 0; an
-        // interior image outside [0, 1] along the axis copies the nearest
-        // image inside (values before fixing)
-        if (i == 0) {
-            o[d] = a.s0[d];
-        } else if (i == n - 1) {
-            for (int k = 0; k < 6; ++k) o[k] = k == d ? a.s0[6 * (n - 1) + d] : pre0[k];
-        } else {
-            const double v = ax[i];
-            int src = -1;
-            if (v < 0) {
-                for (int ii = i + 1; ii < n; ++ii)
-                    if (ax[ii] > 0) {
-                        src = ii;
-                        break;
-                    }
-            } else if (v > 1) {
-                for (int ii = i - 1; ii >= 0; --ii)
-                    if (ax[ii] < 1) {
-                        src = ii;
-                        break;
-                    }
-            }
-            if (src >= 0)
-                for (int k = 0; k < 6; ++k) o[k] = a.s2[6 * src + k];
-        }
+        string_fix(a, i, a.s0, a.s2, 1, ax, o);
         for (int k = 0; k < 6; ++k) a.s1[6 * i + k] = o[k];
         frac_to_cart(a.H, o[0], o[1], o[2], cart[0][i], cart[1][i], cart[2][i]);
     }
@@ -183,31 +234,11 @@ __global__ void __launch_bounds__(1024) string_step_kernel(StringArgs a) {
         cum[i] = sqrt(dx * dx + dy * dy + dz * dz);
     }
     __syncthreads();
-    if (i == 0) {   // running sum in image order
-        double c = 0;
-        cum[0] = 0;
-        for (int k = 1; k < n; ++k) {
-            c += cum[k];
-            cum[k] = c;
-        }
-    }
+    if (i == 0) running_sum(cum, n);
     __syncthreads();
     if (i < n) {   // (s2 is read above only, three barriers back: rewrite it now)
-        const double L = cum[n - 1];
-        const double t = (double)i / (n - 1);
-        // segment ii with cum[ii]/L <= t <= cum[ii+1]/L (binary search)
-        int lo = 0, hi = n - 2;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) / 2;
-            if (cum[mid] / L <= t) lo = mid;
-            else hi = mid - 1;
-        }
-        const int ii = lo;
-        const double l0 = cum[ii] / L, l1 = cum[ii + 1] / L;
         double *out = a.s2 + 6 * i;
-        const double *p0 = a.s1 + 6 * ii, *p1 = a.s1 + 6 * (ii + 1);
-        for (int k = 0; k < 3; ++k)
-            out[k] = l1 > l0 ? p0[k] + (t - l0) * ((p1[k] - p0[k]) / (l1 - l0)) : p0[k];
+        string_reparametrise(i, n, cum, a.s1, out);
         for (int k = 3; k < 6; ++k) out[k] = o[k];
         pose_of(a, out, a.centers2 + 3 * i, a.quats2 + 4 * i);
     }
@@ -221,6 +252,18 @@ __device__ __forceinline__ double smooth_one(double prev, double cur, double nex
     else if (dn > kPi) wrap = -1 * 2 * kPi;
     else if (dn < -kPi) wrap = 1 * 2 * kPi;
     return (1 - k) * cur + 0.5 * k * (prev + next + wrap);
+}
+
+// Angle k of the smoothed path at image i, wrapped into [0, 2 pi].
+__device__ __forceinline__ double string_smooth(const StringArgs &a, int i, int n,
+                                                const double *s2, int k) {
+    double v = (i == 0 || i == n - 1)
+                   ? s2[6 * i + k]
+                   : smooth_one(s2[6 * (i - 1) + k], s2[6 * i + k], s2[6 * (i + 1) + k],
+                                a.smooth);
+    if (v > 2 * kPi) v -= 2 * kPi;
+    else if (v < 0) v += 2 * kPi;
+    return v;
 }
 
 // Steps 5-8.  One CTA.  check != 0 on convergence-test iterations.
@@ -265,15 +308,7 @@ __global__ void string_finish_kernel(StringArgs a, int check) {
         double *s0 = a.s1 + 6 * i;   // s1 is free now: build the new path there
         const double *s2 = a.s2 + 6 * i;
         for (int k = 0; k < 3; ++k) s0[k] = s2[k];
-        for (int k = 3; k < 6; ++k) {
-            double v = (i == 0 || i == n - 1)
-                           ? s2[k]
-                           : smooth_one(a.s2[6 * (i - 1) + k], s2[k], a.s2[6 * (i + 1) + k],
-                                        a.smooth);
-            if (v > 2 * kPi) v -= 2 * kPi;
-            else if (v < 0) v += 2 * kPi;
-            s0[k] = v;
-        }
+        for (int k = 3; k < 6; ++k) s0[k] = string_smooth(a, i, n, a.s2, k);
     }
     __syncthreads();
     for (int k = threadIdx.x; k < 6 * n; k += blockDim.x) a.s0[k] = a.s1[k];
@@ -282,9 +317,234 @@ __global__ void string_finish_kernel(StringArgs a, int check) {
         pose_of(a, a.s0 + 6 * i, a.centers + 3 * i, a.quats + 4 * i);
 }
 
+// ---------------------------------------------------------------- path loop
+
+// Images a CTA each of which fits the GPU at once with eight warps per pose
+// (warps_per_pose gives eight up to 296 poses, and the sums' order is the pose
+// kernel's).
+constexpr int kLoopImages = 296;
+constexpr int kLoopIterations = 500;   // per launch: about 6 ms for a 64-image path
+
+// All CTAs of a cooperative launch: false when a wait gave up.
+__device__ __forceinline__ bool grid_barrier(unsigned *counter, unsigned target, int *status) {
+    __syncthreads();
+    bool ok = true;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(counter, 1u);
+        ok = false;
+        for (uint32_t it = 0; it < kWaitLimit; ++it) {
+            unsigned now;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(counter) : "memory");
+            if (now >= target) {
+                ok = true;
+                break;
+            }
+            if ((it & 1023u) == 1023u && *(volatile int *)status == DEV_TIMEOUT) break;
+        }
+        if (!ok) atomicExch(status, DEV_TIMEOUT);
+    }
+    return __syncthreads_and(ok);
+}
+
+struct LoopArgs {
+    StringArgs s;
+    const PoseBatchSys *sys;
+    double band_lo, band_hi;
+    int first, last;          // iterations [first, last)
+    int check_every;
+    unsigned *barrier;        // zero at launch
+    int *status;
+};
+
+// Shared-memory doubles of string_loop_kernel for n images.
+static size_t loop_words(int n) { return 18 * (size_t)n + 5 * (size_t)n + 8; }
+
+// Iterations [first, last) of a path, CTA i = image i.  Bound by latency: the
+// four kernels of an iteration took 30 us for 64 images, most of it launches
+// and their drains; here two grid barriers separate the phases, and what one
+// CTA did alone every CTA does for itself.  Outputs: s0, totals, flags (as
+// the two-kernel iteration leaves them).
+template <bool MIXED>
+__global__ void __launch_bounds__(256, 2) string_loop_kernel(LoopArgs g) {
+    const StringArgs &a = g.s;
+    extern __shared__ double sm[];
+    __shared__ double part[8][7];
+    __shared__ double pose[7];    // this CTA's pose: center, quaternion
+    const int n = a.n, d = a.axis, me = blockIdx.x, tid = threadIdx.x;
+    const int warp = tid >> 5, lane = tid & 31;
+    double *s0 = sm, *s1 = s0 + 6 * n, *s2 = s1 + 6 * n;   // [n][6]
+    double *cum = s2 + 6 * n, *cart = cum + n, *e0 = cart + 3 * n;   // [n], [3][n], [n]
+    unsigned bar = 0;
+    for (int k = tid; k < 6 * n; k += 256) s0[k] = a.s0[k];
+    __syncthreads();
+    auto set_pose = [&](const double *s) {
+        if (tid == 0) pose_of(a, s + 6 * me, pose, pose + 3);
+        __syncthreads();
+    };
+    for (int it = g.first; it < g.last; ++it) {
+        const bool check = it % g.check_every == 0 && it >= g.check_every;
+        PosePoint pt;
+        double v[7];
+        // ---- energies and gradients of s0
+        set_pose(s0);
+        pose_eval<MIXED>(*g.sys, pose + 3, pose, 8, warp, lane, part, g.band_lo, g.band_hi,
+                         g.status, pt, v);
+        if (tid == 0) {
+            a.e0[me] = v[0];
+            for (int k = 0; k < 3; ++k) {
+                a.gc[3 * me + k] = v[1 + k] + v[4 + k];
+                a.gu[3 * me + k] = g.sys->off0 * v[1 + k] + g.sys->off1 * v[4 + k];
+            }
+        }
+        if (!grid_barrier(g.barrier, ++bar * gridDim.x, g.status)) return;
+        // ---- steps 2-4 (string_step_kernel) in every CTA
+        for (int i = tid; i < n; i += 256) {
+            const double *s = s0 + 6 * i;
+            double gr[6], gc[3], gu[3], o[6];
+            e0[i] = __ldcg(a.e0 + i);
+            for (int k = 0; k < 3; ++k) {
+                gc[k] = __ldcg(a.gc + 3 * i + k);
+                gu[k] = __ldcg(a.gu + 3 * i + k);
+            }
+            string_gradient(a, s, gc, gu, gr);
+            string_move(a, s, gr, o);
+            for (int k = 0; k < 6; ++k) s2[6 * i + k] = o[k];
+        }
+        __syncthreads();
+        for (int i = tid; i < n; i += 256) {
+            double o[6];
+            string_fix(a, i, s0, s2, 6, s2 + d, o);
+            for (int k = 0; k < 6; ++k) s1[6 * i + k] = o[k];
+            frac_to_cart(a.H, o[0], o[1], o[2], cart[i], cart[n + i], cart[2 * n + i]);
+        }
+        __syncthreads();
+        for (int i = tid; i < n; i += 256) {
+            if (i == 0) continue;
+            const double dx = cart[i] - cart[i - 1], dy = cart[n + i] - cart[n + i - 1],
+                         dz = cart[2 * n + i] - cart[2 * n + i - 1];
+            cum[i] = sqrt(dx * dx + dy * dy + dz * dz);
+        }
+        __syncthreads();
+        if (tid == 0) running_sum(cum, n);
+        __syncthreads();
+        for (int i = tid; i < n; i += 256) {
+            string_reparametrise(i, n, cum, s1, s2 + 6 * i);
+            for (int k = 3; k < 6; ++k) s2[6 * i + k] = s1[6 * i + k];
+        }
+        __syncthreads();
+        // ---- energies of s2
+        set_pose(s2);
+        pose_eval<MIXED>(*g.sys, pose + 3, pose, 8, warp, lane, part, g.band_lo, g.band_hi,
+                         g.status, pt, v);
+        if (tid == 0) a.e2[me] = v[0];
+        if (!grid_barrier(g.barrier, ++bar * gridDim.x, g.status)) return;
+        // ---- steps 5-8 (string_finish_kernel) in every CTA
+        for (int i = tid; i < n; i += 256)
+            if (__ldcg(a.e2 + i) > e0[i])
+                for (int k = 3; k < 6; ++k) s2[6 * i + k] = s0[6 * i + k];
+        bool stop = false;
+        if (check || it + 1 == g.last) {   // movement: the test, and the launch's last totals
+            for (int i = tid; i < n; i += 256) {
+                double dt = 0, dr = 0;
+                for (int k = 0; k < 3; ++k)
+                    dt += (s0[6 * i + k] - s2[6 * i + k]) * (s0[6 * i + k] - s2[6 * i + k]);
+                for (int k = 3; k < 6; ++k)
+                    dr += (s0[6 * i + k] - s2[6 * i + k]) * (s0[6 * i + k] - s2[6 * i + k]);
+                cart[i] = sqrt(dt);
+                cart[n + i] = sqrt(dr);
+            }
+            __syncthreads();
+            double t = 0, r = 0;
+            for (int k = 0; k < n; ++k) {   // image order, every thread the same sums
+                t += cart[k];
+                r += cart[n + k];
+            }
+            const int ct = isfinite(t) && t >= 0 && a.conv_t > 0 && t < a.conv_t;
+            const int cr = isfinite(r) && r >= 0 && a.conv_r > 0 && r < a.conv_r;
+            stop = check && ct && cr;
+            if (me == 0 && tid == 0) {
+                a.totals[0] = t;
+                a.totals[1] = r;
+                a.flags[1] = ct;
+                a.flags[2] = cr;
+                if (stop) a.flags[0] = 1;
+            }
+        }
+        if (me == 0 && tid == 0 && !stop) a.flags[3] += 1;
+        __syncthreads();
+        if (stop) break;   // the same in every CTA
+        for (int i = tid; i < n; i += 256)
+            for (int k = 0; k < 6; ++k)
+                s1[6 * i + k] = k < 3 ? s2[6 * i + k] : string_smooth(a, i, n, s2, k);
+        __syncthreads();
+        for (int k = tid; k < 6 * n; k += 256) s0[k] = s1[k];
+        __syncthreads();
+    }
+    if (me == 0)
+        for (int k = tid; k < 6 * n; k += 256) a.s0[k] = s0[k];
+}
+
 }  // namespace vext
 
 using namespace vext;
+
+namespace vext {
+
+// Run the iterations of a path in string_loop_kernel launches.  *used = 0 (and
+// nothing has run) when the path or the device does not allow it; otherwise
+// *it is the number of iterations started and *stop whether a test converged
+// (counted as the graph loop counts them).
+static int string_loop(System *sys, StringArgs &a, const Options &o, const vext_string_params &p,
+                       cudaStream_t st, int *it, int *stop, int *used) {
+    *used = 0;
+    const bool mixed = o.mode == VEXT_MODE_MIXED;
+    RegionSet *rs = nullptr;
+    VEXT_TRY(get_bin_regions(sys, mixed ? o.r_split : 1e30, &rs, st));
+    // the conditions under which pose_enqueue takes eight warps per pose
+    if (a.n > kLoopImages || (long long)a.n >= 64LL * rs->n_regions || warps_per_pose(a.n) != 8)
+        return 0;
+    auto kernel = mixed ? string_loop_kernel<true> : string_loop_kernel<false>;
+    const size_t smem = sizeof(double) * loop_words(a.n);
+    int occ = 0, sms = 0, coop = 0;
+    VEXT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    VEXT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, 256, smem));
+    VEXT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, sys->device));
+    VEXT_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, sys->device));
+    if (!coop || (long long)occ * sms < a.n) return 0;
+    const PoseBatchSys *d_sys = nullptr;
+    VEXT_TRY(pose_upload_desc(sys, rs, &d_sys));
+    LoopArgs g;
+    g.s = a;
+    g.sys = d_sys;
+    const bool band = mixed && o.band_hi > o.band_lo;
+    g.band_lo = band ? o.band_lo : 0.0;
+    g.band_hi = band ? o.band_hi : 0.0;
+    g.check_every = p.check_every;
+    g.barrier = reinterpret_cast<unsigned *>(a.flags + 4);
+    g.status = sys->d_status;
+    *used = 1;
+    *stop = 0;
+    for (int done = 0; done < p.max_iterations && !*stop;) {
+        g.first = done;
+        g.last = std::min(p.max_iterations, done + kLoopIterations);
+        VEXT_CUDA(cudaMemsetAsync(g.barrier, 0, sizeof(unsigned), st));
+        void *args[] = {&g};
+        VEXT_CUDA(cudaLaunchCooperativeKernel((const void *)kernel, dim3(a.n), dim3(256), args, smem,
+                                              st));
+        done = g.last;
+        *it = done;
+        if (done < p.max_iterations) {   // converged in this launch?
+            int h[4] = {0, 0, 0, 0};
+            VEXT_CUDA(cudaMemcpyAsync(h, a.flags, sizeof h, cudaMemcpyDeviceToHost, st));
+            VEXT_CUDA(cudaStreamSynchronize(st));
+            *stop = h[0];
+        }
+    }
+    return 0;
+}
+
+}  // namespace vext
 
 extern "C" void vext_string_default_params(vext_string_params *p) {
     p->direction = 1;
@@ -391,15 +651,21 @@ extern "C" int vext_string_run(vext_system h, int n, double *path, double *energ
             VEXT_CUDA(cudaGetLastError());
             return 0;
         };
+        int it = 0, stop = 0;
+        const bool looped = !a.fd && p.max_iterations > 0;
+        if (looped) {
+            int used = 0;
+            VEXT_TRY(string_loop(sys, a, o, p, st, &it, &stop, &used));
+            if (!used) it = 0;
+        }
         // first iteration eagerly (builds lists and scratch), then graphs
-        int it = 0;
-        if (p.max_iterations > 0) {
+        if (it == 0 && p.max_iterations > 0) {
             VEXT_TRY(iteration(0));
             VEXT_TRY(pose_status(sys, st));
             it = 1;
         }
         cudaGraphExec_t plain = nullptr, checked = nullptr;
-        for (int variant = 0; variant < 2 && p.max_iterations > 1; ++variant) {
+        for (int variant = 0; variant < 2 && it < p.max_iterations && !stop; ++variant) {
             cudaGraph_t g = nullptr;
             VEXT_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
             const int irc = iteration(variant);
@@ -415,7 +681,6 @@ extern "C" int vext_string_run(vext_system h, int n, double *path, double *energ
             VEXT_CUDA(ie);
             (variant ? checked : plain) = ex;
         }
-        int stop = 0;
         for (; it < p.max_iterations && !stop; ++it) {
             const bool check = it % p.check_every == 0 && it >= p.check_every;
             VEXT_CUDA(cudaGraphLaunch(check ? checked : plain, st));
@@ -438,7 +703,8 @@ extern "C" int vext_string_run(vext_system h, int n, double *path, double *energ
         VEXT_CUDA(cudaMemcpyAsync(ht, a.totals, sizeof ht, cudaMemcpyDeviceToHost, st));
         VEXT_TRY(pose_status(sys, st));
         if (result) {
-            result->iterations = hf[0] ? it - 1 : it;
+            // a converged iteration is not counted (flags[3] holds the others)
+            result->iterations = hf[0] ? (looped ? hf[3] : it - 1) : it;
             result->converged = hf[1] && hf[2] && result->iterations >= p.check_every;
             result->converged_translation = hf[1];
             result->converged_rotation = hf[2];
