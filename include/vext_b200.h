@@ -203,6 +203,10 @@ VEXT_API int vext_field(vext_system sys, int size, int n_axes, const double *axe
                const vext_options *opt, float *orientation_K, double *energy_f64,
                float *marginal_K, float *site_K, float *grid, vext_field_stats *stats);
 
+/* Whether every value of the float32 outputs of the system's last vext_field
+ * call is finite (1) or not (0); looked at while they were copied out. */
+VEXT_API int vext_field_finite(vext_system sys, int *finite);
+
 /* Same, with DEVICE output pointers on the caller's stream (cudaStream_t
  * passed as void*; NULL = legacy default stream).  The call returns once the
  * work is enqueued and the region lists for (size, shape) exist. */

@@ -124,6 +124,8 @@ def load(path=None) -> ctypes.CDLL:
     lib.vext_field.argtypes = [vp, ci, ci, vp, ctypes.POINTER(Options), vp, vp, vp, vp, vp,
                                ctypes.POINTER(FieldStats)]
     lib.vext_field.restype = ci
+    lib.vext_field_finite.argtypes = [vp, ctypes.POINTER(ci)]
+    lib.vext_field_finite.restype = ci
     lib.vext_field_device.argtypes = [vp, ci, ci, vp, ctypes.POINTER(Options), vp, vp, vp, vp,
                                       vp, vp]
     lib.vext_field_device.restype = ci

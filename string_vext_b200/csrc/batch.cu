@@ -788,15 +788,15 @@ struct vext_batch_s {
     ~vext_batch_s() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
-        cudaFree(d_sys);
-        cudaFree(d_items);
-        cudaFree(d_sample);
-        cudaFree(d_counter);
-        cudaFree(d_refine);
-        cudaFree(d_axes);
-        cudaFree(d_status);
-        cudaFree(d_sums);
-        cudaFree(d_slab_counts);
+        device_free(d_sys);
+        device_free(d_items);
+        device_free(d_sample);
+        device_free(d_counter);
+        device_free(d_refine);
+        device_free(d_axes);
+        device_free(d_status);
+        device_free(d_sums);
+        device_free(d_slab_counts);
         for (TaylorPlan &p : plans) p.release();
         if (stream) cudaStreamDestroy(stream);
     }
@@ -917,7 +917,7 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
     int dev = 0;
     VEXT_CUDA(cudaGetDevice(&dev));
     VEXT_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
-    VEXT_CUDA(cudaMalloc(&b->d_axes, sizeof(double) * 3 * n_axes));
+    VEXT_CUDA(device_malloc(&b->d_axes, sizeof(double) * 3 * n_axes));
     VEXT_CUDA(cudaMemcpy(b->d_axes, axes, sizeof(double) * 3 * n_axes, cudaMemcpyHostToDevice));
     // regions of 16 centers x items of 32 directors, or 8 x 64 (kinds 6-9)
     const int kOB = batch_item_directors(b->opt, b->adj), cb = 512 / kOB;
@@ -1033,7 +1033,7 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
             const int end = (int)(((long long)(k + 1) * rs.n_ri + slabs - 1) / slabs);
             b->slab_plane[k + 1] = std::min(size, end * rs.bi);
         }
-        VEXT_CUDA(cudaMalloc(&b->d_slab_counts, sizeof(int) * slabs));
+        VEXT_CUDA(device_malloc(&b->d_slab_counts, sizeof(int) * slabs));
     }
     // the tuning sample: a strided subset of the queue (so it keeps the mix of
     // long and short items), every 128th item for large queues but at least
@@ -1080,20 +1080,20 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
         hs[k].poly = b->plans[k].poly;
     }
     for (const BatchSys &y : hs) b->targets.push_back({y.out, y.grad, y.init, y.init_grad});
-    VEXT_CUDA(cudaMalloc(&b->d_sys, sizeof(BatchSys) * n_systems));
+    VEXT_CUDA(device_malloc(&b->d_sys, sizeof(BatchSys) * n_systems));
     VEXT_CUDA(cudaMemcpy(b->d_sys, hs.data(), sizeof(BatchSys) * n_systems, cudaMemcpyHostToDevice));
-    VEXT_CUDA(cudaMalloc(&b->d_items, sizeof(int4) * hitems.size()));
+    VEXT_CUDA(device_malloc(&b->d_items, sizeof(int4) * hitems.size()));
     VEXT_CUDA(cudaMemcpy(b->d_items, hitems.data(), sizeof(int4) * hitems.size(),
                          cudaMemcpyHostToDevice));
-    VEXT_CUDA(cudaMalloc(&b->d_sample, sizeof(int4) * sample.size()));
+    VEXT_CUDA(device_malloc(&b->d_sample, sizeof(int4) * sample.size()));
     VEXT_CUDA(cudaMemcpy(b->d_sample, sample.data(), sizeof(int4) * sample.size(),
                          cudaMemcpyHostToDevice));
-    VEXT_CUDA(cudaMalloc(&b->d_counter, sizeof(int)));
+    VEXT_CUDA(device_malloc(&b->d_counter, sizeof(int)));
     // refinement records (2 ints each): one pose in 8 at most, 512 MB at most
     // (the 100-field benchmark batch flags 0.75 % of its poses)
     b->refine_cap = (int)std::min<long long>(b->poses / 8 + 1024, 64LL << 20);
-    VEXT_CUDA(cudaMalloc(&b->d_refine, sizeof(int) * (1 + 2 * (size_t)b->refine_cap)));
-    VEXT_CUDA(cudaMalloc(&b->d_status, sizeof(int)));
+    VEXT_CUDA(device_malloc(&b->d_refine, sizeof(int) * (1 + 2 * (size_t)b->refine_cap)));
+    VEXT_CUDA(device_malloc(&b->d_status, sizeof(int)));
     VEXT_CUDA(cudaMemset(b->d_status, 0, sizeof(int)));
     // ---- autotune: CTA shape x resident CTAs per SM, on the sampled queue
     const size_t smem = batch_smem(b->max_types, b->adj);

@@ -206,7 +206,7 @@ extern "C" int evaluate_reused_neighbors(int n_centers, int n_axes, int n_images
             cudaStreamDestroy(cx.stream);
             for (void *p : {(void *)cx.d_images8, (void *)cx.d_centers, (void *)cx.d_axes,
                             (void *)cx.d_out, (void *)cx.d_starts, (void *)cx.d_indices})
-                cudaFree(p);
+                device_free(p);
             cudaSetDevice(cur);
         }
         cx.d_images8 = cx.d_centers = cx.d_axes = cx.d_out = nullptr;

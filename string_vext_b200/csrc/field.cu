@@ -816,18 +816,23 @@ extern "C" int vext_field(vext_system h, int size, int n_axes, const double *axe
     VEXT_TRY(field_device(sys, size, n_axes, axes, o, orientation_K ? sys->d_f32 : nullptr,
                           energy_f64 ? sys->d_e64T : nullptr, dm, ds, dg, st,
                           stats ? stats : &local));
+    VEXT_CUDA(cudaStreamSynchronize(st));
+    bool finite = true;
     if (orientation_K)
-        VEXT_CUDA(cudaMemcpyAsync(orientation_K, sys->d_f32, sizeof(float) * n,
-                                  cudaMemcpyDeviceToHost, st));
-    if (energy_f64)
-        VEXT_CUDA(cudaMemcpyAsync(energy_f64, sys->d_e64T, sizeof(double) * n,
-                                  cudaMemcpyDeviceToHost, st));
-    if (marginal_K)
-        VEXT_CUDA(cudaMemcpyAsync(marginal_K, dm, sizeof(float) * S3, cudaMemcpyDeviceToHost, st));
-    if (site_K)
-        VEXT_CUDA(cudaMemcpyAsync(site_K, ds, sizeof(float) * 2 * S3, cudaMemcpyDeviceToHost, st));
-    if (grid) VEXT_CUDA(cudaMemcpyAsync(grid, dg, sizeof(float) * S3, cudaMemcpyDeviceToHost, st));
+        VEXT_TRY(copy_to_host(orientation_K, sys->d_f32, sizeof(float) * n, &finite));
+    if (energy_f64) VEXT_TRY(copy_to_host(energy_f64, sys->d_e64T, sizeof(double) * n));
+    if (marginal_K) VEXT_TRY(copy_to_host(marginal_K, dm, sizeof(float) * S3, &finite));
+    if (site_K) VEXT_TRY(copy_to_host(site_K, ds, sizeof(float) * 2 * S3, &finite));
+    if (grid) VEXT_TRY(copy_to_host(grid, dg, sizeof(float) * S3, &finite));
+    sys->outputs_finite = finite;
     return check_nonfinite(sys, st);
+}
+
+extern "C" int vext_field_finite(vext_system h, int *finite) {
+    if (!h || !finite) return fail(VEXT_ERR_ARGUMENT, "null system or output");
+    std::lock_guard<std::mutex> guard(h->sys.lock);
+    *finite = h->sys.outputs_finite;
+    return 0;
 }
 
 extern "C" int vext_field_device(vext_system h, int size, int n_axes, const double *axes_host,
@@ -1104,28 +1109,30 @@ extern "C" int vext_field_adjoint(vext_system h, int size, int n_axes, const dou
             sys->host_g = sys->d_g32;
         }
         for (int k = 0; k < parts; ++k) {
-            const size_t first = blk * (size_t)k * S3,
-                         count = std::min(blk, n_axes - blk * k) * S3;
             VEXT_TRY(batch_replay(sys->host_parts[k], st));
             VEXT_CUDA(cudaEventRecord(sys->host_part_done[k], st));
-            VEXT_CUDA(cudaStreamWaitEvent(sys->aux, sys->host_part_done[k], 0));
-            VEXT_CUDA(cudaMemcpyAsync(energy + first, sys->d_f32 + first, sizeof(float) * count,
-                                      cudaMemcpyDeviceToHost, sys->aux));
-            VEXT_CUDA(cudaMemcpyAsync(gradient + 6 * first, sys->d_g32 + 6 * first,
-                                      sizeof(float) * 6 * count, cudaMemcpyDeviceToHost,
-                                      sys->aux));
         }
-        VEXT_CUDA(cudaStreamSynchronize(sys->aux));
+        // block k's copy while the blocks after it compute
+        int rc = 0;
+        for (int k = 0; k < parts && !rc; ++k) {
+            const size_t first = blk * (size_t)k * S3,
+                         count = std::min(blk, n_axes - blk * k) * S3;
+            VEXT_CUDA(cudaEventSynchronize(sys->host_part_done[k]));
+            rc = copy_to_host(energy + first, sys->d_f32 + first, sizeof(float) * count);
+            if (!rc)
+                rc = copy_to_host(gradient + 6 * first, sys->d_g32 + 6 * first,
+                                  sizeof(float) * 6 * count);
+        }
         VEXT_CUDA(cudaStreamSynchronize(st));
+        VEXT_TRY(rc);
         for (vext_batch b : sys->host_parts) VEXT_TRY(vext_batch_status(b));
         return 0;
     }
     VEXT_TRY(field_adjoint_device(h, size, n_axes, axes, o, opt, sys->d_f32, sys->d_g32, nullptr,
                                   nullptr, st));
-    VEXT_CUDA(cudaMemcpyAsync(energy, sys->d_f32, sizeof(float) * n, cudaMemcpyDeviceToHost, st));
-    VEXT_CUDA(cudaMemcpyAsync(gradient, sys->d_g32, sizeof(float) * 6 * n,
-                              cudaMemcpyDeviceToHost, st));
     VEXT_CUDA(cudaStreamSynchronize(st));
+    VEXT_TRY(copy_to_host(energy, sys->d_f32, sizeof(float) * n));
+    VEXT_TRY(copy_to_host(gradient, sys->d_g32, sizeof(float) * 6 * n));
     return check_status(sys, st);   // the FP64 modes (the mixed mode returned above)
 }
 

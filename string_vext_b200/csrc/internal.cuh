@@ -25,6 +25,24 @@
 
 namespace vext {
 
+// Device memory (memory.cu).  Allocations come from a pool per device that
+// keeps up to kPoolKeep bytes of what was freed; device_free waits for the
+// device first, as cudaFree does.
+cudaError_t device_malloc_bytes(void **p, size_t bytes);
+template <typename T>
+cudaError_t device_malloc(T **p, size_t bytes) {
+    return device_malloc_bytes(reinterpret_cast<void **>(p), bytes);
+}
+void device_free(void *p);
+
+// Copy finished device memory to host memory, through page-locked staging by
+// several threads when `dst` is pageable and large; *finite (when given, FP32
+// data) is cleared if a value is not finite.
+int copy_to_host(void *dst, const void *src, size_t bytes, bool *finite = nullptr);
+
+// Unique id of the calling thread's current context (0 when unavailable).
+unsigned long long current_context_id();
+
 constexpr int kMaxTypes = 1024;     // distinct framework (sigma, epsilon) pairs
 constexpr double kDefaultRSplit = 5.0;
 
@@ -80,8 +98,8 @@ struct TaylorPlan {
     int rows = 0;               // outputs of a region's poses, padded to the tile
     int outs = 0;               // outputs per pose: 1 (energy) or 7
     void release() {
-        cudaFree(poly);
-        cudaFree(matrix);
+        device_free(poly);
+        device_free(matrix);
         poly = nullptr;
         matrix = nullptr;
         poly_cap = matrix_cap = 0;
@@ -114,13 +132,15 @@ struct System {
     // guest, so one region-list set serves them all when it is built for the
     // largest site offset among them
     uint64_t frame_hash = 0;
+    void *d_base = nullptr;    // one allocation holding the five arrays below
     double *d_frac = nullptr;
     int *d_type = nullptr;
     float4 *d_tf = nullptr;
     double *d_td = nullptr;
+    int *d_status = nullptr;   // device status word
     std::vector<double> h_td;  // n_types x 4
     std::vector<RegionSet *> sets;
-    int *d_status = nullptr;   // device status word
+    bool outputs_finite = true;    // float32 outputs of the last vext_field call
     // scratch of the field path
     double *d_e64 = nullptr;
     size_t e64_cap = 0;
@@ -212,13 +232,13 @@ double block_radius(const Mat3 &H, int size, int ni, int nj, int nk);
 template <typename T>
 int ensure_capacity(T *&ptr, size_t &cap, size_t need) {
     if (need <= cap && ptr) return 0;
-    if (ptr) cudaFree(ptr);
+    if (ptr) device_free(ptr);
     ptr = nullptr;
     cap = 0;
     size_t n = need < 1 ? 1 : need;
-    cudaError_t err = cudaMalloc((void **)&ptr, n * sizeof(T));
+    cudaError_t err = device_malloc((void **)&ptr, n * sizeof(T));
     if (err != cudaSuccess)
-        return fail(VEXT_ERR_MEMORY, "cudaMalloc of %zu bytes failed: %s", n * sizeof(T),
+        return fail(VEXT_ERR_MEMORY, "device allocation of %zu bytes failed: %s", n * sizeof(T),
                     cudaGetErrorString(err));
     cap = n;
     return 0;

@@ -139,8 +139,8 @@ int pose_upload_desc(System *sys, const RegionSet *rs, const PoseBatchSys **out)
     const bool upload =
         !sys->d_pose_desc || std::memcmp(&sys->h_pose_desc, &y, sizeof y) != 0;
     if (!sys->d_pose_desc) {
-        VEXT_CUDA(cudaMalloc(&sys->d_pose_desc, sizeof(PoseBatchSys)));
-        VEXT_CUDA(cudaMalloc(&sys->d_pose_offsets, 2 * sizeof(long long)));
+        VEXT_CUDA(device_malloc(&sys->d_pose_desc, sizeof(PoseBatchSys)));
+        VEXT_CUDA(device_malloc(&sys->d_pose_offsets, 2 * sizeof(long long)));
         const long long off[2] = {0, 0};   // one system: the kernel never reads them
         VEXT_CUDA(cudaMemcpy(sys->d_pose_offsets, off, sizeof off, cudaMemcpyHostToDevice));
     }
@@ -188,9 +188,9 @@ struct vext_pose_batch_s {
     long long *d_offsets = nullptr;
     int *d_status = nullptr;
     ~vext_pose_batch_s() {
-        cudaFree(d_sys);
-        cudaFree(d_offsets);
-        cudaFree(d_status);
+        device_free(d_sys);
+        device_free(d_offsets);
+        device_free(d_status);
     }
 };
 
@@ -228,13 +228,13 @@ extern "C" int vext_pose_batch_create(int n_systems, const vext_system *systems,
         hs[k] = pose_describe(sys, rs);
     }
     std::vector<long long> offs(pose_offsets, pose_offsets + n_systems + 1);
-    VEXT_CUDA(cudaMalloc(&b->d_sys, sizeof(PoseBatchSys) * n_systems));
+    VEXT_CUDA(device_malloc(&b->d_sys, sizeof(PoseBatchSys) * n_systems));
     VEXT_CUDA(cudaMemcpy(b->d_sys, hs.data(), sizeof(PoseBatchSys) * n_systems,
                          cudaMemcpyHostToDevice));
-    VEXT_CUDA(cudaMalloc(&b->d_offsets, sizeof(long long) * (n_systems + 1)));
+    VEXT_CUDA(device_malloc(&b->d_offsets, sizeof(long long) * (n_systems + 1)));
     VEXT_CUDA(cudaMemcpy(b->d_offsets, offs.data(), sizeof(long long) * (n_systems + 1),
                          cudaMemcpyHostToDevice));
-    VEXT_CUDA(cudaMalloc(&b->d_status, sizeof(int)));
+    VEXT_CUDA(device_malloc(&b->d_status, sizeof(int)));
     VEXT_CUDA(cudaMemset(b->d_status, 0, sizeof(int)));
     *out = guard.release();
     return 0;

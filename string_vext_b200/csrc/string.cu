@@ -585,11 +585,11 @@ extern "C" int vext_string_run(vext_system h, int n, double *path, double *energ
     // centers2 (3n each), quats quats2 (4n each), centers7 quats7 e7 (21n,
     // 28n, 7n)
     const size_t words = 3 * 6 * nd + 4 * nd + 4 * 3 * nd + 2 * 4 * nd + 56 * nd;
-    VEXT_CUDA(cudaMalloc(&buf, sizeof(double) * words));
+    VEXT_CUDA(device_malloc(&buf, sizeof(double) * words));
     int *flags = nullptr;
-    cudaError_t e = cudaMalloc(&flags, sizeof(int) * 8);
+    cudaError_t e = device_malloc(&flags, sizeof(int) * 8);
     if (e != cudaSuccess) {
-        cudaFree(buf);
+        device_free(buf);
         return fail(VEXT_ERR_MEMORY, "cudaMalloc failed");
     }
     StringArgs a;
@@ -621,8 +621,8 @@ extern "C" int vext_string_run(vext_system h, int n, double *path, double *energ
     a.e7 = q; q += 7 * nd;
     a.fd = p.gradient == VEXT_STRING_REFERENCE_FD;
     if ((size_t)(q - buf) != words) {   // the carve-out must match the allocation exactly
-        cudaFree(buf);
-        cudaFree(flags);
+        device_free(buf);
+        device_free(flags);
         return fail(VEXT_ERR_CAPACITY, "String workspace layout mismatch");
     }
     a.flags = flags;
@@ -717,7 +717,7 @@ extern "C" int vext_string_run(vext_system h, int n, double *path, double *energ
     };
     rc = run();
     cudaStreamSynchronize(st);
-    cudaFree(buf);
-    cudaFree(flags);
+    device_free(buf);
+    device_free(flags);
     return rc;
 }

@@ -310,9 +310,9 @@ __global__ void __launch_bounds__(NT, 512 / NT)
 // ------------------------------------------------------------ region sets
 
 RegionSet::~RegionSet() {
-    cudaFree(d_info);
-    cudaFree(d_hi);
-    cudaFree(d_lo);
+    device_free(d_info);
+    device_free(d_hi);
+    device_free(d_lo);
 }
 
 // Per-device scratch of the per-(region, thread) class counts that the count
@@ -327,32 +327,6 @@ struct BuildScratch {
     size_t cap = 0;
     unsigned long long ctx_id = 0;
 };
-// Unique id of the calling thread's current context (0 when unavailable).
-unsigned long long current_context_id() {
-    using GetCurrentFn = CUresult (*)(CUcontext *);
-    using GetIdFn = CUresult (*)(CUcontext, unsigned long long *);
-    static const std::pair<GetCurrentFn, GetIdFn> fns = [] {
-        void *a = nullptr, *b = nullptr;
-        cudaDriverEntryPointQueryResult qa = cudaDriverEntryPointSymbolNotFound, qb = qa;
-        const bool ok =
-            cudaGetDriverEntryPoint("cuCtxGetCurrent", &a, cudaEnableDefault, &qa) ==
-                cudaSuccess &&
-            qa == cudaDriverEntryPointSuccess &&
-            cudaGetDriverEntryPoint("cuCtxGetId", &b, cudaEnableDefault, &qb) == cudaSuccess &&
-            qb == cudaDriverEntryPointSuccess;
-        if (!ok) {
-            cudaGetLastError();
-            return std::pair<GetCurrentFn, GetIdFn>(nullptr, nullptr);
-        }
-        return std::pair<GetCurrentFn, GetIdFn>(reinterpret_cast<GetCurrentFn>(a),
-                                                reinterpret_cast<GetIdFn>(b));
-    }();
-    CUcontext ctx = nullptr;
-    unsigned long long id = 0;
-    if (!fns.first || fns.first(&ctx) != CUDA_SUCCESS || !ctx || fns.second(ctx, &id) != CUDA_SUCCESS)
-        return 0;
-    return id;
-}
 BuildScratch &build_scratch(int device) {
     static BuildScratch scratch[64];
     return scratch[device & 63];
@@ -388,7 +362,7 @@ static int build_lists(System *sys, RegionSet *rs, cudaStream_t stream) {
     const double ra2 = sys->cutoff * sys->cutoff - sys->max_offset * sys->max_offset;
     a.r_shella0 = rs->d_taylor < sys->cutoff && ra2 > 0 ? std::sqrt(ra2) - 1e-3 : 0.0;
     const int n = rs->n_regions;
-    if (!rs->d_info) VEXT_CUDA(cudaMalloc(&rs->d_info, sizeof(RegionInfo) * n));
+    if (!rs->d_info) VEXT_CUDA(device_malloc(&rs->d_info, sizeof(RegionInfo) * n));
     VEXT_CUDA(cudaMemcpyAsync(rs->d_info, rs->h_info.data(), sizeof(RegionInfo) * n,
                               cudaMemcpyHostToDevice, stream));
     cudaEvent_t e0 = sys->ev[3], e1 = sys->ev[4];
@@ -429,12 +403,12 @@ static int build_lists(System *sys, RegionSet *rs, cudaStream_t stream) {
     VEXT_CUDA(cudaMemcpyAsync(rs->d_info, rs->h_info.data(), sizeof(RegionInfo) * n,
                               cudaMemcpyHostToDevice, stream));
     if (off > rs->capacity || !rs->d_hi) {
-        cudaFree(rs->d_hi);
-        cudaFree(rs->d_lo);
+        device_free(rs->d_hi);
+        device_free(rs->d_lo);
         rs->d_hi = rs->d_lo = nullptr;
         rs->capacity = 0;
-        VEXT_CUDA(cudaMalloc(&rs->d_hi, sizeof(float4) * std::max<long long>(off, 1)));
-        VEXT_CUDA(cudaMalloc(&rs->d_lo, sizeof(float4) * std::max<long long>(off, 1)));
+        VEXT_CUDA(device_malloc(&rs->d_hi, sizeof(float4) * std::max<long long>(off, 1)));
+        VEXT_CUDA(device_malloc(&rs->d_lo, sizeof(float4) * std::max<long long>(off, 1)));
         rs->capacity = std::max<long long>(off, 1);
     }
     if (field)
@@ -611,25 +585,21 @@ void System::drop_host_parts() {
 System::~System() {
     drop_adjoint_batch();   // it points into the region sets
     for (RegionSet *rs : sets) delete rs;
-    cudaFree(d_g32);
+    device_free(d_g32);
     field_plan.release();
-    cudaFree(d_sums);
-    cudaFree(d_frac);
-    cudaFree(d_type);
-    cudaFree(d_tf);
-    cudaFree(d_td);
-    cudaFree(d_status);
-    cudaFree(d_e64);
-    cudaFree(d_refine);
-    cudaFree(d_axes);
-    cudaFree(d_f32);
-    cudaFree(d_small);
-    cudaFree(d_e64T);
-    cudaFree(d_flags);
-    cudaFree(d_pose_scratch);
-    cudaFree(d_pose_io);
-    cudaFree(d_pose_desc);
-    cudaFree(d_pose_offsets);
+    device_free(d_sums);
+    device_free(d_base);
+    device_free(d_e64);
+    device_free(d_refine);
+    device_free(d_axes);
+    device_free(d_f32);
+    device_free(d_small);
+    device_free(d_e64T);
+    device_free(d_flags);
+    device_free(d_pose_scratch);
+    device_free(d_pose_io);
+    device_free(d_pose_desc);
+    device_free(d_pose_offsets);
     for (auto &e : ev)
         if (e) cudaEventDestroy(e);
     if (aux) cudaStreamDestroy(aux);
@@ -763,18 +733,31 @@ extern "C" int vext_system_create(const vext_system_desc *d, vext_system *out) {
     chk(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
     chk(cudaStreamCreateWithFlags(&s.aux, cudaStreamNonBlocking));
     for (auto &e : s.ev) chk(cudaEventCreate(&e));
-    chk(cudaMalloc(&s.d_frac, sizeof(double) * frac.size()));
-    chk(cudaMalloc(&s.d_type, sizeof(int) * type.size()));
-    chk(cudaMalloc(&s.d_tf, sizeof(float4) * tf.size()));
-    chk(cudaMalloc(&s.d_td, sizeof(double) * s.h_td.size()));
-    chk(cudaMalloc(&s.d_status, sizeof(int)));
+    // one allocation and one upload
+    size_t bytes = 0;
+    auto place = [&bytes](size_t n) {
+        const size_t at = bytes;
+        bytes = (bytes + n + 255) & ~(size_t)255;
+        return at;
+    };
+    const size_t at_frac = place(sizeof(double) * frac.size()),
+                 at_type = place(sizeof(int) * type.size()),
+                 at_tf = place(sizeof(float4) * tf.size()),
+                 at_td = place(sizeof(double) * s.h_td.size()), at_status = place(sizeof(int));
+    chk(device_malloc(&s.d_base, bytes));
     if (err == cudaSuccess) {
-        chk(cudaMemcpy(s.d_frac, frac.data(), sizeof(double) * frac.size(), cudaMemcpyHostToDevice));
-        chk(cudaMemcpy(s.d_type, type.data(), sizeof(int) * type.size(), cudaMemcpyHostToDevice));
-        chk(cudaMemcpy(s.d_tf, tf.data(), sizeof(float4) * tf.size(), cudaMemcpyHostToDevice));
-        chk(cudaMemcpy(s.d_td, s.h_td.data(), sizeof(double) * s.h_td.size(),
-                       cudaMemcpyHostToDevice));
-        chk(cudaMemset(s.d_status, 0, sizeof(int)));
+        std::vector<char> up(bytes, 0);
+        std::memcpy(&up[at_frac], frac.data(), sizeof(double) * frac.size());
+        std::memcpy(&up[at_type], type.data(), sizeof(int) * type.size());
+        std::memcpy(&up[at_tf], tf.data(), sizeof(float4) * tf.size());
+        std::memcpy(&up[at_td], s.h_td.data(), sizeof(double) * s.h_td.size());
+        char *base = static_cast<char *>(s.d_base);
+        s.d_frac = reinterpret_cast<double *>(base + at_frac);
+        s.d_type = reinterpret_cast<int *>(base + at_type);
+        s.d_tf = reinterpret_cast<float4 *>(base + at_tf);
+        s.d_td = reinterpret_cast<double *>(base + at_td);
+        s.d_status = reinterpret_cast<int *>(base + at_status);
+        chk(cudaMemcpy(base, up.data(), bytes, cudaMemcpyHostToDevice));
     }
     if (err != cudaSuccess) {
         delete handle;

@@ -113,6 +113,12 @@ class VextSystem:
                 out[key] = value
         return out
 
+    def outputs_finite(self) -> bool:
+        """Whether all float32 values the last ``field`` call returned are finite."""
+        finite = ctypes.c_int()
+        _lib.check(self._lib.vext_field_finite(self.handle, ctypes.byref(finite)))
+        return bool(finite.value)
+
     def field_device(self, size: int, axes, out_orientation, mode: int = _lib.VEXT_MODE_MIXED,
                      out_energy=None, out_marginal=None, out_site=None, out_grid=None,
                      stream=None, **opts) -> None:

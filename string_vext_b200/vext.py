@@ -37,11 +37,13 @@ def calculate_vext(case: dict, size: int = 60, orientations: int = 64,
     """The Vext field of ``case`` on a ``size``^3 grid x ``orientations``
     Fibonacci directors, in the reference's output layout."""
     from .system import VextSystem
-    _, axes = regular_pose_grid(size, orientations)
+    # the directors (and the size check) without the centers, which the library forms
+    _, axes = regular_pose_grid(min(size, 2), orientations)
     with VextSystem(case) as system:
         out = system.field(size, normalized_directors(axes), mode=mode, orientation=True,
                            marginal=True, site=True, grid=True)
         stats = system.last_stats
+        finite = system.outputs_finite()
     result = {"orientation_K": out["orientation_K"], "marginal_K": out["marginal_K"],
               "site_K": out["site_K"], "axes": axes.astype(np.float32),
               "cell_matrix": np.asarray(case["cell"], dtype=np.float64),
@@ -50,6 +52,8 @@ def calculate_vext(case: dict, size: int = 60, orientations: int = 64,
               "framework_epsilon_K": np.asarray(case["frame_epsilon"], dtype=np.float64),
               "grid": out["grid"]}
     for name, value in result.items():
+        if finite and name in out:   # looked at while the library copied it
+            continue
         if not np.isfinite(value).all():
             raise ValueError(f"nonfinite Vext output ({name})")
     return (result, stats) if return_stats else result
