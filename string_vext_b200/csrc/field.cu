@@ -342,24 +342,64 @@ __global__ void refine_kernel(FieldArgs a, const int *list) {
 }
 
 // Single-site field at the grid centers (site 0 parameters, no offset):
-// the reference's site_K (src/string_vext/vext.py:27-29, 33).
-__global__ void site_kernel(FieldArgs a, float *site_K) {
-    const int lane = threadIdx.x & 31;
-    const long long S3 = (long long)a.S * a.S * a.S;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < S3;
-         c += nwarps) {
-        const int gi = (int)(c / ((long long)a.S * a.S)), gj = (int)((c / a.S) % a.S),
-                  gk = (int)(c % a.S);
-        const RegionInfo r = a.regs[region_of(a, gi, gj, gk)];
-        double cx, cy, cz;
+// the reference's site_K (src/string_vext/vext.py:27-29, 33).  One CTA per
+// region: each thread takes every 128th entry of the list with all CB centers,
+// so an entry is read once for the region.  FP64 pipe-bound; a warp per
+// center, reading the whole list for it, and a division per pair took 1.56 ms
+// for the 60^3 layered field.
+template <int CB>
+__global__ void __launch_bounds__(128, 4) site_kernel(FieldArgs a, float *site_K) {
+    constexpr int NC = CB < 8 ? CB : 8;   // centers at a time
+    __shared__ double part[4][NC];
+    __shared__ double cen[CB][3];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const RegionInfo r = a.regs[blockIdx.x];
+    const int nc = r.ni * r.nj * r.nk;
+    if (tid < CB) {
+        int gi, gj, gk;
+        center_of(a, r, min(tid, nc - 1), gi, gj, gk);
         frac_to_cart(a.H, (gi + .5) / a.S - r.of[0], (gj + .5) / a.S - r.of[1],
-                     (gk + .5) / a.S - r.of[2], cx, cy, cz);
-        const double e = warp_sum(site_sum_fp64(a, r, cx, cy, cz, lane));
-        if (lane == 0) {
+                     (gk + .5) / a.S - r.of[2], cen[tid][0], cen[tid][1], cen[tid][2]);
+    }
+    __syncthreads();
+    for (int c0 = 0; c0 < nc; c0 += NC) {
+        double sum[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) sum[c] = 0.0;
+#pragma unroll 1
+        for (int e = tid; e < r.n_total; e += 128) {
+            const float4 h = a.hi[r.off + e], l = a.lo[r.off + e];
+            const double x = (double)h.x + (double)l.x, y = (double)h.y + (double)l.y,
+                         z = (double)h.z + (double)l.z;
+            const double2 *td = reinterpret_cast<const double2 *>(a.td) + 2 * __float_as_int(h.w);
+            const double2 cc = td[0], sf = td[1];   // (c12, c6), (shift, floor2)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                const double dx = cen[c0 + c][0] - x, dy = cen[c0 + c][1] - y,
+                             dz = cen[c0 + c][2] - z;
+                const double d2 = fma(dx, dx, fma(dy, dy, dz * dz));
+                const double i2 = rcp64_nr<2>(fmax(d2, sf.y));
+                const double i6 = i2 * i2 * i2;
+                const double en = fma(i6, fma(cc.x, i6, -cc.y), sf.x);
+                sum[c] += d2 < a.rc2 ? en : 0.0;
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            sum[c] = warp_sum(sum[c]);
+            if (lane == 0) part[warp][c] = sum[c];
+        }
+        __syncthreads();
+        if (tid < NC && c0 + tid < nc) {
+            const double e = part[0][tid] + part[1][tid] + part[2][tid] + part[3][tid];
+            int gi, gj, gk;
+            center_of(a, r, c0 + tid, gi, gj, gk);
+            const long long S3 = (long long)a.S * a.S * a.S;
+            const long long c = ((long long)gi * a.S + gj) * a.S + gk;
             site_K[c] = (float)e;
             site_K[S3 + c] = (float)e;
         }
+        __syncthreads();
     }
 }
 
@@ -752,7 +792,9 @@ static int field_device(System *sys, int size, int n_axes, const double *axes_ho
         VEXT_CUDA(cudaGetLastError());
     }
     if (d_site) {
-        site_kernel<<<1184, 256, 0, stream>>>(a, d_site);
+        if (cb == 8) site_kernel<8><<<rs->n_regions, 128, 0, stream>>>(a, d_site);
+        else if (cb == 16) site_kernel<16><<<rs->n_regions, 128, 0, stream>>>(a, d_site);
+        else site_kernel<32><<<rs->n_regions, 128, 0, stream>>>(a, d_site);
         VEXT_CUDA(cudaGetLastError());
     }
     finalize_kernel<<<592, 256, 0, stream>>>(sys->d_e64, size, n_axes, sys->temperature, d_oK,

@@ -382,32 +382,39 @@ struct EvalArgs {
     double *e64;
 };
 
-constexpr int kEvalThreads = 128, kEvalCols = 64, kEvalK = 16;
-__host__ __device__ constexpr int eval_rows(int outs) { return outs == 1 ? 16 : 14; }   // rows per thread
+constexpr int kEvalK = 16;
+__host__ __device__ constexpr int eval_rows(int outs) { return outs == 1 ? 16 : 14; }   // per thread
 __host__ __device__ constexpr int eval_tile(int outs) { return 16 * eval_rows(outs); }
 
-// Tile: eval_tile rows (32 poses x 7 outputs, or 256 poses) x 64 regions; a
-// thread holds 14 or 16 rows (packed in pairs: two poses) x 8 regions.  Bound
-// by the FMA pipe: 56-64 packed FMA per 11-12 shared-memory wavefronts.
-template <int OUTS>
-__global__ void __launch_bounds__(kEvalThreads, 2) taylor_eval_kernel(EvalArgs a) {
+// Tile: eval_tile rows (32 poses x 7 outputs, or 256 poses) x NT / 16 CT
+// regions; a thread holds 14 or 16 rows (packed in pairs: two poses) x CT
+// regions.  Bound by the FMA pipe.  28,800 regions: energy and gradient
+// 1.99 ms as 128 threads x 8 regions (256 x 4: 2.12; 6 regions at 3 CTAs/SM:
+// 2.09; unpacked FMA: 2.07); 14,400 regions of 16 centers, energy alone: 0.46
+// ms as 256 x 4 (128 x 8: 0.53).
+template <int OUTS, int NT, int CT>
+__global__ void __launch_bounds__(NT, 2) taylor_eval_kernel(EvalArgs a) {
     constexpr int RT = eval_rows(OUTS), RP = RT / 2, TILE = eval_tile(OUTS);
+    constexpr int COLS = NT / 16 * CT;   // regions per tile
     __shared__ __align__(16) float ms[2][kEvalK][TILE];
-    __shared__ __align__(16) float2 ss[2][kEvalK][kEvalCols];
-    const int tid = threadIdx.x, rg = tid >> 3, cg = tid & 7;
-    const int row0 = blockIdx.x * TILE, reg0 = blockIdx.y * kEvalCols;
-    float2 acc[RP][8];
+    __shared__ __align__(16) float2 ss[2][kEvalK][COLS];
+    // warps 4 (rows) x NT / 128 (regions), lanes 4 x 8: one wavefront per
+    // shared-memory load
+    const int tid = threadIdx.x, rg = (tid >> 5 & 3) * 4 + (tid >> 3 & 3),
+              cg = (tid >> 7) * 8 + (tid & 7);
+    const int row0 = blockIdx.x * TILE, reg0 = blockIdx.y * COLS;
+    float2 acc[RP][CT];
 #pragma unroll
     for (int i = 0; i < RP; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = make_float2(0.f, 0.f);
-    // region columns this thread stages: 2 x 4 consecutive sums
-    const int sr0 = tid >> 2, sk = (tid & 3) * 4;
-    float4 hold[2];
+        for (int j = 0; j < CT; ++j) acc[i][j] = make_float2(0.f, 0.f);
+    constexpr int SV = COLS * kEvalK / 4, SL = (SV + NT - 1) / NT;   // float4 of sums, per thread
+    float4 hold[SL];
     auto load_m = [&](int buf, int k0) {
 #pragma unroll
-        for (int i = 0; i < kEvalK * TILE / 4 / kEvalThreads; ++i) {
-            const int v = tid + i * kEvalThreads, k = v / (TILE / 4), c = v % (TILE / 4) * 4;
+        for (int i = 0; i < (kEvalK * TILE / 4 + NT - 1) / NT; ++i) {
+            const int v = tid + i * NT, k = v / (TILE / 4), c = v % (TILE / 4) * 4;
+            if (k >= kEvalK) break;
             const uint32_t dst = smem_addr(&ms[buf][k][c]);
             const float *src = a.matrix + (size_t)(k0 + k) * a.rows + row0 + c;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
@@ -416,30 +423,34 @@ __global__ void __launch_bounds__(kEvalThreads, 2) taylor_eval_kernel(EvalArgs a
     };
     auto load_s = [&](int k0) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int r = min(reg0 + sr0 + 32 * i, a.n_regions - 1);
-            hold[i] = *reinterpret_cast<const float4 *>(a.sums + (size_t)r * kTaylorPad + k0 + sk);
+        for (int i = 0; i < SL; ++i) {
+            const int v = min(tid + i * NT, SV - 1);
+            const int r = min(reg0 + (v >> 2), a.n_regions - 1);
+            hold[i] = *reinterpret_cast<const float4 *>(a.sums + (size_t)r * kTaylorPad + k0 +
+                                                        (v & 3) * 4);
         }
     };
     auto store_s = [&](int buf) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int c = sr0 + 32 * i;
-            ss[buf][sk][c] = make_float2(hold[i].x, hold[i].x);
-            ss[buf][sk + 1][c] = make_float2(hold[i].y, hold[i].y);
-            ss[buf][sk + 2][c] = make_float2(hold[i].z, hold[i].z);
-            ss[buf][sk + 3][c] = make_float2(hold[i].w, hold[i].w);
+        for (int i = 0; i < SL; ++i) {
+            const int v = tid + i * NT, c = v >> 2, k = (v & 3) * 4;
+            if (v >= SV) break;
+            ss[buf][k][c] = make_float2(hold[i].x, hold[i].x);
+            ss[buf][k + 1][c] = make_float2(hold[i].y, hold[i].y);
+            ss[buf][k + 2][c] = make_float2(hold[i].z, hold[i].z);
+            ss[buf][k + 3][c] = make_float2(hold[i].w, hold[i].w);
         }
     };
     // one k of operands ahead of the FMAs that use them
-    float2 m[2][RP], v[2][8];
-    auto fetch = [&](int buf, int k, float2 (&mk)[RP], float2 (&vk)[8]) {
+    float2 m[2][RP], v[2][CT];
+    auto fetch = [&](int buf, int k, float2 (&mk)[RP], float2 (&vk)[CT]) {
 #pragma unroll
         for (int i = 0; i < RP; ++i)
             mk[i] = *reinterpret_cast<const float2 *>(&ms[buf][k][rg * RT + 2 * i]);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float4 q = *reinterpret_cast<const float4 *>(&ss[buf][k][16 * j + 2 * cg]);
+        for (int j = 0; j < CT / 2; ++j) {
+            const float4 q =
+                *reinterpret_cast<const float4 *>(&ss[buf][k][NT / 8 * j + 2 * cg]);
             vk[2 * j] = make_float2(q.x, q.y);
             vk[2 * j + 1] = make_float2(q.z, q.w);
         }
@@ -462,7 +473,7 @@ __global__ void __launch_bounds__(kEvalThreads, 2) taylor_eval_kernel(EvalArgs a
 #pragma unroll
             for (int i = 0; i < RP; ++i)
 #pragma unroll
-                for (int j = 0; j < 8; ++j)
+                for (int j = 0; j < CT; ++j)
                     acc[i][j] = __ffma2_rn(m[k & 1][i], v[k & 1][j], acc[i][j]);
         }
         if (more) store_s(buf ^ 1);
@@ -471,8 +482,8 @@ __global__ void __launch_bounds__(kEvalThreads, 2) taylor_eval_kernel(EvalArgs a
     const long long S3 = (long long)a.S * a.S * a.S;
     float *e32 = a.e32 ? *a.e32 : nullptr, *g32 = OUTS == 7 ? *a.g32 : nullptr;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int reg = reg0 + 16 * (j >> 1) + 2 * cg + (j & 1);
+    for (int j = 0; j < CT; ++j) {
+        const int reg = reg0 + NT / 8 * (j >> 1) + 2 * cg + (j & 1);
         if (reg >= a.n_regions) continue;
         const RegionInfo &r = a.regs[reg];
         const int i0 = r.i0, j0 = r.j0, kk0 = r.k0;
@@ -628,9 +639,11 @@ int taylor_enqueue(const System &sys, const RegionSet &rs, int n_axes, const Tay
     a.e32 = e32;
     a.g32 = g32;
     a.e64 = e64;
-    const dim3 grid(plan.rows / eval_tile(plan.outs), (rs.n_regions + kEvalCols - 1) / kEvalCols);
-    if (plan.outs == 7) taylor_eval_kernel<7><<<grid, kEvalThreads, 0, stream>>>(a);
-    else taylor_eval_kernel<1><<<grid, kEvalThreads, 0, stream>>>(a);
+    const int tiles = plan.rows / eval_tile(plan.outs);
+    if (plan.outs == 7)
+        taylor_eval_kernel<7, 128, 8><<<dim3(tiles, (rs.n_regions + 63) / 64), 128, 0, stream>>>(a);
+    else
+        taylor_eval_kernel<1, 256, 4><<<dim3(tiles, (rs.n_regions + 63) / 64), 256, 0, stream>>>(a);
     VEXT_CUDA(cudaGetLastError());
     return 0;
 }
