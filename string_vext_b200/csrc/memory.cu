@@ -4,9 +4,10 @@
 // system again: about twenty cudaMalloc and cudaFree, 4 ms of its 5.5 ms for
 // a small framework.  Device memory therefore comes from a stream-ordered pool
 // per device, used on a stream of its own that every allocation waits for, so
-// the memory may be used on any stream and by any thread.  The pool returns
-// what is freed beyond kPoolKeep bytes to the device, all of it when an
-// allocation fails, and belongs to the context it was made in.
+// the memory may be used on any stream and by any thread.  What is freed beyond
+// kPoolKeep bytes goes back to the device at once (not by the pool's own
+// threshold, which every synchronisation of the process would look at), all of
+// it when an allocation fails; the pool belongs to the context it was made in.
 //
 // Large results go to pageable memory through page-locked buffers: a few
 // threads each copy their chunks from the device and on to the destination
@@ -85,7 +86,7 @@ void open_pool(DevicePool &p, int device) {
     props.handleTypes = cudaMemHandleTypeNone;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = device;
-    unsigned long long keep = kPoolKeep;
+    unsigned long long keep = ~0ull;   // device_free trims
     if (ctx == 0 ||
         cudaDeviceGetAttribute(&supported, cudaDevAttrMemoryPoolsSupported, device) !=
             cudaSuccess ||
@@ -145,6 +146,13 @@ void device_free(void *ptr) {
         } else {
             cudaDeviceSynchronize();   // no stream uses it any more
             cudaFreeAsync(ptr, p.stream);
+            unsigned long long held = 0;
+            if (cudaMemPoolGetAttribute(p.pool, cudaMemPoolAttrReservedMemCurrent, &held) ==
+                    cudaSuccess &&
+                held > kPoolKeep) {
+                cudaStreamSynchronize(p.stream);
+                cudaMemPoolTrimTo(p.pool, kPoolKeep);
+            }
         }
     }
     if (at.device != current) cudaSetDevice(current);

@@ -41,7 +41,7 @@ struct PoseBatchArgs {
 // list together, so that small batches (a String path) still fill the GPU;
 // the warps' sums are added in shared memory in a fixed order.  MIXED = false:
 // the FP64 mode (every entry near, evaluated as in refinement).
-template <bool MIXED>
+template <bool MIXED, int LOADS>
 __global__ void __launch_bounds__(256, 2) pose_batch_kernel(PoseBatchArgs a) {
     __shared__ double part[8][7];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(256, 2) pose_batch_kernel(PoseBatchArgs a) {
         const PoseBatchSys &y = a.sys[lo];
         PosePoint pt;
         double v[7];
-        pose_eval<MIXED>(y, a.quats + 4 * p, a.centers + 3 * p, W, warp, lane, part, a.band_lo,
+        pose_eval<MIXED, LOADS>(y, a.quats + 4 * p, a.centers + 3 * p, W, warp, lane, part, a.band_lo,
                          a.band_hi, a.status, pt, v);
         if (sub != 0) continue;
         if (live && lane == 0) {
@@ -101,12 +101,26 @@ int warps_per_pose(long long n) {
     return w;
 }
 
-static int pose_batch_launch(PoseBatchArgs a, bool mixed, cudaStream_t st) {
+// Lists from this mean length on are worth loading ahead.
+constexpr double kLongList = 512;
+
+// mean_list: entries of a bin list, over the batch's poses; max_list: the mean
+// of the system with the longest.  Long lists load several entries at a time.
+// Uneven ones (the longest 1.5 times the mean and more) take two warps per
+// pose up to about 96 warps per SM in all: the halves shorten the tail that the
+// poses of dense systems leave (6,545 String poses of 12 frameworks: 118 us
+// with one warp, 83 with two, 112 with four), while 100 paths of one framework
+// lose (42 us with one, 55 with two).
+static int pose_batch_launch(PoseBatchArgs a, bool mixed, double mean_list, double max_list,
+                             cudaStream_t st) {
     a.wpp = warps_per_pose(a.n);
+    const bool long_lists = mean_list >= kLongList && a.wpp <= 2;
+    if (long_lists && max_list >= 1.5 * mean_list && a.n * 2 <= 148LL * 96) a.wpp = 2;
     const long long groups = (a.n + 8 / a.wpp - 1) / (8 / a.wpp);
     const int blocks = (int)std::min<long long>(groups, 148LL * 16);
-    if (mixed) pose_batch_kernel<true><<<blocks, 256, 0, st>>>(a);
-    else pose_batch_kernel<false><<<blocks, 256, 0, st>>>(a);
+    auto kernel = mixed ? long_lists ? pose_batch_kernel<true, 4> : pose_batch_kernel<true, 1>
+                        : long_lists ? pose_batch_kernel<false, 4> : pose_batch_kernel<false, 1>;
+    kernel<<<blocks, 256, 0, st>>>(a);
     VEXT_CUDA(cudaGetLastError());
     return 0;
 }
@@ -172,7 +186,8 @@ int pose_warp_enqueue(System *sys, const RegionSet *rs, int n, const double *cen
     a.band_lo = band ? o.band_lo : 0.0;
     a.band_hi = band ? o.band_hi : 0.0;
     a.status = sys->d_status;
-    return pose_batch_launch(a, o.mode == VEXT_MODE_MIXED, st);
+    const double list = (double)rs->n_entries / std::max(rs->n_regions, 1);
+    return pose_batch_launch(a, o.mode == VEXT_MODE_MIXED, list, list, st);
 }
 
 }  // namespace vext
@@ -183,6 +198,7 @@ struct vext_pose_batch_s {
     std::vector<vext_system> systems;
     long long n = 0;
     int n_systems = 0;
+    double mean_list = 0, max_list = 0;   // entries of a bin list (pose_batch_launch)
     Options opt;
     PoseBatchSys *d_sys = nullptr;
     long long *d_offsets = nullptr;
@@ -226,6 +242,9 @@ extern "C" int vext_pose_batch_create(int n_systems, const vext_system *systems,
         RegionSet *rs = nullptr;
         VEXT_TRY(get_bin_regions(sys, r_split, &rs, sys->stream));
         hs[k] = pose_describe(sys, rs);
+        const double list = (double)rs->n_entries / std::max(rs->n_regions, 1);
+        b->mean_list += (double)(pose_offsets[k + 1] - pose_offsets[k]) / std::max(b->n, 1LL) * list;
+        if (pose_offsets[k + 1] > pose_offsets[k]) b->max_list = std::max(b->max_list, list);
     }
     std::vector<long long> offs(pose_offsets, pose_offsets + n_systems + 1);
     VEXT_CUDA(device_malloc(&b->d_sys, sizeof(PoseBatchSys) * n_systems));
@@ -261,7 +280,8 @@ extern "C" int vext_pose_batch_run(vext_pose_batch b, const double *centers, con
     a.band_lo = band ? b->opt.band_lo : 0.0;
     a.band_hi = band ? b->opt.band_hi : 0.0;
     a.status = b->d_status;
-    return pose_batch_launch(a, b->opt.mode == VEXT_MODE_MIXED, (cudaStream_t)stream);
+    return pose_batch_launch(a, b->opt.mode == VEXT_MODE_MIXED, b->mean_list, b->max_list,
+                             (cudaStream_t)stream);
 }
 
 extern "C" int vext_pose_batch_status(vext_pose_batch b) {

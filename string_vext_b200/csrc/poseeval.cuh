@@ -6,8 +6,6 @@
 
 namespace vext {
 
-constexpr int kPoseLoads = 4, kPoseNearLoads = 2;   // entries loaded together per lane
-
 // This lane's far entries begin + lane + stride i < end of one pose, the two
 // sites in the two lanes of the packed FP32x2 instructions (pose.cu's far loop):
 // d = x - r_s, n1 = hardware reciprocal of d2, n3 = n1^3, e = n3 (c12 n3 - c6),
@@ -18,7 +16,9 @@ constexpr int kPoseLoads = 4, kPoseNearLoads = 2;   // entries loaded together p
 // kBorderTol of rc^2 -- where the FP32 test might decide the pair unlike the
 // FP64 one -- leaves the FP32 sums and takes the pair in FP64
 // (fp64_border_pair, from the hi + lo position and the FP64 site sd).
-template <bool MASK>
+// LOADS: entries a lane loads together (long lists only: a short one would
+// mostly load its last entry again).
+template <bool MASK, int LOADS>
 __device__ __forceinline__ void far_lane_sums(const PoseBatchSys &y, long long base, int begin,
                                               int end, int lane, int stride, float2 nsx,
                                               float2 nsy, float2 nsz, const double (&sd)[2][3],
@@ -29,22 +29,7 @@ __device__ __forceinline__ void far_lane_sums(const PoseBatchSys &y, long long b
         float2 fe = make_float2(0.f, 0.f), gx = fe, gy = fe, gz = fe;
         float fs = 0.f;
         const int i1 = min(i0 + 16, mine);
-#pragma unroll 1
-        for (int j0 = i0; j0 < i1; j0 += kPoseLoads) {
-        // the loads of kPoseLoads entries in flight together (each entry is a
-        // chain of list, table and arithmetic latencies), summed in order
-        float4 hv[kPoseLoads], tv[kPoseLoads];
-#pragma unroll
-        for (int j = 0; j < kPoseLoads; ++j)
-            hv[j] = y.hi[base + begin + lane + (long long)stride * min(j0 + j, i1 - 1)];
-#pragma unroll
-        for (int j = 0; j < kPoseLoads; ++j) tv[j] = y.tf[__float_as_int(hv[j].w)];
-#pragma unroll
-        for (int j = 0; j < kPoseLoads; ++j) {
-            if (j0 + j >= i1) break;
-            const long long k = base + begin + lane + (long long)stride * (j0 + j);
-            const float4 h = hv[j];
-            const float4 tp = tv[j];   // (c12, c6, shift, floor2)
+        auto add = [&](long long k, const float4 &h, const float4 &tp) {
             const float2 dx = __fadd2_rn(make_float2(h.x, h.x), nsx),
                          dy = __fadd2_rn(make_float2(h.y, h.y), nsy),
                          dz = __fadd2_rn(make_float2(h.z, h.z), nsz);
@@ -88,7 +73,27 @@ __device__ __forceinline__ void far_lane_sums(const PoseBatchSys &y, long long b
             gx = __ffma2_rn(fp, dx, gx);
             gy = __ffma2_rn(fp, dy, gy);
             gz = __ffma2_rn(fp, dz, gz);
-        }
+        };
+        auto entry = [&](int i) { return base + begin + lane + (long long)stride * i; };
+        if constexpr (LOADS == 1) {
+            for (int i = i0; i < i1; ++i) {
+                const float4 h = y.hi[entry(i)];
+                add(entry(i), h, y.tf[__float_as_int(h.w)]);   // (c12, c6, shift, floor2)
+            }
+        } else {
+            // LOADS entries in flight together (each is a chain of list, table
+            // and arithmetic latencies), summed in order
+#pragma unroll 1
+            for (int j0 = i0; j0 < i1; j0 += LOADS) {
+                float4 hv[LOADS], tv[LOADS];
+#pragma unroll
+                for (int j = 0; j < LOADS; ++j) hv[j] = y.hi[entry(min(j0 + j, i1 - 1))];
+#pragma unroll
+                for (int j = 0; j < LOADS; ++j) tv[j] = y.tf[__float_as_int(hv[j].w)];
+#pragma unroll
+                for (int j = 0; j < LOADS; ++j)
+                    if (j0 + j < i1) add(entry(j0 + j), hv[j], tv[j]);
+            }
         }
         v[0] += (double)fe.x + (double)fe.y;
         if (!MASK) shift_sum += (double)fs;
@@ -108,24 +113,13 @@ __device__ __forceinline__ void far_lane_sums(const PoseBatchSys &y, long long b
 // hardware seed + two Newton steps, within an ulp or two of it); otherwise
 // near entries in FP64 with the hardware reciprocal seed + one Newton step
 // (relative error <= 2^-46) and far entries in packed FP32.
-template <bool FAR64, bool IEEE = FAR64>
+template <bool FAR64, int LOADS, bool IEEE = FAR64>
 __device__ __forceinline__ void pose_sums(const PoseBatchSys &y, const RegionInfo &r,
                                           const double (&sd)[2][3], int lane, int stride,
                                           double (&v)[7]) {
+    constexpr int NEAR = LOADS > 1 ? LOADS / 2 : 1;
     const int end = FAR64 ? r.n_total : r.n_near;
-#pragma unroll 1
-    for (int e0 = lane; e0 < end; e0 += kPoseNearLoads * stride) {
-    float4 hv[kPoseNearLoads], lv[kPoseNearLoads];
-#pragma unroll
-    for (int j = 0; j < kPoseNearLoads; ++j) {
-        const int e = min(e0 + j * stride, end - 1);
-        hv[j] = y.hi[r.off + e];
-        lv[j] = y.lo[r.off + e];
-    }
-#pragma unroll
-    for (int j = 0; j < kPoseNearLoads; ++j) {
-        if (e0 + j * stride >= end) break;
-        const float4 h = hv[j], l = lv[j];
+    auto add = [&](const float4 &h, const float4 &l) {
         const double x = (double)h.x + (double)l.x, yy = (double)h.y + (double)l.y,
                      z = (double)h.z + (double)l.z;
         const int t = __float_as_int(h.w);
@@ -148,7 +142,23 @@ __device__ __forceinline__ void pose_sums(const PoseBatchSys &y, const RegionInf
                 v[3 + 3 * s] = fma(w, dz, v[3 + 3 * s]);
             }
         }
-    }
+    };
+    if constexpr (LOADS == 1) {
+        for (int e = lane; e < end; e += stride) add(y.hi[r.off + e], y.lo[r.off + e]);
+    } else {
+#pragma unroll 1
+        for (int e0 = lane; e0 < end; e0 += NEAR * stride) {
+            float4 hv[NEAR], lv[NEAR];
+#pragma unroll
+            for (int j = 0; j < NEAR; ++j) {
+                const int e = min(e0 + j * stride, end - 1);
+                hv[j] = y.hi[r.off + e];
+                lv[j] = y.lo[r.off + e];
+            }
+#pragma unroll
+            for (int j = 0; j < NEAR; ++j)
+                if (e0 + j * stride < end) add(hv[j], lv[j]);
+        }
     }
     if (FAR64) return;
     // far entries lie beyond r_split of every site: no contact floor
@@ -156,9 +166,9 @@ __device__ __forceinline__ void pose_sums(const PoseBatchSys &y, const RegionInf
                  nsy = make_float2(-(float)sd[0][1], -(float)sd[1][1]),
                  nsz = make_float2(-(float)sd[0][2], -(float)sd[1][2]);
     double shift_sum = 0.0;
-    far_lane_sums<false>(y, r.off, r.n_near, r.n_near + r.n_inner, lane, stride, nsx, nsy, nsz,
+    far_lane_sums<false, LOADS>(y, r.off, r.n_near, r.n_near + r.n_inner, lane, stride, nsx, nsy, nsz,
                          sd, v, shift_sum);
-    far_lane_sums<true>(y, r.off, r.n_near + r.n_inner, r.n_total, lane, stride, nsx, nsy, nsz,
+    far_lane_sums<true, LOADS>(y, r.off, r.n_near + r.n_inner, r.n_total, lane, stride, nsx, nsy, nsz,
                         sd, v, shift_sum);
     v[0] += 2.0 * shift_sum;
 }
@@ -181,7 +191,7 @@ struct PosePoint {
 // (W = 1, 2, 4, 8 consecutive warps of a 256-thread CTA share the pose; every
 // warp of the CTA calls this together and gets its pose's whole sums).  part:
 // shared memory [8][7].  MIXED = false: the FP64 mode (every entry near).
-template <bool MIXED>
+template <bool MIXED, int LOADS>
 __device__ __forceinline__ void pose_eval(const PoseBatchSys &y, const double *q,
                                           const double *center, int W, int warp, int lane,
                                           double (*part)[7], double band_lo, double band_hi,
@@ -226,7 +236,7 @@ __device__ __forceinline__ void pose_eval(const PoseBatchSys &y, const double *q
     }
 #pragma unroll
     for (int k = 0; k < 7; ++k) v[k] = 0.0;
-    pose_sums<!MIXED>(y, r, sd, lane + 32 * sub, 32 * W, v);
+    pose_sums<!MIXED, LOADS>(y, r, sd, lane + 32 * sub, 32 * W, v);
     warp_reduce7(v);
     if (W > 1) {   // (W is a launch argument: uniform over the CTA)
         if (lane == 0)
@@ -249,7 +259,7 @@ __device__ __forceinline__ void pose_eval(const PoseBatchSys &y, const double *q
         if (again) {
 #pragma unroll
             for (int k = 0; k < 7; ++k) v[k] = 0.0;
-            pose_sums<true, false>(y, r, sd, lane + 32 * sub, 32 * W, v);
+            pose_sums<true, LOADS, false>(y, r, sd, lane + 32 * sub, 32 * W, v);
             warp_reduce7(v);
         }
         if (W > 1) {   // every warp of the CTA passes both barriers

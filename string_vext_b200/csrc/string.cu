@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(256, 2) string_loop_kernel(LoopArgs g) {
         double v[7];
         // ---- energies and gradients of s0
         set_pose(s0);
-        pose_eval<MIXED>(*g.sys, pose + 3, pose, 8, warp, lane, part, g.band_lo, g.band_hi,
+        pose_eval<MIXED, 1>(*g.sys, pose + 3, pose, 8, warp, lane, part, g.band_lo, g.band_hi,
                          g.status, pt, v);
         if (tid == 0) {
             a.e0[me] = v[0];
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(256, 2) string_loop_kernel(LoopArgs g) {
         __syncthreads();
         // ---- energies of s2
         set_pose(s2);
-        pose_eval<MIXED>(*g.sys, pose + 3, pose, 8, warp, lane, part, g.band_lo, g.band_hi,
+        pose_eval<MIXED, 1>(*g.sys, pose + 3, pose, 8, warp, lane, part, g.band_lo, g.band_hi,
                          g.status, pt, v);
         if (tid == 0) a.e2[me] = v[0];
         if (!grid_barrier(g.barrier, ++bar * gridDim.x, g.status)) return;
