@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "pair.cuh"
+#include "sitepose.cuh"
 #include "taylor.cuh"
 
 namespace vext {
@@ -60,6 +61,7 @@ struct BatchSys {
                                 // device scratch when those are host memory)
     const double *poly;         // [regions][kTaylorPolyPad], or null: inner pairs are summed here
     double *out64;              // FP64 copy of the energies [O][S^3], or null
+    const SiteView *site;       // summed site by site (sites.cuh; no items), or null
 };
 
 // Refinement record flag: the pose is outside the refinement band but has a
@@ -489,6 +491,16 @@ __global__ void batch_refine_kernel(BatchArgs a) {
         const long long c = idx % S3;
         const int gi = (int)(c / ((long long)y.S * y.S)), gj = (int)((c / y.S) % y.S),
                   gk = (int)(c % y.S);
+        if (y.site) {
+            double e, g[6];
+            site_pose_fp64(*y.site, o, gi, gj, gk, lane, e, g);
+            e = warp_total(e);
+            if (lane == 0) {
+                y.out[idx] = (float)e;
+                if (y.out64) y.out64[idx] = e;
+            }
+            continue;
+        }
         const RegionInfo r = y.regs[((gi / y.bi) * y.nrj + gj / y.bj) * y.nrk + gk / y.bk];
         double cx, cy, cz;
         frac_to_cart(y.H, (gi + .5) / y.S - r.of[0], (gj + .5) / y.S - r.of[1],
@@ -549,13 +561,17 @@ __global__ void batch_refine_adj_kernel(BatchArgs a) {
         const long long c = idx % S3;
         const int gi = (int)(c / ((long long)y.S * y.S)), gj = (int)((c / y.S) % y.S),
                   gk = (int)(c % y.S);
-        const RegionInfo r = y.regs[((gi / y.bi) * y.nrj + gj / y.bj) * y.nrk + gk / y.bk];
-        double cx, cy, cz;
-        frac_to_cart(y.H, (gi + .5) / y.S - r.of[0], (gj + .5) / y.S - r.of[1],
-                     (gk + .5) / y.S - r.of[2], cx, cy, cz);
         const double u[3] = {y.axes[3 * o], y.axes[3 * o + 1], y.axes[3 * o + 2]};
-        double e = 0.0, g[6];
-        if (repair)
+        double e = 0.0, g[6], cx, cy, cz;
+        RegionInfo r;
+        if (!y.site) {
+            r = y.regs[((gi / y.bi) * y.nrj + gj / y.bj) * y.nrk + gk / y.bk];
+            frac_to_cart(y.H, (gi + .5) / y.S - r.of[0], (gj + .5) / y.S - r.of[1],
+                         (gk + .5) / y.S - r.of[2], cx, cy, cz);
+        }
+        if (y.site)
+            site_pose_fp64(*y.site, o, gi, gj, gk, lane, e, g);
+        else if (repair)
             shell_border_repair(y.hi, y.lo, y.td, r.off + r.n_near + r.n_inner,
                                 r.n_total - r.n_near - r.n_inner, lane, 32, y.rc2, y.rc2f,
                                 y.off0, y.off1, cx, cy, cz, u, e, g);
@@ -587,6 +603,51 @@ __global__ void batch_refine_adj_kernel(BatchArgs a) {
                 gd[1] = make_float2((float)g[2], (float)g[3]);
                 gd[2] = make_float2((float)g[4], (float)g[5]);
             }
+        }
+    }
+}
+
+// The poses of a system summed site by site: V (and its gradient) at both
+// sites -> energy and [dE/dc, tangent dE/du]; refinement records for the band.
+// Pairs at the cutoff were decided in FP64 already.  Bound by memory.
+template <bool ADJ>
+__global__ void __launch_bounds__(256)
+    site_pose_kernel(BatchArgs a, int k, const double *value, int plane0, int plane1) {
+    const BatchSys &y = a.sys[k];
+    const long long S2 = (long long)y.S * y.S, S3 = S2 * y.S;
+    long long c = plane0 * S2 + blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const int o = blockIdx.y;
+    if (c >= plane1 * S2) return;
+    if (c >= S3) c -= S3;   // planes from S on are the first ones
+    const long long idx = o * S3 + c, s0 = 2 * o * S3 + c, s1 = s0 + S3;
+    double e;
+    if constexpr (ADJ) {
+        const double2 *p = reinterpret_cast<const double2 *>(value + 4 * s0),
+                      *q = reinterpret_cast<const double2 *>(value + 4 * s1);
+        const double2 a0 = p[0], a1 = p[1], b0 = q[0], b1 = q[1];
+        e = a0.x + b0.x;
+        double g[6] = {a0.y + b0.y,
+                       a1.x + b1.x,
+                       a1.y + b1.y,
+                       y.off0 * a0.y + y.off1 * b0.y,
+                       y.off0 * a1.x + y.off1 * b1.x,
+                       y.off0 * a1.y + y.off1 * b1.y};
+        const double u[3] = {y.axes[3 * o], y.axes[3 * o + 1], y.axes[3 * o + 2]};
+        fp64_tangent(u, g);
+        float2 *gd = reinterpret_cast<float2 *>(y.grad + 6 * idx);
+        gd[0] = make_float2((float)g[0], (float)g[1]);
+        gd[1] = make_float2((float)g[2], (float)g[3]);
+        gd[2] = make_float2((float)g[4], (float)g[5]);
+    } else {
+        e = value[s0] + value[s1];
+    }
+    y.out[idx] = (float)e;
+    if (y.out64) y.out64[idx] = e;
+    if (e > a.band_lo && e < a.band_hi) {
+        const int n = atomicAdd(&a.refine[0], 1);
+        if (n < a.refine_cap) {
+            a.refine[1 + 2 * n] = k;
+            a.refine[2 + 2 * n] = (int)idx;
         }
     }
 }
@@ -765,6 +826,9 @@ struct vext_batch_s {
     std::vector<int> slab_items, slab_plane;   // first item and first grid plane of each slab,
                                                // then the ends (see batch_run_slab)
     int *d_slab_counts = nullptr;              // refinement records of each slab
+    std::vector<SitePlan> sites;          // systems summed site by site (rs null: by items)
+    SiteView *d_sites = nullptr;
+    SiteScratch site_scratch;
     float *d_sums = nullptr;              // expansion sums of one system at a time
     size_t sums_cap = 0;
     int4 *d_items = nullptr, *d_sample = nullptr;
@@ -798,6 +862,9 @@ struct vext_batch_s {
         device_free(d_sums);
         device_free(d_slab_counts);
         for (TaylorPlan &p : plans) p.release();
+        for (SitePlan &p : sites) p.release();
+        site_scratch.release();
+        device_free(d_sites);
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -817,17 +884,7 @@ static size_t batch_smem(int max_types, bool adj) {
            (adj ? (size_t)kGradWords * 16 * 32 * sizeof(double) : 0);
 }
 
-// expand: evaluate the local expansions into the outputs first (a whole
-// pass; the tuner's samples run without).
-static int batch_launch(vext_batch b, const BatchConfig &cfg, const int4 *items, int n_items,
-                        bool expand, cudaStream_t st) {
-    for (size_t k = 0; expand && k < b->plans.size(); ++k) {
-        if (!b->plans[k].poly) continue;
-        const System &sys = b->systems[k]->sys;
-        VEXT_TRY(taylor_enqueue(sys, *b->lists[k], b->n_axes, b->plans[k], batch_trims(b, sys),
-                                b->d_sums, &b->d_sys[k].init, nullptr, &b->d_sys[k].init_grad,
-                                st));
-    }
+static BatchArgs batch_args(vext_batch b, const int4 *items, int n_items) {
     BatchArgs a;
     a.sys = b->d_sys;
     a.items = items;
@@ -839,20 +896,56 @@ static int batch_launch(vext_batch b, const BatchConfig &cfg, const int4 *items,
     a.band_hi = b->opt.band_hi;
     a.full_refine = (b->opt.variant & kVariantFullRefine) != 0;
     a.status = b->d_status;
+    return a;
+}
+
+static int launch_refine(vext_batch b, const BatchArgs &a, cudaStream_t st) {
+    if (b->adj) batch_refine_adj_kernel<<<1184, 256, 0, st>>>(a);
+    else if (b->opt.band_hi > b->opt.band_lo) batch_refine_kernel<<<1184, 256, 0, st>>>(a);
+    VEXT_CUDA(cudaGetLastError());
+    return 0;
+}
+
+// System k site by site: the sites of region planes [region0, region1), then
+// the poses of grid planes [plane0, plane1).
+static int launch_sites(vext_batch b, size_t k, const BatchArgs &a, int region0, int region1,
+                        int plane0, int plane1, cudaStream_t st) {
+    VEXT_TRY(site_enqueue(b->systems[k]->sys, b->sites[k], b->adj, b->site_scratch, region0,
+                          region1, st));
+    if (plane1 <= plane0) return 0;
+    const long long n = (long long)(plane1 - plane0) * b->size * b->size;
+    const dim3 grid((unsigned)((n + 255) / 256), b->n_axes);
+    const double *value = b->site_scratch.value;
+    if (b->adj) site_pose_kernel<true><<<grid, 256, 0, st>>>(a, (int)k, value, plane0, plane1);
+    else site_pose_kernel<false><<<grid, 256, 0, st>>>(a, (int)k, value, plane0, plane1);
+    VEXT_CUDA(cudaGetLastError());
+    return 0;
+}
+
+// expand: a whole pass (systems summed site by site, and the local expansions
+// into the outputs first); the tuner's samples run without.
+static int batch_launch(vext_batch b, const BatchConfig &cfg, const int4 *items, int n_items,
+                        bool expand, cudaStream_t st) {
+    for (size_t k = 0; expand && k < b->plans.size(); ++k) {
+        if (!b->plans[k].poly) continue;
+        const System &sys = b->systems[k]->sys;
+        VEXT_TRY(taylor_enqueue(sys, *b->lists[k], b->n_axes, b->plans[k], batch_trims(b, sys),
+                                b->d_sums, &b->d_sys[k].init, nullptr, &b->d_sys[k].init_grad,
+                                st));
+    }
+    const BatchArgs a = batch_args(b, items, n_items);
     const size_t smem = batch_smem(b->max_types, b->adj);
     VEXT_CUDA(cudaMemsetAsync(b->d_counter, 0, sizeof(int), st));
     VEXT_CUDA(cudaMemsetAsync(b->d_refine, 0, sizeof(int), st));
-    const BatchKernel &k = batch_kernel(b->kind, cfg.shape);
-    (b->d_sums ? k.fn_expand : k.fn)<<<cfg.grid, k.threads, smem, st>>>(a);
-    VEXT_CUDA(cudaGetLastError());
-    if (b->adj) {
-        batch_refine_adj_kernel<<<1184, 256, 0, st>>>(a);
-        VEXT_CUDA(cudaGetLastError());
-    } else if (b->opt.band_hi > b->opt.band_lo) {
-        batch_refine_kernel<<<1184, 256, 0, st>>>(a);
+    for (size_t k = 0; expand && k < b->sites.size(); ++k)
+        if (b->sites[k].rs)
+            VEXT_TRY(launch_sites(b, k, a, 0, b->sites[k].rs->n_ri, 0, b->size, st));
+    if (n_items) {
+        const BatchKernel &k = batch_kernel(b->kind, cfg.shape);
+        (b->d_sums ? k.fn_expand : k.fn)<<<cfg.grid, k.threads, smem, st>>>(a);
         VEXT_CUDA(cudaGetLastError());
     }
-    return 0;
+    return launch_refine(b, a, st);
 }
 
 namespace vext {
@@ -945,6 +1038,13 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
             }
         }
     }
+    // systems summed site by site (all members of a framework, or none)
+    std::vector<char> by_site(n_systems, 1);
+    for (int k = 0; k < n_systems; ++k)
+        if (!sites_worthwhile(systems[k]->sys, size, rule_axes ? rule_axes : n_axes,
+                                           b->opt, b->adj))
+            by_site[owner[k]] = 0;
+    for (int k = 0; k < n_systems; ++k) by_site[k] = by_site[owner[k]];
     std::vector<RegionSet *> lists(n_systems, nullptr);
     for (int k = 0; k < n_systems; ++k) {
         if (owner[k] != k) continue;
@@ -953,13 +1053,16 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
             return fail(VEXT_ERR_ARGUMENT, "system %d lives on another device", k);
         std::unique_lock<std::mutex> lock(sys->lock, std::defer_lock);
         if (lock_systems) lock.lock();
-        VEXT_TRY(get_field_regions(sys, size, cb, b->opt.r_split, &lists[k], sys->stream));
+        VEXT_TRY(by_site[k]
+                     ? get_site_regions(sys, size, kBatchVoxels, b->opt.r_split, &lists[k],
+                                        sys->stream)
+                     : get_field_regions(sys, size, cb, b->opt.r_split, &lists[k], sys->stream));
         b->list_bytes += lists[k]->n_entries * 32;
     }
     {
         size_t n = 0;
         for (int k = 0; k < n_systems; ++k)
-            n += (size_t)lists[owner[k]]->n_regions * ((n_axes + kOB - 1) / kOB);
+            if (!by_site[k]) n += (size_t)lists[owner[k]]->n_regions * ((n_axes + kOB - 1) / kOB);
         items.reserve(n);
     }
     for (int k = 0; k < n_systems; ++k) {
@@ -1000,10 +1103,11 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
         y.init_grad = init ? init[1] : y.grad;
         y.poly = nullptr;
         y.out64 = outputs_f64 ? outputs_f64[k] : nullptr;
+        y.site = nullptr;
         b->max_types = std::max(b->max_types, sys->n_types);
         b->poses += S3 * n_axes;
         const int n_ob = (n_axes + kOB - 1) / kOB;
-        for (int ri = 0; ri < rs->n_regions; ++ri)
+        for (int ri = 0; !by_site[k] && ri < rs->n_regions; ++ri)
             for (int ob = 0; ob < n_ob; ++ob)
                 items.push_back({(long long)rs->h_info[ri].n_total, make_int4(k, ri, ob, 0)});
     }
@@ -1020,18 +1124,20 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
     if (slabs > 1) {
         // slab by slab (region planes along the slowest axis), longest first in each
         const RegionSet &rs = *lists[owner[0]];
+        b->slab_items.assign(slabs + 1, 0);
+        b->slab_plane.assign(slabs + 1, 0);
+        // first region plane I with I * slabs / n_ri > k
+        auto slab_end = [&](int k) {
+            return (int)(((long long)(k + 1) * rs.n_ri + slabs - 1) / slabs);
+        };
         const int per = rs.n_rj * rs.n_rk;
         auto slab_of = [&](const int4 &it) { return (int)((long long)(it.y / per) * slabs / rs.n_ri); };
         std::stable_sort(hitems.begin(), hitems.end(),
                          [&](const int4 &x, const int4 &y) { return slab_of(x) < slab_of(y); });
-        b->slab_items.assign(slabs + 1, 0);
-        b->slab_plane.assign(slabs + 1, 0);
         for (const int4 &it : hitems) ++b->slab_items[slab_of(it) + 1];
         for (int k = 0; k < slabs; ++k) {
-            b->slab_items[k + 1] += b->slab_items[k];
-            // first region plane I with I * slabs / n_ri > k
-            const int end = (int)(((long long)(k + 1) * rs.n_ri + slabs - 1) / slabs);
-            b->slab_plane[k + 1] = std::min(size, end * rs.bi);
+            b->slab_items[k + 1] = by_site[0] ? slab_end(k) : b->slab_items[k] + b->slab_items[k + 1];
+            b->slab_plane[k + 1] = std::min(size, slab_end(k) * rs.bi);
         }
         VEXT_CUDA(device_malloc(&b->d_slab_counts, sizeof(int) * slabs));
     }
@@ -1072,20 +1178,44 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
         b->lists.push_back(lists[owner[k]]);
         const System &sys = systems[k]->sys;
         const RegionSet &rs = *b->lists[k];
-        if (!expands || !taylor_worthwhile(sys, rs, rule_axes ? rule_axes : n_axes, b->adj) ||
+        if (by_site[k] || !expands || !taylor_worthwhile(sys, rs, rule_axes ? rule_axes : n_axes, b->adj) ||
             !device_memory(hs[k].init) || (b->adj && !device_memory(hs[k].init_grad)))
             continue;
         VEXT_TRY(taylor_prepare(sys, rs, n_axes, b->d_axes, b->adj, b->plans[k], b->stream));
         VEXT_TRY(ensure_capacity(b->d_sums, b->sums_cap, taylor_workspace(rs)));
         hs[k].poly = b->plans[k].poly;
     }
+    b->sites.resize(n_systems);
+    std::vector<SiteView> views(n_systems);
+    for (int k = 0; k < n_systems; ++k) {
+        if (!by_site[k]) continue;
+        if (!b->d_sites) VEXT_CUDA(device_malloc(&b->d_sites, sizeof(SiteView) * n_systems));
+        VEXT_TRY(site_plan_build(systems[k]->sys, *b->lists[k], n_axes, axes, b->d_axes, b->adj,
+                                 b->sites[k], b->stream));
+        VEXT_TRY(site_scratch_reserve(b->sites[k], b->adj, b->site_scratch));
+        views[k] = b->sites[k].view;
+        hs[k].site = b->d_sites + k;
+    }
+    if (slabs > 1 && by_site[0]) {
+        // a pose is final once both its sites are: with the regions of voxel
+        // planes [0, V) done, those of planes [reach_lo, V - reach_hi); the
+        // last slab goes on to the first planes (counted from `size` on)
+        const SitePlan &p = b->sites[0];
+        const int first = std::min(p.reach_lo, size);
+        for (int &v : b->slab_plane) v = std::max(first, v - p.reach_hi);
+        b->slab_plane[0] = first;
+        b->slab_plane[slabs] = size + first;
+    }
+    if (b->d_sites)
+        VEXT_CUDA(cudaMemcpy(b->d_sites, views.data(), sizeof(SiteView) * n_systems,
+                             cudaMemcpyHostToDevice));
     for (const BatchSys &y : hs) b->targets.push_back({y.out, y.grad, y.init, y.init_grad});
     VEXT_CUDA(device_malloc(&b->d_sys, sizeof(BatchSys) * n_systems));
     VEXT_CUDA(cudaMemcpy(b->d_sys, hs.data(), sizeof(BatchSys) * n_systems, cudaMemcpyHostToDevice));
-    VEXT_CUDA(device_malloc(&b->d_items, sizeof(int4) * hitems.size()));
+    VEXT_CUDA(device_malloc(&b->d_items, sizeof(int4) * std::max<size_t>(hitems.size(), 1)));
     VEXT_CUDA(cudaMemcpy(b->d_items, hitems.data(), sizeof(int4) * hitems.size(),
                          cudaMemcpyHostToDevice));
-    VEXT_CUDA(device_malloc(&b->d_sample, sizeof(int4) * sample.size()));
+    VEXT_CUDA(device_malloc(&b->d_sample, sizeof(int4) * std::max<size_t>(sample.size(), 1)));
     VEXT_CUDA(cudaMemcpy(b->d_sample, sample.data(), sizeof(int4) * sample.size(),
                          cudaMemcpyHostToDevice));
     VEXT_CUDA(device_malloc(&b->d_counter, sizeof(int)));
@@ -1136,6 +1266,11 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
                     cached = true;
                 }
         }
+    }
+    if (!n_all) {
+        b->config = cands[0];   // nothing queued
+        b->n_cands = 1;
+        cached = true;
     }
     if (!cached) {
         cudaEvent_t e0, e1;
@@ -1219,13 +1354,20 @@ int batch_replay(vext_batch b, cudaStream_t stream) {
 }
 
 // Run slab k (of a batch built with slabs > 1) on `stream`, slabs in order: the
-// poses of grid planes [*plane0, *plane1) along the slowest axis are final
-// once it is done, so a caller can copy them while the next slab runs.
+// poses of grid planes [*plane0, *plane1) along the slowest axis (those from
+// `size` on are the first ones) are final once it is done, so a caller can copy them while the next slab runs.
 int batch_run_slab(vext_batch b, int k, cudaStream_t stream, int *plane0, int *plane1) {
     const int first = b->slab_items[k], n = b->slab_items[k + 1] - first;
     *plane0 = b->slab_plane[k];
     *plane1 = b->slab_plane[k + 1];
-    VEXT_TRY(batch_launch(b, b->config, b->d_items + first, n, k == 0, stream));
+    if (b->sites[0].rs) {
+        const BatchArgs a = batch_args(b, nullptr, 0);
+        VEXT_CUDA(cudaMemsetAsync(b->d_refine, 0, sizeof(int), stream));
+        VEXT_TRY(launch_sites(b, 0, a, first, first + n, *plane0, *plane1, stream));
+        VEXT_TRY(launch_refine(b, a, stream));
+    } else {
+        VEXT_TRY(batch_launch(b, b->config, b->d_items + first, n, k == 0, stream));
+    }
     VEXT_CUDA(cudaMemcpyAsync(b->d_slab_counts + k, b->d_refine, sizeof(int),
                               cudaMemcpyDeviceToDevice, stream));
     return 0;
@@ -1308,7 +1450,8 @@ extern "C" int vext_batch_tuning(vext_batch b, int max_candidates, int *n_candid
         if (shapes) shapes[c] = b->cands[c].shape;
         if (grids) grids[c] = b->cands[c].grid;
         if (ms) ms[c] = b->tune_ms[c];
-        if (names) names[c] = batch_kernel(b->kind, b->cands[c].shape).name;
+        if (names) names[c] = b->n_items ? batch_kernel(b->kind, b->cands[c].shape).name
+                                     : "64-site clusters";
     }
     return 0;
 }
@@ -1316,7 +1459,11 @@ extern "C" int vext_batch_tuning(vext_batch b, int max_candidates, int *n_candid
 extern "C" int vext_batch_info(vext_batch b, int64_t *work_items, int64_t *poses,
                                int64_t *list_bytes, int *shape, int *grid) {
     if (!b) return fail(VEXT_ERR_ARGUMENT, "null batch");
-    if (work_items) *work_items = b->n_items;
+    if (work_items) {
+        *work_items = b->n_items;
+        for (const SitePlan &p : b->sites)
+            if (p.rs) *work_items += (int64_t)p.view.n_regions * p.view.n_clusters;
+    }
     if (poses) *poses = b->poses;
     if (list_bytes) *list_bytes = b->list_bytes;
     if (shape) *shape = b->config.shape;

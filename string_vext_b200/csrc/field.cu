@@ -20,6 +20,7 @@
 #include <cuda.h>
 
 #include "pair.cuh"
+#include "sitepose.cuh"
 #include "taylor.cuh"
 
 namespace vext {
@@ -338,6 +339,24 @@ __global__ void refine_kernel(FieldArgs a, const int *list) {
         e += site_sum_fp64(a, r, cx + a.off1 * ux, cy + a.off1 * uy, cz + a.off1 * uz, lane);
         e = warp_sum(e);
         if (lane == 0) a.e64[idx] = e;
+    }
+}
+
+// refine_kernel on the lists of the site-by-site sum.
+__global__ void refine_sites_kernel(SiteView v, const int *list, double *e64) {
+    const int lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const int count = list[0];
+    const long long S3 = (long long)v.S * v.S * v.S;
+    for (int q = warp; q < count; q += nwarps) {
+        const long long idx = list[1 + q];
+        const long long c = idx % S3;
+        double e, g[6];
+        site_pose_fp64(v, (int)(idx / S3), (int)(c / ((long long)v.S * v.S)),
+                       (int)((c / v.S) % v.S), (int)(c % v.S), lane, e, g);
+        e = warp_sum(e);
+        if (lane == 0) e64[idx] = e;
     }
 }
 
@@ -743,6 +762,24 @@ int launch_field(System *sys, const RegionSet *rs, int n_axes, const double *axe
                   : launch_far<false>(a, cb, variant, stream);
 }
 
+// The site-by-site sum into e64 (sites.cuh), its plan kept for the last
+// (lists, directors).
+static int launch_sites(System *sys, const RegionSet *rs, int n_axes, const double *axes_host,
+                        const double *d_axes, double *d_e64, cudaStream_t stream) {
+    if (!sys->site_field) sys->site_field = new SiteField();
+    SiteField &f = *sys->site_field;
+    sys->split_timed = false;
+    if (f.plan.rs != rs || f.axes.size() != 3 * (size_t)n_axes ||
+        !std::equal(axes_host, axes_host + 3 * n_axes, f.axes.begin())) {
+        f.plan.rs = nullptr;
+        VEXT_TRY(site_plan_build(*sys, *rs, n_axes, axes_host, d_axes, false, f.plan, stream));
+        f.axes.assign(axes_host, axes_host + 3 * n_axes);
+    }
+    VEXT_TRY(site_scratch_reserve(f.plan, false, f.scratch));
+    VEXT_TRY(site_enqueue(*sys, f.plan, false, f.scratch, 0, rs->n_ri, stream));
+    return site_energies(f.plan, f.scratch, d_e64, stream);
+}
+
 // Everything on device pointers and `stream`; region lists are built (with
 // a host synchronisation) on first use of (size, shape, r_split).
 static int field_device(System *sys, int size, int n_axes, const double *axes_host,
@@ -765,8 +802,10 @@ static int field_device(System *sys, int size, int n_axes, const double *axes_ho
     // 8-center regions for 5 % less pair work, so 16 stays the default here
     const int cb = o.cb == 32 ? 32 : o.cb == 8 && !fp64 ? 8 : 16;
     const double r_split = fp64 ? 1e30 : o.r_split;
+    const bool by_site = sites_worthwhile(*sys, size, n_axes, o, false);
     RegionSet *rs = nullptr;
-    VEXT_TRY(get_field_regions(sys, size, cb, r_split, &rs, stream));
+    VEXT_TRY(by_site ? get_site_regions(sys, size, kFieldVoxels, r_split, &rs, stream)
+                     : get_field_regions(sys, size, cb, r_split, &rs, stream));
     const size_t n = (size_t)S3 * n_axes;
     VEXT_TRY(ensure_capacity(sys->d_axes, sys->axes_cap, 3 * (size_t)n_axes));
     VEXT_TRY(ensure_capacity(sys->d_e64, sys->e64_cap, n));
@@ -778,7 +817,10 @@ static int field_device(System *sys, int size, int n_axes, const double *axes_ho
     VEXT_CUDA(cudaMemsetAsync(sys->d_refine, 0, sizeof(int), stream));
     const FieldArgs a = make_args(sys, rs, n_axes, sys->d_axes, sys->d_e64);
     VEXT_CUDA(cudaEventRecord(sys->ev[0], stream));
-    VEXT_TRY(launch_field(sys, rs, n_axes, axes_host, sys->d_axes, sys->d_e64, cb,
+    if (by_site)
+        VEXT_TRY(launch_sites(sys, rs, n_axes, axes_host, sys->d_axes, sys->d_e64, stream));
+    else
+        VEXT_TRY(launch_field(sys, rs, n_axes, axes_host, sys->d_axes, sys->d_e64, cb,
                           o.mode == VEXT_MODE_FP64_PLAIN   ? kPlainVariant
                           : o.mode == VEXT_MODE_FP32_NAIVE ? kNaiveVariant
                                                            : o.variant,
@@ -788,12 +830,17 @@ static int field_device(System *sys, int size, int n_axes, const double *axes_ho
         flag_kernel<<<592, 256, 0, stream>>>(sys->d_e64, (long long)n, o.band_lo, o.band_hi,
                                               sys->d_refine);
         VEXT_CUDA(cudaGetLastError());
-        refine_kernel<<<1184, 256, 0, stream>>>(a, sys->d_refine);
+        if (by_site)
+            refine_sites_kernel<<<1184, 256, 0, stream>>>(site_view(sys->site_field->plan),
+                                                          sys->d_refine, sys->d_e64);
+        else
+            refine_kernel<<<1184, 256, 0, stream>>>(a, sys->d_refine);
         VEXT_CUDA(cudaGetLastError());
     }
     if (d_site) {
-        if (cb == 8) site_kernel<8><<<rs->n_regions, 128, 0, stream>>>(a, d_site);
-        else if (cb == 16) site_kernel<16><<<rs->n_regions, 128, 0, stream>>>(a, d_site);
+        const int per = rs->bi * rs->bj * rs->bk;   // centers of a region
+        if (per <= 8) site_kernel<8><<<rs->n_regions, 128, 0, stream>>>(a, d_site);
+        else if (per <= 16) site_kernel<16><<<rs->n_regions, 128, 0, stream>>>(a, d_site);
         else site_kernel<32><<<rs->n_regions, 128, 0, stream>>>(a, d_site);
         VEXT_CUDA(cudaGetLastError());
     }
@@ -1074,9 +1121,13 @@ static int adjoint_pinned(vext_system h, int size, int n_axes, const double *axe
             VEXT_TRY(batch_run_slab(sys->slab_batch, k, st, &p0, &p1));
             VEXT_CUDA(cudaEventRecord(sys->ev[5], st));
             VEXT_CUDA(cudaStreamWaitEvent(sys->aux, sys->ev[5], 0));
-            if (p1 <= p0) continue;
-            VEXT_CUDA(copy_rows(energy, sys->d_f32, 1, p0, p1));
-            VEXT_CUDA(copy_rows(gradient, sys->d_g32, 6, p0, p1));
+            // [p0, p1), the planes from `size` on are the first ones
+            const int range[2][2] = {{p0, std::min(p1, size)}, {0, p1 - size}};
+            for (const auto &r : range) {
+                if (r[1] <= r[0]) continue;
+                VEXT_CUDA(copy_rows(energy, sys->d_f32, 1, r[0], r[1]));
+                VEXT_CUDA(copy_rows(gradient, sys->d_g32, 6, r[0], r[1]));
+            }
         }
         return 0;
     };
@@ -1119,7 +1170,12 @@ extern "C" int vext_field_adjoint(vext_system h, int size, int n_axes, const dou
         for (int k = 0; k < 3 * n_axes; ++k)
             if (!std::isfinite(axes[k])) return fail(VEXT_ERR_ARGUMENT, "non-finite director");
         const size_t S3 = (size_t)size * size * size;
-        const int blk = batch_item_directors(o, true), parts = (n_axes + blk - 1) / blk;
+        // (one batch when poses are summed site by site: a cluster of sites
+        // takes all directors)
+        const int blk = sites_worthwhile(*sys, size, n_axes, o, true)
+                            ? n_axes
+                            : batch_item_directors(o, true),
+                  parts = (n_axes + blk - 1) / blk;
         const bool same = (int)sys->host_parts.size() == parts && sys->host_size == size &&
                           sys->host_axes.size() == 3 * (size_t)n_axes &&
                           std::equal(axes, axes + 3 * n_axes, sys->host_axes.begin()) &&

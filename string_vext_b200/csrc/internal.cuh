@@ -72,6 +72,7 @@ struct RegionSet {
     int nb[3] = {0, 0, 0};                  // bins per axis (pose regions)
     double bin_width = 0;                   // target bin width (A, pose regions)
     double r_split = 0;
+    bool sites = false;                     // regions of voxels: lists about single sites
     // data
     int n_regions = 0;
     int n_ri = 0, n_rj = 0, n_rk = 0;       // regions per axis
@@ -119,6 +120,9 @@ struct PoseBatchSys {
     const float4 *tf;
 };
 
+struct SiteField;
+void site_field_free(SiteField *f);
+
 struct System {
     int device = 0;
     Mat3 H, Hinv;
@@ -162,6 +166,8 @@ struct System {
     std::vector<double> field_plan_axes;
     float *d_sums = nullptr;
     size_t sums_cap = 0;
+    // site-by-site sums of the field path (sites.cuh)
+    SiteField *site_field = nullptr;
     // scratch of the pose path
     void *d_pose_scratch = nullptr;
     size_t pose_scratch_cap = 0;
@@ -222,6 +228,8 @@ int batch_retarget(vext_batch b, int k, float *out, float *grad, float *init, fl
 // Region sets (system.cu)
 int get_field_regions(System *sys, int size, int cb, double r_split, RegionSet **out,
                       cudaStream_t stream);
+int get_block_regions(System *sys, int size, int bi, int bj, int bk, double rho, double offset,
+                      bool sites, double r_split, RegionSet **out, cudaStream_t stream);
 constexpr double kBinWidth = 0.75;  // pose-bin width between lattice planes (A)
 int get_bin_regions(System *sys, double r_split, RegionSet **out, cudaStream_t stream,
                     double bin_width = kBinWidth);

@@ -351,16 +351,17 @@ static int build_lists(System *sys, RegionSet *rs, cudaStream_t stream) {
     a.n_atoms = sys->n_atoms;
     // 1e-6 A margins keep every pair within rc (resp. r_split) listed despite
     // FP64 rounding of the distances (~1e-14 A).
-    a.r_list0 = sys->cutoff + sys->max_offset + 1e-6;
-    a.r_near0 = rs->r_split + sys->max_offset + 1e-6;
-    a.r_inner0 = sys->cutoff - sys->max_offset - 1e-6;
+    const double offset = rs->sites ? 0.0 : sys->max_offset;
+    a.r_list0 = sys->cutoff + offset + 1e-6;
+    a.r_near0 = rs->r_split + offset + 1e-6;
+    a.r_inner0 = sys->cutoff - offset - 1e-6;
     a.r_outer0 = sys->cutoff + 1e-3;
     // field lists set the entries of the local expansion apart, and those near
     // shell entries whose nearer site is always inside: |d0|^2 + o^2 < rc^2
     // for every center (|d0| the entry's distance from it)
     a.r_taylor = rs->d_taylor;
     const double ra2 = sys->cutoff * sys->cutoff - sys->max_offset * sys->max_offset;
-    a.r_shella0 = rs->d_taylor < sys->cutoff && ra2 > 0 ? std::sqrt(ra2) - 1e-3 : 0.0;
+    a.r_shella0 = rs->d_taylor < sys->cutoff && ra2 > 0 && !rs->sites ? std::sqrt(ra2) - 1e-3 : 0.0;
     const int n = rs->n_regions;
     if (!rs->d_info) VEXT_CUDA(device_malloc(&rs->d_info, sizeof(RegionInfo) * n));
     VEXT_CUDA(cudaMemcpyAsync(rs->d_info, rs->h_info.data(), sizeof(RegionInfo) * n,
@@ -434,8 +435,20 @@ static double det3(const Mat3 &m) {
 
 int get_field_regions(System *sys, int size, int cb, double r_split, RegionSet **out,
                       cudaStream_t stream) {
+    int bi, bj, bk;
+    choose_block_shape(sys->H, size, cb, bi, bj, bk);
+    const double rho = block_radius(sys->H, size, bi, bj, bk) + 1e-9;
+    return get_block_regions(sys, size, bi, bj, bk, rho, sys->max_offset, false, r_split, out,
+                             stream);
+}
+
+// Lists of blocks of bi x bj x bk grid centers (sites: voxels) for sites within
+// rho + offset of a block's middle.
+int get_block_regions(System *sys, int size, int bi, int bj, int bk, double rho, double offset,
+                      bool sites, double r_split, RegionSet **out, cudaStream_t stream) {
     for (RegionSet *rs : sys->sets)
-        if (rs->size == size && rs->bi * rs->bj * rs->bk == cb && rs->r_split == r_split) {
+        if (rs->size == size && rs->bi == bi && rs->bj == bj && rs->bk == bk &&
+            rs->sites == sites && rs->r_split == r_split) {
             if (rs->stale) {
                 for (auto &r : rs->h_info)
                     r.n_near = r.n_total = r.n_inner = r.n_outer = r.n_mid = r.n_shella = 0;
@@ -447,13 +460,15 @@ int get_field_regions(System *sys, int size, int cb, double r_split, RegionSet *
     RegionSet *rs = new RegionSet();
     rs->size = size;
     rs->r_split = r_split;
-    choose_block_shape(sys->H, size, cb, rs->bi, rs->bj, rs->bk);
+    rs->sites = sites;
+    rs->bi = bi;
+    rs->bj = bj;
+    rs->bk = bk;
     rs->n_ri = (size + rs->bi - 1) / rs->bi;
     rs->n_rj = (size + rs->bj - 1) / rs->bj;
     rs->n_rk = (size + rs->bk - 1) / rs->bk;
     rs->n_regions = rs->n_ri * rs->n_rj * rs->n_rk;
     rs->h_info.resize(rs->n_regions);
-    const double rho = block_radius(sys->H, size, rs->bi, rs->bj, rs->bk) + 1e-9;
     int idx = 0;
     for (int I = 0; I < rs->n_ri; ++I)
         for (int J = 0; J < rs->n_rj; ++J)
@@ -475,7 +490,7 @@ int get_field_regions(System *sys, int size, int cb, double r_split, RegionSet *
                 r.rho = rho;
             }
     if (r_split < 1e29) {
-        rs->taylor_radius = sys->max_offset + rho;
+        rs->taylor_radius = offset + rho;
         const double start = std::max(taylor_start(*sys, rs->taylor_radius),
                                       r_split + rs->taylor_radius);
         const double inner = sys->cutoff - rs->taylor_radius;
@@ -587,6 +602,7 @@ System::~System() {
     for (RegionSet *rs : sets) delete rs;
     device_free(d_g32);
     field_plan.release();
+    site_field_free(site_field);
     device_free(d_sums);
     device_free(d_base);
     device_free(d_e64);

@@ -292,7 +292,8 @@ struct MatrixArgs {
     int poses, rows;         // poses of a region, padded row length
     const double *axes;
     double off0, off1, inv_r;
-    int outs;                // 1 (energy) or 7
+    int outs;                // 1 (energy) or 7; sites: 1 or 4
+    const double *sites;     // [poses][3]: single sites instead of poses
     float *matrix;
 };
 
@@ -341,6 +342,20 @@ __global__ void __launch_bounds__(128) taylor_matrix_kernel(MatrixArgs a, SumInd
     const int pose = blockIdx.x * blockDim.x + threadIdx.x;
     if (pose >= a.poses) return;
     const uchar4 w = index.at[blockIdx.y];
+    float *row = a.matrix + (size_t)blockIdx.y * a.rows;
+    if (a.sites) {
+        double v, g[3];
+        const double *p = a.sites + 3 * pose;
+        solid_term(w.x, w.y, w.z, w.w, p[0] * a.inv_r, p[1] * a.inv_r, p[2] * a.inv_r, v, g);
+        if (a.outs == 1) {
+            row[pose] = (float)v;
+            return;
+        }
+        row[(pose >> 1) * 8 + (pose & 1)] = (float)v;
+        for (int k = 0; k < 3; ++k)
+            row[(pose >> 1) * 8 + 2 + 2 * k + (pose & 1)] = (float)(g[k] * a.inv_r);
+        return;
+    }
     const int cb = a.bi * a.bj * a.bk, o = pose / cb, c = pose % cb;
     const int ck = c % a.bk, cj = (c / a.bk) % a.bj, ci = c / (a.bk * a.bj);
     double cx, cy, cz;
@@ -359,7 +374,6 @@ __global__ void __launch_bounds__(128) taylor_matrix_kernel(MatrixArgs a, SumInd
             out[4 + k] += off * g[k] * a.inv_r;
         }
     }
-    float *row = a.matrix + (size_t)blockIdx.y * a.rows;
     if (a.outs == 1) {
         row[pose] = (float)out[0];
         return;
@@ -380,10 +394,11 @@ struct EvalArgs {
     float *const *e32;       // device words holding the output pointers
     float *const *g32;
     double *e64;
+    float *site_out;         // single sites: [n_regions][poses] x OUTS
 };
 
 constexpr int kEvalK = 16;
-__host__ __device__ constexpr int eval_rows(int outs) { return outs == 1 ? 16 : 14; }   // per thread
+__host__ __device__ constexpr int eval_rows(int outs) { return outs == 7 ? 14 : 16; }   // per thread
 __host__ __device__ constexpr int eval_tile(int outs) { return 16 * eval_rows(outs); }
 
 // Tile: eval_tile rows (32 poses x 7 outputs, or 256 poses) x NT / 16 CT
@@ -392,7 +407,9 @@ __host__ __device__ constexpr int eval_tile(int outs) { return 16 * eval_rows(ou
 // 1.99 ms as 128 threads x 8 regions (256 x 4: 2.12; 6 regions at 3 CTAs/SM:
 // 2.09; unpacked FMA: 2.07); 14,400 regions of 16 centers, energy alone: 0.46
 // ms as 256 x 4 (128 x 8: 0.53).
-template <int OUTS, int NT, int CT>
+// SITES: single sites (sites.cuh) instead of poses, OUTS 1 or 4 (value and
+// gradient).
+template <int OUTS, int NT, int CT, bool SITES = false>
 __global__ void __launch_bounds__(NT, 2) taylor_eval_kernel(EvalArgs a) {
     constexpr int RT = eval_rows(OUTS), RP = RT / 2, TILE = eval_tile(OUTS);
     constexpr int COLS = NT / 16 * CT;   // regions per tile
@@ -477,6 +494,31 @@ __global__ void __launch_bounds__(NT, 2) taylor_eval_kernel(EvalArgs a) {
                     acc[i][j] = __ffma2_rn(m[k & 1][i], v[k & 1][j], acc[i][j]);
         }
         if (more) store_s(buf ^ 1);
+    }
+    if constexpr (SITES) {
+#pragma unroll
+        for (int j = 0; j < CT; ++j) {
+            const int reg = reg0 + NT / 8 * (j >> 1) + 2 * cg + (j & 1);
+            if (reg >= a.n_regions) continue;
+            const int first = (row0 + rg * RT) / OUTS;   // this thread's RT / OUTS sites
+            if (first >= a.poses) continue;
+            float4 *out = reinterpret_cast<float4 *>(a.site_out +
+                                                     ((size_t)reg * a.poses + first) * OUTS);
+#pragma unroll
+            for (int q = 0; q < RT / 4; ++q) {
+                if (OUTS == 1)
+                    out[q] = make_float4(acc[2 * q][j].x, acc[2 * q][j].y, acc[2 * q + 1][j].x,
+                                         acc[2 * q + 1][j].y);
+                else {
+                    const int p = q / 2 * 4;
+                    out[q] = q & 1 ? make_float4(acc[p][j].y, acc[p + 1][j].y, acc[p + 2][j].y,
+                                                 acc[p + 3][j].y)
+                                   : make_float4(acc[p][j].x, acc[p + 1][j].x, acc[p + 2][j].x,
+                                                 acc[p + 3][j].x);
+                }
+            }
+        }
+        return;
     }
     const int cb = a.bi * a.bj * a.bk;
     const long long S3 = (long long)a.S * a.S * a.S;
@@ -563,10 +605,14 @@ double taylor_start(const System &sys, double radius) {
     return hi;
 }
 
-bool taylor_worthwhile(const System &sys, const RegionSet &rs, int n_axes, bool adjoint) {
+bool taylor_allowed(const System &sys, const RegionSet &rs) {
     if (!(rs.d_taylor < sys.cutoff) || rs.n_regions < 1) return false;
     // another guest of the same framework on shared lists: its own bound
-    if (worst_truncation(sys, rs.taylor_radius, rs.d_taylor) > 1.05 * kTruncation) return false;
+    return worst_truncation(sys, rs.taylor_radius, rs.d_taylor) <= 1.05 * kTruncation;
+}
+
+bool taylor_worthwhile(const System &sys, const RegionSet &rs, int n_axes, bool adjoint) {
+    if (!taylor_allowed(sys, rs)) return false;
     const double n = (double)rs.n_taylor / rs.n_regions;
     const double poses = (double)n_axes * rs.bi * rs.bj * rs.bk;
     const double direct = n * poses * 2.0 * (adjoint ? 19.0 : 9.3);
@@ -574,11 +620,9 @@ bool taylor_worthwhile(const System &sys, const RegionSet &rs, int n_axes, bool 
     return direct > taylor;
 }
 
-int taylor_prepare(const System &sys, const RegionSet &rs, int n_axes, const double *d_axes,
-                   bool adjoint, TaylorPlan &plan, cudaStream_t stream) {
-    const int outs = adjoint ? 7 : 1;
-    const int poses = n_axes * rs.bi * rs.bj * rs.bk;
-    const int rows_used = adjoint ? (poses + 1) / 2 * 14 : poses;
+static int prepare(const System &sys, const RegionSet &rs, int poses, const double *d_axes,
+                   const double *d_sites, int outs, TaylorPlan &plan, cudaStream_t stream) {
+    const int rows_used = outs == 1 ? poses : (poses + 1) / 2 * 2 * outs;
     const int tile = eval_tile(outs);
     const int rows = (rows_used + tile - 1) / tile * tile;
     VEXT_TRY(ensure_capacity(plan.matrix, plan.matrix_cap, (size_t)kTaylorPad * rows));
@@ -599,6 +643,7 @@ int taylor_prepare(const System &sys, const RegionSet &rs, int n_axes, const dou
     a.off1 = sys.offsets[1];
     a.inv_r = 1.0 / rs.taylor_radius;
     a.outs = outs;
+    a.sites = d_sites;
     a.matrix = plan.matrix;
     taylor_matrix_kernel<<<dim3((poses + 127) / 128, kTaylorSums), 128, 0, stream>>>(a,
                                                                                    sum_index());
@@ -606,9 +651,20 @@ int taylor_prepare(const System &sys, const RegionSet &rs, int n_axes, const dou
     return 0;
 }
 
-int taylor_enqueue(const System &sys, const RegionSet &rs, int n_axes, const TaylorPlan &plan,
-                   bool symmetric, float *sums, float *const *e32, double *e64,
-                   float *const *g32, cudaStream_t stream) {
+int taylor_prepare(const System &sys, const RegionSet &rs, int n_axes, const double *d_axes,
+                   bool adjoint, TaylorPlan &plan, cudaStream_t stream) {
+    return prepare(sys, rs, n_axes * rs.bi * rs.bj * rs.bk, d_axes, nullptr, adjoint ? 7 : 1, plan,
+                   stream);
+}
+
+int taylor_prepare_sites(const System &sys, const RegionSet &rs, int n_sites,
+                         const double *d_sites, bool adjoint, TaylorPlan &plan,
+                         cudaStream_t stream) {
+    return prepare(sys, rs, n_sites, nullptr, d_sites, adjoint ? 4 : 1, plan, stream);
+}
+
+static int sum_expansions(const System &sys, const RegionSet &rs, const TaylorPlan &plan,
+                          bool symmetric, float *sums, cudaStream_t stream) {
     SumArgs s;
     s.regs = rs.d_info;
     s.n_regions = rs.n_regions;
@@ -624,11 +680,19 @@ int taylor_enqueue(const System &sys, const RegionSet &rs, int n_axes, const Tay
     taylor_sums_kernel<<<chunks * (kSumChunk / kSumWarps) * (kTaylorRoles + 1), 32 * kSumWarps, 0,
                          stream>>>(s);
     VEXT_CUDA(cudaGetLastError());
+    return 0;
+}
+
+int taylor_enqueue(const System &sys, const RegionSet &rs, int n_axes, const TaylorPlan &plan,
+                   bool symmetric, float *sums, float *const *e32, double *e64,
+                   float *const *g32, cudaStream_t stream) {
+    VEXT_TRY(sum_expansions(sys, rs, plan, symmetric, sums, stream));
     EvalArgs a;
     a.matrix = plan.matrix;
     a.sums = sums;
     a.rows = plan.rows;
     a.poses = n_axes * rs.bi * rs.bj * rs.bk;
+    a.site_out = nullptr;
     a.n_regions = rs.n_regions;
     a.regs = rs.d_info;
     a.S = rs.size;
@@ -644,6 +708,23 @@ int taylor_enqueue(const System &sys, const RegionSet &rs, int n_axes, const Tay
         taylor_eval_kernel<7, 128, 8><<<dim3(tiles, (rs.n_regions + 63) / 64), 128, 0, stream>>>(a);
     else
         taylor_eval_kernel<1, 256, 4><<<dim3(tiles, (rs.n_regions + 63) / 64), 256, 0, stream>>>(a);
+    VEXT_CUDA(cudaGetLastError());
+    return 0;
+}
+
+int taylor_enqueue_sites(const System &sys, const RegionSet &rs, int n_sites,
+                         const TaylorPlan &plan, float *sums, float *out, cudaStream_t stream) {
+    VEXT_TRY(sum_expansions(sys, rs, plan, false, sums, stream));
+    EvalArgs a{};
+    a.matrix = plan.matrix;
+    a.sums = sums;
+    a.rows = plan.rows;
+    a.poses = n_sites;
+    a.n_regions = rs.n_regions;
+    a.site_out = out;
+    const dim3 grid(plan.rows / eval_tile(plan.outs), (rs.n_regions + 63) / 64);
+    if (plan.outs == 4) taylor_eval_kernel<4, 128, 8, true><<<grid, 128, 0, stream>>>(a);
+    else taylor_eval_kernel<1, 256, 4, true><<<grid, 256, 0, stream>>>(a);
     VEXT_CUDA(cudaGetLastError());
     return 0;
 }

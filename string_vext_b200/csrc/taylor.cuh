@@ -135,6 +135,18 @@ bool taylor_worthwhile(const System &sys, const RegionSet &rs, int n_axes, bool 
 int taylor_prepare(const System &sys, const RegionSet &rs, int n_axes, const double *d_axes,
                    bool adjoint, TaylorPlan &plan, cudaStream_t stream);
 
+// The same for single sites: `d_sites` [n_sites][3] relative to a region's
+// origin (sites.cuh), outputs value (and gradient) per site.
+int taylor_prepare_sites(const System &sys, const RegionSet &rs, int n_sites,
+                         const double *d_sites, bool adjoint, TaylorPlan &plan,
+                         cudaStream_t stream);
+int taylor_enqueue_sites(const System &sys, const RegionSet &rs, int n_sites,
+                         const TaylorPlan &plan, float *sums, float *out, cudaStream_t stream);
+
+// Whether a pair's truncation error stays within tolerance for `sys` on lists
+// that another guest of the same framework may have built.
+bool taylor_allowed(const System &sys, const RegionSet &rs);
+
 // Floats of the per-region sums taylor_enqueue needs as workspace.
 inline size_t taylor_workspace(const RegionSet &rs) { return (size_t)rs.n_regions * kTaylorPad; }
 
