@@ -62,7 +62,8 @@ struct alignas(16) RegionInfo {
                         // expansion (taylor.cuh), which covers the rest
     int n_shella;       // the first of the shell entries: so near that a symmetric director's
                         // site on the entry's side is inside the cutoff for every pose
-    int pad[2];
+    int n_tnear;        // the first of the expansion's entries: the others need fewer degrees
+    int pad[1];
 };
 static_assert(sizeof(RegionInfo) % 16 == 0, "RegionInfo must stay 16-byte aligned");
 
@@ -79,6 +80,7 @@ struct RegionSet {
     long long n_entries = 0, n_near = 0, n_outer = 0;
     long long n_taylor = 0;                 // inner entries of the expansions (taylor.cuh)
     double d_taylor = 1e30;                 // their smallest distance from the origin
+    double d_tfar = 1e30;                   // from here on kTaylorFarOrder degrees do
     double taylor_radius = 0;               // every site of a region lies this near its origin
     RegionInfo *d_info = nullptr;
     float4 *d_hi = nullptr, *d_lo = nullptr;

@@ -112,14 +112,16 @@ struct BuildArgs {
     double r_inner0;  // cutoff - max|offset| (- margin): inner entries lie within r_inner0 - rho
     double r_outer0;  // cutoff + 1e-3 A: outer shell entries lie beyond r_outer0 + rho
     double r_taylor;  // inner entries beyond it belong to the local expansion
+    double r_tfar;    // and those beyond this one need fewer of its degrees
     double r_shella0; // shell entries within r_shella0 - rho: the nearer of two symmetric sites
                       // is inside the cutoff for every pose (0: none are set apart)
 };
 
 // Class boundaries (squared distance from the origin) of one region, in
-// increasing order: near | mid | taylor | shell a | shell | outer is the order
-// of the classes and of the entries.
-constexpr int kClasses = 6;
+// increasing order: near | mid | taylor | taylor far | shell a | shell | outer
+// is the order of the classes and of the entries (an eighth one, always empty,
+// for the scans in pairs).
+constexpr int kClasses = 8;
 struct ClassRadii {
     double rl, at[kClasses - 1];
     __device__ ClassRadii(const BuildArgs &a, const RegionInfo &r) {
@@ -127,10 +129,12 @@ struct ClassRadii {
         const double rn = a.r_near0 + r.rho, ri = fmax(a.r_inner0 - r.rho, 0.0),
                      ra = fmax(a.r_shella0 - r.rho, 0.0), ro = a.r_outer0 + r.rho;
         at[0] = rn * rn;
-        at[2] = fmax(ri * ri, at[0]);
-        at[1] = fmin(fmax(a.r_taylor * a.r_taylor, at[0]), at[2]);
-        at[3] = fmax(ra * ra, at[2]);
-        at[4] = fmax(ro * ro, at[3]);
+        at[3] = fmax(ri * ri, at[0]);
+        at[1] = fmin(fmax(a.r_taylor * a.r_taylor, at[0]), at[3]);
+        at[2] = fmin(fmax(a.r_tfar * a.r_tfar, at[1]), at[3]);
+        at[4] = fmax(ra * ra, at[3]);
+        at[5] = fmax(ro * ro, at[4]);
+        at[6] = 1e300;
     }
 };
 struct ClassCounts {
@@ -221,7 +225,7 @@ __global__ void __launch_bounds__(NT)
     if (region >= n_regions) return;
     const RegionInfo r = regs[region];
     const ClassRadii cls(a, r);
-    int from[kClasses] = {0, 0, 0, 0, 0, 0};   // entries at or beyond each boundary
+    int from[kClasses] = {0, 0, 0, 0, 0, 0, 0, 0};   // entries at or beyond each boundary
     for (int j = threadIdx.x; j < a.n_atoms; j += NT)
         for_each_image(a, r, j, cls.rl, [&](double q, double, double, double) {
             ++from[0];
@@ -241,10 +245,11 @@ __global__ void __launch_bounds__(NT)
         RegionInfo &w = regs[region];
         w.n_near = t[0];
         w.n_mid = t[1];
-        w.n_inner = t[1] + t[2];
-        w.n_shella = t[3];
-        w.n_outer = t[5];
-        w.n_total = t[0] + t[1] + t[2] + t[3] + t[4] + t[5];
+        w.n_inner = t[1] + t[2] + t[3];
+        w.n_tnear = t[2];
+        w.n_shella = t[4];
+        w.n_outer = t[6];
+        w.n_total = t[0] + t[1] + t[2] + t[3] + t[4] + t[5] + t[6];
     }
 }
 
@@ -268,9 +273,10 @@ __global__ void __launch_bounds__(NT, 512 / NT)
 #pragma unroll
     for (int i = 0; i < kClasses; i += 2)
         block_scan2<NT>(c.n[i], c.n[i + 1], w[i], w[i + 1], t[i], t[i + 1], sh);
-    if (threadIdx.x == 0 && (t[0] != r.n_near || t[1] != r.n_mid || t[1] + t[2] != r.n_inner ||
-                             t[3] != r.n_shella || t[5] != r.n_outer ||
-                             t[0] + t[1] + t[2] + t[3] + t[4] + t[5] != r.n_total))
+    if (threadIdx.x == 0 &&
+        (t[0] != r.n_near || t[1] != r.n_mid || t[2] != r.n_tnear ||
+         t[1] + t[2] + t[3] != r.n_inner || t[4] != r.n_shella || t[6] != r.n_outer ||
+         t[0] + t[1] + t[2] + t[3] + t[4] + t[5] + t[6] != r.n_total))
         atomicExch(status, DEV_BAD_LIST);
     int base = 0;
 #pragma unroll
@@ -360,6 +366,7 @@ static int build_lists(System *sys, RegionSet *rs, cudaStream_t stream) {
     // shell entries whose nearer site is always inside: |d0|^2 + o^2 < rc^2
     // for every center (|d0| the entry's distance from it)
     a.r_taylor = rs->d_taylor;
+    a.r_tfar = rs->d_tfar;
     const double ra2 = sys->cutoff * sys->cutoff - sys->max_offset * sys->max_offset;
     a.r_shella0 = rs->d_taylor < sys->cutoff && ra2 > 0 && !rs->sites ? std::sqrt(ra2) - 1e-3 : 0.0;
     const int n = rs->n_regions;
@@ -451,7 +458,8 @@ int get_block_regions(System *sys, int size, int bi, int bj, int bk, double rho,
             rs->sites == sites && rs->r_split == r_split) {
             if (rs->stale) {
                 for (auto &r : rs->h_info)
-                    r.n_near = r.n_total = r.n_inner = r.n_outer = r.n_mid = r.n_shella = 0;
+                    r.n_near = r.n_total = r.n_inner = r.n_outer = r.n_mid = r.n_tnear =
+                        r.n_shella = 0;
                 VEXT_TRY(build_lists(sys, rs, stream));
             }
             *out = rs;
@@ -499,6 +507,8 @@ int get_block_regions(System *sys, int size, int bi, int bj, int bk, double rho,
         if (start < inner && 4.18879 * (inner * inner * inner - start * start * start) *
                                      sys->n_atoms / volume >= kTaylorMinEntries)
             rs->d_taylor = start;
+        rs->d_tfar = std::max(rs->d_taylor,
+                              taylor_start(*sys, rs->taylor_radius, kTaylorFarOrder));
     }
     int rc = build_lists(sys, rs, stream);
     if (rc) {
@@ -518,7 +528,8 @@ int get_bin_regions(System *sys, double r_split, RegionSet **out, cudaStream_t s
         if (rs->size == 0 && rs->r_split == r_split && rs->bin_width == bin_width) {
             if (rs->stale) {
                 for (auto &r : rs->h_info)
-                    r.n_near = r.n_total = r.n_inner = r.n_outer = r.n_mid = r.n_shella = 0;
+                    r.n_near = r.n_total = r.n_inner = r.n_outer = r.n_mid = r.n_tnear =
+                        r.n_shella = 0;
                 VEXT_TRY(build_lists(sys, rs, stream));
             }
             *out = rs;

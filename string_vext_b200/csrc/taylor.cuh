@@ -21,6 +21,7 @@
 namespace vext {
 
 constexpr int kTaylorOrder = 12;
+constexpr int kTaylorFarOrder = 8;   // degrees that entries from RegionSet::d_tfar on need
 constexpr int kTaylorLow = 4;        // degrees below this: the FP64 polynomial
 constexpr int kTaylorPoly = 20;      // its coefficients
 constexpr int kTaylorPolyPad = 24;   // doubles per region
@@ -121,10 +122,11 @@ __device__ __forceinline__ double taylor_pair(const double *p, double cx, double
 
 // ---------------------------------------------------------------- host side
 
-// Smallest distance from the origin at which the expansion's truncation
-// error is within tolerance for sites within `radius` (system.cu builds the
-// lists with it); a value beyond the cutoff when there is none.
-double taylor_start(const System &sys, double radius);
+// Smallest distance from the origin at which the truncation error of an
+// expansion of this order is within tolerance for sites within `radius`
+// (system.cu builds the lists with it); a value beyond the cutoff when there is
+// none.
+double taylor_start(const System &sys, double radius, int order = kTaylorOrder);
 
 // Whether summing the inner pairs of `rs` by expansion is the faster way for
 // `n_axes` directors (the rule is explained at its definition), and allowed
