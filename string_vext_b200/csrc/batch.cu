@@ -911,7 +911,7 @@ static int launch_refine(vext_batch b, const BatchArgs &a, cudaStream_t st) {
 static int launch_sites(vext_batch b, size_t k, const BatchArgs &a, int region0, int region1,
                         int plane0, int plane1, cudaStream_t st) {
     VEXT_TRY(site_enqueue(b->systems[k]->sys, b->sites[k], b->adj, b->site_scratch, region0,
-                          region1, st));
+                          region1, b->d_status, st));
     if (plane1 <= plane0) return 0;
     const long long n = (long long)(plane1 - plane0) * b->size * b->size;
     const dim3 grid((unsigned)((n + 255) / 256), b->n_axes);

@@ -776,7 +776,7 @@ static int launch_sites(System *sys, const RegionSet *rs, int n_axes, const doub
         f.axes.assign(axes_host, axes_host + 3 * n_axes);
     }
     VEXT_TRY(site_scratch_reserve(f.plan, false, f.scratch));
-    VEXT_TRY(site_enqueue(*sys, f.plan, false, f.scratch, 0, rs->n_ri, stream));
+    VEXT_TRY(site_enqueue(*sys, f.plan, false, f.scratch, 0, rs->n_ri, sys->d_status, stream));
     return site_energies(f.plan, f.scratch, d_e64, stream);
 }
 

@@ -615,11 +615,12 @@ int site_plan_build(const System &sys, const RegionSet &rs, int n_axes, const do
     v.floor = reinterpret_cast<const int4 *>(base + at_floor);
     v.poly = nullptr;
     v.eval = nullptr;
-    // an expansion's cost per region: 2,100 operations an entry and 580 per
-    // output; it takes 12 (forward 9) off every (site, entry) pair
+    // an expansion costs about 1,000 operations an entry and 140 an output (the
+    // 28,800 regions of the 60^3 x 64 layered field: 1.56 and 0.49 ms); it takes 12
+    // (forward 9) off every (site, entry) pair
     const double n = (double)rs.n_taylor / std::max(rs.n_regions, 1);
     if (taylor_allowed(sys, rs) && n * v.n_sites * (adjoint ? 12.0 : 9.0) >
-                                       n * 2100.0 + v.n_sites * (adjoint ? 4 : 1) * 580.0) {
+                                       n * 1000.0 + v.n_sites * (adjoint ? 4 : 1) * 140.0) {
         VEXT_TRY(taylor_prepare_sites(sys, rs, v.n_sites, v.pos, adjoint, plan.expansion, stream));
         v.poly = plan.expansion.poly;
     }
@@ -637,7 +638,7 @@ int site_scratch_reserve(const SitePlan &plan, bool adjoint, SiteScratch &s) {
     const size_t S3 = (size_t)v.S * v.S * v.S, words = adjoint ? 4 : 1;
     VEXT_TRY(ensure_capacity(s.value, s.value_cap, 2 * v.O * S3 * words));
     if (v.poly) {
-        VEXT_TRY(ensure_capacity(s.sums, s.sums_cap, taylor_workspace(*plan.rs)));
+        VEXT_TRY(ensure_capacity(s.sums, s.sums_cap, taylor_workspace_sites(*plan.rs)));
         VEXT_TRY(ensure_capacity(s.eval, s.eval_cap, (size_t)v.n_regions * v.n_sites * words));
     }
     return 0;
@@ -652,7 +653,8 @@ SiteView site_view(const SitePlan &plan) {
 }
 
 int site_enqueue(const System &sys, const SitePlan &plan, bool adjoint,
-                 const SiteScratch &scratch, int plane0, int plane1, cudaStream_t stream) {
+                 const SiteScratch &scratch, int plane0, int plane1, int *status,
+                 cudaStream_t stream) {
     SiteArgs g;
     g.v = site_view(plan);
     g.v.eval = scratch.eval;
@@ -662,7 +664,7 @@ int site_enqueue(const System &sys, const SitePlan &plan, bool adjoint,
     if (plane1 <= plane0) return 0;
     if (v.poly && plane0 == 0)
         VEXT_TRY(taylor_enqueue_sites(sys, *plan.rs, v.n_sites, plan.expansion, scratch.sums,
-                                      scratch.eval, stream));
+                                      scratch.eval, status, stream));
     const int per_plane = v.nrj * v.nrk;
     g.region0 = plane0 * per_plane;
     const unsigned blocks =

@@ -105,7 +105,8 @@ int site_scratch_reserve(const SitePlan &plan, bool adjoint, SiteScratch &scratc
 // V (and its gradient) into scratch.value at the sites of region planes
 // [plane0, plane1) along the slowest axis (with plane 0: all the expansions).
 int site_enqueue(const System &sys, const SitePlan &plan, bool adjoint,
-                 const SiteScratch &scratch, int plane0, int plane1, cudaStream_t stream);
+                 const SiteScratch &scratch, int plane0, int plane1, int *status,
+                 cudaStream_t stream);
 
 // The view with the lists where they stand now (a rebuild may have moved them).
 SiteView site_view(const SitePlan &plan);

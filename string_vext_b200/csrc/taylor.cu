@@ -7,7 +7,8 @@
 //                       relative to the origin in every region of a system,
 //                       so values and gradients at all poses are one matrix
 //                       product: [outputs of a region x sums] . [sums x
-//                       regions], register-tiled packed FP32
+//                       regions], register-tiled packed FP32; single sites
+//                       take taylor_mma_kernel (taylormma.cu) instead
 //   taylor_matrix_kernel  that matrix: solid harmonics and their gradients
 //                       at the poses' sites, in FP64, rounded once
 //
@@ -20,6 +21,7 @@
 
 #include "pair.cuh"
 #include "taylor.cuh"
+#include "taylormma.cuh"
 
 namespace vext {
 
@@ -32,7 +34,8 @@ struct SumArgs {
     float inv_r;          // 1 / unit length
     int symmetric;        // near shell entries (RegionInfo::n_shella) belong to the expansion
     int far;              // entries after the first n_tnear lie beyond RegionSet::d_tfar
-    float *sums;          // [n_regions][kTaylorPad]
+    float *sums;          // [n_regions][kTaylorPad]; split: the operand of taylor_mma_kernel
+    int split;
     double *poly;         // [n_regions][kTaylorPolyPad]
 };
 
@@ -150,7 +153,7 @@ __device__ __forceinline__ void role_entries(const SumArgs &s, const float4 *hi,
 // ms; with order 7, which starts farther out, 14.21, with 9 14.20).
 template <int ROLE>
 __device__ __forceinline__ void role_sum(const SumArgs &s, const float4 *hi, int n_full, int n,
-                                         int lane, float *out) {
+                                         int lane, int region, float *out) {
     constexpr int N = role_sums(ROLE), NP = (N + 31) / 32 * 32;
     float acc[NP];
 #pragma unroll
@@ -160,7 +163,10 @@ __device__ __forceinline__ void role_sum(const SumArgs &s, const float4 *hi, int
 #pragma unroll
     for (int g = 0; g < NP / 32; ++g) {
         const float t = transpose_sum(acc + 32 * g, lane);
-        if (32 * g + lane < N) out[role_start(ROLE) + 32 * g + lane] = t;
+        const int i = role_start(ROLE) + 32 * g + lane;
+        if (32 * g + lane >= N) continue;
+        if (s.split) mma_store_split<kMmaN>(s.sums, region, kMmaOrder.at[i], t);
+        else out[i] = t;
     }
 }
 
@@ -262,14 +268,17 @@ __global__ void __launch_bounds__(32 * kSumWarps, 4) taylor_sums_kernel(SumArgs 
     const float4 *hi = s.hi + first;
     float *out = s.sums + (size_t)region * kTaylorPad;
     switch (role) {
-    case 0: role_sum<0>(s, hi, n_full, n, lane, out); break;
-    case 1: role_sum<1>(s, hi, n_full, n, lane, out); break;
-    case 2: role_sum<2>(s, hi, n_full, n, lane, out); break;
-    case 3: role_sum<3>(s, hi, n_full, n, lane, out); break;
-    case 4: role_sum<4>(s, hi, n_full, n, lane, out); break;
-    case 5: role_sum<5>(s, hi, n_full, n, lane, out); break;
+    case 0: role_sum<0>(s, hi, n_full, n, lane, region, out); break;
+    case 1: role_sum<1>(s, hi, n_full, n, lane, region, out); break;
+    case 2: role_sum<2>(s, hi, n_full, n, lane, region, out); break;
+    case 3: role_sum<3>(s, hi, n_full, n, lane, region, out); break;
+    case 4: role_sum<4>(s, hi, n_full, n, lane, region, out); break;
+    case 5: role_sum<5>(s, hi, n_full, n, lane, region, out); break;
     default:
-        if (lane < kTaylorPad - kTaylorSums) out[kTaylorSums + lane] = 0.f;
+        if (lane < kTaylorPad - kTaylorSums) {
+            if (s.split) mma_store_split<kMmaN>(s.sums, region, lane, 0.f);
+            else out[kTaylorSums + lane] = 0.f;
+        }
         poly_sum(s, hi, s.lo + first, n, lane, s.poly + (size_t)region * kTaylorPolyPad);
     }
 }
@@ -360,17 +369,14 @@ __global__ void __launch_bounds__(128) taylor_matrix_kernel(MatrixArgs a, SumInd
     if (pose >= a.poses) return;
     const uchar4 w = index.at[blockIdx.y];
     float *row = a.matrix + (size_t)blockIdx.y * a.rows;
-    if (a.sites) {
+    if (a.sites) {   // the other operand of taylor_mma_kernel
         double v, g[3];
         const double *p = a.sites + 3 * pose;
         solid_term(w.x, w.y, w.z, w.w, p[0] * a.inv_r, p[1] * a.inv_r, p[2] * a.inv_r, v, g);
-        if (a.outs == 1) {
-            row[pose] = (float)v;
-            return;
-        }
-        row[(pose >> 1) * 8 + (pose & 1)] = (float)v;
-        for (int k = 0; k < 3; ++k)
-            row[(pose >> 1) * 8 + 2 + 2 * k + (pose & 1)] = (float)(g[k] * a.inv_r);
+        const int k = kMmaOrder.at[blockIdx.y];
+        mma_store_split<kMmaM>(a.matrix, pose * a.outs, k, (float)v);
+        for (int d = 0; d < 3 && a.outs == 4; ++d)
+            mma_store_split<kMmaM>(a.matrix, pose * 4 + 1 + d, k, (float)(g[d] * a.inv_r));
         return;
     }
     const int cb = a.bi * a.bj * a.bk, o = pose / cb, c = pose % cb;
@@ -411,11 +417,11 @@ struct EvalArgs {
     float *const *e32;       // device words holding the output pointers
     float *const *g32;
     double *e64;
-    float *site_out;         // single sites: [n_regions][poses] x OUTS
 };
 
 constexpr int kEvalK = 16;
-__host__ __device__ constexpr int eval_rows(int outs) { return outs == 7 ? 14 : 16; }   // per thread
+// rows per thread
+__host__ __device__ constexpr int eval_rows(int outs) { return outs == 1 ? 16 : 14; }
 __host__ __device__ constexpr int eval_tile(int outs) { return 16 * eval_rows(outs); }
 
 // Tile: eval_tile rows (32 poses x 7 outputs, or 256 poses) x NT / 16 CT
@@ -424,9 +430,7 @@ __host__ __device__ constexpr int eval_tile(int outs) { return 16 * eval_rows(ou
 // 1.99 ms as 128 threads x 8 regions (256 x 4: 2.12; 6 regions at 3 CTAs/SM:
 // 2.09; unpacked FMA: 2.07); 14,400 regions of 16 centers, energy alone: 0.46
 // ms as 256 x 4 (128 x 8: 0.53).
-// SITES: single sites (sites.cuh) instead of poses, OUTS 1 or 4 (value and
-// gradient).
-template <int OUTS, int NT, int CT, bool SITES = false>
+template <int OUTS, int NT, int CT>
 __global__ void __launch_bounds__(NT, 2) taylor_eval_kernel(EvalArgs a) {
     constexpr int RT = eval_rows(OUTS), RP = RT / 2, TILE = eval_tile(OUTS);
     constexpr int COLS = NT / 16 * CT;   // regions per tile
@@ -511,31 +515,6 @@ __global__ void __launch_bounds__(NT, 2) taylor_eval_kernel(EvalArgs a) {
                     acc[i][j] = __ffma2_rn(m[k & 1][i], v[k & 1][j], acc[i][j]);
         }
         if (more) store_s(buf ^ 1);
-    }
-    if constexpr (SITES) {
-#pragma unroll
-        for (int j = 0; j < CT; ++j) {
-            const int reg = reg0 + NT / 8 * (j >> 1) + 2 * cg + (j & 1);
-            if (reg >= a.n_regions) continue;
-            const int first = (row0 + rg * RT) / OUTS;   // this thread's RT / OUTS sites
-            if (first >= a.poses) continue;
-            float4 *out = reinterpret_cast<float4 *>(a.site_out +
-                                                     ((size_t)reg * a.poses + first) * OUTS);
-#pragma unroll
-            for (int q = 0; q < RT / 4; ++q) {
-                if (OUTS == 1)
-                    out[q] = make_float4(acc[2 * q][j].x, acc[2 * q][j].y, acc[2 * q + 1][j].x,
-                                         acc[2 * q + 1][j].y);
-                else {
-                    const int p = q / 2 * 4;
-                    out[q] = q & 1 ? make_float4(acc[p][j].y, acc[p + 1][j].y, acc[p + 2][j].y,
-                                                 acc[p + 3][j].y)
-                                   : make_float4(acc[p][j].x, acc[p + 1][j].x, acc[p + 2][j].x,
-                                                 acc[p + 3][j].x);
-                }
-            }
-        }
-        return;
     }
     const int cb = a.bi * a.bj * a.bk;
     const long long S3 = (long long)a.S * a.S * a.S;
@@ -643,14 +622,15 @@ bool taylor_worthwhile(const System &sys, const RegionSet &rs, int n_axes, bool 
 
 static int prepare(const System &sys, const RegionSet &rs, int poses, const double *d_axes,
                    const double *d_sites, int outs, TaylorPlan &plan, cudaStream_t stream) {
-    const int rows_used = outs == 1 ? poses : (poses + 1) / 2 * 2 * outs;
-    const int tile = eval_tile(outs);
+    const int rows_used = d_sites || outs == 1 ? poses * outs : (poses + 1) / 2 * 14;
+    const int tile = d_sites ? kMmaM : eval_tile(outs);
     const int rows = (rows_used + tile - 1) / tile * tile;
-    VEXT_TRY(ensure_capacity(plan.matrix, plan.matrix_cap, (size_t)kTaylorPad * rows));
+    const size_t words = (size_t)kTaylorPad * rows * (d_sites ? 2 : 1);
+    VEXT_TRY(ensure_capacity(plan.matrix, plan.matrix_cap, words));
     VEXT_TRY(ensure_capacity(plan.poly, plan.poly_cap, (size_t)rs.n_regions * kTaylorPolyPad));
     plan.rows = rows;
     plan.outs = outs;
-    VEXT_CUDA(cudaMemsetAsync(plan.matrix, 0, sizeof(float) * kTaylorPad * (size_t)rows, stream));
+    VEXT_CUDA(cudaMemsetAsync(plan.matrix, 0, sizeof(float) * words, stream));
     MatrixArgs a;
     a.H = sys.H;
     a.S = rs.size;
@@ -685,7 +665,7 @@ int taylor_prepare_sites(const System &sys, const RegionSet &rs, int n_sites,
 }
 
 static int sum_expansions(const System &sys, const RegionSet &rs, const TaylorPlan &plan,
-                          bool symmetric, float *sums, cudaStream_t stream) {
+                          bool symmetric, bool split, float *sums, cudaStream_t stream) {
     SumArgs s;
     s.regs = rs.d_info;
     s.n_regions = rs.n_regions;
@@ -697,6 +677,7 @@ static int sum_expansions(const System &sys, const RegionSet &rs, const TaylorPl
     s.symmetric = symmetric;
     s.far = rs.d_tfar < sys.cutoff - rs.taylor_radius;   // the inner entries' bound
     s.sums = sums;
+    s.split = split;
     s.poly = plan.poly;
     const int chunks = (rs.n_regions + kSumChunk - 1) / kSumChunk;
     taylor_sums_kernel<<<chunks * (kSumChunk / kSumWarps) * (kTaylorRoles + 1), 32 * kSumWarps, 0,
@@ -708,13 +689,12 @@ static int sum_expansions(const System &sys, const RegionSet &rs, const TaylorPl
 int taylor_enqueue(const System &sys, const RegionSet &rs, int n_axes, const TaylorPlan &plan,
                    bool symmetric, float *sums, float *const *e32, double *e64,
                    float *const *g32, cudaStream_t stream) {
-    VEXT_TRY(sum_expansions(sys, rs, plan, symmetric, sums, stream));
+    VEXT_TRY(sum_expansions(sys, rs, plan, symmetric, false, sums, stream));
     EvalArgs a;
     a.matrix = plan.matrix;
     a.sums = sums;
     a.rows = plan.rows;
     a.poses = n_axes * rs.bi * rs.bj * rs.bk;
-    a.site_out = nullptr;
     a.n_regions = rs.n_regions;
     a.regs = rs.d_info;
     a.S = rs.size;
@@ -735,20 +715,11 @@ int taylor_enqueue(const System &sys, const RegionSet &rs, int n_axes, const Tay
 }
 
 int taylor_enqueue_sites(const System &sys, const RegionSet &rs, int n_sites,
-                         const TaylorPlan &plan, float *sums, float *out, cudaStream_t stream) {
-    VEXT_TRY(sum_expansions(sys, rs, plan, false, sums, stream));
-    EvalArgs a{};
-    a.matrix = plan.matrix;
-    a.sums = sums;
-    a.rows = plan.rows;
-    a.poses = n_sites;
-    a.n_regions = rs.n_regions;
-    a.site_out = out;
-    const dim3 grid(plan.rows / eval_tile(plan.outs), (rs.n_regions + 63) / 64);
-    if (plan.outs == 4) taylor_eval_kernel<4, 128, 8, true><<<grid, 128, 0, stream>>>(a);
-    else taylor_eval_kernel<1, 256, 4, true><<<grid, 256, 0, stream>>>(a);
-    VEXT_CUDA(cudaGetLastError());
-    return 0;
+                         const TaylorPlan &plan, float *sums, float *out, int *status,
+                         cudaStream_t stream) {
+    VEXT_TRY(sum_expansions(sys, rs, plan, false, true, sums, stream));
+    return taylor_mma(plan.matrix, plan.rows / kMmaM, sums, rs.n_regions, n_sites * plan.outs, out,
+                      status, stream);
 }
 
 }  // namespace vext

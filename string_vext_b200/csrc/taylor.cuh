@@ -143,7 +143,9 @@ int taylor_prepare_sites(const System &sys, const RegionSet &rs, int n_sites,
                          const double *d_sites, bool adjoint, TaylorPlan &plan,
                          cudaStream_t stream);
 int taylor_enqueue_sites(const System &sys, const RegionSet &rs, int n_sites,
-                         const TaylorPlan &plan, float *sums, float *out, cudaStream_t stream);
+                         const TaylorPlan &plan, float *sums, float *out, int *status,
+                         cudaStream_t stream);
+size_t taylor_workspace_sites(const RegionSet &rs);   // floats of `sums`
 
 // Whether a pair's truncation error stays within tolerance for `sys` on lists
 // that another guest of the same framework may have built.

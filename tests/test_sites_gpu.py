@@ -18,7 +18,8 @@ pytestmark = pytest.mark.gpu
 
 CELLS = {"skewed": ([14.0, 12.0, 13.0], [75.0, 85.0, 115.0], 90),
          "flat": ([16.0, 15.0, 3.6], [90.0, 90.0, 120.0], 60),
-         "sparse": ([9.0, 11.0, 8.0], [90.0, 90.0, 90.0], 6)}
+         "sparse": ([9.0, 11.0, 8.0], [90.0, 90.0, 90.0], 6),
+         "dense": ([11.0, 12.0, 10.0], [80.0, 95.0, 100.0], 220)}
 
 
 def directors(n):
@@ -99,6 +100,13 @@ def check(case, size, axes, **options):
     ("skewed", 25, 17), ("skewed", 24, 64), ("flat", 27, 33), ("sparse", 16, 50)])
 def test_fields_by_sites_match_fp64(cell, size, n_axes, masses):
     check(make_case(cell, masses), size, directors(n_axes))
+
+
+@pytest.mark.parametrize("masses", [None, (15.0, 25.0)])
+@pytest.mark.parametrize("size,n_axes", [(19, 17), (23, 33), (18, 96)])
+def test_expansions_at_sites(size, n_axes, masses):
+    """Local expansions by matrix product: partial tiles of sites and regions."""
+    check(make_case("dense", masses), size, directors(n_axes))
 
 
 @pytest.mark.parametrize("r_split", [6.0, 8.5])
