@@ -61,7 +61,8 @@ struct alignas(16) RegionInfo {
     int n_mid;          // the first of the inner entries: too near the origin for its local
                         // expansion (taylor.cuh), which covers the rest
     int n_shella;       // the first of the shell entries: so near that a symmetric director's
-                        // site on the entry's side is inside the cutoff for every pose
+                        // site on the entry's side is inside the cutoff for every pose (site
+                        // lists: within the cutoff of the origin)
     int n_tnear;        // the first of the expansion's entries: the others need fewer degrees
     int pad[1];
 };

@@ -20,7 +20,7 @@ struct SiteArgs {
     int region0;              // first region
 };
 
-constexpr int kSiteWarps = 4;     // clusters per CTA
+constexpr int kSiteWarps = 2;     // clusters per CTA
 constexpr int kFarQueue = 32;     // entries a far queue gathers before they are taken
 constexpr int kNearQueue = 8;
 
@@ -38,7 +38,7 @@ constexpr double kNearMargin = 0.9;
 struct SiteQueue {
     float4 xy[kFarQueue + 32], zc[kFarQueue + 32];       // inside: (x,x,y,y), (z,z,c12,c12)
     float4 sxy[kFarQueue + 32], szc[kFarQueue + 32];     // shell
-    float4 scs[kFarQueue + 32];                          // (-c6,-c6,shift,index)
+    float4 scs[kFarQueue + 32];                          // (-c6, limit, shift, index)
     double2 near[kNearQueue + 32][4];                    // (x,y), (z,c12), (c6,shift), (floor2,
                                                          // test: 1)
     float2 c6[kFarQueue + 32];                           // inside: (-c6,-c6)
@@ -57,11 +57,11 @@ struct SitePartial {
 };
 
 // One far entry (a, b: queue entry; c6: minus the coefficient), both sites of
-// the lane.  MASK: added where d2 < inside; near_rc collects the least |d2 -
-// rc2f|.
+// the lane.  MASK: added where d2 < limit, or, with a limit above rc2f, taken
+// off where d2 >= limit; near_rc collects the least |d2 - rc2f|.
 template <bool ADJ, bool MASK>
 __device__ __forceinline__ void site_pair(float4 a, float4 b, float2 mc6, float shift,
-                                          const SitePoint &t, float inside, float rc2f,
+                                          const SitePoint &t, float limit, float rc2f,
                                           SitePartial &s, float &near_rc) {
     const float2 dx = __fadd2_rn(make_float2(a.x, a.y), t.nx),
                  dy = __fadd2_rn(make_float2(a.z, a.w), t.ny),
@@ -73,15 +73,17 @@ __device__ __forceinline__ void site_pair(float4 a, float4 b, float2 mc6, float 
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(d2.y));
     const float2 n1 = make_float2(r0, r1);
     float2 n3 = __fmul2_rn(__fmul2_rn(n1, n1), n1);
+    // e = n3 (c12 n3 - c6), dE/dd2 = -3 n1 n3 (2 c12 n3 - c6)
+    const float2 w = __fmul2_rn(c12, n3);
+    const float2 x = __fadd2_rn(w, mc6);
     if (MASK) {
-        const float2 m = make_float2(set_lt(d2.x, inside), set_lt(d2.y, inside));
+        const float all = limit > rc2f ? -1.f : 0.f;
+        const float2 m = __fadd2_rn(make_float2(set_lt(d2.x, limit), set_lt(d2.y, limit)),
+                                    make_float2(all, all));
         near_rc = fminf(near_rc, fminf(fabsf(d2.x - rc2f), fabsf(d2.y - rc2f)));
         n3 = __fmul2_rn(n3, m);
         s.e = __ffma2_rn(m, make_float2(shift, shift), s.e);
     }
-    // e = n3 (c12 n3 - c6), dE/dd2 = -3 n1 n3 (2 c12 n3 - c6)
-    const float2 w = __fmul2_rn(c12, n3);
-    const float2 x = __fadd2_rn(w, mc6);
     s.e = __ffma2_rn(n3, x, s.e);
     if (ADJ) {
         const float2 f = __fmul2_rn(__fmul2_rn(n1, n3), __fadd2_rn(w, x));
@@ -179,55 +181,63 @@ __device__ __forceinline__ void take_inside(const SiteQueue &q, int n, const Sit
     add_gradient<ADJ>(s, sum);
 }
 
-// Entries of the cutoff shell.  Pairs whose FP32 d2 lies within kBorderTol of
-// rc^2 stay out of the FP32 sums and are decided and added in FP64 (rare: the
-// queue is gone through again for them).
+// Entries of the cutoff shell; those in the expansion have a limit above rc^2
+// and are taken off where they lie outside.  Pairs whose FP32 d2 lies within
+// kBorderTol of rc^2 stay out of the FP32 sums and are decided and added in
+// FP64 (rare: the queue is gone through again for them).
 template <bool ADJ>
 __device__ __forceinline__ void take_shell(const SiteQueue &q, int n, const SitePoint &t,
                                            const SiteView &v, long long off, SiteSum &sum) {
     SitePartial s;
     s.e = s.gx = s.gy = s.gz = make_float2(0.f, 0.f);
     float near_rc = 1.f;
-    const float inside = v.rc2f - kBorderTol;
     int j = 0;
 #pragma unroll 1
     for (; j + 4 <= n; j += 4) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const float4 c = q.scs[j + k];
-            site_pair<ADJ, true>(q.sxy[j + k], q.szc[j + k], make_float2(c.x, c.y), c.z, t,
-                                 inside, v.rc2f, s, near_rc);
+            site_pair<ADJ, true>(q.sxy[j + k], q.szc[j + k], make_float2(c.x, c.x), c.z, t, c.y,
+                                 v.rc2f, s, near_rc);
         }
     }
 #pragma unroll 1
     for (; j < n; ++j) {
         const float4 c = q.scs[j];
-        site_pair<ADJ, true>(q.sxy[j], q.szc[j], make_float2(c.x, c.y), c.z, t, inside, v.rc2f,
-                             s, near_rc);
+        site_pair<ADJ, true>(q.sxy[j], q.szc[j], make_float2(c.x, c.x), c.z, t, c.y, v.rc2f, s,
+                             near_rc);
     }
     add_energy<ADJ>(s, sum);
     add_gradient<ADJ>(s, sum);
-    if (near_rc <= kBorderTol) {
+    const float lo = v.rc2f - kBorderTol, hi = v.rc2f + kBorderTol;
+    if (near_rc <= fmaxf(v.rc2f - lo, hi - v.rc2f)) {
 #pragma unroll 1
         for (int k = 0; k < n; ++k) {
-            const float4 a = q.sxy[k], b = q.szc[k];
+            const float4 a = q.sxy[k], b = q.szc[k], c = q.scs[k];
             const float2 dx = __fadd2_rn(make_float2(a.x, a.y), t.nx),
                          dy = __fadd2_rn(make_float2(a.z, a.w), t.ny),
                          dz = __fadd2_rn(make_float2(b.x, b.y), t.nz);
             const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+            const double taken = c.y > v.rc2f ? 1.0 : 0.0;   // by the expansion
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const float d = h ? d2.y : d2.x;
-                // what the FP32 sums left out and may be inside
-                if (d < inside || d > v.rc2f + kBorderTol) continue;
-                const int at = __float_as_int(q.scs[k].w);
+                if (d < lo || d >= hi) continue;   // the FP32 sums decided it
+                const int at = __float_as_int(c.w);
                 const float4 hh = v.hi[off + at], l = v.lo[off + at];
-                double f[3] = {0, 0, 0};
-                fp64_border_pair(t.p[h][0], t.p[h][1], t.p[h][2], (double)hh.x + (double)l.x,
-                                 (double)hh.y + (double)l.y, (double)hh.z + (double)l.z, v.td,
-                                 __float_as_int(hh.w), v.rc2, sum.e[h], f);
-#pragma unroll
-                for (int i = 0; i < 3; ++i) sum.g[h][i] -= f[i] / 6.0;
+                const double *td = v.td + 4 * __float_as_int(hh.w);
+                const double x = t.p[h][0] - ((double)hh.x + (double)l.x),
+                             y = t.p[h][1] - ((double)hh.y + (double)l.y),
+                             z = t.p[h][2] - ((double)hh.z + (double)l.z);
+                const double r2 = fma(x, x, fma(y, y, z * z));
+                const double wt = (r2 < v.rc2 ? 1.0 : 0.0) - taken;
+                const double i2 = rcp64_nr<2>(r2);
+                const double i6 = i2 * i2 * i2, w = td[0] * i6;
+                sum.e[h] += wt * fma(i6, w - td[1], td[2]);
+                const double f = wt * (i2 * i6) * (2.0 * w - td[1]);
+                sum.g[h][0] = fma(f, x, sum.g[h][0]);
+                sum.g[h][1] = fma(f, y, sum.g[h][1]);
+                sum.g[h][2] = fma(f, z, sum.g[h][2]);
             }
         }
     }
@@ -241,15 +251,22 @@ __device__ __forceinline__ void take_shell(const SiteQueue &q, int n, const Site
 // full all lanes take its entries, two sites each.  No barrier, no staging: the
 // entries come from L1/L2, the warps are independent.
 //
-// 60^3 x 64 layered forward + adjoint: 9.9 ms here (with the expansions 14.7;
-// pose by pose, on lists about regions of poses, 18.1), about 1.2 of it
-// classification and 3.5 / 2.4 / 2.4 near, inside and shell entries; bound by
-// the latency of the FP64 and FP32 chains at 16 warps per SM (20 with spills:
-// 14.3 against 13.9 in all).  Hence eight inside entries, four shell entries
-// and two near ones side by side (half as many: 14.2), taken from full queues:
-// straight from each group of 32 the sums took 0.8 ms more.
+// The expansion holds all entries within rc of the region's origin, also those
+// in its shell: a cluster takes off the few that lie outside for its sites,
+// instead of adding the many that lie inside (in all: layered adjoint 12.5 ->
+// 11.2 ms; up to rc - 0.4 radius of the region 11.5, to rc + 0.3 radius 11.5).
+//
+// 60^3 x 64 layered forward + adjoint: 8.7 of 11.2 ms (pose by pose, on lists
+// about regions of poses, 18.1 in all), about 1.3 of it classification and 3.6
+// near entries.  Bound by the latency of the FP64 and FP32 chains at 16 warps
+// per SM (issue slots 57 %, FP64 pipe 33 %, FMA pipe 39 % busy; 20 warps with
+// spills are slower, forward 20 beat 24 by 1-2 %).  Hence eight inside entries,
+// four shell entries and two near ones side by side (half as many: 2 % slower,
+// one near entry: 3 %), taken from full queues: straight from each group of 32
+// the sums took 0.8 ms more.  Two warps a CTA leave fewer idle than four at odd
+// cluster counts (47^3 x 50 skewed field 1 %).
 template <bool ADJ>
-__global__ void __launch_bounds__(32 * kSiteWarps, (ADJ ? 16 : 24) / kSiteWarps)
+__global__ void __launch_bounds__(32 * kSiteWarps, (ADJ ? 16 : 20) / kSiteWarps)
     site_cluster_kernel(SiteArgs g) {
     __shared__ SiteQueue queue[kSiteWarps];
     const SiteView &v = g.v;
@@ -283,6 +300,8 @@ __global__ void __launch_bounds__(32 * kSiteWarps, (ADJ ? 16 : 24) / kSiteWarps)
     const long long off = r.off;
     const int near_end = v.poly ? r.n_near + r.n_mid : r.n_total;
     const int far_from = v.poly ? r.n_near + r.n_inner : r.n_total, total = r.n_total;
+    // shell entries that the expansion holds
+    const int taken_from = v.poly ? far_from : 0, taken_to = v.poly ? far_from + r.n_shella : 0;
     int n_near = 0, n_in = 0, n_shell = 0;
 #pragma unroll 1
     for (int part = 0; part < 2; ++part) {
@@ -296,9 +315,10 @@ __global__ void __launch_bounds__(32 * kSiteWarps, (ADJ ? 16 : 24) / kSiteWarps)
             if (base + 32 + lane < end) next = v.hi[off + base + 32 + lane];
             const float cx = h.x - mid.x, cy = h.y - mid.y, cz = h.z - mid.z;
             const float d2c = fmaf(cx, cx, fmaf(cy, cy, cz * cz));
-            const bool near = mine && d2c < rn2;
-            const bool in = mine && !near && d2c < ri2;
-            const bool shell = mine && !near && !in && d2c < ro2;
+            const bool taken = base + lane >= taken_from && base + lane < taken_to;
+            const bool near = mine && !taken && d2c < rn2;
+            const bool in = mine && !near && !taken && d2c < ri2;
+            const bool shell = mine && !near && d2c >= ri2 && (taken || d2c < ro2);
             const unsigned mn = __ballot_sync(0xffffffffu, near),
                            mi = __ballot_sync(0xffffffffu, in),
                            ms = __ballot_sync(0xffffffffu, shell), below = (1u << lane) - 1;
@@ -314,7 +334,8 @@ __global__ void __launch_bounds__(32 * kSiteWarps, (ADJ ? 16 : 24) / kSiteWarps)
                     const int at = n_shell + __popc(ms & below);
                     q.sxy[at] = make_float4(h.x, h.x, h.y, h.y);
                     q.szc[at] = make_float4(h.z, h.z, tp.x, tp.x);
-                    q.scs[at] = make_float4(-tp.y, -tp.y, tp.z, __int_as_float(base + lane));
+                    q.scs[at] = make_float4(-tp.y, taken ? v.rc2f + kBorderTol : v.rc2f - kBorderTol,
+                                            tp.z, __int_as_float(base + lane));
                 }
             } else if (near) {
                 const float4 l = v.lo[off + base + lane];
@@ -402,10 +423,10 @@ __global__ void site_energy_kernel(const double *value, long long S3, int O, dou
 // ---------------------------------------------------------------- plan
 
 // Radius of a cluster (A) up to which poses are summed site by site: the
-// region's by the cube root of its share of the 16 n_axes sites.  The finer the grid, the
-// more is gained (18.1 -> 14.7 ms at 0.25 A); four uneven frameworks at 35^3 x 64
-// with clusters of 0.4-1.4 A, forward + adjoint: none by sites 19.6 ms, up to
-// 0.65 A 19.3, up to 0.8 A 18.7, up to 1 A or all 18.9.
+// region's by the cube root of its share of the 16 n_axes sites.  The finer the
+// grid, the more is gained (18.1 -> 11.2 ms at 0.25 A); four uneven frameworks at
+// 35^3 x 64 with clusters of 0.4-1.4 A, forward + adjoint: none by sites 19.6 ms,
+// up to 0.8 A 16.4, up to 1 A or all 16.75.
 constexpr double kSiteRadius = 0.8;
 
 // Bytes of scratch beyond which a field is summed pose by pose.

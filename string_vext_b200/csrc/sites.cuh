@@ -93,8 +93,8 @@ int get_site_regions(System *sys, int size, int block, double r_split, RegionSet
                      cudaStream_t stream);
 // Voxels of a region: 8 in batches; a field call that builds its lists pays
 // twice the list work and memory for them (the 60^3 x 64 layered calculate_vext
-// 26.9 ms with 8, 16.6 with 16) while the sums differ little (adjoint 13.9 and
-// 14.2 ms; 47^3 x 50 skewed field 8.19 and 8.24).
+// 28.4 ms with 8, 16.0 with 16).  The sums with 8 and 16: layered adjoint 11.2 and
+// 11.6 ms, uneven batch adjoint 16.4 and 20.0; 47^3 x 50 skewed field 7.67 and 7.48.
 constexpr int kBatchVoxels = 8, kFieldVoxels = 16;
 
 int site_plan_build(const System &sys, const RegionSet &rs, int n_axes, const double *axes,

@@ -368,7 +368,9 @@ static int build_lists(System *sys, RegionSet *rs, cudaStream_t stream) {
     a.r_taylor = rs->d_taylor;
     a.r_tfar = rs->d_tfar;
     const double ra2 = sys->cutoff * sys->cutoff - sys->max_offset * sys->max_offset;
-    a.r_shella0 = rs->d_taylor < sys->cutoff && ra2 > 0 && !rs->sites ? std::sqrt(ra2) - 1e-3 : 0.0;
+    a.r_shella0 = rs->d_taylor < sys->cutoff && ra2 > 0 ? std::sqrt(ra2) - 1e-3 : 0.0;
+    // (site lists: those within rc; a cluster takes the ones outside off again)
+    if (rs->sites && rs->d_taylor < sys->cutoff) a.r_shella0 = sys->cutoff + rs->taylor_radius;
     const int n = rs->n_regions;
     if (!rs->d_info) VEXT_CUDA(device_malloc(&rs->d_info, sizeof(RegionInfo) * n));
     VEXT_CUDA(cudaMemcpyAsync(rs->d_info, rs->h_info.data(), sizeof(RegionInfo) * n,

@@ -717,7 +717,7 @@ int taylor_enqueue(const System &sys, const RegionSet &rs, int n_axes, const Tay
 int taylor_enqueue_sites(const System &sys, const RegionSet &rs, int n_sites,
                          const TaylorPlan &plan, float *sums, float *out, int *status,
                          cudaStream_t stream) {
-    VEXT_TRY(sum_expansions(sys, rs, plan, false, true, sums, stream));
+    VEXT_TRY(sum_expansions(sys, rs, plan, true, true, sums, stream));
     return taylor_mma(plan.matrix, plan.rows / kMmaM, sums, rs.n_regions, n_sites * plan.outs, out,
                       status, stream);
 }
