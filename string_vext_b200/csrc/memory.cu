@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <set>
 #include <thread>
 #include <utility>
 
@@ -26,6 +27,10 @@
 namespace vext {
 
 constexpr size_t kPoolKeep = 1536ull << 20;   // a 60^3 x 64 field's lists and buffers: 1.0 GB
+// Larger arrays than this would hardly stay in the pool, and it maps memory
+// more slowly than cudaMalloc does: the 27 GB of pose lists of 24 systems took
+// 0.4-0.8 s from it, 0.2 s by cudaMalloc.
+constexpr size_t kPoolLargest = 512ull << 20;
 
 unsigned long long current_context_id() {
     using GetCurrentFn = CUresult (*)(CUcontext *);
@@ -62,6 +67,7 @@ struct DevicePool {
     cudaStream_t stream = nullptr;
     unsigned long long ctx_id = 0;
     bool plain = false;   // no pool on this device: cudaMalloc and cudaFree
+    std::set<void *> direct;   // allocations beyond kPoolLargest, by cudaMalloc
 };
 
 DevicePool &device_pool(int device) {
@@ -77,6 +83,7 @@ void open_pool(DevicePool &p, int device) {
     if (p.pool && ctx != 0 && ctx != p.ctx_id) {
         p.pool = nullptr;   // went with its context
         p.stream = nullptr;
+        p.direct.clear();
     }
     if (p.pool || p.plain) return;
     int supported = 0;
@@ -113,6 +120,22 @@ cudaError_t device_malloc_bytes(void **out, size_t bytes) {
     std::lock_guard<std::mutex> guard(p.lock);
     open_pool(p, device);
     if (p.plain) return cudaMalloc(out, bytes);
+    if (bytes > kPoolLargest) {
+        e = cudaMalloc(out, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            cudaDeviceSynchronize();
+            cudaMemPoolTrimTo(p.pool, 0);
+            e = cudaMalloc(out, bytes);
+        }
+        if (e == cudaSuccess) {
+            p.direct.insert(*out);
+        } else {
+            cudaGetLastError();
+            *out = nullptr;
+        }
+        return e;
+    }
     e = cudaMallocFromPoolAsync(out, bytes, p.pool, p.stream);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
@@ -141,7 +164,7 @@ void device_free(void *ptr) {
     DevicePool &p = device_pool(at.device);
     {
         std::lock_guard<std::mutex> guard(p.lock);
-        if (p.plain || !p.pool) {
+        if (p.plain || !p.pool || p.direct.erase(ptr)) {
             cudaFree(ptr);
         } else {
             cudaDeviceSynchronize();   // no stream uses it any more
