@@ -124,7 +124,8 @@ VEXT_API int vext_system_invalidate(vext_system sys);
  * system's most recent list build and of the most recent field call's near
  * (FP64) pair kernel, far (FP32) pair kernel and epilogue; waits for those
  * events.  list_ms is 0 if no list was built since the previous query; in
- * the FP64 modes near_ms is the whole pair kernel and far_ms 0. */
+ * the FP64 modes near_ms is the whole pair kernel and far_ms 0; of fields
+ * summed site by site (fine grids) far_ms is the whole sum. */
 VEXT_API int vext_last_timings(vext_system sys, double *list_ms, double *near_ms,
                                double *far_ms, double *epilogue_ms);
 
@@ -147,7 +148,9 @@ typedef struct {
     double band_lo, band_hi; /* refinement band for E (K); band_hi <= band_lo
                                 disables refinement; defaults via
                                 vext_default_options                          */
-    int centers_per_region;  /* 16 or 32; 0 = default (16)                    */
+    int centers_per_region;  /* 0 = default: fine grids are summed site by site,
+                                others pose by pose on regions of 16 centers
+                                (batches 8); 8, 16 or 32 sum pose by pose      */
     int variant;             /* 0 = default.  Forward + adjoint batches
                                 (studies and checks): bit 32 / 64 the
                                 reciprocal of q^3 with / without a Newton
@@ -186,7 +189,8 @@ typedef struct {
     double list_build_ms, kernel_ms, epilogue_ms;  /* device time (events)   */
     int64_t outer_entries;   /* shell entries beyond rc + the region radius of
                                 their region's origin (at most one site of a
-                                director inside the cutoff)                   */
+                                director inside the cutoff); 0 for fields
+                                summed site by site                           */
 } vext_field_stats;
 
 /* Full Vext field on a size^3 fractional grid (centers ((i+.5)/S, ...),
@@ -239,9 +243,10 @@ VEXT_API int vext_field_adjoint_device(vext_system sys, int size, int n_axes,
                                        float *energy, float *gradient, double *energy_f64,
                                        double *gradient_f64, void *stream);
 /* Same with HOST float32 outputs (staged on the device, copied back before
- * the call returns).  In the mixed mode with more than 32 directors the poses
- * run as one batch per 32-director block and each block's outputs are copied
- * back while the next block computes. */
+ * the call returns).  In the mixed mode large page-locked outputs leave by slabs
+ * of grid planes while the next slab computes; pageable ones by blocks of 64
+ * directors (whole for fields summed site by site), through page-locked staging
+ * by several threads. */
 VEXT_API int vext_field_adjoint(vext_system sys, int size, int n_axes, const double *axes,
                                 const vext_options *opt, float *energy, float *gradient);
 
@@ -335,10 +340,10 @@ VEXT_API int vext_tst_log_score(int n, const double *frac, const double *energy,
 
 /* ------------------------------------------------------------------------ */
 /* Batched fields: many systems (frameworks x guests of uneven sizes and cell
- * shapes) in one persistent launch over a work queue of (system, region,
- * 32-director block) items, longest first, captured in a CUDA graph.  The
- * CTA shape and resident-CTA count are autotuned at creation on a sample of
- * the queue.  outputs[k] is a DEVICE float32 field [n_axes][S^3] for
+ * shapes) in one graph launch.  Systems on fine grids are summed site by site,
+ * one after another; the others share one persistent launch over a work queue of
+ * (system, region, director block) items, longest first, whose CTA shape and
+ * resident-CTA count are autotuned at creation on a sample of the queue.  outputs[k] is a DEVICE float32 field [n_axes][S^3] for
  * systems[k] (mixed precision, with FP64 re-evaluation of the refinement
  * band).  The systems must outlive the batch and must not be invalidated
  * while it exists.  No reference counterpart: the reference runs one field
@@ -414,9 +419,9 @@ VEXT_API int vext_measure_pipes(int iterations, double *ffma_per_s, double *ffma
 
 /* Exact FP64 number of (site, image) pairs closer than the cutoff over the
  * size^3 x n_axes field (the algorithmic unit of work); far_pairs (may be
- * NULL) receives those whose image is a far entry of the default 16-center
- * regions for the given r_split (<= 0: the default), i.e. the pairs the FP32
- * far kernel of the mixed field evaluates. */
+ * NULL) receives those whose image is a far entry of 16-center regions for the
+ * given r_split (<= 0: the default), i.e. the pairs outside the FP64 near lists
+ * of a field summed pose by pose. */
 VEXT_API int vext_count_pairs(vext_system sys, int size, int n_axes, const double *axes,
                               double r_split, int64_t *pairs, int64_t *far_pairs);
 

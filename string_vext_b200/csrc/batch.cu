@@ -1,6 +1,7 @@
 // Batched fields: many systems (frameworks x guests of uneven sizes and cell
-// shapes) in ONE persistent launch over a work queue, captured in a CUDA
-// graph and replayed.
+// shapes) captured in one CUDA graph and replayed.  Systems on fine grids are
+// summed site by site (sites.cuh), one after another; the others in ONE
+// persistent launch over a work queue.
 //
 // Work item = (system, region, director block): by default an 8-center
 // region x 64 directors (16 x 32 with centers_per_region 16; either way one
@@ -823,8 +824,9 @@ struct vext_batch_s {
     std::vector<Target> targets;          // current outputs of each system
     std::vector<TaylorPlan> plans;        // local expansions (poly null: none)
     std::vector<const RegionSet *> lists; // each system's region lists
-    std::vector<int> slab_items, slab_plane;   // first item and first grid plane of each slab,
-                                               // then the ends (see batch_run_slab)
+    std::vector<int> slab_items, slab_plane;   // first item (by sites: region plane) and first
+                                               // grid plane of each slab, then the ends (see
+                                               // batch_run_slab)
     int *d_slab_counts = nullptr;              // refinement records of each slab
     std::vector<SitePlan> sites;          // systems summed site by site (rs null: by items)
     SiteView *d_sites = nullptr;
@@ -1131,12 +1133,15 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
             return (int)(((long long)(k + 1) * rs.n_ri + slabs - 1) / slabs);
         };
         const int per = rs.n_rj * rs.n_rk;
-        auto slab_of = [&](const int4 &it) { return (int)((long long)(it.y / per) * slabs / rs.n_ri); };
+        auto slab_of = [&](const int4 &it) {
+            return (int)((long long)(it.y / per) * slabs / rs.n_ri);
+        };
         std::stable_sort(hitems.begin(), hitems.end(),
                          [&](const int4 &x, const int4 &y) { return slab_of(x) < slab_of(y); });
         for (const int4 &it : hitems) ++b->slab_items[slab_of(it) + 1];
         for (int k = 0; k < slabs; ++k) {
-            b->slab_items[k + 1] = by_site[0] ? slab_end(k) : b->slab_items[k] + b->slab_items[k + 1];
+            b->slab_items[k + 1] =
+                by_site[0] ? slab_end(k) : b->slab_items[k] + b->slab_items[k + 1];
             b->slab_plane[k + 1] = std::min(size, slab_end(k) * rs.bi);
         }
         VEXT_CUDA(device_malloc(&b->d_slab_counts, sizeof(int) * slabs));
@@ -1178,7 +1183,8 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
         b->lists.push_back(lists[owner[k]]);
         const System &sys = systems[k]->sys;
         const RegionSet &rs = *b->lists[k];
-        if (by_site[k] || !expands || !taylor_worthwhile(sys, rs, rule_axes ? rule_axes : n_axes, b->adj) ||
+        if (by_site[k] || !expands ||
+            !taylor_worthwhile(sys, rs, rule_axes ? rule_axes : n_axes, b->adj) ||
             !device_memory(hs[k].init) || (b->adj && !device_memory(hs[k].init_grad)))
             continue;
         VEXT_TRY(taylor_prepare(sys, rs, n_axes, b->d_axes, b->adj, b->plans[k], b->stream));
@@ -1355,7 +1361,8 @@ int batch_replay(vext_batch b, cudaStream_t stream) {
 
 // Run slab k (of a batch built with slabs > 1) on `stream`, slabs in order: the
 // poses of grid planes [*plane0, *plane1) along the slowest axis (those from
-// `size` on are the first ones) are final once it is done, so a caller can copy them while the next slab runs.
+// `size` on are the first ones) are final once it is done, so a caller can copy
+// them while the next slab runs.
 int batch_run_slab(vext_batch b, int k, cudaStream_t stream, int *plane0, int *plane1) {
     const int first = b->slab_items[k], n = b->slab_items[k + 1] - first;
     *plane0 = b->slab_plane[k];

@@ -1,4 +1,5 @@
 // Vext field kernels: every (grid center, director) pose of a size^3 grid.
+// Fine grids are summed site by site (sites.cuh); pose by pose:
 //
 // One CTA = one region (a block of CB grid centers) x one block of G*P
 // directors; thread (cl, og) owns center cl and directors og + G p (p < P).
@@ -768,7 +769,6 @@ static int launch_sites(System *sys, const RegionSet *rs, int n_axes, const doub
                         const double *d_axes, double *d_e64, cudaStream_t stream) {
     if (!sys->site_field) sys->site_field = new SiteField();
     SiteField &f = *sys->site_field;
-    sys->split_timed = false;
     if (f.plan.rs != rs || f.axes.size() != 3 * (size_t)n_axes ||
         !std::equal(axes_host, axes_host + 3 * n_axes, f.axes.begin())) {
         f.plan.rs = nullptr;
@@ -776,6 +776,8 @@ static int launch_sites(System *sys, const RegionSet *rs, int n_axes, const doub
         f.axes.assign(axes_host, axes_host + 3 * n_axes);
     }
     VEXT_TRY(site_scratch_reserve(f.plan, false, f.scratch));
+    VEXT_CUDA(cudaEventRecord(sys->ev[5], stream));   // timed as one (far) sum
+    sys->split_timed = true;
     VEXT_TRY(site_enqueue(*sys, f.plan, false, f.scratch, 0, rs->n_ri, sys->d_status, stream));
     return site_energies(f.plan, f.scratch, d_e64, stream);
 }

@@ -334,8 +334,9 @@ __global__ void __launch_bounds__(32 * kSiteWarps, (ADJ ? 16 : 20) / kSiteWarps)
                     const int at = n_shell + __popc(ms & below);
                     q.sxy[at] = make_float4(h.x, h.x, h.y, h.y);
                     q.szc[at] = make_float4(h.z, h.z, tp.x, tp.x);
-                    q.scs[at] = make_float4(-tp.y, taken ? v.rc2f + kBorderTol : v.rc2f - kBorderTol,
-                                            tp.z, __int_as_float(base + lane));
+                    q.scs[at] =
+                        make_float4(-tp.y, taken ? v.rc2f + kBorderTol : v.rc2f - kBorderTol, tp.z,
+                                    __int_as_float(base + lane));
                 }
             } else if (near) {
                 const float4 l = v.lo[off + base + lane];
@@ -428,6 +429,15 @@ __global__ void site_energy_kernel(const double *value, long long S3, int O, dou
 // 35^3 x 64 with clusters of 0.4-1.4 A, forward + adjoint: none by sites 19.6 ms,
 // up to 0.8 A 16.4, up to 1 A or all 16.75.
 constexpr double kSiteRadius = 0.8;
+
+// Images within rc of a site from which on the sum site by site pays: its values
+// pass through memory once more (0.5 ms forward, 0.8 forward + adjoint at 60^3 x
+// 64), its clusters win on the pairs.  Pose by pose against site by site, forward
+// and forward + adjoint, at 60^3 x 64 in a 30 A cell: 70 images 1.36 / 1.93 and
+// 2.39 / 2.98 ms, 140 images 2.45 / 2.29 and 3.66 / 3.48, 280 images 3.71 / 3.37 and
+// 7.40 / 4.83; at 42^3 x 43 in 20 and 28 A cells the ratio is 0.83-0.89 and 1.02-1.04
+// with 70 images, 1.20-1.28 and 1.20-1.31 with 140.
+constexpr double kSiteImages = 110;
 
 // Bytes of scratch beyond which a field is summed pose by pose.
 constexpr long long kSiteScratch = 8LL << 30;
@@ -562,6 +572,11 @@ bool sites_worthwhile(const System &sys, int size, int n_axes, const Options &o,
     if (o.variant || o.batch_shape || o.cb || o.mode != VEXT_MODE_MIXED) return false;
     if (size < 8 || n_axes < 16) return false;   // fewer than four clusters a region
     const long long S3 = (long long)size * size * size;
+    const double *h = sys.H.m;
+    const double volume = h[0] * (h[4] * h[8] - h[5] * h[7]) - h[1] * (h[3] * h[8] - h[5] * h[6]) +
+                          h[2] * (h[3] * h[7] - h[4] * h[6]);
+    if (4.18879 * sys.cutoff * sys.cutoff * sys.cutoff * sys.n_atoms < kSiteImages * volume)
+        return false;
     // scratch: V (and its gradient) at every site, and the expansions' part of it
     if (S3 * n_axes * 2 * (adjoint ? 48 : 12) > kSiteScratch) return false;
     int bi = 0, bj = 0, bk = 0;

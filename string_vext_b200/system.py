@@ -137,9 +137,9 @@ class VextSystem:
         """Forward + adjoint over the field poses (host arrays).  Returns the
         float32 energy [O, S, S, S] and gradient [O, S, S, S, 6] = (dE/dcenter,
         dE/du projected on the plane normal to u).  ``pinned=True`` returns
-        them in page-locked memory (torch's pinned host allocator), which the
-        kernels of the mixed mode write directly: the call then costs about
-        the device time instead of device time plus a copy."""
+        them in page-locked memory (torch's pinned host allocator): large
+        results of the mixed mode are then copied out by slabs of grid planes
+        while the next slab computes."""
         axes = _c(axes)
         n_axes = len(axes)
         if pinned:

@@ -18,7 +18,8 @@ pytestmark = pytest.mark.gpu
 
 CELLS = {"skewed": ([14.0, 12.0, 13.0], [75.0, 85.0, 115.0], 90),
          "flat": ([16.0, 15.0, 3.6], [90.0, 90.0, 120.0], 60),
-         "sparse": ([9.0, 11.0, 8.0], [90.0, 90.0, 90.0], 6),
+         "sparse": ([9.0, 11.0, 8.0], [90.0, 90.0, 90.0], 12),
+         "dilute": ([9.0, 11.0, 8.0], [90.0, 90.0, 90.0], 4),
          "dense": ([11.0, 12.0, 10.0], [80.0, 95.0, 100.0], 220)}
 
 
@@ -107,6 +108,29 @@ def test_fields_by_sites_match_fp64(cell, size, n_axes, masses):
 def test_expansions_at_sites(size, n_axes, masses):
     """Local expansions by matrix product: partial tiles of sites and regions."""
     check(make_case("dense", masses), size, directors(n_axes))
+
+
+def test_batch_of_both_routes():
+    """A system by sites beside a dilute one by poses in one batch."""
+    size, axes = 20, directors(40)
+    shape = (40,) + (size,) * 3
+    with VextSystem(make_case("skewed")) as a, VextSystem(make_case("dilute")) as b:
+        exact = [adjoint(s, size, axes, mode=_lib.VEXT_MODE_FP64_PLAIN) for s in (a, b)]
+        for adj in (False, True):
+            outs = [torch.empty(shape, dtype=torch.float32, device="cuda") for _ in range(2)]
+            grads = [torch.empty(shape + (6,), dtype=torch.float32, device="cuda")
+                     for _ in range(2)]
+            batch = VextBatch([a, b], size, axes, outs, gradients=grads if adj else None)
+            assert batch.info()["cta_shape"] != "64-site clusters"
+            for _ in range(2):
+                batch.run()
+            batch.check()
+            torch.cuda.synchronize()
+            for k, (ex, gx) in enumerate(exact):
+                assert_energy(outs[k].cpu().numpy().astype(np.float64), ex, storage=1.2e-7)
+                if adj:
+                    assert_gradient(grads[k].cpu().numpy().astype(np.float64), gx)
+            batch.close()
 
 
 @pytest.mark.parametrize("r_split", [6.0, 8.5])
