@@ -486,22 +486,13 @@ __global__ void batch_refine_kernel(BatchArgs a) {
     const int count = min(a.refine[0], a.refine_cap);
     for (int q = warp; q < count; q += nwarps) {
         const BatchSys &y = a.sys[a.refine[1 + 2 * q]];
+        if (y.site) continue;
         const long long idx = a.refine[2 + 2 * q];
         const long long S3 = (long long)y.S * y.S * y.S;
         const int o = (int)(idx / S3);
         const long long c = idx % S3;
         const int gi = (int)(c / ((long long)y.S * y.S)), gj = (int)((c / y.S) % y.S),
                   gk = (int)(c % y.S);
-        if (y.site) {
-            double e, g[6];
-            site_pose_fp64(*y.site, o, gi, gj, gk, lane, e, g);
-            e = warp_total(e);
-            if (lane == 0) {
-                y.out[idx] = (float)e;
-                if (y.out64) y.out64[idx] = e;
-            }
-            continue;
-        }
         const RegionInfo r = y.regs[((gi / y.bi) * y.nrj + gj / y.bj) * y.nrk + gk / y.bk];
         double cx, cy, cz;
         frac_to_cart(y.H, (gi + .5) / y.S - r.of[0], (gj + .5) / y.S - r.of[1],
@@ -556,23 +547,20 @@ __global__ void batch_refine_adj_kernel(BatchArgs a) {
         const int tag = a.refine[1 + 2 * q];
         const bool repair = (tag & kRepairOnly) != 0;
         const BatchSys &y = a.sys[tag & ~kRepairOnly];
+        if (y.site) continue;
         const long long idx = a.refine[2 + 2 * q];
         const long long S3 = (long long)y.S * y.S * y.S;
         const int o = (int)(idx / S3);
         const long long c = idx % S3;
         const int gi = (int)(c / ((long long)y.S * y.S)), gj = (int)((c / y.S) % y.S),
                   gk = (int)(c % y.S);
+        const RegionInfo r = y.regs[((gi / y.bi) * y.nrj + gj / y.bj) * y.nrk + gk / y.bk];
+        double cx, cy, cz;
+        frac_to_cart(y.H, (gi + .5) / y.S - r.of[0], (gj + .5) / y.S - r.of[1],
+                     (gk + .5) / y.S - r.of[2], cx, cy, cz);
         const double u[3] = {y.axes[3 * o], y.axes[3 * o + 1], y.axes[3 * o + 2]};
-        double e = 0.0, g[6], cx, cy, cz;
-        RegionInfo r;
-        if (!y.site) {
-            r = y.regs[((gi / y.bi) * y.nrj + gj / y.bj) * y.nrk + gk / y.bk];
-            frac_to_cart(y.H, (gi + .5) / y.S - r.of[0], (gj + .5) / y.S - r.of[1],
-                         (gk + .5) / y.S - r.of[2], cx, cy, cz);
-        }
-        if (y.site)
-            site_pose_fp64(*y.site, o, gi, gj, gk, lane, e, g);
-        else if (repair)
+        double e = 0.0, g[6];
+        if (repair)
             shell_border_repair(y.hi, y.lo, y.td, r.off + r.n_near + r.n_inner,
                                 r.n_total - r.n_near - r.n_inner, lane, 32, y.rc2, y.rc2f,
                                 y.off0, y.off1, cx, cy, cz, u, e, g);
@@ -604,6 +592,43 @@ __global__ void batch_refine_adj_kernel(BatchArgs a) {
                 gd[1] = make_float2((float)g[2], (float)g[3]);
                 gd[2] = make_float2((float)g[4], (float)g[5]);
             }
+        }
+    }
+}
+
+// The flagged poses of systems summed site by site (in a kernel of its own: as
+// a branch of the two above it took registers from them, 73 -> 114 and 112 -> 195
+// us for a dilute framework's poses in the band).
+template <bool ADJ>
+__global__ void batch_refine_sites_kernel(BatchArgs a) {
+    const int lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const int count = min(a.refine[0], a.refine_cap);
+    for (int q = warp; q < count; q += nwarps) {
+        const BatchSys &y = a.sys[a.refine[1 + 2 * q] & ~kRepairOnly];
+        if (!y.site) continue;
+        const long long idx = a.refine[2 + 2 * q];
+        const long long S3 = (long long)y.S * y.S * y.S, c = idx % S3;
+        const int o = (int)(idx / S3);
+        double e, g[6];
+        site_pose_fp64(*y.site, o, (int)(c / ((long long)y.S * y.S)), (int)((c / y.S) % y.S),
+                       (int)(c % y.S), lane, e, g);
+        e = warp_total(e);
+        if constexpr (ADJ) {
+#pragma unroll
+            for (int k = 0; k < 6; ++k) g[k] = warp_total(g[k]);
+        }
+        if (lane != 0) continue;
+        y.out[idx] = (float)e;
+        if (y.out64) y.out64[idx] = e;
+        if constexpr (ADJ) {
+            const double u[3] = {y.axes[3 * o], y.axes[3 * o + 1], y.axes[3 * o + 2]};
+            fp64_tangent(u, g);
+            float2 *gd = reinterpret_cast<float2 *>(y.grad + 6 * idx);
+            gd[0] = make_float2((float)g[0], (float)g[1]);
+            gd[1] = make_float2((float)g[2], (float)g[3]);
+            gd[2] = make_float2((float)g[4], (float)g[5]);
         }
     }
 }
@@ -902,8 +927,15 @@ static BatchArgs batch_args(vext_batch b, const int4 *items, int n_items) {
 }
 
 static int launch_refine(vext_batch b, const BatchArgs &a, cudaStream_t st) {
-    if (b->adj) batch_refine_adj_kernel<<<1184, 256, 0, st>>>(a);
-    else if (b->opt.band_hi > b->opt.band_lo) batch_refine_kernel<<<1184, 256, 0, st>>>(a);
+    const bool band = b->opt.band_hi > b->opt.band_lo;
+    if (b->n_items) {
+        if (b->adj) batch_refine_adj_kernel<<<1184, 256, 0, st>>>(a);
+        else if (band) batch_refine_kernel<<<1184, 256, 0, st>>>(a);
+    }
+    if (b->d_sites && band) {
+        if (b->adj) batch_refine_sites_kernel<true><<<1184, 256, 0, st>>>(a);
+        else batch_refine_sites_kernel<false><<<1184, 256, 0, st>>>(a);
+    }
     VEXT_CUDA(cudaGetLastError());
     return 0;
 }
@@ -1329,6 +1361,7 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
     VEXT_CUDA(end);
     b->graph = g;
     VEXT_CUDA(cudaGraphInstantiate(&b->exec, b->graph, 0));
+    VEXT_CUDA(cudaStreamSynchronize(b->stream));   // the plans, for replays on any stream
     *out = guard.release();
     return 0;
 }

@@ -256,7 +256,7 @@ __device__ __forceinline__ void take_shell(const SiteQueue &q, int n, const Site
 // instead of adding the many that lie inside (in all: layered adjoint 12.5 ->
 // 11.2 ms; up to rc - 0.4 radius of the region 11.5, to rc + 0.3 radius 11.5).
 //
-// 60^3 x 64 layered forward + adjoint: 8.7 of 11.2 ms (pose by pose, on lists
+// 60^3 x 64 layered forward + adjoint: 8.8 of 11.2 ms (pose by pose, on lists
 // about regions of poses, 18.1 in all), about 1.3 of it classification and 3.6
 // near entries.  Bound by the latency of the FP64 and FP32 chains at 16 warps
 // per SM (issue slots 57 %, FP64 pipe 33 %, FMA pipe 39 % busy; 20 warps with
@@ -570,7 +570,8 @@ static void site_layout(const System &sys, const RegionSet &rs, int n_axes, cons
 bool sites_worthwhile(const System &sys, int size, int n_axes, const Options &o, bool adjoint) {
     // pinned kernels and region sizes keep the sum pose by pose
     if (o.variant || o.batch_shape || o.cb || o.mode != VEXT_MODE_MIXED) return false;
-    if (size < 8 || n_axes < 16) return false;   // fewer than four clusters a region
+    // fewer than four clusters a region; a plan of more than 0.25 GB
+    if (size < 8 || n_axes < 16 || n_axes > 1024) return false;
     const long long S3 = (long long)size * size * size;
     const double *h = sys.H.m;
     const double volume = h[0] * (h[4] * h[8] - h[5] * h[7]) - h[1] * (h[3] * h[8] - h[5] * h[6]) +
@@ -616,7 +617,8 @@ int site_plan_build(const System &sys, const RegionSet &rs, int n_axes, const do
     char *base = static_cast<char *>(plan.arena);
     VEXT_TRY(ensure_capacity(base, plan.arena_cap, bytes));
     plan.arena = base;
-    VEXT_CUDA(cudaMemcpy(base, up.data(), bytes, cudaMemcpyHostToDevice));
+    // in stream order: calls before this one may still read the old plan
+    VEXT_CUDA(cudaMemcpyAsync(base, up.data(), bytes, cudaMemcpyHostToDevice, stream));
     SiteView &v = plan.view;
     v.H = sys.H;
     v.rc2 = sys.cutoff * sys.cutoff;
@@ -652,7 +654,7 @@ int site_plan_build(const System &sys, const RegionSet &rs, int n_axes, const do
     v.poly = nullptr;
     v.eval = nullptr;
     // an expansion costs about 1,000 operations an entry and 140 an output (the
-    // 28,800 regions of the 60^3 x 64 layered field: 1.56 and 0.49 ms); it takes 12
+    // 28,800 regions of the 60^3 x 64 layered field: 1.83 and 0.44 ms); it takes 12
     // (forward 9) off every (site, entry) pair
     const double n = (double)rs.n_taylor / std::max(rs.n_regions, 1);
     if (taylor_allowed(sys, rs) && n * v.n_sites * (adjoint ? 12.0 : 9.0) >

@@ -149,7 +149,8 @@ __device__ __forceinline__ void role_entries(const SumArgs &s, const float4 *hi,
 
 // n entries, the first `n_full` of which need every degree.  The others, four
 // fifths of a fine grid's, take a third of the sums: 2.17 -> 1.55 ms for the
-// 28,800 regions of the 60^3 x 64 layered field (the whole field 14.67 -> 14.08
+// 28,800 regions of the 60^3 x 64 layered field (1.83 with the shell entries that
+// the expansion has held since; the whole field 14.67 -> 14.08
 // ms; with order 7, which starts farther out, 14.21, with 9 14.20).
 template <int ROLE>
 __device__ __forceinline__ void role_sum(const SumArgs &s, const float4 *hi, int n_full, int n,

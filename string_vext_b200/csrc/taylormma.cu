@@ -1,7 +1,7 @@
 // The matrix product of taylormma.cuh on the fifth-generation tensor cores.
 //
 // 4,096 rows x 28,800 regions x 448 sums (60^3 x 64 layered field, forward +
-// adjoint): 0.49 ms, 317 GFLOP in three TF32 products, against 2.06 ms as packed
+// adjoint): 0.44 ms, 317 GFLOP in three TF32 products, against 2.06 ms as packed
 // FP32 FMA (taylor_eval_kernel's tiles) that two thirds of the FMA pipe bounded.
 // Bound by the tensor pipe, 73 % of its cycles active (44^3), then by the
 // operands' way from L2: 96 KB a chunk of 32 sums against about 1,600 cycles of
