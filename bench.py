@@ -48,12 +48,11 @@ from string_vext_b200 import ranks  # noqa: E402  (no CUDA work at import)
 FLOP_FWD = 16          # algorithmic FLOP per in-cutoff (site, image) pair, forward
 FLOP_FWD_ADJ = 28      # forward + adjoint
 METRIC = "Vext pose evals/s at <=1e-4 K vs FP64, fwd+adjoint evals/s; % FP32 peak"
-# dram__bytes_read.sum + dram__bytes_write.sum of one field_far2_kernel launch on
-# full_field, from an ncu capture (--set full) of `bench.py --profile field`.
-FAR_DRAM_BYTES_FULL_FIELD = 776_213_504 + 100_771_584
-# the same for one forward + adjoint batch_field_kernel launch on full_field,
-# from an ncu capture (--set full) of `bench.py --profile adjoint`.
-ADJ_DRAM_BYTES_FULL_FIELD = 771_922_688 + 367_529_216
+# dram__bytes_read.sum + dram__bytes_write.sum of the kernels of one forward
+# field's sum on full_field (expansions, clusters, energies; ncu).
+FAR_DRAM_BYTES_FULL_FIELD = 1_087_278_432 + 372_915_200
+# the same for one forward + adjoint step (expansions, clusters, poses).
+ADJ_DRAM_BYTES_FULL_FIELD = 2_798_525_440 + 1_698_379_520
 CPU_CENTERS_PER_CORE_S = 900.0   # reference driver throughput estimate used to size the sample
 
 
@@ -376,10 +375,10 @@ def run_ours(args, rank, world, local_rank):
                                         "(forward + adjoint) per field",
                          "traffic": (ADJ_DRAM_BYTES_FULL_FIELD
                                      if args.workload == "full_field" else None),
-                         "traffic_unit": "bytes per launch (ncu dram__bytes_read+write)",
-                         "bound_note": "non-tensor FP32 SIMT pipe: pairwise LJ is not a dense "
-                                       "contraction, so neither the HBM nor the tensor-core "
-                                       "roofline applies; see hbm_check",
+                         "traffic_unit": "bytes per step (ncu dram__bytes_read+write)",
+                         "bound_note": "FP32 and FP64 pipes of the pair sums (latency-bound); the "
+                                       "expansions' product runs on the tensor cores; see "
+                                       "hbm_check",
                          "hbm_check": hbm_check(ADJ_DRAM_BYTES_FULL_FIELD
                                                 if args.workload == "full_field" else None,
                                                 ms_step),
