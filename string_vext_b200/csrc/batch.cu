@@ -1228,8 +1228,8 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
     for (int k = 0; k < n_systems; ++k) {
         if (!by_site[k]) continue;
         if (!b->d_sites) VEXT_CUDA(device_malloc(&b->d_sites, sizeof(SiteView) * n_systems));
-        VEXT_TRY(site_plan_build(systems[k]->sys, *b->lists[k], n_axes, axes, b->d_axes, b->adj,
-                                 b->sites[k], b->stream));
+        VEXT_TRY(site_plan_build(systems[k]->sys, *b->lists[k], n_axes, axes, b->adj, b->sites[k],
+                                 b->stream));
         VEXT_TRY(site_scratch_reserve(b->sites[k], b->adj, b->site_scratch));
         views[k] = b->sites[k].view;
         hs[k].site = b->d_sites + k;

@@ -766,13 +766,13 @@ int launch_field(System *sys, const RegionSet *rs, int n_axes, const double *axe
 // The site-by-site sum into e64 (sites.cuh), its plan kept for the last
 // (lists, directors).
 static int launch_sites(System *sys, const RegionSet *rs, int n_axes, const double *axes_host,
-                        const double *d_axes, double *d_e64, cudaStream_t stream) {
+                        double *d_e64, cudaStream_t stream) {
     if (!sys->site_field) sys->site_field = new SiteField();
     SiteField &f = *sys->site_field;
     if (f.plan.rs != rs || f.axes.size() != 3 * (size_t)n_axes ||
         !std::equal(axes_host, axes_host + 3 * n_axes, f.axes.begin())) {
         f.plan.rs = nullptr;
-        VEXT_TRY(site_plan_build(*sys, *rs, n_axes, axes_host, d_axes, false, f.plan, stream));
+        VEXT_TRY(site_plan_build(*sys, *rs, n_axes, axes_host, false, f.plan, stream));
         f.axes.assign(axes_host, axes_host + 3 * n_axes);
     }
     VEXT_TRY(site_scratch_reserve(f.plan, false, f.scratch));
@@ -820,7 +820,7 @@ static int field_device(System *sys, int size, int n_axes, const double *axes_ho
     const FieldArgs a = make_args(sys, rs, n_axes, sys->d_axes, sys->d_e64);
     VEXT_CUDA(cudaEventRecord(sys->ev[0], stream));
     if (by_site)
-        VEXT_TRY(launch_sites(sys, rs, n_axes, axes_host, sys->d_axes, sys->d_e64, stream));
+        VEXT_TRY(launch_sites(sys, rs, n_axes, axes_host, sys->d_e64, stream));
     else
         VEXT_TRY(launch_field(sys, rs, n_axes, axes_host, sys->d_axes, sys->d_e64, cb,
                           o.mode == VEXT_MODE_FP64_PLAIN   ? kPlainVariant

@@ -594,7 +594,7 @@ int get_site_regions(System *sys, int size, int block, double r_split, RegionSet
 }
 
 int site_plan_build(const System &sys, const RegionSet &rs, int n_axes, const double *axes,
-                    const double *d_axes, bool adjoint, SitePlan &plan, cudaStream_t stream) {
+                    bool adjoint, SitePlan &plan, cudaStream_t stream) {
     SiteLayout l;
     site_layout(sys, rs, n_axes, axes, l);
     size_t bytes = 0;
@@ -632,7 +632,6 @@ int site_plan_build(const System &sys, const RegionSet &rs, int n_axes, const do
     v.floor_out = std::sqrt(fl);
     v.S = rs.size;
     v.O = n_axes;
-    v.axes = d_axes;
     v.regs = rs.d_info;
     v.hi = rs.d_hi;
     v.lo = rs.d_lo;

@@ -28,7 +28,6 @@ struct SiteView {
     float rc, rc2f;
     double floor_out;           // site-atom distance beyond which no contact floor applies
     int S, O;
-    const double *axes;         // [O][3]
     const RegionInfo *regs;     // regions of voxels
     const float4 *hi, *lo;
     const float4 *tf;
@@ -98,7 +97,7 @@ int get_site_regions(System *sys, int size, int block, double r_split, RegionSet
 constexpr int kBatchVoxels = 8, kFieldVoxels = 16;
 
 int site_plan_build(const System &sys, const RegionSet &rs, int n_axes, const double *axes,
-                    const double *d_axes, bool adjoint, SitePlan &plan, cudaStream_t stream);
+                    bool adjoint, SitePlan &plan, cudaStream_t stream);
 
 int site_scratch_reserve(const SitePlan &plan, bool adjoint, SiteScratch &scratch);
 

@@ -27,8 +27,10 @@ constexpr int kTaylorPoly = 20;      // its coefficients
 constexpr int kTaylorPolyPad = 24;   // doubles per region
 
 // Expected entries per region below which lists are built without a class for
-// the expansion (forward fields begin to gain from about 40).
-constexpr double kTaylorMinEntries = 40;
+// the expansion: site lists gain from about 40; lists for poses need 120 before
+// forward + adjoint takes the expansion (taylor_worthwhile), and sorted lists
+// that do without it lose 2 % to their shorter partial sums (list_flush).
+constexpr double kTaylorMinEntries = 40, kTaylorMinEntriesPoses = 120;
 
 // Columns |m| of the expansion that one warp sums (balanced: 66-76 sums).
 constexpr int kTaylorRoles = 6;
