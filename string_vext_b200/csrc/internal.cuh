@@ -27,7 +27,8 @@ namespace vext {
 
 // Device memory (memory.cu).  Allocations come from a pool per device that
 // keeps up to kPoolKeep bytes of what was freed; device_free waits for the
-// device first, as cudaFree does.
+// device first, as cudaFree does (a block whose wait is refused, during a stream
+// capture, is kept for the next free).
 cudaError_t device_malloc_bytes(void **p, size_t bytes);
 template <typename T>
 cudaError_t device_malloc(T **p, size_t bytes) {
