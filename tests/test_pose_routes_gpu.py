@@ -1,0 +1,138 @@
+"""Calls that are summed pose by pose although finer ones go site by site:
+local expansions in forward + adjoint, page-locked outputs by slabs of work
+items, and String paths too long for the cooperative loop, which iterate by
+graphs.  The bars are the mixed mode's: 1e-4 K where E <= 0, 1e-6 relative
+above, gradients 1e-5 relative (floor 1 K/A); the String iteration is held to
+its CPU restatement as in the other String tests."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import string_oracle
+from string_vext_b200 import _lib, synth
+from string_vext_b200.orientation import normalized_directors
+from string_vext_b200.string_path import euler_from_quaternions, run_string
+from string_vext_b200.system import VextBatch, VextSystem
+
+pytestmark = pytest.mark.gpu
+
+
+def directors(n):
+    return normalized_directors(np.random.default_rng(n).normal(size=(n, 3)))
+
+
+def random_case(lengths, angles, n, masses=None):
+    rng = np.random.default_rng(n)
+    kind = rng.integers(0, 4, n)
+    case = synth.make_case(lengths, angles, rng.random((n, 3)), synth.TYPE_TABLE[kind, 1],
+                           synth.TYPE_TABLE[kind, 0], synth.GUEST_A, 12.8)
+    if masses:
+        case["guest_mass"], case["total_mass"] = np.array(masses), float(sum(masses))
+    return case
+
+
+def dense(masses=None):
+    return random_case([11.0, 12.0, 10.0], [80.0, 95.0, 100.0], 220, masses)
+
+
+def dilute():
+    return random_case([9.0, 11.0, 8.0], [90.0, 90.0, 90.0], 4)
+
+
+def layered(masses=None):
+    case = synth.full_field()
+    if masses:
+        case["guest_mass"], case["total_mass"] = np.array(masses), float(sum(masses))
+    return case
+
+
+def assert_energy(got, exact, storage=0.0):
+    err = np.abs(got - exact) - storage * np.abs(exact)
+    neg = exact <= 0
+    assert err[neg].max(initial=0) < 1e-4
+    assert (err / np.maximum(np.abs(exact), 1))[~neg].max(initial=0) < 1e-6
+
+
+def assert_gradient(got, exact):
+    err = np.linalg.norm(got - exact, axis=-1) / np.maximum(np.linalg.norm(exact, axis=-1), 1.0)
+    assert err.max() < 1e-5
+
+
+def adjoint(system, size, axes, **options):
+    shape = (len(axes),) + (size,) * 3
+    exact = options.get("mode") == _lib.VEXT_MODE_FP64_PLAIN
+    e = None if exact else torch.empty(shape, dtype=torch.float32, device="cuda")
+    g = None if exact else torch.empty(shape + (6,), dtype=torch.float32, device="cuda")
+    e64 = torch.empty(shape, dtype=torch.float64, device="cuda")
+    g64 = torch.empty(shape + (6,), dtype=torch.float64, device="cuda") if exact else None
+    system.field_adjoint_device(size, axes, e, g, e64, g64, **options)
+    torch.cuda.synchronize()
+    return e64.cpu().numpy(), (g64 if exact else g).cpu().numpy().astype(np.float64)
+
+
+@pytest.mark.parametrize("masses", [None, (15.0, 25.0)])
+@pytest.mark.parametrize("maker,size,n_axes,options", [
+    (dense, 13, 64, {"centers_per_region": 8}), (dense, 16, 33, {"centers_per_region": 8}),
+    (dense, 21, 65, {"centers_per_region": 8}), (layered, 21, 25, {})])
+def test_adjoint_expansions_pose_by_pose(maker, size, n_axes, options, masses):
+    axes = directors(n_axes)
+    with VextSystem(maker(masses)) as system:
+        ex, gx = adjoint(system, size, axes, mode=_lib.VEXT_MODE_FP64_PLAIN)
+        e, g = adjoint(system, size, axes, **options)
+        assert_energy(e, ex)
+        assert_gradient(g, gx)
+        # a batch of it, replayed
+        out = torch.empty(e.shape, dtype=torch.float32, device="cuda")
+        grad = torch.empty(g.shape, dtype=torch.float32, device="cuda")
+        batch = VextBatch([system], size, axes, [out], gradients=[grad], **options)
+        assert batch.info()["cta_shape"] != "64-site clusters"
+        for _ in range(2):
+            batch.run()
+        batch.check()
+        torch.cuda.synchronize()
+        assert_energy(out.cpu().numpy().astype(np.float64), ex, storage=1.2e-7)
+        assert_gradient(grad.cpu().numpy().astype(np.float64), gx)
+        batch.close()
+
+
+@pytest.mark.parametrize("maker,size,n_axes,options", [
+    (dilute, 41, 90, {}), (dense, 33, 70, {"centers_per_region": 8})])
+def test_slabs_pose_by_pose(maker, size, n_axes, options):
+    """Page-locked outputs of two and more slabs, without and with local
+    expansions (which the first slab evaluates for all): the device entry's
+    bits, twice, and the FP64 values."""
+    axes = directors(n_axes)
+    shape = (n_axes,) + (size,) * 3
+    with VextSystem(maker()) as system:
+        ex, gx = adjoint(system, size, axes, mode=_lib.VEXT_MODE_FP64_PLAIN)
+        e = torch.empty(shape, dtype=torch.float32, device="cuda")
+        g = torch.empty(shape + (6,), dtype=torch.float32, device="cuda")
+        system.field_adjoint_device(size, axes, e, g, **options)
+        torch.cuda.synchronize()
+        for _ in range(2):
+            he, hg = system.field_adjoint(size, axes, pinned=True, **options)
+            np.testing.assert_array_equal(he, e.cpu().numpy())
+            np.testing.assert_array_equal(hg, g.cpu().numpy())
+        assert_energy(he.astype(np.float64), ex, storage=1.2e-7)
+        assert_gradient(hg.astype(np.float64), gx)
+
+
+@pytest.mark.parametrize("n_images", [296, 297, 400])
+def test_long_paths_match_cpu_restatement(n_images):
+    """The longest path of the cooperative loop and paths by graphs, plain and
+    checked iterations."""
+    case, frac, quat, _, _ = synth.string_path()
+    path = np.column_stack([frac, np.mod(euler_from_quaternions(quat), 2 * np.pi)])
+    at = np.linspace(0, len(path) - 1, n_images)
+    low = np.minimum(at.astype(int), len(path) - 2)
+    s = path[low] + (at - low)[:, None] * (path[low + 1] - path[low])
+    with VextSystem(case) as system:
+        gpu, e_gpu, res = run_string(system, s, mode=_lib.VEXT_MODE_FP64, direction=3,
+                                     max_iterations=4, check_every=2, conv_trans_percent=0.0)
+    ref = s.copy()
+    for _ in range(4):
+        ref = string_oracle.iteration(case, ref, direction=3)[0]
+    assert res["iterations"] == 4 and not res["converged"]
+    np.testing.assert_allclose(gpu[:, :3], ref[:, :3], rtol=0, atol=1e-10)
+    np.testing.assert_allclose(gpu[:, 3:], ref[:, 3:], rtol=0, atol=1e-9)
+    np.testing.assert_allclose(e_gpu, string_oracle.pose_energy(case, gpu), rtol=1e-10, atol=1e-8)
