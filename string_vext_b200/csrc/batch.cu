@@ -58,9 +58,8 @@ struct BatchSys {
     int bi, bj, bk, nrj, nrk;   // region grid (pose -> region)
     float *out;                 // [O][S^3]
     float *grad;                // [O][S^3][6] (forward + adjoint batches), else null
-    float *init, *init_grad;    // where the local expansions' values stand (out and grad, or
-                                // device scratch when those are host memory)
-    const double *poly;         // [regions][kTaylorPolyPad], or null: inner pairs are summed here
+    const double *poly;         // local expansions [regions][kTaylorPolyPad], whose further
+                                // degrees stand in out and grad; null: inner pairs are summed here
     double *out64;              // FP64 copy of the energies [O][S^3], or null
     const SiteView *site;       // summed site by site (sites.cuh; no items), or null
 };
@@ -103,8 +102,8 @@ __device__ __forceinline__ void add_expansion(const BatchSys &y, int reg, long l
     double a[3], b[3];
     e += taylor_poly_grad(p, cx + y.off0 * u[0], cy + y.off0 * u[1], cz + y.off0 * u[2], a) +
          taylor_poly_grad(p, cx + y.off1 * u[0], cy + y.off1 * u[1], cz + y.off1 * u[2], b);
-    e += (double)y.init[idx];
-    const float2 *gi = reinterpret_cast<const float2 *>(y.init_grad + 6 * idx);
+    e += (double)y.out[idx];
+    const float2 *gi = reinterpret_cast<const float2 *>(y.grad + 6 * idx);
     const float2 g0 = gi[0], g1 = gi[1], g2 = gi[2];
     const double w[3] = {y.off0 * a[0] + y.off1 * b[0], y.off0 * a[1] + y.off1 * b[1],
                          y.off0 * a[2] + y.off1 * b[2]};
@@ -368,7 +367,7 @@ __global__ void __launch_bounds__(CB *G, MINB) batch_field_kernel(BatchArgs a) {
                 if (EXPAND && y.poly && cvalid && obase + G * p < y.O) {
                     const double *tp = y.poly + (size_t)w.y * kTaylorPolyPad;
                     e[p] += taylor_pair(tp, cx, cy, cz, y.off0, y.off1, ux[p], uy[p], uz[p]);
-                    e[p] += (double)y.init[pose_index(y, obase + G * p, gi, gj, gk)];
+                    e[p] += (double)y.out[pose_index(y, obase + G * p, gi, gj, gk)];
                 }
             }
         }
@@ -841,10 +840,8 @@ struct vext_batch_s {
     Options opt;
     BatchSys *d_sys = nullptr;
     struct Target {   // (the layout of these words in BatchSys)
-        float *out, *grad, *init, *init_grad;
-        bool operator==(const Target &o) const {
-            return out == o.out && grad == o.grad && init == o.init && init_grad == o.init_grad;
-        }
+        float *out, *grad;
+        bool operator==(const Target &o) const { return out == o.out && grad == o.grad; }
     };
     std::vector<Target> targets;          // current outputs of each system
     std::vector<TaylorPlan> plans;        // local expansions (poly null: none)
@@ -964,8 +961,7 @@ static int batch_launch(vext_batch b, const BatchConfig &cfg, const int4 *items,
         if (!b->plans[k].poly) continue;
         const System &sys = b->systems[k]->sys;
         VEXT_TRY(taylor_enqueue(sys, *b->lists[k], b->n_axes, b->plans[k], batch_trims(b, sys),
-                                b->d_sums, &b->d_sys[k].init, nullptr, &b->d_sys[k].init_grad,
-                                st));
+                                b->d_sums, &b->d_sys[k].out, nullptr, &b->d_sys[k].grad, st));
     }
     const BatchArgs a = batch_args(b, items, n_items);
     const size_t smem = batch_smem(b->max_types, b->adj);
@@ -1001,7 +997,7 @@ static std::map<TuneKey, TunePick> g_tune_cache;
 // pick for this class (the pick is then replaced)
 constexpr int kVariantTuneAfresh = 2048;
 
-static bool device_memory(const void *p) {
+bool device_memory(const void *p) {
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();
@@ -1013,13 +1009,12 @@ static bool device_memory(const void *p) {
 // Shared by vext_batch_create, vext_batch_create_adjoint and the cached
 // one-system batch of vext_field_adjoint_device (which already holds its
 // system's lock: lock_systems = false, and says with `rule_axes` how many
-// directors the whole call has and with `init` where expansion values may
-// stand when the outputs are host memory; slabs > 1 orders the queue of a
-// one-system batch for batch_run_slab).
+// directors the whole call has; slabs > 1 orders the queue of a one-system batch
+// for batch_run_slab).
 int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
                 const double *axes, const vext_options *opt, float *const *outputs,
                 float *const *gradients, double *const *outputs_f64, bool lock_systems,
-                vext_batch *out, int rule_axes, float *const *init, int slabs) {
+                vext_batch *out, int rule_axes, int slabs) {
     if (!out || n_systems < 1 || !systems || !outputs || size < 1 || n_axes < 1 || !axes)
         return fail(VEXT_ERR_ARGUMENT, "bad batch arguments");
     for (int k = 0; k < n_systems; ++k)
@@ -1133,8 +1128,6 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
         y.nrk = rs->n_rk;
         y.out = outputs[k];
         y.grad = gradients ? gradients[k] : nullptr;
-        y.init = init ? init[0] : y.out;
-        y.init_grad = init ? init[1] : y.grad;
         y.poly = nullptr;
         y.out64 = outputs_f64 ? outputs_f64[k] : nullptr;
         y.site = nullptr;
@@ -1207,7 +1200,8 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
         for (const BatchSys &y : hs)
             if (y.off0 == 0.0 || y.off1 != -y.off0) b->kind = 9;
     // local expansions: the kinds whose kernels use them, where the rule of
-    // taylor_worthwhile says so and their values can stand in device memory
+    // taylor_worthwhile says so and the outputs, where their values stand first,
+    // are device memory
     b->plans.resize(n_systems);
     const bool expands = b->kind == 0 || b->kind == 6 || b->kind == 7 || b->kind == 9 ||
                          b->kind == 10;
@@ -1217,7 +1211,7 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
         const RegionSet &rs = *b->lists[k];
         if (by_site[k] || !expands ||
             !taylor_worthwhile(sys, rs, rule_axes ? rule_axes : n_axes, b->adj) ||
-            !device_memory(hs[k].init) || (b->adj && !device_memory(hs[k].init_grad)))
+            !device_memory(hs[k].out) || (b->adj && !device_memory(hs[k].grad)))
             continue;
         VEXT_TRY(taylor_prepare(sys, rs, n_axes, b->d_axes, b->adj, b->plans[k], b->stream));
         VEXT_TRY(ensure_capacity(b->d_sums, b->sums_cap, taylor_workspace(rs)));
@@ -1247,7 +1241,7 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
     if (b->d_sites)
         VEXT_CUDA(cudaMemcpy(b->d_sites, views.data(), sizeof(SiteView) * n_systems,
                              cudaMemcpyHostToDevice));
-    for (const BatchSys &y : hs) b->targets.push_back({y.out, y.grad, y.init, y.init_grad});
+    for (const BatchSys &y : hs) b->targets.push_back({y.out, y.grad});
     VEXT_CUDA(device_malloc(&b->d_sys, sizeof(BatchSys) * n_systems));
     VEXT_CUDA(cudaMemcpy(b->d_sys, hs.data(), sizeof(BatchSys) * n_systems, cudaMemcpyHostToDevice));
     VEXT_CUDA(device_malloc(&b->d_items, sizeof(int4) * std::max<size_t>(hitems.size(), 1)));
@@ -1372,7 +1366,7 @@ extern "C" int vext_batch_create(int n_systems, const vext_system *systems, int 
                                  int n_axes, const double *axes, const vext_options *opt,
                                  float *const *outputs, vext_batch *out) {
     return batch_build(n_systems, systems, size, n_axes, axes, opt, outputs, nullptr, nullptr,
-                       true, out, 0, nullptr, 1);
+                       true, out, 0, 1);
 }
 
 extern "C" int vext_batch_create_adjoint(int n_systems, const vext_system *systems, int size,
@@ -1381,7 +1375,7 @@ extern "C" int vext_batch_create_adjoint(int n_systems, const vext_system *syste
                                          float *const *gradients, vext_batch *out) {
     if (!gradients) return fail(VEXT_ERR_ARGUMENT, "gradient outputs required");
     return batch_build(n_systems, systems, size, n_axes, axes, opt, energies, gradients, nullptr,
-                       true, out, 0, nullptr, 1);
+                       true, out, 0, 1);
 }
 
 namespace vext {
@@ -1425,22 +1419,16 @@ int batch_slab_status(vext_batch b) {
     return vext_batch_status(b);
 }
 
-// Point system k's float32 energy / gradient outputs at `out` / `grad` (and
-// its expansion values at `init` / `init_grad`) for the replays that follow on
-// `stream`: a stream-ordered update of the device copy of its BatchSys, which
-// the captured kernels read at run time (no rebuild).
-int batch_retarget(vext_batch b, int k, float *out, float *grad, float *init, float *init_grad,
-                   cudaStream_t stream) {
+// Point system k's float32 energy / gradient outputs at `out` / `grad` for the
+// replays that follow on `stream`: a stream-ordered update of the device copy of
+// its BatchSys, which the captured kernels read at run time (no rebuild).
+int batch_retarget(vext_batch b, int k, float *out, float *grad, cudaStream_t stream) {
     if (k < 0 || k >= (int)b->systems.size()) return fail(VEXT_ERR_ARGUMENT, "bad system index");
     if (!out || (b->adj && !grad)) return fail(VEXT_ERR_ARGUMENT, "null output");
     using Target = vext_batch_s::Target;
-    static_assert(offsetof(BatchSys, grad) - offsetof(BatchSys, out) == offsetof(Target, grad) &&
-                      offsetof(BatchSys, init) - offsetof(BatchSys, out) ==
-                          offsetof(Target, init) &&
-                      offsetof(BatchSys, init_grad) - offsetof(BatchSys, out) ==
-                          offsetof(Target, init_grad),
+    static_assert(offsetof(BatchSys, grad) - offsetof(BatchSys, out) == offsetof(Target, grad),
                   "the output words must be adjacent");
-    const Target to{out, b->adj ? grad : nullptr, init, b->adj ? init_grad : nullptr};
+    const Target to{out, b->adj ? grad : nullptr};
     if (b->targets[k] == to) return 0;
     VEXT_CUDA(cudaMemcpyAsync(reinterpret_cast<char *>(b->d_sys + k) + offsetof(BatchSys, out),
                               &to, sizeof to, cudaMemcpyHostToDevice, stream));

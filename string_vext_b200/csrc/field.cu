@@ -964,30 +964,21 @@ static int field_adjoint_device(vext_system h, int size, int n_axes, const doubl
             return fail(VEXT_ERR_ARGUMENT, "the mixed adjoint writes float32 energy and gradient");
         if (gradient_f64)
             return fail(VEXT_ERR_ARGUMENT, "the FP64 gradient needs an FP64 mode");
+        // (outputs in host memory: a batch without local expansions)
+        const bool device = device_memory(energy) && device_memory(gradient);
         const bool same = sys->adj_batch && sys->adj_size == size &&
                           sys->adj_axes.size() == 3 * (size_t)n_axes &&
                           std::equal(axes, axes + 3 * n_axes, sys->adj_axes.begin()) &&
                           sys->adj_key[0] == o.r_split && sys->adj_key[1] == o.band_lo &&
                           sys->adj_key[2] == o.band_hi &&
                           sys->adj_key[3] == batch_key(o) &&
-                          sys->adj_energy64 == energy_f64;
-        // outputs in host memory: expansion values stand in device scratch
-        float *init[2] = {energy, gradient};
-        cudaPointerAttributes at;
-        if (cudaPointerGetAttributes(&at, energy) != cudaSuccess) cudaGetLastError();
-        else if (at.type == cudaMemoryTypeHost) {
-            const size_t n = (size_t)(S3 * n_axes);
-            VEXT_TRY(ensure_capacity(sys->d_f32, sys->f32_cap, n));
-            VEXT_TRY(ensure_capacity(sys->d_g32, sys->g32_cap, 6 * n));
-            init[0] = sys->d_f32;
-            init[1] = sys->d_g32;
-        }
+                          sys->adj_energy64 == energy_f64 && sys->adj_device == device;
         if (!same) {
             if (sys->adj_batch) vext_batch_destroy(sys->adj_batch);   // (host parts stay)
             sys->adj_batch = nullptr;
             vext_batch b = nullptr;
             VEXT_TRY(batch_build(1, &h, size, n_axes, axes, opt, &energy, &gradient,
-                                 energy_f64 ? &energy_f64 : nullptr, false, &b, n_axes, init, 1));
+                                 energy_f64 ? &energy_f64 : nullptr, false, &b, n_axes, 1));
             sys->adj_batch = b;
             sys->adj_size = size;
             sys->adj_axes.assign(axes, axes + 3 * n_axes);
@@ -996,10 +987,11 @@ static int field_adjoint_device(vext_system h, int size, int n_axes, const doubl
             sys->adj_key[2] = o.band_hi;
             sys->adj_key[3] = batch_key(o);
             sys->adj_energy64 = energy_f64;
+            sys->adj_device = device;
         }
         // other float32 outputs than the last call's: a stream-ordered update
         // of the batch's output pointers, no rebuild
-        VEXT_TRY(batch_retarget(sys->adj_batch, 0, energy, gradient, init[0], init[1], stream));
+        VEXT_TRY(batch_retarget(sys->adj_batch, 0, energy, gradient, stream));
         return batch_replay(sys->adj_batch, stream);
     }
     if (o.mode != VEXT_MODE_FP64 && o.mode != VEXT_MODE_FP64_PLAIN)
@@ -1101,14 +1093,13 @@ static int adjoint_pinned(vext_system h, int size, int n_axes, const double *axe
         if (sys->slab_batch) vext_batch_destroy(sys->slab_batch);
         sys->slab_batch = nullptr;
         VEXT_TRY(batch_build(1, &h, size, n_axes, axes, opt, &sys->d_f32, &sys->d_g32, nullptr,
-                             false, &sys->slab_batch, n_axes, nullptr, slabs));
+                             false, &sys->slab_batch, n_axes, slabs));
         sys->slab_size = size;
         sys->slab_count = slabs;
         sys->slab_axes.assign(axes, axes + 3 * n_axes);
         std::copy(key, key + 4, sys->slab_key);
     }
-    VEXT_TRY(batch_retarget(sys->slab_batch, 0, sys->d_f32, sys->d_g32, sys->d_f32, sys->d_g32,
-                            st));
+    VEXT_TRY(batch_retarget(sys->slab_batch, 0, sys->d_f32, sys->d_g32, st));
     // a slab of the [directors][S][S][S] arrays: one row of consecutive planes
     // per director
     auto copy_rows = [&](float *to, const float *from, size_t words, int p0, int p1) {
@@ -1193,7 +1184,7 @@ extern "C" int vext_field_adjoint(vext_system h, int size, int n_axes, const dou
                 float *gk = sys->d_g32 + 6 * blk * (size_t)k * S3;
                 vext_batch b = nullptr;
                 VEXT_TRY(batch_build(1, &h, size, nk, axes + 3 * blk * k, opt, &ek, &gk, nullptr,
-                                     false, &b, n_axes, nullptr, 1));
+                                     false, &b, n_axes, 1));
                 sys->host_parts.push_back(b);
                 cudaEvent_t ev;
                 VEXT_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));

@@ -194,6 +194,7 @@ struct System {
     int adj_size = 0;
     std::vector<double> adj_axes;
     double adj_key[4] = {0, 0, 0, 0};   // r_split, band_lo, band_hi, variant
+    bool adj_device = false;            // outputs in device memory
     double *adj_energy64 = nullptr;
     float *d_g32 = nullptr;          // host-output staging of the float32 gradient
     size_t g32_cap = 0;
@@ -222,12 +223,12 @@ struct System {
 int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
                 const double *axes, const vext_options *opt, float *const *outputs,
                 float *const *gradients, double *const *outputs_f64, bool lock_systems,
-                vext_batch *out, int rule_axes, float *const *init, int slabs);
+                vext_batch *out, int rule_axes, int slabs);
 int batch_replay(vext_batch b, cudaStream_t stream);
 int batch_run_slab(vext_batch b, int k, cudaStream_t stream, int *plane0, int *plane1);
 int batch_slab_status(vext_batch b);
-int batch_retarget(vext_batch b, int k, float *out, float *grad, float *init, float *init_grad,
-                   cudaStream_t stream);
+int batch_retarget(vext_batch b, int k, float *out, float *grad, cudaStream_t stream);
+bool device_memory(const void *p);   // device or managed, not host memory
 
 // Region sets (system.cu)
 int get_field_regions(System *sys, int size, int cb, double r_split, RegionSet **out,

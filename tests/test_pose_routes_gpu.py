@@ -136,3 +136,29 @@ def test_long_paths_match_cpu_restatement(n_images):
     np.testing.assert_allclose(gpu[:, :3], ref[:, :3], rtol=0, atol=1e-10)
     np.testing.assert_allclose(gpu[:, 3:], ref[:, 3:], rtol=0, atol=1e-9)
     np.testing.assert_allclose(e_gpu, string_oracle.pose_energy(case, gpu), rtol=1e-10, atol=1e-8)
+
+
+def test_adjoint_into_host_memory_beside_other_calls():
+    """Device-pointer calls into page-locked memory (both outputs or one) keep
+    their results when the next call of the system starts before they end, and
+    device outputs are as before afterwards."""
+    size, axes, other = 33, directors(70), directors(24)
+    shape = (len(axes),) + (size,) * 3
+    options = {"centers_per_region": 8}
+    with VextSystem(dense()) as system:
+        ex, gx = adjoint(system, size, axes, mode=_lib.VEXT_MODE_FP64_PLAIN)
+        first = adjoint(system, size, axes, **options)
+        system.field(size, other, **options)   # scratch and lists in place
+        for pin_energy, pin_gradient in ((True, True), (False, True), (True, False)):
+            e = torch.empty(shape, dtype=torch.float32, pin_memory=pin_energy,
+                            device="cpu" if pin_energy else "cuda")
+            g = torch.empty(shape + (6,), dtype=torch.float32, pin_memory=pin_gradient,
+                            device="cpu" if pin_gradient else "cuda")
+            for _ in range(2):
+                system.field_adjoint_device(size, axes, e, g, **options)
+                system.field(size, other, **options)
+                torch.cuda.synchronize()
+                assert_energy(e.cpu().numpy().astype(np.float64), ex, storage=1.2e-7)
+                assert_gradient(g.cpu().numpy().astype(np.float64), gx)
+        for a, b in zip(adjoint(system, size, axes, **options), first):
+            np.testing.assert_array_equal(a, b)
