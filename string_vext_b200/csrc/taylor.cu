@@ -412,7 +412,8 @@ __global__ void __launch_bounds__(128) taylor_matrix_kernel(MatrixArgs a, SumInd
 struct EvalArgs {
     const float *matrix;     // [kTaylorPad][rows]
     const float *sums;       // [n_regions][kTaylorPad]
-    int rows, poses, n_regions;
+    int rows, tiles;         // padded row length, tiles of rows
+    int poses, n_regions;
     const RegionInfo *regs;
     int S, O, bi, bj, bk;
     float *const *e32;       // device words holding the output pointers
@@ -441,7 +442,9 @@ __global__ void __launch_bounds__(NT, 2) taylor_eval_kernel(EvalArgs a) {
     // shared-memory load
     const int tid = threadIdx.x, rg = (tid >> 5 & 3) * 4 + (tid >> 3 & 3),
               cg = (tid >> 7) * 8 + (tid & 7);
-    const int row0 = blockIdx.x * TILE, reg0 = blockIdx.y * COLS;
+    // one grid dimension for both: 65,535 region tiles would be 4.2 M regions
+    const int row0 = (int)(blockIdx.x % a.tiles) * TILE,
+              reg0 = (int)(blockIdx.x / a.tiles) * COLS;
     float2 acc[RP][CT];
 #pragma unroll
     for (int i = 0; i < RP; ++i)
@@ -706,11 +709,12 @@ int taylor_enqueue(const System &sys, const RegionSet &rs, int n_axes, const Tay
     a.e32 = e32;
     a.g32 = g32;
     a.e64 = e64;
-    const int tiles = plan.rows / eval_tile(plan.outs);
+    a.tiles = plan.rows / eval_tile(plan.outs);
+    const unsigned blocks = (unsigned)a.tiles * ((rs.n_regions + 63) / 64);
     if (plan.outs == 7)
-        taylor_eval_kernel<7, 128, 8><<<dim3(tiles, (rs.n_regions + 63) / 64), 128, 0, stream>>>(a);
+        taylor_eval_kernel<7, 128, 8><<<blocks, 128, 0, stream>>>(a);
     else
-        taylor_eval_kernel<1, 256, 4><<<dim3(tiles, (rs.n_regions + 63) / 64), 256, 0, stream>>>(a);
+        taylor_eval_kernel<1, 256, 4><<<blocks, 256, 0, stream>>>(a);
     VEXT_CUDA(cudaGetLastError());
     return 0;
 }

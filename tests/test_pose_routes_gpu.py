@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 import torch
 
-from oracle import string_oracle
+from oracle import oracle, string_oracle
 from string_vext_b200 import _lib, synth
 from string_vext_b200.orientation import normalized_directors
 from string_vext_b200.string_path import euler_from_quaternions, run_string
@@ -162,3 +162,20 @@ def test_adjoint_into_host_memory_beside_other_calls():
                 assert_gradient(g.cpu().numpy().astype(np.float64), gx)
         for a, b in zip(adjoint(system, size, axes, **options), first):
             np.testing.assert_array_equal(a, b)
+
+
+def test_expansions_of_more_than_four_million_regions():
+    """More region tiles than one of the smaller grid dimensions holds."""
+    size, axes = 324, directors(32)
+    case = random_case([36.0] * 3, [90.0] * 3, 1100)
+    with VextSystem(case) as system:
+        out = torch.empty((len(axes),) + (size,) * 3, dtype=torch.float32, device="cuda")
+        system.field_device(size, axes, out, centers_per_region=8)
+        torch.cuda.synchronize()
+        rng = np.random.default_rng(5)
+        o = rng.integers(0, len(axes), 2000)
+        at = rng.integers(0, size, (2000, 3))
+        at[:8] = [[i, j, k] for i in (0, size - 1) for j in (0, size - 1) for k in (0, size - 1)]
+        got = out[tuple(torch.from_numpy(x).cuda() for x in (o, *at.T))].cpu().numpy()
+    exact = oracle.pose_energy_grad(case, (at + 0.5) / size @ case["cell"], axes[o])[0]
+    assert_energy(got.astype(np.float64), exact, storage=1.2e-7)
