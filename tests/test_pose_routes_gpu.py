@@ -179,3 +179,26 @@ def test_expansions_of_more_than_four_million_regions():
         got = out[tuple(torch.from_numpy(x).cuda() for x in (o, *at.T))].cpu().numpy()
     exact = oracle.pose_energy_grad(case, (at + 0.5) / size @ case["cell"], axes[o])[0]
     assert_energy(got.astype(np.float64), exact, storage=1.2e-7)
+
+
+@pytest.mark.parametrize("n_axes", [10600, 10800, 1900000])
+def test_many_directors_on_a_small_grid(n_axes):
+    """Directors up to and beyond what an expansion's evaluation matrix holds."""
+    size, axes = 4, directors(n_axes)
+    case = random_case([4.0, 4.2, 3.9], [90.0, 90.0, 90.0], 8)
+    with VextSystem(case) as system:
+        e = torch.empty((n_axes,) + (size,) * 3, dtype=torch.float32, device="cuda")
+        g = torch.empty(tuple(e.shape) + (6,), dtype=torch.float32, device="cuda")
+        free = torch.cuda.mem_get_info()[0]
+        system.field_adjoint_device(size, axes, e, g)
+        torch.cuda.synchronize()
+        assert free - torch.cuda.mem_get_info()[0] < 2 << 30
+        rng = np.random.default_rng(6)
+        o = rng.integers(0, n_axes, 500)
+        at = rng.integers(0, size, (500, 3))
+        where = tuple(torch.from_numpy(x).cuda() for x in (o, *at.T))
+        got, grad = e[where].cpu().numpy(), g[where].cpu().numpy()
+    exact, gc, gu = oracle.pose_energy_grad(case, (at + 0.5) / size @ case["cell"], axes[o])
+    gu = gu - (gu * axes[o]).sum(1)[:, None] * axes[o]
+    assert_energy(got.astype(np.float64), exact, storage=1.2e-7)
+    assert_gradient(grad.astype(np.float64), np.concatenate([gc, gu], 1))
