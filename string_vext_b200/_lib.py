@@ -121,6 +121,8 @@ def load(path=None) -> ctypes.CDLL:
     lib.vext_system_create.restype = ci
     lib.vext_system_destroy.argtypes = [vp]
     lib.vext_system_destroy.restype = ci
+    lib.vext_release_memory.argtypes = []
+    lib.vext_release_memory.restype = ci
     lib.vext_field.argtypes = [vp, ci, ci, vp, ctypes.POINTER(Options), vp, vp, vp, vp, vp,
                                ctypes.POINTER(FieldStats)]
     lib.vext_field.restype = ci

@@ -36,6 +36,9 @@ cudaError_t device_malloc(T **p, size_t bytes) {
 }
 void device_free(void *p);
 
+// Free the list builds' scratch on a device (system.cu).
+void release_build_scratch(int device);
+
 // Copy finished device memory to host memory, through page-locked staging by
 // several threads when `dst` is pageable and large; *finite (when given, FP32
 // data) is cleared if a value is not finite.

@@ -360,3 +360,23 @@ int copy_to_host(void *dst, const void *src, size_t bytes, bool *finite) {
 }
 
 }  // namespace vext
+
+using namespace vext;
+
+extern "C" int vext_release_memory(void) {
+    int device = 0;
+    VEXT_CUDA(cudaGetDevice(&device));
+    release_build_scratch(device);
+    DevicePool &p = device_pool(device);
+    std::lock_guard<std::mutex> guard(p.lock);
+    open_pool(p, device);
+    settle(p);
+    if (p.pool) {
+        VEXT_CUDA(cudaStreamSynchronize(p.stream));
+        VEXT_CUDA(cudaMemPoolTrimTo(p.pool, 0));
+    }
+    if (!p.freed.empty())
+        return fail(VEXT_ERR_CUDA, "%zu blocks may still be in use (a stream capture?)",
+                    p.freed.size());
+    return 0;
+}

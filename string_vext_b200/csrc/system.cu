@@ -345,6 +345,14 @@ struct StreamDrain {
 };
 }  // namespace
 
+void release_build_scratch(int device) {
+    BuildScratch &scratch = build_scratch(device);
+    std::lock_guard<std::mutex> guard(scratch.lock);
+    if (scratch.ptr && current_context_id() == scratch.ctx_id) device_free(scratch.ptr);
+    scratch.ptr = nullptr;
+    scratch.cap = 0;
+}
+
 static int build_lists(System *sys, RegionSet *rs, cudaStream_t stream) {
     BuildScratch &scratch = build_scratch(sys->device);
     std::lock_guard<std::mutex> scratch_guard(scratch.lock);

@@ -17,6 +17,13 @@ def _c(a, dtype=np.float64):
     return np.ascontiguousarray(a, dtype=dtype)
 
 
+def release_memory() -> None:
+    """Give back the device memory that the library keeps for later calls (up to
+    1.5 GiB of what dropped systems and batches held, and list-build scratch) on
+    the current device."""
+    _lib.check(_lib.load().vext_release_memory())
+
+
 class VextSystem:
     """Device-resident framework + guest.  ``case`` uses the reference's case
     dictionary layout (src/string_vext/input.py:49-55)."""

@@ -16,7 +16,9 @@ namespace vext {   // as in string_vext_b200/csrc/internal.cuh
 cudaError_t device_malloc_bytes(void **p, size_t bytes);
 void device_free(void *p);
 int fail(int code, const char *, ...) { return code; }
+void release_build_scratch(int) {}
 }  // namespace vext
+extern "C" int vext_release_memory(void);
 
 // ---------------------------------------------------------------- the runtime
 
@@ -203,10 +205,27 @@ static int refused_wait(size_t bytes) {
     return 0;
 }
 
+// What was freed goes back to the device on request, all of it or with an error.
+static int released() {
+    void *a = take((size_t)300 << 20), *b = take((size_t)300 << 20);
+    const size_t others = mapped() - ((size_t)600 << 20);
+    device_free(a);
+    CHECK(mapped() > others + ((size_t)500 << 20));
+    CHECK(vext_release_memory() == 0);
+    CHECK(mapped() == others + ((size_t)300 << 20) && blocks.count(b));
+    refuse_waits = true;
+    device_free(b);
+    CHECK(vext_release_memory() != 0 && blocks.count(b) && !captures_ended);
+    refuse_waits = false;
+    CHECK(vext_release_memory() == 0 && mapped() == others);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "refused_wait") return refused_wait(1 << 20);
     if (what == "refused_wait_large") return refused_wait((size_t)600 << 20);
+    if (what == "released") return released();
     std::printf("unknown scenario\n");
     return 2;
 }

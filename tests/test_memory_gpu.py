@@ -7,7 +7,7 @@ import torch
 
 from string_vext_b200 import synth
 from string_vext_b200.orientation import normalized_directors
-from string_vext_b200.system import VextSystem
+from string_vext_b200.system import VextSystem, release_memory
 
 pytestmark = pytest.mark.gpu
 
@@ -53,3 +53,21 @@ def test_systems_dropped_beside_another_threads_capture():
     assert len(seen) == 3
     for field in seen:
         np.testing.assert_array_equal(field, expected)
+
+
+def test_release_memory_gives_back_what_dropped_systems_held():
+    case, axes = synth.full_field(), directors(64)
+    release_memory()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    for _ in range(2):
+        with VextSystem(case) as system:
+            kept = system.field(40, axes)["orientation_K"]
+        assert free - torch.cuda.mem_get_info()[0] > 50 << 20   # kept for the next one
+        release_memory()
+        assert abs(free - torch.cuda.mem_get_info()[0]) < 16 << 20
+    with VextSystem(case) as system:
+        release_memory()   # what is in use stays
+        np.testing.assert_array_equal(system.field(40, axes)["orientation_K"], kept)
+        release_memory()
+        np.testing.assert_array_equal(system.field(40, axes)["orientation_K"], kept)
