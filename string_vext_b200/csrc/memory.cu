@@ -248,13 +248,13 @@ struct CopyLanes {
     std::mutex lock;
     char *pinned = nullptr;                      // [kCopyThreads][2][kCopyChunk]
     cudaStream_t stream[kCopyThreads] = {};
-    int device = -1;
+    int device = 0;
     unsigned long long ctx_id = 0;
 };
 
-CopyLanes &copy_lanes() {
-    static CopyLanes lanes;
-    return lanes;
+CopyLanes &copy_lanes(int device) {
+    static CopyLanes lanes[64];
+    return lanes[device & 63];
 }
 
 bool all_finite(const char *bytes, size_t n) {
@@ -264,25 +264,20 @@ bool all_finite(const char *bytes, size_t n) {
     return bad == 0;
 }
 
-// Buffers and streams for the current device; false when there are none.
-bool open_lanes(CopyLanes &l) {
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess) return false;
+// Buffers and streams for `device`, the current one; false when there are none.
+bool open_lanes(CopyLanes &l, int device) {
     const unsigned long long ctx = current_context_id();
     if (l.pinned && ctx == l.ctx_id && device == l.device) return true;
-    if (l.pinned && ctx == l.ctx_id) {
-        for (auto &s : l.stream) cudaStreamDestroy(s);
-        cudaFreeHost(l.pinned);
-    }
-    l.pinned = nullptr;
+    l.pinned = nullptr;   // (went with its context)
     void *p = nullptr;
     if (cudaHostAlloc(&p, 2 * kCopyThreads * kCopyChunk, cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    for (auto &s : l.stream)
-        if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
+    for (int t = 0; t < kCopyThreads; ++t)
+        if (cudaStreamCreateWithFlags(&l.stream[t], cudaStreamNonBlocking) != cudaSuccess) {
             cudaGetLastError();
+            while (t > 0) cudaStreamDestroy(l.stream[--t]);
             cudaFreeHost(p);
             return false;
         }
@@ -328,10 +323,12 @@ int copy_to_host(void *dst, const void *src, size_t bytes, bool *finite) {
         pageable = at.type == cudaMemoryTypeUnregistered;
     else
         cudaGetLastError();
-    CopyLanes &l = copy_lanes();
+    int device = 0;
+    VEXT_CUDA(cudaGetDevice(&device));
+    CopyLanes &l = copy_lanes(device);
     std::unique_lock<std::mutex> guard(l.lock, std::defer_lock);
     if (pageable && bytes >= kCopyDirect) guard.lock();
-    if (!guard.owns_lock() || !open_lanes(l)) {
+    if (!guard.owns_lock() || !open_lanes(l, device)) {
         VEXT_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost));
         if (finite && !all_finite(static_cast<const char *>(dst), bytes)) *finite = false;
         return 0;

@@ -17,6 +17,7 @@ cudaError_t device_malloc_bytes(void **p, size_t bytes);
 void device_free(void *p);
 int fail(int code, const char *, ...) { return code; }
 void release_build_scratch(int) {}
+int copy_to_host(void *dst, const void *src, size_t bytes, bool *finite = nullptr);
 }  // namespace vext
 extern "C" int vext_release_memory(void);
 
@@ -221,11 +222,25 @@ static int released() {
     return 0;
 }
 
+// Large copies from two devices in turn keep their staging buffers.
+static int two_devices() {
+    const size_t bytes = (size_t)6 << 20;
+    char *to = static_cast<char *>(std::malloc(bytes));
+    for (int i = 0; i < 8; ++i) {
+        device = i & 1;
+        std::memset(to, 1, bytes);
+        CHECK(copy_to_host(to, to, bytes) == 0 && to[0] == 0 && to[bytes - 1] == 0);
+    }
+    CHECK(host_allocs - host_frees <= 2);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "refused_wait") return refused_wait(1 << 20);
     if (what == "refused_wait_large") return refused_wait((size_t)600 << 20);
     if (what == "released") return released();
+    if (what == "two_devices") return two_devices();
     std::printf("unknown scenario\n");
     return 2;
 }

@@ -1,6 +1,6 @@
 """The device allocator (string_vext_b200/csrc/memory.cu) on a fake CUDA
 runtime of host memory (tests/fake_cuda.cpp): refused waits, which no GPU test
-brings about, and memory given back."""
+brings about, memory given back, and copies from two devices."""
 import shutil
 import subprocess
 from pathlib import Path
@@ -23,7 +23,8 @@ def fake(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("scenario", ["refused_wait", "refused_wait_large", "released"])
+@pytest.mark.parametrize("scenario", ["refused_wait", "refused_wait_large", "released",
+                                      "two_devices"])
 def test_allocator(fake, scenario):
     run = subprocess.run([str(fake), scenario], capture_output=True, text=True, timeout=60)
     assert run.returncode == 0, run.stdout + run.stderr
