@@ -846,6 +846,7 @@ struct vext_batch_s {
     std::vector<Target> targets;          // current outputs of each system
     std::vector<TaylorPlan> plans;        // local expansions (poly null: none)
     std::vector<const RegionSet *> lists; // each system's region lists
+    std::vector<std::shared_ptr<int>> list_use;
     std::vector<int> slab_items, slab_plane;   // first item (by sites: region plane) and first
                                                // grid plane of each slab, then the ends (see
                                                // batch_run_slab)
@@ -1010,11 +1011,12 @@ bool device_memory(const void *p) {
 // one-system batch of vext_field_adjoint_device (which already holds its
 // system's lock: lock_systems = false, and says with `rule_axes` how many
 // directors the whole call has; slabs > 1 orders the queue of a one-system batch
-// for batch_run_slab).
-int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
-                const double *axes, const vext_options *opt, float *const *outputs,
-                float *const *gradients, double *const *outputs_f64, bool lock_systems,
-                vext_batch *out, int rule_axes, int slabs) {
+// for batch_run_slab).  level: 2 may sum site by site and by expansions, 1 by
+// expansions only, 0 neither; *used: the highest level whose sums it went for.
+static int build_batch(int n_systems, const vext_system *systems, int size, int n_axes,
+                       const double *axes, const vext_options *opt, float *const *outputs,
+                       float *const *gradients, double *const *outputs_f64, bool lock_systems,
+                       vext_batch *out, int rule_axes, int slabs, int level, int *used) {
     if (!out || n_systems < 1 || !systems || !outputs || size < 1 || n_axes < 1 || !axes)
         return fail(VEXT_ERR_ARGUMENT, "bad batch arguments");
     for (int k = 0; k < n_systems; ++k)
@@ -1070,10 +1072,13 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
     // systems summed site by site (all members of a framework, or none)
     std::vector<char> by_site(n_systems, 1);
     for (int k = 0; k < n_systems; ++k)
-        if (!sites_worthwhile(systems[k]->sys, size, rule_axes ? rule_axes : n_axes,
-                                           b->opt, b->adj))
+        if (level < 2 || !sites_worthwhile(systems[k]->sys, size,
+                                           rule_axes ? rule_axes : n_axes, b->opt, b->adj))
             by_site[owner[k]] = 0;
-    for (int k = 0; k < n_systems; ++k) by_site[k] = by_site[owner[k]];
+    for (int k = 0; k < n_systems; ++k) {
+        by_site[k] = by_site[owner[k]];
+        if (by_site[k]) *used = 2;
+    }
     std::vector<RegionSet *> lists(n_systems, nullptr);
     for (int k = 0; k < n_systems; ++k) {
         if (owner[k] != k) continue;
@@ -1087,6 +1092,7 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
                                         sys->stream)
                      : get_field_regions(sys, size, cb, b->opt.r_split, &lists[k], sys->stream));
         b->list_bytes += lists[k]->n_entries * 32;
+        b->list_use.push_back(lists[k]->use);
     }
     {
         size_t n = 0;
@@ -1209,10 +1215,11 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
         b->lists.push_back(lists[owner[k]]);
         const System &sys = systems[k]->sys;
         const RegionSet &rs = *b->lists[k];
-        if (by_site[k] || !expands ||
+        if (by_site[k] || !expands || level < 1 ||
             !taylor_worthwhile(sys, rs, rule_axes ? rule_axes : n_axes, b->adj) ||
             !device_memory(hs[k].out) || (b->adj && !device_memory(hs[k].grad)))
             continue;
+        *used = std::max(*used, 1);
         VEXT_TRY(taylor_prepare(sys, rs, n_axes, b->d_axes, b->adj, b->plans[k], b->stream));
         VEXT_TRY(ensure_capacity(b->d_sums, b->sums_cap, taylor_workspace(rs)));
         hs[k].poly = b->plans[k].poly;
@@ -1358,6 +1365,26 @@ int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
     VEXT_CUDA(cudaStreamSynchronize(b->stream));   // the plans, for replays on any stream
     *out = guard.release();
     return 0;
+}
+
+// build_batch; where the scratch of the faster sums cannot be had, the plainer
+// ones, which do without it.
+int batch_build(int n_systems, const vext_system *systems, int size, int n_axes,
+                const double *axes, const vext_options *opt, float *const *outputs,
+                float *const *gradients, double *const *outputs_f64, bool lock_systems,
+                vext_batch *out, int rule_axes, int slabs) {
+    for (int level = 2;;) {
+        int used = 0;
+        const int rc = build_batch(n_systems, systems, size, n_axes, axes, opt, outputs, gradients,
+                                   outputs_f64, lock_systems, out, rule_axes, slabs, level, &used);
+        if (rc == 0 || used == 0 || !memory_failure(rc)) return rc;
+        level = used - 1;
+        for (int k = 0; used == 2 && k < n_systems; ++k) {
+            std::unique_lock<std::mutex> lock(systems[k]->sys.lock, std::defer_lock);
+            if (lock_systems) lock.lock();
+            drop_idle_site_lists(&systems[k]->sys);
+        }
+    }
 }
 
 }  // namespace vext

@@ -720,9 +720,11 @@ static FieldArgs make_args(System *sys, const RegionSet *rs, int n_axes, const d
 }
 
 // Local expansions (when they pay) into e64, the near kernel adds to them or
-// writes e64, the far kernel adds its sums to it.
+// writes e64, the far kernel adds its sums to it.  *expanded (may be null): whether
+// it went for expansions.
 int launch_field(System *sys, const RegionSet *rs, int n_axes, const double *axes_host,
-                 const double *d_axes, double *d_e64, int cb, int variant, cudaStream_t stream) {
+                 const double *d_axes, double *d_e64, int cb, int variant, cudaStream_t stream,
+                 bool *expanded) {
     FieldArgs a = make_args(sys, rs, n_axes, d_axes, d_e64);
     sys->split_timed = false;
     if (rs->r_split >= 1e29 && variant == kPlainVariant) {            // plain FP64 baseline
@@ -740,7 +742,10 @@ int launch_field(System *sys, const RegionSet *rs, int n_axes, const double *axe
     double rho = 0;
     for (const RegionInfo &r : rs->h_info) rho = std::max(rho, r.rho);
     const int near_mode = rs->r_split + 2.0 * (rho + sys->max_offset) + 1e-6 < sys->cutoff ? 2 : 1;
-    if (variant != 9 && cb != 32 && taylor_worthwhile(*sys, *rs, n_axes, false)) {
+    const long long poses = (long long)rs->size * rs->size * rs->size * n_axes;
+    if (variant != 9 && cb != 32 && poses < sys->no_expansions_from &&
+        taylor_worthwhile(*sys, *rs, n_axes, false)) {
+        if (expanded) *expanded = true;
         TaylorPlan &plan = sys->field_plan;
         if (sys->field_plan_set != rs || sys->field_plan_axes.size() != 3 * (size_t)n_axes ||
             !std::equal(axes_host, axes_host + 3 * n_axes, sys->field_plan_axes.begin())) {
@@ -783,31 +788,23 @@ static int launch_sites(System *sys, const RegionSet *rs, int n_axes, const doub
 }
 
 // Everything on device pointers and `stream`; region lists are built (with
-// a host synchronisation) on first use of (size, shape, r_split).
-static int field_device(System *sys, int size, int n_axes, const double *axes_host,
-                        const Options &o, float *d_oK, double *d_e64_out, float *d_marg,
-                        float *d_site, float *d_grid, cudaStream_t stream,
-                        vext_field_stats *stats) {
-    if (size < 1 || n_axes < 1 || !axes_host)
-        return fail(VEXT_ERR_ARGUMENT, "size >= 1, n_axes >= 1 and axes required");
+// a host synchronisation) on first use of (size, shape, r_split).  *by_site,
+// *expanded: which of the sums with scratch of their own it went for.
+static int field_pass(System *sys, int size, int n_axes, const double *axes_host,
+                      const Options &o, float *d_oK, double *d_e64_out, float *d_marg,
+                      float *d_site, float *d_grid, cudaStream_t stream,
+                      vext_field_stats *stats, bool *by_site, bool *expanded) {
     const long long S3 = (long long)size * size * size;
-    if (S3 * n_axes >= (1LL << 31) - 1)
-        return fail(VEXT_ERR_CAPACITY, "size^3 * n_axes must stay below 2^31");
-    for (int k = 0; k < 3 * n_axes; ++k)
-        if (!std::isfinite(axes_host[k])) return fail(VEXT_ERR_ARGUMENT, "non-finite director");
-    if (o.mode != VEXT_MODE_MIXED && o.mode != VEXT_MODE_FP64 && o.mode != VEXT_MODE_FP64_PLAIN &&
-        o.mode != VEXT_MODE_FP32_NAIVE)
-        return fail(VEXT_ERR_ARGUMENT, "unknown precision mode %d", o.mode);
     const bool fp64 = o.mode != VEXT_MODE_MIXED;   // all-entry region lists
     // regions of 16 grid centers by default (8 or 32 on request; 8 only in the
     // mixed mode): a call that builds its lists pays twice the list work on
     // 8-center regions for 5 % less pair work, so 16 stays the default here
     const int cb = o.cb == 32 ? 32 : o.cb == 8 && !fp64 ? 8 : 16;
     const double r_split = fp64 ? 1e30 : o.r_split;
-    const bool by_site = sites_worthwhile(*sys, size, n_axes, o, false);
+    *by_site = S3 * n_axes < sys->no_sites_from && sites_worthwhile(*sys, size, n_axes, o, false);
     RegionSet *rs = nullptr;
-    VEXT_TRY(by_site ? get_site_regions(sys, size, kFieldVoxels, r_split, &rs, stream)
-                     : get_field_regions(sys, size, cb, r_split, &rs, stream));
+    VEXT_TRY(*by_site ? get_site_regions(sys, size, kFieldVoxels, r_split, &rs, stream)
+                      : get_field_regions(sys, size, cb, r_split, &rs, stream));
     const size_t n = (size_t)S3 * n_axes;
     VEXT_TRY(ensure_capacity(sys->d_axes, sys->axes_cap, 3 * (size_t)n_axes));
     VEXT_TRY(ensure_capacity(sys->d_e64, sys->e64_cap, n));
@@ -819,20 +816,20 @@ static int field_device(System *sys, int size, int n_axes, const double *axes_ho
     VEXT_CUDA(cudaMemsetAsync(sys->d_refine, 0, sizeof(int), stream));
     const FieldArgs a = make_args(sys, rs, n_axes, sys->d_axes, sys->d_e64);
     VEXT_CUDA(cudaEventRecord(sys->ev[0], stream));
-    if (by_site)
+    if (*by_site)
         VEXT_TRY(launch_sites(sys, rs, n_axes, axes_host, sys->d_e64, stream));
     else
         VEXT_TRY(launch_field(sys, rs, n_axes, axes_host, sys->d_axes, sys->d_e64, cb,
                           o.mode == VEXT_MODE_FP64_PLAIN   ? kPlainVariant
                           : o.mode == VEXT_MODE_FP32_NAIVE ? kNaiveVariant
                                                            : o.variant,
-                          stream));
+                          stream, expanded));
     VEXT_CUDA(cudaEventRecord(sys->ev[1], stream));
     if (o.mode == VEXT_MODE_MIXED && o.band_hi > o.band_lo) {
         flag_kernel<<<592, 256, 0, stream>>>(sys->d_e64, (long long)n, o.band_lo, o.band_hi,
                                               sys->d_refine);
         VEXT_CUDA(cudaGetLastError());
-        if (by_site)
+        if (*by_site)
             refine_sites_kernel<<<1184, 256, 0, stream>>>(site_view(sys->site_field->plan),
                                                           sys->d_refine, sys->d_e64);
         else
@@ -873,6 +870,49 @@ static int field_device(System *sys, int size, int n_axes, const double *axes_ho
         stats->epilogue_ms = e_ms;
     }
     return 0;
+}
+
+// field_pass; where the scratch of the faster sums cannot be had, the plainer
+// ones, from then on for fields of this size and larger.
+static int field_device(System *sys, int size, int n_axes, const double *axes_host,
+                        const Options &o, float *d_oK, double *d_e64_out, float *d_marg,
+                        float *d_site, float *d_grid, cudaStream_t stream,
+                        vext_field_stats *stats) {
+    if (size < 1 || n_axes < 1 || !axes_host)
+        return fail(VEXT_ERR_ARGUMENT, "size >= 1, n_axes >= 1 and axes required");
+    const long long S3 = (long long)size * size * size;
+    if (S3 * n_axes >= (1LL << 31) - 1)
+        return fail(VEXT_ERR_CAPACITY, "size^3 * n_axes must stay below 2^31");
+    for (int k = 0; k < 3 * n_axes; ++k)
+        if (!std::isfinite(axes_host[k])) return fail(VEXT_ERR_ARGUMENT, "non-finite director");
+    if (o.mode != VEXT_MODE_MIXED && o.mode != VEXT_MODE_FP64 && o.mode != VEXT_MODE_FP64_PLAIN &&
+        o.mode != VEXT_MODE_FP32_NAIVE)
+        return fail(VEXT_ERR_ARGUMENT, "unknown precision mode %d", o.mode);
+    const long long sites_from = sys->no_sites_from, expansions_from = sys->no_expansions_from;
+    for (;;) {
+        bool by_site = false, expanded = false;
+        const int rc = field_pass(sys, size, n_axes, axes_host, o, d_oK, d_e64_out, d_marg, d_site,
+                                  d_grid, stream, stats, &by_site, &expanded);
+        if (rc == 0) return 0;
+        if (!memory_failure(rc) || !(by_site || expanded)) {
+            sys->no_sites_from = sites_from;
+            sys->no_expansions_from = expansions_from;
+            return rc;
+        }
+        if (by_site) {
+            sys->no_sites_from = S3 * n_axes;
+            site_field_free(sys->site_field);
+            sys->site_field = nullptr;
+            drop_idle_site_lists(sys);
+        } else {
+            sys->no_expansions_from = S3 * n_axes;
+            sys->field_plan.release();
+            sys->field_plan_set = nullptr;
+            device_free(sys->d_sums);
+            sys->d_sums = nullptr;
+            sys->sums_cap = 0;
+        }
+    }
 }
 
 static int check_nonfinite(System *sys, cudaStream_t stream) {

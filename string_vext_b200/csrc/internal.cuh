@@ -18,6 +18,7 @@
 // beyond rc + rho + 1e-3 A of the origin.
 #pragma once
 
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -43,6 +44,9 @@ void release_build_scratch(int device);
 // several threads when `dst` is pageable and large; *finite (when given, FP32
 // data) is cleared if a value is not finite.
 int copy_to_host(void *dst, const void *src, size_t bytes, bool *finite = nullptr);
+
+// Whether a call that failed so may succeed with less device memory.
+inline bool memory_failure(int code) { return code == VEXT_ERR_MEMORY || code == VEXT_ERR_CUDA; }
 
 // Unique id of the calling thread's current context (0 when unavailable).
 unsigned long long current_context_id();
@@ -89,6 +93,7 @@ struct RegionSet {
     double taylor_radius = 0;               // every site of a region lies this near its origin
     RegionInfo *d_info = nullptr;
     float4 *d_hi = nullptr, *d_lo = nullptr;
+    std::shared_ptr<int> use = std::make_shared<int>(0);   // batches on it hold a copy
     std::vector<RegionInfo> h_info;
     long long capacity = 0;                 // allocated entries (hi and lo)
     bool stale = false;                     // rebuild before the next use
@@ -175,6 +180,9 @@ struct System {
     size_t sums_cap = 0;
     // site-by-site sums of the field path (sites.cuh)
     SiteField *site_field = nullptr;
+    // poses from which on the field path does without site-by-site sums and
+    // without expansions, because their scratch could not be had
+    long long no_sites_from = 1LL << 62, no_expansions_from = 1LL << 62;
     // scratch of the pose path
     void *d_pose_scratch = nullptr;
     size_t pose_scratch_cap = 0;
@@ -238,6 +246,9 @@ int get_field_regions(System *sys, int size, int cb, double r_split, RegionSet *
                       cudaStream_t stream);
 int get_block_regions(System *sys, int size, int bi, int bj, int bk, double rho, double offset,
                       bool sites, double r_split, RegionSet **out, cudaStream_t stream);
+// Delete the lists for single sites that neither a batch nor the field path's
+// plan uses (under the system's lock).
+void drop_idle_site_lists(System *sys);
 constexpr double kBinWidth = 0.75;  // pose-bin width between lattice planes (A)
 int get_bin_regions(System *sys, double r_split, RegionSet **out, cudaStream_t stream,
                     double bin_width = kBinWidth);
@@ -317,7 +328,8 @@ int pose_upload_desc(System *sys, const RegionSet *rs, const PoseBatchSys **out)
 
 // Field kernel launcher (field.cu): computes E64 [O][S^3] for all regions.
 int launch_field(System *sys, const RegionSet *rs, int n_axes, const double *axes_host,
-                 const double *d_axes, double *d_e64, int cb, int variant, cudaStream_t stream);
+                 const double *d_axes, double *d_e64, int cb, int variant, cudaStream_t stream,
+                 bool *expanded);
 
 }  // namespace vext
 

@@ -670,13 +670,30 @@ int site_plan_build(const System &sys, const RegionSet &rs, int n_axes, const do
     return 0;
 }
 
+// Scratch from which on it has to leave as much again free: the sum pose by pose
+// needs none of it, and what the rest of the call and the program allocate later
+// should still fit.  (Not less: cudaMemGetInfo takes 70 us, and calls that make
+// and drop a system would pay it each time.)
+constexpr size_t kSiteScratchCareful = 1u << 30;
+
 int site_scratch_reserve(const SitePlan &plan, bool adjoint, SiteScratch &s) {
     const SiteView &v = plan.view;
-    const size_t S3 = (size_t)v.S * v.S * v.S, words = adjoint ? 4 : 1;
-    VEXT_TRY(ensure_capacity(s.value, s.value_cap, 2 * v.O * S3 * words));
+    const size_t S3 = (size_t)v.S * v.S * v.S, words = adjoint ? 4 : 1,
+                 value = 2 * v.O * S3 * words,
+                 sums = v.poly ? taylor_workspace_sites(*plan.rs) : 0,
+                 eval = v.poly ? (size_t)v.n_regions * v.n_sites * words : 0;
+    const size_t more = (value > s.value_cap ? 8 * value : 0) +
+                        (sums > s.sums_cap ? 4 * sums : 0) + (eval > s.eval_cap ? 4 * eval : 0);
+    if (more >= kSiteScratchCareful) {
+        size_t free = 0, total = 0;
+        VEXT_CUDA(cudaMemGetInfo(&free, &total));
+        if (2 * more > free)
+            return fail(VEXT_ERR_MEMORY, "%zu bytes of scratch, %zu free", more, free);
+    }
+    VEXT_TRY(ensure_capacity(s.value, s.value_cap, value));
     if (v.poly) {
-        VEXT_TRY(ensure_capacity(s.sums, s.sums_cap, taylor_workspace_sites(*plan.rs)));
-        VEXT_TRY(ensure_capacity(s.eval, s.eval_cap, (size_t)v.n_regions * v.n_sites * words));
+        VEXT_TRY(ensure_capacity(s.sums, s.sums_cap, sums));
+        VEXT_TRY(ensure_capacity(s.eval, s.eval_cap, eval));
     }
     return 0;
 }

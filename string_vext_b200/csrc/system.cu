@@ -20,7 +20,7 @@
 #include <map>
 
 #include "internal.cuh"
-#include "taylor.cuh"
+#include "sites.cuh"
 
 namespace vext {
 
@@ -542,6 +542,19 @@ int get_block_regions(System *sys, int size, int bi, int bj, int bk, double rho,
 
 // Width (A, between lattice planes) of the pose bins.
 
+void drop_idle_site_lists(System *sys) {
+    auto idle = [sys](const RegionSet *rs) {
+        return rs->sites && rs->use.use_count() == 1 &&
+               !(sys->site_field && sys->site_field->plan.rs == rs);
+    };
+    for (RegionSet *&rs : sys->sets)
+        if (idle(rs)) {
+            delete rs;
+            rs = nullptr;
+        }
+    sys->sets.erase(std::remove(sys->sets.begin(), sys->sets.end(), nullptr), sys->sets.end());
+}
+
 int get_bin_regions(System *sys, double r_split, RegionSet **out, cudaStream_t stream,
                     double bin_width) {
     for (RegionSet *rs : sys->sets)
@@ -818,6 +831,7 @@ extern "C" int vext_system_invalidate(vext_system h) {
     if (!h) return fail(VEXT_ERR_ARGUMENT, "null system");
     std::lock_guard<std::mutex> guard(h->sys.lock);
     for (RegionSet *rs : h->sys.sets) rs->stale = true;
+    h->sys.no_sites_from = h->sys.no_expansions_from = 1LL << 62;
     h->sys.drop_adjoint_batch();
     return 0;
 }

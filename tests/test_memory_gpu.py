@@ -1,13 +1,14 @@
 """Device memory of calls that come and go (string_vext_b200/csrc/memory.cu)."""
 import threading
+from contextlib import contextmanager
 
 import numpy as np
 import pytest
 import torch
 
-from string_vext_b200 import synth
+from string_vext_b200 import _lib, synth
 from string_vext_b200.orientation import normalized_directors
-from string_vext_b200.system import VextSystem, release_memory
+from string_vext_b200.system import VextBatch, VextSystem, release_memory
 
 pytestmark = pytest.mark.gpu
 
@@ -71,3 +72,115 @@ def test_release_memory_gives_back_what_dropped_systems_held():
         np.testing.assert_array_equal(system.field(40, axes)["orientation_K"], kept)
         release_memory()
         np.testing.assert_array_equal(system.field(40, axes)["orientation_K"], kept)
+
+
+# ---- scratch of the faster sums that cannot be had: the plainer ones serve
+
+@contextmanager
+def hog(leave):
+    """Hold all device memory but `leave` bytes."""
+    torch.cuda.synchronize()
+    release_memory()
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        torch.cuda.synchronize()
+        held.untyped_storage().resize_(0)
+        torch.cuda.empty_cache()
+
+
+def outputs(size, n_axes):
+    shape = (n_axes,) + (size,) * 3
+    return (torch.empty(shape, dtype=torch.float32, device="cuda"),
+            torch.empty(shape + (6,), dtype=torch.float32, device="cuda"))
+
+
+def exact_adjoint(system, size, axes):
+    shape = (len(axes),) + (size,) * 3
+    e = torch.empty(shape, dtype=torch.float64, device="cuda")
+    g = torch.empty(shape + (6,), dtype=torch.float64, device="cuda")
+    system.field_adjoint_device(size, axes, None, None, e, g, mode=_lib.VEXT_MODE_FP64_PLAIN)
+    torch.cuda.synchronize()
+    return e.cpu().numpy(), g.cpu().numpy()
+
+
+def assert_mixed(e, g, exact):
+    ex, gx = exact
+    err = np.abs(e - ex) - 1.2e-7 * np.abs(ex)
+    neg = ex <= 0
+    assert err[neg].max(initial=0) < 1e-4
+    assert (err / np.maximum(np.abs(ex), 1))[~neg].max(initial=0) < 1e-6
+    if g is not None:
+        err = np.linalg.norm(g - gx, axis=-1) / np.maximum(np.linalg.norm(gx, axis=-1), 1.0)
+        assert err.max() < 1e-5
+
+
+@pytest.fixture(scope="module")
+def fine_field():
+    size, axes = 40, directors(64)
+    with VextSystem(synth.small_field()) as system:
+        return size, axes, exact_adjoint(system, size, axes)
+
+
+def test_adjoint_field_without_room_for_site_sums(fine_field):
+    size, axes, exact = fine_field
+    e, g = outputs(size, len(axes))
+    with VextSystem(synth.small_field()) as system:
+        with hog(500 << 20):
+            system.field_adjoint_device(size, axes, e, g)
+            torch.cuda.synchronize()
+            assert_mixed(e.cpu().numpy(), g.cpu().numpy(), exact)
+        for pinned in (False, True):   # with room again
+            assert_mixed(*system.field_adjoint(size, axes, pinned=pinned), exact)
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+def test_host_adjoint_without_room_for_site_sums(fine_field, pinned):
+    size, axes, exact = fine_field
+    with VextSystem(synth.small_field()) as system:
+        with hog(640 << 20):
+            assert_mixed(*system.field_adjoint(size, axes, pinned=pinned), exact)
+
+
+def test_batch_without_room_for_site_sums(fine_field):
+    size, axes, exact = fine_field
+    outs = [outputs(size, len(axes)) for _ in range(2)]
+    with VextSystem(synth.small_field()) as a, VextSystem(synth.small_field()) as b, \
+            hog(500 << 20):
+        batch = VextBatch([a, b], size, axes, [o[0] for o in outs],
+                          gradients=[o[1] for o in outs])
+        assert batch.info()["cta_shape"] != "64-site clusters"
+        batch.run()
+        batch.check()
+        torch.cuda.synchronize()
+        for e, g in outs:
+            assert_mixed(e.cpu().numpy(), g.cpu().numpy(), exact)
+        batch.close()
+
+
+def test_field_without_room_for_site_sums(fine_field):
+    size, axes, exact = fine_field
+    with VextSystem(synth.small_field()) as system:
+        with hog(260 << 20):
+            small = system.field(20, axes)["orientation_K"]
+            for _ in range(2):
+                assert_mixed(system.field(size, axes)["orientation_K"], None, exact)
+            np.testing.assert_array_equal(system.field(20, axes)["orientation_K"], small)
+
+
+def test_adjoint_without_room_for_expansions():
+    size, axes = 4, directors(10600)   # an evaluation matrix of 1 GB
+    rng = np.random.default_rng(8)
+    kind = rng.integers(0, 4, 8)
+    case = synth.make_case([4.0, 4.2, 3.9], [90.0, 90.0, 90.0], rng.random((8, 3)),
+                           synth.TYPE_TABLE[kind, 1], synth.TYPE_TABLE[kind, 0],
+                           synth.GUEST_A, 12.8)
+    with VextSystem(case) as system:
+        exact = exact_adjoint(system, size, axes)
+        e, g = outputs(size, len(axes))
+        with hog(600 << 20):
+            system.field_adjoint_device(size, axes, e, g)
+            torch.cuda.synchronize()
+        assert_mixed(e.cpu().numpy(), g.cpu().numpy(), exact)
