@@ -875,6 +875,7 @@ struct vext_batch_s {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     ~vext_batch_s() {
+        FreeTogether together;
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
         device_free(d_sys);

@@ -37,6 +37,13 @@ cudaError_t device_malloc(T **p, size_t bytes) {
 }
 void device_free(void *p);
 
+// While one is alive on a thread, its device_free calls wait together, when the
+// last one goes.
+struct FreeTogether {
+    FreeTogether();
+    ~FreeTogether();
+};
+
 // Free the list builds' scratch on a device (system.cu).
 void release_build_scratch(int device);
 

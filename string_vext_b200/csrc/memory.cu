@@ -165,7 +165,41 @@ void settle(DevicePool &p) {
     p.freed.swap(left);
 }
 
+// settle, and no more than kPoolKeep bytes stay in the pool.
+void give_back(DevicePool &p) {
+    settle(p);
+    unsigned long long held = 0;
+    if (p.pool &&
+        cudaMemPoolGetAttribute(p.pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+        held > kPoolKeep) {
+        cudaStreamSynchronize(p.stream);
+        cudaMemPoolTrimTo(p.pool, kPoolKeep);
+    }
+}
+
+thread_local int frees_together = 0;
+thread_local unsigned long long frees_devices = 0;   // with blocks to give back
+
 }  // namespace
+
+FreeTogether::FreeTogether() { ++frees_together; }
+
+FreeTogether::~FreeTogether() {
+    if (--frees_together > 0) return;
+    int current = 0;
+    if (cudaGetDevice(&current) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    for (int d = 0; frees_devices; ++d, frees_devices >>= 1) {
+        if (!(frees_devices & 1)) continue;
+        if (d != current) cudaSetDevice(d);
+        DevicePool &p = device_pool(d);
+        std::lock_guard<std::mutex> guard(p.lock);
+        give_back(p);
+        if (d != current) cudaSetDevice(current);
+    }
+}
 
 cudaError_t device_malloc_bytes(void **out, size_t bytes) {
     *out = nullptr;
@@ -223,15 +257,8 @@ void device_free(void *ptr) {
     {
         std::lock_guard<std::mutex> guard(p.lock);
         p.freed.push_back(ptr);
-        settle(p);
-        unsigned long long held = 0;
-        if (p.pool &&
-            cudaMemPoolGetAttribute(p.pool, cudaMemPoolAttrReservedMemCurrent, &held) ==
-                cudaSuccess &&
-            held > kPoolKeep) {
-            cudaStreamSynchronize(p.stream);
-            cudaMemPoolTrimTo(p.pool, kPoolKeep);
-        }
+        if (frees_together > 0) frees_devices |= 1ull << (at.device & 63);
+        else give_back(p);
     }
     if (at.device != current) cudaSetDevice(current);
 }

@@ -642,6 +642,7 @@ void System::drop_host_parts() {
 }
 
 System::~System() {
+    FreeTogether together;
     drop_adjoint_batch();   // it points into the region sets
     for (RegionSet *rs : sets) delete rs;
     device_free(d_g32);

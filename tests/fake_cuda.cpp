@@ -16,6 +16,10 @@ namespace vext {   // as in string_vext_b200/csrc/internal.cuh
 cudaError_t device_malloc_bytes(void **p, size_t bytes);
 void device_free(void *p);
 int fail(int code, const char *, ...) { return code; }
+struct FreeTogether {
+    FreeTogether();
+    ~FreeTogether();
+};
 void release_build_scratch(int) {}
 int copy_to_host(void *dst, const void *src, size_t bytes, bool *finite = nullptr);
 }  // namespace vext
@@ -37,6 +41,7 @@ thread_local int device = 0;
 bool refuse_waits = false;               // as while another stream is being captured
 bool captures_ended = false;             // a wait for the whole device ends such captures
 size_t limit = ~(size_t)0;               // device memory in all
+int waits = 0;
 int host_allocs = 0, host_frees = 0;
 
 size_t mapped() {
@@ -89,6 +94,7 @@ cudaError_t cudaFree(void *p) {
     std::lock_guard<std::recursive_mutex> g(lock);
     if (!p) return cudaSuccess;
     if (refuse_waits) return cudaErrorStreamCaptureUnsupported;
+    ++waits;
     if (!blocks.count(p)) std::abort();
     blocks.erase(p);
     return cudaSuccess;
@@ -235,12 +241,37 @@ static int two_devices() {
     return 0;
 }
 
+// Blocks freed together are waited for once, whichever device they are on.
+static int together() {
+    void *p[6];
+    for (int i = 0; i < 6; ++i) {
+        device = i & 1;
+        CHECK(p[i] = take((size_t)(i + 1) << 20));
+    }
+    device = 0;
+    waits = 0;
+    {
+        FreeTogether outer;
+        {
+            FreeTogether inner;
+            for (int i = 0; i < 3; ++i) device_free(p[i]);
+        }
+        for (int i = 0; i < 3; ++i) CHECK(blocks.count(p[i]));
+        for (int i = 3; i < 6; ++i) device_free(p[i]);
+        CHECK(waits == 0);
+    }
+    for (int i = 0; i < 6; ++i) CHECK(!blocks.count(p[i]));
+    CHECK(waits == 2 && device == 0);
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "refused_wait") return refused_wait(1 << 20);
     if (what == "refused_wait_large") return refused_wait((size_t)600 << 20);
     if (what == "released") return released();
     if (what == "two_devices") return two_devices();
+    if (what == "together") return together();
     std::printf("unknown scenario\n");
     return 2;
 }

@@ -24,7 +24,7 @@ def fake(tmp_path_factory):
 
 
 @pytest.mark.parametrize("scenario", ["refused_wait", "refused_wait_large", "released",
-                                      "two_devices"])
+                                      "two_devices", "together"])
 def test_allocator(fake, scenario):
     run = subprocess.run([str(fake), scenario], capture_output=True, text=True, timeout=60)
     assert run.returncode == 0, run.stdout + run.stderr
