@@ -118,7 +118,7 @@ VEXT_API int vext_system_destroy(vext_system sys);
 
 /* Device memory of dropped systems and batches is kept for the next ones, up to
  * 1.5 GiB per device, as is the scratch of the largest list build (4 KB per
- * region, 8 KB per pose bin).  This call gives it all back on the calling
+ * region or pose bin).  This call gives it all back on the calling
  * thread's current device, after waiting for the device; VEXT_ERR_CUDA when some
  * of it may still be in use because that wait was refused (during a stream
  * capture). */

@@ -137,8 +137,34 @@ struct ClassRadii {
         at[6] = 1e300;
     }
 };
+// A thread's counts: all classes, or those of lists without an expansion (pose
+// bins), whose other ones are empty.  Either way 4 KB per region of a list build.
 struct ClassCounts {
     int n[kClasses];
+    __device__ void put(const int (&from)[kClasses]) {
+#pragma unroll
+        for (int i = 0; i < kClasses; ++i) n[i] = from[i];
+    }
+    __device__ void get(int (&to)[kClasses]) const {
+#pragma unroll
+        for (int i = 0; i < kClasses; ++i) to[i] = n[i];
+    }
+};
+struct BinCounts {
+    int n[4];   // near, mid, shell, outer
+    __device__ void put(const int (&from)[kClasses]) {
+        n[0] = from[0];
+        n[1] = from[1];
+        n[2] = from[5];
+        n[3] = from[6];
+    }
+    __device__ void get(int (&to)[kClasses]) const {
+        to[0] = n[0];
+        to[1] = n[1];
+        to[2] = to[3] = to[4] = to[7] = 0;
+        to[5] = n[2];
+        to[6] = n[3];
+    }
 };
 
 // Visit every candidate image of atom j for a region; f(dist2, rel) per image.
@@ -218,9 +244,9 @@ constexpr int kBuildThreads = 256, kFieldBuildThreads = 128;
 
 // Per region: the entries of each class, and per thread (atoms j = tid, tid +
 // NT, ...) its counts per class for the fill.
-template <int NT>
+template <int NT, typename Counts>
 __global__ void __launch_bounds__(NT)
-    region_count_kernel(BuildArgs a, RegionInfo *regs, int n_regions, ClassCounts *counts) {
+    region_count_kernel(BuildArgs a, RegionInfo *regs, int n_regions, Counts *counts) {
     const int region = blockIdx.x;
     if (region >= n_regions) return;
     const RegionInfo r = regs[region];
@@ -232,15 +258,15 @@ __global__ void __launch_bounds__(NT)
 #pragma unroll
             for (int i = 1; i < kClasses; ++i) from[i] += q >= cls.at[i - 1];
         });
-    ClassCounts c;
+    int c[kClasses];
 #pragma unroll
-    for (int i = 0; i < kClasses; ++i) c.n[i] = from[i] - (i + 1 < kClasses ? from[i + 1] : 0);
-    counts[(long long)region * NT + threadIdx.x] = c;
+    for (int i = 0; i < kClasses; ++i) c[i] = from[i] - (i + 1 < kClasses ? from[i + 1] : 0);
+    counts[(long long)region * NT + threadIdx.x].put(c);
     __shared__ int sh[128];
     int p, q, t[kClasses];
 #pragma unroll
     for (int i = 0; i < kClasses; i += 2)
-        block_scan2<NT>(c.n[i], c.n[i + 1], p, q, t[i], t[i + 1], sh);
+        block_scan2<NT>(c[i], c[i + 1], p, q, t[i], t[i + 1], sh);
     if (threadIdx.x == 0) {
         RegionInfo &w = regs[region];
         w.n_near = t[0];
@@ -257,22 +283,23 @@ __global__ void __launch_bounds__(NT)
 // ... in turn, each atom's images in enumeration order), so a thread's slots
 // follow from a block scan of the per-thread counts that region_count_kernel
 // stored and the candidates are enumerated once here.
-template <int NT>
+template <int NT, typename Counts>
 __global__ void __launch_bounds__(NT, 512 / NT)
     region_fill_kernel(BuildArgs a, const RegionInfo *regs, int n_regions,
-                       const ClassCounts *counts, float4 *hi, float4 *lo, int *status) {
+                       const Counts *counts, float4 *hi, float4 *lo, int *status) {
     const int region = blockIdx.x;
     if (region >= n_regions) return;
     const RegionInfo r = regs[region];
     const ClassRadii cls(a, r);
     __shared__ int sh[128];
-    const ClassCounts c = counts[(long long)region * NT + threadIdx.x];
+    int c[kClasses];
+    counts[(long long)region * NT + threadIdx.x].get(c);
     // this thread's next slot and end per class (indexed by unrolled loops
     // only: a runtime index would put them in local memory)
     int w[kClasses], end[kClasses], t[kClasses];
 #pragma unroll
     for (int i = 0; i < kClasses; i += 2)
-        block_scan2<NT>(c.n[i], c.n[i + 1], w[i], w[i + 1], t[i], t[i + 1], sh);
+        block_scan2<NT>(c[i], c[i + 1], w[i], w[i + 1], t[i], t[i + 1], sh);
     if (threadIdx.x == 0 &&
         (t[0] != r.n_near || t[1] != r.n_mid || t[2] != r.n_tnear ||
          t[1] + t[2] + t[3] != r.n_inner || t[4] != r.n_shella || t[6] != r.n_outer ||
@@ -282,7 +309,7 @@ __global__ void __launch_bounds__(NT, 512 / NT)
 #pragma unroll
     for (int i = 0; i < kClasses; ++i) {
         w[i] += base;
-        end[i] = w[i] + c.n[i];
+        end[i] = w[i] + c[i];
         base += t[i];
     }
     for (int j = threadIdx.x; j < a.n_atoms; j += NT) {
@@ -329,7 +356,7 @@ RegionSet::~RegionSet() {
 namespace {
 struct BuildScratch {
     std::mutex lock;
-    ClassCounts *ptr = nullptr;
+    unsigned char *ptr = nullptr;
     size_t cap = 0;
     unsigned long long ctx_id = 0;
 };
@@ -394,14 +421,17 @@ static int build_lists(System *sys, RegionSet *rs, cudaStream_t stream) {
     }
     const bool field = rs->size > 0;
     VEXT_TRY(ensure_capacity(scratch.ptr, scratch.cap,
-                             (size_t)n * (field ? kFieldBuildThreads : kBuildThreads)));
+                             (size_t)n * (field ? kFieldBuildThreads * sizeof(ClassCounts)
+                                                : kBuildThreads * sizeof(BinCounts))));
     scratch.ctx_id = ctx;
+    ClassCounts *field_counts = reinterpret_cast<ClassCounts *>(scratch.ptr);
+    BinCounts *bin_counts = reinterpret_cast<BinCounts *>(scratch.ptr);
     if (field)
         region_count_kernel<kFieldBuildThreads>
-            <<<n, kFieldBuildThreads, 0, stream>>>(a, rs->d_info, n, scratch.ptr);
+            <<<n, kFieldBuildThreads, 0, stream>>>(a, rs->d_info, n, field_counts);
     else
         region_count_kernel<kBuildThreads>
-            <<<n, kBuildThreads, 0, stream>>>(a, rs->d_info, n, scratch.ptr);
+            <<<n, kBuildThreads, 0, stream>>>(a, rs->d_info, n, bin_counts);
     VEXT_CUDA(cudaGetLastError());
     VEXT_CUDA(cudaMemcpyAsync(rs->h_info.data(), rs->d_info, sizeof(RegionInfo) * n,
                               cudaMemcpyDeviceToHost, stream));
@@ -431,10 +461,10 @@ static int build_lists(System *sys, RegionSet *rs, cudaStream_t stream) {
     }
     if (field)
         region_fill_kernel<kFieldBuildThreads><<<n, kFieldBuildThreads, 0, stream>>>(
-            a, rs->d_info, n, scratch.ptr, rs->d_hi, rs->d_lo, sys->d_status);
+            a, rs->d_info, n, field_counts, rs->d_hi, rs->d_lo, sys->d_status);
     else
         region_fill_kernel<kBuildThreads><<<n, kBuildThreads, 0, stream>>>(
-            a, rs->d_info, n, scratch.ptr, rs->d_hi, rs->d_lo, sys->d_status);
+            a, rs->d_info, n, bin_counts, rs->d_hi, rs->d_lo, sys->d_status);
     VEXT_CUDA(cudaGetLastError());
     VEXT_CUDA(cudaEventRecord(e1, stream));
     VEXT_CUDA(cudaEventSynchronize(e1));

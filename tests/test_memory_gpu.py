@@ -8,7 +8,7 @@ import torch
 
 from string_vext_b200 import _lib, synth
 from string_vext_b200.orientation import normalized_directors
-from string_vext_b200.system import VextBatch, VextSystem, release_memory
+from string_vext_b200.system import VextBatch, VextPoseBatch, VextSystem, release_memory
 
 pytestmark = pytest.mark.gpu
 
@@ -72,6 +72,24 @@ def test_release_memory_gives_back_what_dropped_systems_held():
         np.testing.assert_array_equal(system.field(40, axes)["orientation_K"], kept)
         release_memory()
         np.testing.assert_array_equal(system.field(40, axes)["orientation_K"], kept)
+
+
+def test_pose_list_build_scratch():
+    """4 KB of scratch per pose bin (0.75 A between lattice planes) beside the
+    lists, which a cell without images in reach of most bins keeps small."""
+    rng = np.random.default_rng(9)
+    edge, n = 45.0, 12
+    case = synth.make_case([edge] * 3, [90.0] * 3, rng.random((n, 3)),
+                           np.full(n, 3.0), np.full(n, 40.0), synth.GUEST_A, 6.0)
+    release_memory()
+    free = torch.cuda.mem_get_info()[0]
+    with VextSystem(case) as system:
+        batch = VextPoseBatch([system], [4])
+        held = free - torch.cuda.mem_get_info()[0]
+        batch.close()
+    bins = round(edge / 0.75) ** 3
+    listed = 4 / 3 * np.pi * (6.0 + 0.8 + 0.7) ** 3 * n / edge ** 3
+    assert held < bins * (4096 + 200 + 32 * 1.5 * listed) + (64 << 20)
 
 
 # ---- scratch of the faster sums that cannot be had: the plainer ones serve
