@@ -364,9 +364,9 @@ __global__ void refine_sites_kernel(SiteView v, const int *list, double *e64) {
 // Single-site field at the grid centers (site 0 parameters, no offset):
 // the reference's site_K (src/string_vext/vext.py:27-29, 33).  One CTA per
 // region: each thread takes every 128th entry of the list with all CB centers,
-// so an entry is read once for the region.  FP64 pipe-bound; a warp per
-// center, reading the whole list for it, and a division per pair took 1.56 ms
-// for the 60^3 layered field.
+// so an entry is read once for the region.  FP64 pipe-bound: 0.72 ms for the 60^3
+// layered field (a warp per center, reading the whole list for it: 1.56 ms), with
+// the correctly rounded reciprocal (the hardware seed and two Newton steps: 0.61).
 template <int CB>
 __global__ void __launch_bounds__(128, 4) site_kernel(FieldArgs a, float *site_K) {
     constexpr int NC = CB < 8 ? CB : 8;   // centers at a time
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(128, 4) site_kernel(FieldArgs a, float *site_K
                 const double dx = cen[c0 + c][0] - x, dy = cen[c0 + c][1] - y,
                              dz = cen[c0 + c][2] - z;
                 const double d2 = fma(dx, dx, fma(dy, dy, dz * dz));
-                const double i2 = rcp64_nr<2>(fmax(d2, sf.y));
+                const double i2 = __drcp_rn(fmax(d2, sf.y));
                 const double i6 = i2 * i2 * i2;
                 const double en = fma(i6, fma(cc.x, i6, -cc.y), sf.x);
                 sum[c] += d2 < a.rc2 ? en : 0.0;
