@@ -21,7 +21,8 @@ __device__ __forceinline__ int wrap(int x, int n) {
 
 // Energy and gradient sums of pose (director o, center gi gj gk) over the lists of
 // its two sites in FP64, with the correctly rounded reciprocal; partial over the
-// lanes.  Few poses come here: 64 us more than with two Newton steps in the 47^3 x 50 skewed field's 7.4 ms.
+// lanes.  Few poses come here: 64 us more than with two Newton steps in the
+// 47^3 x 50 skewed field's 7.4 ms.
 __device__ __forceinline__ void site_pose_fp64(const SiteView &v, int o, int gi, int gj, int gk,
                                                int lane, double &e, double (&g)[6]) {
     e = 0.0;

@@ -200,6 +200,7 @@ __device__ __forceinline__ void take_shell(const SiteQueue &q, int n, const Site
             site_pair<ADJ, true>(q.sxy[j + k], q.szc[j + k], make_float2(c.x, c.x), c.z, t, c.y,
                                  v.rc2f, s, near_rc);
         }
+        if ((j & 12) == 12) add_energy<ADJ>(s, sum);   // partials over 16, as pose by pose
     }
 #pragma unroll 1
     for (; j < n; ++j) {
