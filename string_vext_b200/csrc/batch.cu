@@ -53,7 +53,6 @@ struct BatchSys {
     const float4 *tf;
     const double *td;
     int n_types;
-    int flush;                  // list_flush
     int near_mode;              // 1: cutoff test on near pairs, 2: none needed
     int bi, bj, bk, nrj, nrk;   // region grid (pose -> region)
     float *out;                 // [O][S^3]
@@ -249,7 +248,8 @@ __device__ __forceinline__ bool batch_item_adj(const BatchArgs &a, const BatchSy
                         hb, stf, len, g, ux, uy, uz, acc, shift_sum, gsum, border);
                 } else {
                     far_chunk_adj<P, NEWTON, FLUSH, false, RCP1, UNROLL, GNT, 0, SYM>(
-                        hb, stf, len, g, ux, uy, uz, acc, shift_sum, gsum, nullptr, y.flush);
+                        hb, stf, len, g, ux, uy, uz, acc, shift_sum, gsum, nullptr,
+                        expand ? kExpandFlush : kFlush);
                 }
                 stage_next(st, plan, y.hi, y.lo, c, seq);
             }
@@ -415,12 +415,13 @@ __global__ void __launch_bounds__(CB *G, MINB) batch_field_kernel(BatchArgs a) {
                         far_chunk_trim<P, 16>(hb, stf, len, g, ux, uy, uz, acc);
                     else if (pass && sym)
                         far_chunk_fwd<P, true, true>(hb, stf, len, g, ux, uy, uz, acc, shift_sum,
-                                                     16, outer_at - start);
+                                                     kFlush, outer_at - start);
                     else if (pass)
-                        far_chunk_fwd<P, true>(hb, stf, len, g, ux, uy, uz, acc, shift_sum, 16);
+                        far_chunk_fwd<P, true>(hb, stf, len, g, ux, uy, uz, acc, shift_sum,
+                                               kFlush);
                     else
                         far_chunk_fwd<P, false>(hb, stf, len, g, ux, uy, uz, acc, shift_sum,
-                                                y.flush);
+                                                expand ? kExpandFlush : kFlush);
                     stage_next(st, plan, y.hi, y.lo, c, seq);
                 }
                 seq += plan.n_chunks;
@@ -1080,6 +1081,9 @@ static int build_batch(int n_systems, const vext_system *systems, int size, int 
         by_site[k] = by_site[owner[k]];
         if (by_site[k]) *used = 2;
     }
+    // local expansions: the kinds whose kernels use them
+    const bool expands = level >= 1 && (b->kind == 0 || b->kind == 6 || b->kind == 7 ||
+                                        b->kind == 9 || b->kind == 10);
     std::vector<RegionSet *> lists(n_systems, nullptr);
     for (int k = 0; k < n_systems; ++k) {
         if (owner[k] != k) continue;
@@ -1088,10 +1092,27 @@ static int build_batch(int n_systems, const vext_system *systems, int size, int 
             return fail(VEXT_ERR_ARGUMENT, "system %d lives on another device", k);
         std::unique_lock<std::mutex> lock(sys->lock, std::defer_lock);
         if (lock_systems) lock.lock();
-        VEXT_TRY(by_site[k]
-                     ? get_site_regions(sys, size, kBatchVoxels, b->opt.r_split, &lists[k],
-                                        sys->stream)
-                     : get_field_regions(sys, size, cb, b->opt.r_split, &lists[k], sys->stream));
+        if (by_site[k]) {
+            VEXT_TRY(get_site_regions(sys, size, kBatchVoxels, b->opt.r_split, &lists[k],
+                                      sys->stream));
+        } else {
+            // expansions for all members of a framework or none: their values
+            // stand in the outputs first, which have to be device memory
+            int expand_axes = expands ? (rule_axes ? rule_axes : n_axes) : 0;
+            for (int j = 0; j < n_systems; ++j)
+                if (owner[j] == k && !(device_memory(outputs[j]) &&
+                                       (!gradients || device_memory(gradients[j]))))
+                    expand_axes = 0;
+            VEXT_TRY(get_field_regions(sys, size, cb, b->opt.r_split, expand_axes, b->adj,
+                                       &lists[k], sys->stream));
+            bool pay = true;
+            for (int j = 0; lists[k]->expand && j < n_systems; ++j)
+                if (owner[j] == k)
+                    pay = pay && taylor_worthwhile(systems[j]->sys, *lists[k], expand_axes, b->adj);
+            if (!pay)
+                VEXT_TRY(get_field_regions(sys, size, cb, b->opt.r_split, 0, b->adj, &lists[k],
+                                           sys->stream));
+        }
         b->list_bytes += lists[k]->n_entries * 32;
         b->list_use.push_back(lists[k]->use);
     }
@@ -1127,7 +1148,6 @@ static int build_batch(int n_systems, const vext_system *systems, int size, int 
         for (const RegionInfo &r : rs->h_info) rho = std::max(rho, r.rho);
         y.near_mode =
             rs->r_split + 2.0 * (rho + list_sys->max_offset) + 1e-6 < sys->cutoff ? 2 : 1;
-        y.flush = list_flush(*rs, sys->cutoff);
         y.bi = rs->bi;
         y.bj = rs->bj;
         y.bk = rs->bk;
@@ -1206,20 +1226,12 @@ static int build_batch(int n_systems, const vext_system *systems, int size, int 
     if (b->kind == 6 || b->kind == 10)
         for (const BatchSys &y : hs)
             if (y.off0 == 0.0 || y.off1 != -y.off0) b->kind = 9;
-    // local expansions: the kinds whose kernels use them, where the rule of
-    // taylor_worthwhile says so and the outputs, where their values stand first,
-    // are device memory
     b->plans.resize(n_systems);
-    const bool expands = b->kind == 0 || b->kind == 6 || b->kind == 7 || b->kind == 9 ||
-                         b->kind == 10;
     for (int k = 0; k < n_systems; ++k) {
         b->lists.push_back(lists[owner[k]]);
         const System &sys = systems[k]->sys;
         const RegionSet &rs = *b->lists[k];
-        if (by_site[k] || !expands || level < 1 ||
-            !taylor_worthwhile(sys, rs, rule_axes ? rule_axes : n_axes, b->adj) ||
-            !device_memory(hs[k].out) || (b->adj && !device_memory(hs[k].grad)))
-            continue;
+        if (by_site[k] || !rs.expand) continue;
         *used = std::max(*used, 1);
         VEXT_TRY(taylor_prepare(sys, rs, n_axes, b->d_axes, b->adj, b->plans[k], b->stream));
         VEXT_TRY(ensure_capacity(b->d_sums, b->sums_cap, taylor_workspace(rs)));

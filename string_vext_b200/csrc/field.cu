@@ -44,7 +44,6 @@ struct FieldArgs {
     const float4 *tf;
     const double *td;
     int n_types;
-    int flush;                // list_flush
     const double *poly;       // [regions][kTaylorPolyPad] local expansions, whose further
                               // degrees stand in e64; null: inner pairs are summed directly
     double *e64;              // [O][S^3]
@@ -255,8 +254,10 @@ __global__ void __launch_bounds__(CB *G, MINB) field_far2_kernel(FieldArgs a) {
             plan.chunk(c, start, len, near);
             const float4 *hb = st.hib + ((seq + c) % kStages) * kCH;
             if (trim) far_chunk_trim<P, 16>(hb, stf, len, g, ux, uy, uz, acc);
-            else if (pass) far_chunk_fwd<P, true>(hb, stf, len, g, ux, uy, uz, acc, shift_sum, 16);
-            else far_chunk_fwd<P, false>(hb, stf, len, g, ux, uy, uz, acc, shift_sum, a.flush);
+            else if (pass) far_chunk_fwd<P, true>(hb, stf, len, g, ux, uy, uz, acc, shift_sum, kFlush);
+            else
+                far_chunk_fwd<P, false>(hb, stf, len, g, ux, uy, uz, acc, shift_sum,
+                                        EXPAND ? kExpandFlush : kFlush);
             stage_next(st, plan, a.hi, a.lo, c, seq);
         }
         seq += plan.n_chunks;
@@ -712,7 +713,6 @@ static FieldArgs make_args(System *sys, const RegionSet *rs, int n_axes, const d
     a.tf = sys->d_tf;
     a.td = sys->d_td;
     a.n_types = sys->n_types;
-    a.flush = list_flush(*rs, sys->cutoff);
     a.poly = nullptr;
     a.e64 = d_e64;
     a.status = sys->d_status;
@@ -742,9 +742,7 @@ int launch_field(System *sys, const RegionSet *rs, int n_axes, const double *axe
     double rho = 0;
     for (const RegionInfo &r : rs->h_info) rho = std::max(rho, r.rho);
     const int near_mode = rs->r_split + 2.0 * (rho + sys->max_offset) + 1e-6 < sys->cutoff ? 2 : 1;
-    const long long poses = (long long)rs->size * rs->size * rs->size * n_axes;
-    if (variant != 9 && cb != 32 && poses < sys->no_expansions_from &&
-        taylor_worthwhile(*sys, *rs, n_axes, false)) {
+    if (rs->expand) {
         if (expanded) *expanded = true;
         TaylorPlan &plan = sys->field_plan;
         if (sys->field_plan_set != rs || sys->field_plan_axes.size() != 3 * (size_t)n_axes ||
@@ -802,9 +800,12 @@ static int field_pass(System *sys, int size, int n_axes, const double *axes_host
     const int cb = o.cb == 32 ? 32 : o.cb == 8 && !fp64 ? 8 : 16;
     const double r_split = fp64 ? 1e30 : o.r_split;
     *by_site = S3 * n_axes < sys->no_sites_from && sites_worthwhile(*sys, size, n_axes, o, false);
+    const bool expands = !fp64 && cb != 32 && o.variant != 9 &&
+                         S3 * n_axes < sys->no_expansions_from;
     RegionSet *rs = nullptr;
     VEXT_TRY(*by_site ? get_site_regions(sys, size, kFieldVoxels, r_split, &rs, stream)
-                      : get_field_regions(sys, size, cb, r_split, &rs, stream));
+                      : get_field_regions(sys, size, cb, r_split,
+                                          expands ? n_axes : 0, false, &rs, stream));
     const size_t n = (size_t)S3 * n_axes;
     VEXT_TRY(ensure_capacity(sys->d_axes, sys->axes_cap, 3 * (size_t)n_axes));
     VEXT_TRY(ensure_capacity(sys->d_e64, sys->e64_cap, n));
@@ -1037,7 +1038,7 @@ static int field_adjoint_device(vext_system h, int size, int n_axes, const doubl
     if (o.mode != VEXT_MODE_FP64 && o.mode != VEXT_MODE_FP64_PLAIN)
         return fail(VEXT_ERR_ARGUMENT, "unknown precision mode %d", o.mode);
     RegionSet *rs = nullptr;
-    VEXT_TRY(get_field_regions(sys, size, 16, 1e30, &rs, stream));
+    VEXT_TRY(get_field_regions(sys, size, 16, 1e30, 0, true, &rs, stream));
     VEXT_TRY(ensure_capacity(sys->d_axes, sys->axes_cap, 3 * (size_t)n_axes));
     VEXT_CUDA(cudaMemcpyAsync(sys->d_axes, axes, sizeof(double) * 3 * n_axes,
                               cudaMemcpyHostToDevice, stream));
@@ -1282,7 +1283,7 @@ extern "C" int vext_count_pairs(vext_system h, int size, int n_axes, const doubl
     RegionSet *rs = nullptr;
     // the mixed field's default region set (16 centers): far_pairs counts the
     // pairs its far kernel evaluates
-    VEXT_TRY(get_field_regions(sys, size, 16, o.r_split, &rs, st));
+    VEXT_TRY(get_field_regions(sys, size, 16, o.r_split, 0, false, &rs, st));
     VEXT_TRY(ensure_capacity(sys->d_axes, sys->axes_cap, 3 * (size_t)n_axes));
     VEXT_TRY(ensure_capacity(sys->d_flags, sys->flags_cap, 4));
     VEXT_CUDA(cudaMemcpyAsync(sys->d_axes, axes, sizeof(double) * 3 * n_axes,

@@ -18,8 +18,10 @@
 // beyond rc + rho + 1e-3 A of the origin.
 #pragma once
 
+#include <map>
 #include <memory>
 #include <mutex>
+#include <tuple>
 #include <vector>
 
 #include "common.cuh"
@@ -90,6 +92,7 @@ struct RegionSet {
     double bin_width = 0;                   // target bin width (A, pose regions)
     double r_split = 0;
     bool sites = false;                     // regions of voxels: lists about single sites
+    bool expand = false;                    // classes for local expansions (taylor.cuh)
     // data
     int n_regions = 0;
     int n_ri = 0, n_rj = 0, n_rk = 0;       // regions per axis
@@ -163,6 +166,8 @@ struct System {
     int *d_status = nullptr;   // device status word
     std::vector<double> h_td;  // n_types x 4
     std::vector<RegionSet *> sets;
+    // expected expansion entries per region of field lists: (size, cb, r_split)
+    std::map<std::tuple<int, int, double>, double> expansion_entries;
     bool outputs_finite = true;    // float32 outputs of the last vext_field call
     // scratch of the field path
     double *d_e64 = nullptr;
@@ -249,10 +254,13 @@ int batch_retarget(vext_batch b, int k, float *out, float *grad, cudaStream_t st
 bool device_memory(const void *p);   // device or managed, not host memory
 
 // Region sets (system.cu)
-int get_field_regions(System *sys, int size, int cb, double r_split, RegionSet **out,
-                      cudaStream_t stream);
+// expand_axes: directors of a call that sums by local expansions where they pay
+// (adjoint: forward + adjoint); 0: lists without classes for them.
+int get_field_regions(System *sys, int size, int cb, double r_split, int expand_axes,
+                      bool adjoint, RegionSet **out, cudaStream_t stream);
 int get_block_regions(System *sys, int size, int bi, int bj, int bk, double rho, double offset,
-                      bool sites, double r_split, RegionSet **out, cudaStream_t stream);
+                      bool sites, bool expand, double r_split, RegionSet **out,
+                      cudaStream_t stream);
 // Delete the lists for single sites that neither a batch nor the field path's
 // plan uses (under the system's lock).
 void drop_idle_site_lists(System *sys);
@@ -305,11 +313,11 @@ inline double floor_clear_radius2(const System &sys) {
 }
 
 // Far entries per FP32 energy partial in the unmasked pass over inner entries:
-// 16, or 8 where the lists set the nearer ones apart (RegionInfo::n_mid).  A
-// partial's rounding grows with its sum, and with the nearest entries next to
+// kFlush, or kExpandFlush of those too near for an expansion (RegionInfo::n_mid).
+// A partial's rounding grows with its sum, and with the nearest entries next to
 // one another partials over 16 gave 1.55e-4 instead of 1.26e-4 K at worst in a
 // slab framework whose pairs were summed unsorted to 1.24e-4 K.
-inline int list_flush(const RegionSet &rs, double cutoff) { return rs.d_taylor < cutoff ? 8 : 16; }
+constexpr int kFlush = 16, kExpandFlush = 8;
 
 // Directors per work item of a batch with these options (32 or 64; its
 // regions hold 512 / that many grid centers).

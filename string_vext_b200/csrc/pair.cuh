@@ -843,7 +843,7 @@ __device__ __forceinline__ void grad_load(double *gsum, AdjAcc (&acc)[P]) {
 // pose of the region): no mask, and the shift, the same for every pose, is
 // summed once per entry into shift_sum (the caller adds 2 x shift_sum, both
 // sites, to every energy).  FP32 partials are flushed into the FP64 AdjAcc:
-// the energy every `eb` entries (16, or list_flush's 8), the gradient sums
+// the energy every `eb` entries (kFlush or kExpandFlush), the gradient sums
 // every FLUSH entries.
 // GSUM_NT > 0: the gradient partials go to the shared-memory sums
 // (grad_slot<GSUM_NT>(gsum, ...)) instead of acc (whose energies stay).
@@ -861,7 +861,7 @@ __device__ __forceinline__ void far_chunk_adj(const float4 *hb, const float4 *st
                                               const float2 (&uy)[P / 2],
                                               const float2 (&uz)[P / 2], AdjAcc (&acc)[P],
                                               double &shift_sum, double *gsum = nullptr,
-                                              float *border = nullptr, int eb = 16) {
+                                              float *border = nullptr, int eb = kFlush) {
     constexpr int PP = P / 2;
     const float2 one2 = make_float2(1.f, 1.f);
     const float2 mrc2 = make_float2(-g.rc2f, -g.rc2f);

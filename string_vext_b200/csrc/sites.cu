@@ -165,7 +165,7 @@ __device__ __forceinline__ void take_inside(const SiteQueue &q, int n, const Sit
     s.e = s.gx = s.gy = s.gz = make_float2(0.f, 0.f);
     float unused = 0.f;
     int j = 0;
-    // energy partials over 8 entries (list_flush)
+    // energy partials over 8 entries (kExpandFlush)
 #pragma unroll 1
     for (; j + 8 <= n; j += 8) {
 #pragma unroll
@@ -591,7 +591,8 @@ int get_site_regions(System *sys, int size, int block, double r_split, RegionSet
                      cudaStream_t stream) {
     int bi = 0, bj = 0, bk = 0;
     const double radius = site_block(sys->H, size, block, bi, bj, bk) + 1e-9;
-    return get_block_regions(sys, size, bi, bj, bk, radius, 0.0, true, r_split, out, stream);
+    return get_block_regions(sys, size, bi, bj, bk, radius, 0.0, true, true, r_split, out,
+                             stream);
 }
 
 int site_plan_build(const System &sys, const RegionSet &rs, int n_axes, const double *axes,

@@ -480,22 +480,55 @@ static double det3(const Mat3 &m) {
            h[2] * (h[3] * h[7] - h[4] * h[6]);
 }
 
-int get_field_regions(System *sys, int size, int cb, double r_split, RegionSet **out,
-                      cudaStream_t stream) {
+// Entries per region that an expansion about its origin is expected to hold, for
+// sites within `radius` of it; 0: none.
+static double expansion_entries(const System &sys, double radius, double r_split) {
+    const double start = std::max(taylor_start(sys, radius), r_split + radius);
+    const double inner = sys.cutoff - radius;
+    if (!(start < inner)) return 0.0;
+    return 4.18879 * (inner * inner * inner - start * start * start) * sys.n_atoms *
+           std::fabs(det3(sys.Hinv));
+}
+
+int get_field_regions(System *sys, int size, int cb, double r_split, int expand_axes,
+                      bool adjoint, RegionSet **out, cudaStream_t stream) {
     int bi, bj, bk;
     choose_block_shape(sys->H, size, cb, bi, bj, bk);
     const double rho = block_radius(sys->H, size, bi, bj, bk) + 1e-9;
-    return get_block_regions(sys, size, bi, bj, bk, rho, sys->max_offset, false, r_split, out,
-                             stream);
+    bool expand = false;
+    if (expand_axes > 0 && r_split < 1e29) {
+        const auto key = std::make_tuple(size, cb, r_split);
+        auto known = sys->expansion_entries.find(key);
+        if (known == sys->expansion_entries.end())
+            known = sys->expansion_entries
+                        .emplace(key, expansion_entries(*sys, rho + sys->max_offset, r_split))
+                        .first;
+        expand = known->second >= kTaylorMinEntriesPoses &&
+                 taylor_pays(known->second, (double)expand_axes * bi * bj * bk, adjoint);
+    }
+    VEXT_TRY(get_block_regions(sys, size, bi, bj, bk, rho, sys->max_offset, false, expand, r_split,
+                               out, stream));
+    if (!expand || taylor_worthwhile(*sys, **out, expand_axes, adjoint)) return 0;
+    // fewer entries than expected: plain lists, also in the calls to come
+    RegionSet *rs = *out;
+    sys->expansion_entries[std::make_tuple(size, cb, r_split)] =
+        (double)rs->n_taylor / rs->n_regions;
+    if (rs->use.use_count() == 1 && sys->field_plan_set != rs) {
+        sys->sets.erase(std::find(sys->sets.begin(), sys->sets.end(), rs));
+        delete rs;
+    }
+    return get_block_regions(sys, size, bi, bj, bk, rho, sys->max_offset, false, false, r_split,
+                             out, stream);
 }
 
 // Lists of blocks of bi x bj x bk grid centers (sites: voxels) for sites within
 // rho + offset of a block's middle.
 int get_block_regions(System *sys, int size, int bi, int bj, int bk, double rho, double offset,
-                      bool sites, double r_split, RegionSet **out, cudaStream_t stream) {
+                      bool sites, bool expand, double r_split, RegionSet **out,
+                      cudaStream_t stream) {
     for (RegionSet *rs : sys->sets)
         if (rs->size == size && rs->bi == bi && rs->bj == bj && rs->bk == bk &&
-            rs->sites == sites && rs->r_split == r_split) {
+            rs->sites == sites && rs->expand == expand && rs->r_split == r_split) {
             if (rs->stale) {
                 for (auto &r : rs->h_info)
                     r.n_near = r.n_total = r.n_inner = r.n_outer = r.n_mid = r.n_tnear =
@@ -509,6 +542,7 @@ int get_block_regions(System *sys, int size, int bi, int bj, int bk, double rho,
     rs->size = size;
     rs->r_split = r_split;
     rs->sites = sites;
+    rs->expand = expand;
     rs->bi = bi;
     rs->bj = bj;
     rs->bk = bk;
@@ -537,23 +571,16 @@ int get_block_regions(System *sys, int size, int bi, int bj, int bk, double rho,
                 r.of[2] = (r.k0 + 0.5 * rs->bk) / size;
                 r.rho = rho;
             }
-    if (r_split < 1e29) {
-        rs->taylor_radius = offset + rho;
-        const double start = std::max(taylor_start(*sys, rs->taylor_radius),
-                                      r_split + rs->taylor_radius);
-        const double inner = sys->cutoff - rs->taylor_radius;
-        const double volume = 1.0 / std::fabs(det3(sys->Hinv));
-        // too few entries for an expansion to pay (taylor_worthwhile): unsorted
-        if (start < inner && 4.18879 * (inner * inner * inner - start * start * start) *
-                                     sys->n_atoms / volume >=
-                                 (sites ? kTaylorMinEntries : kTaylorMinEntriesPoses))
-            rs->d_taylor = start;
+    rs->taylor_radius = offset + rho;
+    if (expand && expansion_entries(*sys, rs->taylor_radius, r_split) >= kTaylorMinEntries) {
+        rs->d_taylor = std::max(taylor_start(*sys, rs->taylor_radius),
+                                r_split + rs->taylor_radius);
         rs->d_tfar = std::max(rs->d_taylor,
                               taylor_start(*sys, rs->taylor_radius, kTaylorFarOrder));
     }
     // without expansions a cut block's origin is the mean of its own centers:
     // shorter lists (21^3 and 35^3 grids 2-3 % faster)
-    if (!sites && rs->d_taylor >= sys->cutoff)
+    if (!sites && !expand)
         for (RegionInfo &r : rs->h_info) {
             r.of[0] = (r.i0 + 0.5 * r.ni) / size;
             r.of[1] = (r.j0 + 0.5 * r.nj) / size;

@@ -620,14 +620,17 @@ bool taylor_allowed(const System &sys, const RegionSet &rs) {
 // directors alone (2 M directors on a 4^3 grid: 190 GB).
 constexpr double kTaylorMatrix = 1 << 30;
 
-bool taylor_worthwhile(const System &sys, const RegionSet &rs, int n_axes, bool adjoint) {
-    if (!taylor_allowed(sys, rs)) return false;
-    const double n = (double)rs.n_taylor / rs.n_regions;
-    const double poses = (double)n_axes * rs.bi * rs.bj * rs.bk;
+bool taylor_pays(double n, double poses, bool adjoint) {
     if (poses * (adjoint ? 7.0 : 1.0) * kTaylorPad * sizeof(float) > kTaylorMatrix) return false;
     const double direct = n * poses * 2.0 * (adjoint ? 19.0 : 9.3);
     const double taylor = n * 2100.0 + poses * (adjoint ? 7.0 : 1.0) * 580.0;
     return direct > taylor;
+}
+
+bool taylor_worthwhile(const System &sys, const RegionSet &rs, int n_axes, bool adjoint) {
+    return taylor_allowed(sys, rs) &&
+           taylor_pays((double)rs.n_taylor / rs.n_regions,
+                       (double)n_axes * rs.bi * rs.bj * rs.bk, adjoint);
 }
 
 static int prepare(const System &sys, const RegionSet &rs, int poses, const double *d_axes,

@@ -26,10 +26,9 @@ constexpr int kTaylorLow = 4;        // degrees below this: the FP64 polynomial
 constexpr int kTaylorPoly = 20;      // its coefficients
 constexpr int kTaylorPolyPad = 24;   // doubles per region
 
-// Expected entries per region below which lists are built without a class for
-// the expansion: site lists gain from about 40; lists for poses need 120 before
-// forward + adjoint takes the expansion (taylor_worthwhile), and sorted lists
-// that do without it lose 2 % to their shorter partial sums (list_flush).
+// Expected entries per region below which site lists are built without a class
+// for the expansion (they gain from about 40), and lists for poses without one
+// whatever the directors (taylor_pays).
 constexpr double kTaylorMinEntries = 40, kTaylorMinEntriesPoses = 120;
 
 // Columns |m| of the expansion that one warp sums (balanced: 66-76 sums).
@@ -134,6 +133,8 @@ double taylor_start(const System &sys, double radius, int order = kTaylorOrder);
 // `n_axes` directors (the rule is explained at its definition), and allowed
 // for this system's pair coefficients.
 bool taylor_worthwhile(const System &sys, const RegionSet &rs, int n_axes, bool adjoint);
+// The rule itself, for `entries` per region and `poses` of a region.
+bool taylor_pays(double entries, double poses, bool adjoint);
 
 // Build the evaluation matrix of a (system, region shape, directors) triple.
 int taylor_prepare(const System &sys, const RegionSet &rs, int n_axes, const double *d_axes,

@@ -202,3 +202,23 @@ def test_many_directors_on_a_small_grid(n_axes):
     gu = gu - (gu * axes[o]).sum(1)[:, None] * axes[o]
     assert_energy(got.astype(np.float64), exact, storage=1.2e-7)
     assert_gradient(grad.astype(np.float64), np.concatenate([gc, gu], 1))
+
+
+def test_lists_follow_the_directors():
+    """Few directors are summed on lists without classes for expansions, whose
+    regions cut by the grid's edge are smaller; many ones on lists with them;
+    either way the same call gives the same bits again."""
+    size = 25
+    with VextSystem(dense()) as system:
+        seen = {}
+        for n_axes in (4, 64, 4, 64):
+            out = system.field(size, directors(n_axes), centers_per_region=16)["orientation_K"]
+            entries = system.last_stats["list_entries"]
+            if n_axes in seen:
+                np.testing.assert_array_equal(out, seen[n_axes][0])
+                assert entries == seen[n_axes][1]
+            seen[n_axes] = out, entries
+        assert seen[4][1] < seen[64][1]
+        exact = system.field(size, directors(4), energy=True,
+                             mode=_lib.VEXT_MODE_FP64)["energy"].T.reshape(seen[4][0].shape)
+        assert_energy(seen[4][0].astype(np.float64), exact, storage=1.2e-7)
