@@ -92,12 +92,13 @@ __global__ void __launch_bounds__(256, 2) pose_batch_kernel(PoseBatchArgs a) {
     }
 }
 
-// Warps per pose: the smallest power of two up to 8 that gives about 16
-// resident warps per SM (148 SMs), so small batches spread each pose's list
-// over several warps.
+constexpr long long kWarps = 148 * 16;   // resident warps the launches aim at
+
+// Warps per pose: the smallest power of two up to 8 that gives about kWarps warps,
+// so small batches spread each pose's list over several warps.
 int warps_per_pose(long long n) {
     int w = 1;
-    while (w < 8 && n * (2 * w) <= 148LL * 16) w *= 2;
+    while (w < 8 && n * (2 * w) <= kWarps) w *= 2;
     return w;
 }
 
@@ -106,18 +107,22 @@ constexpr double kLongList = 512;
 
 // mean_list: entries of a bin list, over the batch's poses; max_list: the mean
 // of the system with the longest.  Long lists load several entries at a time.
-// Uneven ones (the longest 1.5 times the mean and more) take two warps per
-// pose up to about 96 warps per SM in all: the halves shorten the tail that the
-// poses of dense systems leave (6,545 String poses of 12 frameworks: 118 us
-// with one warp, 83 with two, 112 with four), while 100 paths of one framework
-// lose (42 us with one, 55 with two).
+// A pose of the densest system takes as long as max_list entries, all poses
+// together at least as long as `load` entries a warp: with one warp per pose the
+// former is a tail where it is well above the latter (of uneven lists, 1.5 times
+// the mean and more), and two warps per pose halve it, but pay twice for what a
+// pose costs beside its entries.  One and two warps, by max_list and load: 8,480
+// and 3,870 102 and 75 us (6,174 String poses of 12 frameworks), 3,540 and 1,280
+// 39.6 and 37.0, 1,760 and 360 18.6 and 16.5; 1,300 and 380 16.5 and 20.0, 1,800
+// and 490 19.3 and 22.6, 1,890 and 2,460 35.6 and 44.0, 1,170 and 1,200 24.9 and 35.1.
 static int pose_batch_launch(PoseBatchArgs a, bool mixed, double mean_list, double max_list,
                              cudaStream_t st) {
     a.wpp = warps_per_pose(a.n);
     const bool long_lists = mean_list >= kLongList && a.wpp <= 2;
-    if (long_lists && max_list >= 1.5 * mean_list && a.n * 2 <= 148LL * 96) a.wpp = 2;
+    const double load = (double)a.n * mean_list / kWarps;
+    if (long_lists && max_list >= 1.5 * mean_list && max_list >= 1.6 * load + 1100.0) a.wpp = 2;
     const long long groups = (a.n + 8 / a.wpp - 1) / (8 / a.wpp);
-    const int blocks = (int)std::min<long long>(groups, 148LL * 16);
+    const int blocks = (int)std::min<long long>(groups, kWarps);
     auto kernel = mixed ? long_lists ? pose_batch_kernel<true, 4> : pose_batch_kernel<true, 1>
                         : long_lists ? pose_batch_kernel<false, 4> : pose_batch_kernel<false, 1>;
     kernel<<<blocks, 256, 0, st>>>(a);

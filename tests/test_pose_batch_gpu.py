@@ -127,3 +127,35 @@ def test_pose_batch_rejects_bad_input():
         VextPoseBatch(systems, [-1] + counts[1:])
     for s in systems:
         s.close()
+
+
+@pytest.mark.parametrize("counts", [(1222, 78), (2256, 144), (3200, 800), (4512, 288)])
+def test_uneven_lists_one_and_two_warps_per_pose(counts):
+    """A dense framework beside a sparse one, on both sides of the rule for two
+    warps per pose."""
+    cases = []
+    for n in (400, 3200):
+        rng = np.random.default_rng(n)
+        kind = rng.integers(0, 4, n)
+        cases.append(synth.make_case([20.0] * 3, [90.0] * 3, rng.random((n, 3)),
+                                     synth.TYPE_TABLE[kind, 1], synth.TYPE_TABLE[kind, 0],
+                                     synth.GUEST_A, 12.8))
+    rng = np.random.default_rng(sum(counts))
+    total = sum(counts)
+    centers = rng.random((total, 3)) * 20.0
+    quats = synth.random_quaternions(rng, total)
+    systems = [VextSystem(c) for c in cases]
+    e, gc, gq, gu = run_batch(systems, counts, centers, quats, _lib.VEXT_MODE_MIXED)
+    start = 0
+    for system, n in zip(systems, counts):
+        part = slice(start, start + n)
+        se, sgc, sgq, sgu = system.pose_energy_grad(centers[part], quats[part],
+                                                    mode=_lib.VEXT_MODE_FP64)
+        neg = se <= 0
+        assert np.abs(e[part] - se)[neg].max(initial=0) < 1e-4
+        assert (np.abs(e[part] - se) / np.maximum(np.abs(se), 1.0))[~neg].max(initial=0) < 1e-6
+        assert rel_rows(gc[part], sgc).max() < 1e-5
+        assert rel_rows(gu[part], sgu).max() < 1e-5
+        start += n
+    for s in systems:
+        s.close()
