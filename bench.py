@@ -10,9 +10,10 @@ lists and outputs resident in HBM.
 Our arm prints one JSON line with: value (poses/s over all ranks, device time
 from CUDA events, max over ranks), e2e (the public host C-ABI call
 vext_field_adjoint: directors up, float32 energy + gradient down into pinned
-host memory, by slabs of grid planes while the next slab computes), roofline of
-the step against the measured FP32 FFMA peak of this GPU, the forward-only
-field (list build + pair kernels + epilogue, with its roofline), the plain and tiled FP64 GPU
+host memory, by slabs of grid planes while the next slab computes), what bounds
+the step (roofline) and the rate of pairs it stands for against the measured FP32
+FFMA peak of this GPU, the forward-only field (list build + pair kernels +
+epilogue, with its rate of pairs), the plain and tiled FP64 GPU
 kernels and the error of the mixed result against FP64, the random-pose
 forward+adjoint path and its error against its FP64 mode, the precision
 study, the GPU String update, the drop-in mode (the reference's driver calling
@@ -53,7 +54,21 @@ METRIC = "Vext pose evals/s at <=1e-4 K vs FP64, fwd+adjoint evals/s; % FP32 pea
 FAR_DRAM_BYTES_FULL_FIELD = 1_087_278_432 + 372_915_200
 # the same for one forward + adjoint step (expansions, clusters, poses).
 ADJ_DRAM_BYTES_FULL_FIELD = 2_798_525_440 + 1_698_379_520
+# site_cluster_kernel's busiest pipe (ncu, forward + adjoint, layered 44^3 x 64).
+CLUSTER_FP64_PIPE = 0.393
 CPU_CENTERS_PER_CORE_S = 900.0   # reference driver throughput estimate used to size the sample
+
+
+def pair_rate(pairs, flop, ms, peak):
+    """In-cutoff pairs a step stands for, as FLOP/s.  Not a fraction of a roofline:
+    local expansions take the place of most of the pairs, so it can exceed 1."""
+    rate = pairs * flop / (ms * 1e-3)
+    return {"value": rate / 1e12, "unit": "TFLOP/s", "of_fp32_peak": rate / peak,
+            "fp32_peak": peak / 1e12,
+            "peak_source": "measured on this GPU: max(FFMA, FFMA2) FMA rate x 2 "
+                           "(vext_measure_pipes); MEASURED_PEAKS.json has no FP32 figure",
+            "algorithmic": f"{pairs} in-cutoff pairs x {flop} FLOP per field, most of them by "
+                           "local expansion instead of one by one"}
 
 
 def ensure_built():
@@ -284,7 +299,7 @@ def run_ours(args, rank, world, local_rank):
     grad = torch.empty(shape + (6,), dtype=torch.float32, device=device)
     system = VextSystem(case)
 
-    pairs, far_pairs = system.count_pairs(size, axes)
+    pairs, _ = system.count_pairs(size, axes)
     pipes = _lib.measure_pipes()
     peak = 2.0 * max(pipes["ffma_per_s"], pipes["ffma2_fma_per_s"])   # FLOP/s, FMA = 2
 
@@ -306,7 +321,6 @@ def run_ours(args, rank, world, local_rank):
     ms_total = ranks.max_over_ranks(ms_total, device)
     ms_step = ms_total / args.steps
     value = world * poses * args.steps / (ms_total * 1e-3)
-    achieved = pairs * FLOP_FWD_ADJ / (ms_step * 1e-3)
 
     # ---- e2e through the public host entry (vext_field_adjoint): directors
     # up, float32 energy + gradient down into pinned host buffers, every call
@@ -334,7 +348,7 @@ def run_ours(args, rank, world, local_rank):
     if rank == 0:
         extra["e2e_cold"] = e2e_cold_field(case, size, axes)
         extra.update(secondary_measurements(args, system, case, size, axes, poses, pairs,
-                                            far_pairs, peak, stream, device, ms_step, energy,
+                                            peak, stream, device, ms_step, energy,
                                             grad))
     ranks.barrier()
     if rank != 0:
@@ -347,8 +361,8 @@ def run_ours(args, rank, world, local_rank):
     line = {"metric": METRIC, "value": value, "unit": "poses/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_step,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": "f32x2+f64 (pairs < 5 A in FP64, beyond in packed FP32 with FP64-flushed "
-                     "partial sums; FP64 energy refinement band; FP64 re-evaluation of poses "
+            "dtype": "f32x2+f64 (pairs < 5.9 A in FP64, beyond in packed FP32 with FP64-flushed "
+                     "partial sums and FP32 local expansions; FP64 energy refinement band; FP64 re-evaluation of poses "
                      "with a shell pair within the FP32 error of the cutoff)",
             "data": "synthetic", "config": config_of(args.workload, size),
             "step": "forward + adjoint of every pose: energy, dE/d(center), tangent dE/du; "
@@ -360,29 +374,21 @@ def run_ours(args, rank, world, local_rank):
                             "slab computes)"},
             "gpu_launches": args.steps * 5,
             "setup_s": setup_s,
-            "roofline": {"bound": "fp32",
-                         "kernel": "the whole step: local expansions of far images (taylor_sums_kernel, "
-                                   "taylor_mma_kernel on the tensor cores), site_cluster_kernel "
-                                   "(FP64 near + FP32x2 far), site_pose_kernel, refinement; the "
-                                   "expansions replace most pair evaluations, so the pairs' "
-                                   "FLOP rate can exceed the FFMA peak",
-                         "achieved": achieved / 1e12, "peak": peak / 1e12, "unit": "TFLOP/s",
-                         "frac": achieved / peak,
-                         "peak_source": "measured on this GPU: max(FFMA, FFMA2) FMA rate x 2 "
-                                        "(vext_measure_pipes); MEASURED_PEAKS.json has no FP32 "
-                                        "figure",
-                         "algorithmic": f"{pairs} in-cutoff pairs x {FLOP_FWD_ADJ} FLOP "
-                                        "(forward + adjoint) per field",
+            "roofline": {"bound": "latency of the FP64 and FP32 chains of site_cluster_kernel "
+                                  "(four fifths of the step)",
+                         "kernel": "site_cluster_kernel (FP64 near + FP32x2 far)",
+                         "achieved": CLUSTER_FP64_PIPE, "peak": 1.0,
+                         "unit": "cycles active of the FP64 pipe", "frac": CLUSTER_FP64_PIPE,
+                         "frac_source": "ncu sm__pipe_fp64_cycles_active, its fullest pipe "
+                                        "(profiles/site_kernels_full_field.md, 44^3 x 64)",
                          "traffic": (ADJ_DRAM_BYTES_FULL_FIELD
                                      if args.workload == "full_field" else None),
                          "traffic_unit": "bytes per step (ncu dram__bytes_read+write)",
-                         "bound_note": "FP32 and FP64 pipes of the pair sums (latency-bound); the "
-                                       "expansions' product runs on the tensor cores; see "
-                                       "hbm_check",
                          "hbm_check": hbm_check(ADJ_DRAM_BYTES_FULL_FIELD
                                                 if args.workload == "full_field" else None,
                                                 ms_step),
                          "pipes": pipes},
+            "pair_rate": pair_rate(pairs, FLOP_FWD_ADJ, ms_step, peak),
             "clocks": clocks.summary(), "cpu_baseline": cpu}
     # the numbers the secondary measurements support, also inside the standard
     # keys (records that keep only those keys still carry them)
@@ -442,7 +448,7 @@ def e2e_cold_field(case, size, axes):
                     "memory); host clock"}
 
 
-def secondary_measurements(args, system, case, size, axes, poses, pairs, far_pairs, peak,
+def secondary_measurements(args, system, case, size, axes, poses, pairs, peak,
                            stream, device, ms_adj, energy, grad):
     """Forward-only field, FP64 baselines, error against FP64, pose path and
     the 100-field batches (rank 0)."""
@@ -469,20 +475,14 @@ def secondary_measurements(args, system, case, size, axes, poses, pairs, far_pai
     far_ms = statistics.mean(t["far_ms"] for t in timings)
     list_ms = statistics.mean(t["list_ms"] for t in timings)
     epi_ms = statistics.mean(t["epilogue_ms"] for t in timings)
-    achieved_far = far_pairs * FLOP_FWD / (far_ms * 1e-3)
     out["forward"] = {
         "value": poses / (fwd_ms * 1e-3), "unit": "poses/s", "ms_per_field": fwd_ms,
         "step": "region-list build + near (FP64) + far (FP32x2) kernels + refinement + "
                 "float32 epilogue",
         "breakdown_ms": {"list_build": list_ms, "near_pairs_fp64": near_ms,
                          "far_pairs_fp32x2": far_ms, "refine_epilogue": epi_ms},
-        "roofline_far_kernel": {"kernel": "site_cluster_kernel with the local expansions (near "
-                                          "pairs included in its time)", "bound": "fp32",
-                                "achieved": achieved_far / 1e12, "peak": peak / 1e12,
-                                "unit": "TFLOP/s", "frac": achieved_far / peak,
-                                "algorithmic": f"{far_pairs} far in-cutoff pairs x {FLOP_FWD} FLOP",
-                                "traffic": (FAR_DRAM_BYTES_FULL_FIELD
-                                            if args.workload == "full_field" else None)}}
+        "pair_rate": pair_rate(pairs, FLOP_FWD, near_ms + far_ms, peak),
+        "traffic": FAR_DRAM_BYTES_FULL_FIELD if args.workload == "full_field" else None}
     del fwd_out
     # FP64 GPU baselines, one field per launch
     e64 = torch.empty(shape, dtype=torch.float64, device=device)
@@ -643,7 +643,7 @@ def bench_string_update():
     return {"iterations": res["iterations"], "images": len(path), "seconds": wall,
             "ms_per_iteration": 1e3 * wall / max(res["iterations"], 1),
             "workload": "config-4 path, 64 images, 200 iterations, host wall time of "
-                        "vext_string_run (graph-replayed iterations)"}
+                        "vext_string_run (one cooperative launch)"}
 
 
 def reference_package_driver():

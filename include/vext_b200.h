@@ -237,11 +237,12 @@ VEXT_API int vext_field_device(vext_system sys, int size, int n_axes, const doub
  *   energy_f64    double [n_axes][S^3]     the energies before float32 rounding
  *                                          (NULL to skip)
  *   gradient_f64  double [n_axes][S^3][6]  FP64 modes only (NULL to skip)
- * VEXT_MODE_MIXED runs the persistent batched kernel (FP64 near pairs, packed
- * FP32 far pairs with FP64-flushed partial sums, FP64 energy refinement band)
- * on a one-system batch that is built, autotuned and graph-captured on the
- * first call and replayed while (size, directors, options, outputs) stay the
- * same; VEXT_MODE_FP64 and VEXT_MODE_FP64_PLAIN run the plain one-thread-per-
+ * VEXT_MODE_MIXED (FP64 near pairs, packed FP32 far pairs with FP64-flushed
+ * partial sums and local expansions, FP64 energy refinement band) runs a
+ * one-system batch that is built and graph-captured on the first call and
+ * replayed while (size, directors, options) stay the same, also into other
+ * float32 outputs; fine grids are summed site by site, others pose by pose by the
+ * persistent kernel, which is autotuned then.  VEXT_MODE_FP64 and VEXT_MODE_FP64_PLAIN run the plain one-thread-per-
  * pose FP64 kernel (IEEE division), the FP64 reference of the adjoint.  No
  * reference counterpart: the reference has no field gradient; its String
  * solver differentiates by forward differences
@@ -376,8 +377,9 @@ VEXT_API int vext_batch_destroy(vext_batch batch);
 VEXT_API int vext_batch_info(vext_batch batch, int64_t *work_items, int64_t *poses,
                              int64_t *list_bytes, int *shape, int *grid);
 /* Poses the last replay re-evaluated in FP64 (energies in the refinement
- * band; for forward + adjoint batches also poses with a shell pair within
- * 1.25e-4 A^2 of the cutoff), after waiting for the device. */
+ * band; of systems summed pose by pose, forward + adjoint, also poses with a
+ * shell pair within 1.25e-4 A^2 of the cutoff: site by site such pairs are
+ * decided in FP64 on the spot), after waiting for the device. */
 VEXT_API int vext_batch_refined(vext_batch batch, int64_t *poses);
 /* The autotuner's candidates (kernel shape index, resident CTAs, sample time
  * in ms, shape name: threads x directors per thread[/CTAs-per-SM bound]),

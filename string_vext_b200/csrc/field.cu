@@ -1199,8 +1199,8 @@ extern "C" int vext_field_adjoint(vext_system h, int size, int n_axes, const dou
     }
     if (o.mode == VEXT_MODE_MIXED) {
         // pageable host outputs: one batch per block of the batch's work-item
-        // directors (64 by default); block k's copy (on aux) overlaps block
-        // k + 1's pair work (on st)
+        // directors (64 by default); block k's copy (copy_to_host's threads)
+        // overlaps the sums of the blocks after it (on st)
         for (int k = 0; k < 3 * n_axes; ++k)
             if (!std::isfinite(axes[k])) return fail(VEXT_ERR_ARGUMENT, "non-finite director");
         const size_t S3 = (size_t)size * size * size;

@@ -260,7 +260,7 @@ __device__ __forceinline__ void take_shell(const SiteQueue &q, int n, const Site
 // 60^3 x 64 layered forward + adjoint: 8.8 of 11.2 ms (pose by pose, on lists
 // about regions of poses, 18.1 in all), about 1.3 of it classification and 3.6
 // near entries.  Bound by the latency of the FP64 and FP32 chains at 16 warps
-// per SM (issue slots 57 %, FP64 pipe 33 %, FMA pipe 39 % busy; 20 warps with
+// per SM (issue slots 58 %, FP64 pipe 39 %, FMA pipe 29 % busy; 20 warps with
 // spills are slower, forward 20 beat 24 by 1-2 %).  Hence eight inside entries,
 // four shell entries and two near ones side by side (half as many: 2 % slower,
 // one near entry: 3 %), taken from full queues: straight from each group of 32

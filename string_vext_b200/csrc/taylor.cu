@@ -610,8 +610,6 @@ static double worst_truncation(const System &sys, double radius, double d,
 double taylor_start(const System &sys, double radius, int order) {
     double lo = 2.0 * radius, hi = sys.cutoff;
     if (!(lo < hi) || worst_truncation(sys, radius, hi, order) > kTruncation) return 1e30;
-    // the largest c12 and c6 bound every type: bisect on the types that lead
-    // at the far end only when there are many
     for (int i = 0; i < 24; ++i) {
         const double mid = 0.5 * (lo + hi);
         (worst_truncation(sys, radius, mid, order) > kTruncation ? lo : hi) = mid;
