@@ -480,10 +480,14 @@ static double det3(const Mat3 &m) {
            h[2] * (h[3] * h[7] - h[4] * h[6]);
 }
 
-// Entries per region that an expansion about its origin is expected to hold, for
-// sites within `radius` of it; 0: none.
-static double expansion_entries(const System &sys, double radius, double r_split) {
-    const double start = std::max(taylor_start(sys, radius), r_split + radius);
+// Where a region's local expansion starts, for sites within `radius` of its origin
+// (taylor_start goes through all types some 24 times: called once per list set).
+static double expansion_start(const System &sys, double radius, double r_split) {
+    return std::max(taylor_start(sys, radius), r_split + radius);
+}
+
+// Entries per region that it is expected to hold; 0: none.
+static double expansion_entries(const System &sys, double radius, double start) {
     const double inner = sys.cutoff - radius;
     if (!(start < inner)) return 0.0;
     return 4.18879 * (inner * inner * inner - start * start * start) * sys.n_atoms *
@@ -499,10 +503,13 @@ int get_field_regions(System *sys, int size, int cb, double r_split, int expand_
     if (expand_axes > 0 && r_split < 1e29) {
         const auto key = std::make_tuple(size, cb, r_split);
         auto known = sys->expansion_entries.find(key);
-        if (known == sys->expansion_entries.end())
+        if (known == sys->expansion_entries.end()) {
+            const double radius = rho + sys->max_offset;
             known = sys->expansion_entries
-                        .emplace(key, expansion_entries(*sys, rho + sys->max_offset, r_split))
+                        .emplace(key, expansion_entries(*sys, radius,
+                                                        expansion_start(*sys, radius, r_split)))
                         .first;
+        }
         expand = known->second >= kTaylorMinEntriesPoses &&
                  taylor_pays(known->second, (double)expand_axes * bi * bj * bk, adjoint);
     }
@@ -572,9 +579,9 @@ int get_block_regions(System *sys, int size, int bi, int bj, int bk, double rho,
                 r.rho = rho;
             }
     rs->taylor_radius = offset + rho;
-    if (expand && expansion_entries(*sys, rs->taylor_radius, r_split) >= kTaylorMinEntries) {
-        rs->d_taylor = std::max(taylor_start(*sys, rs->taylor_radius),
-                                r_split + rs->taylor_radius);
+    const double start = expand ? expansion_start(*sys, rs->taylor_radius, r_split) : 1e30;
+    if (expansion_entries(*sys, rs->taylor_radius, start) >= kTaylorMinEntries) {
+        rs->d_taylor = start;
         rs->d_tfar = std::max(rs->d_taylor,
                               taylor_start(*sys, rs->taylor_radius, kTaylorFarOrder));
     }
